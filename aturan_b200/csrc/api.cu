@@ -104,6 +104,15 @@ struct aturan_ctx {
     HydroConst hc;
     SatConst sc;
     PressConst pc;
+    // the GS sweep: its plan (nb = 0: the column does not fit, a captured graph of hyperplanes instead),
+    // the bands' edge buffer and block ticket, the sweeps launched so far; a device word that a wait
+    // which ran out sets, and whether a sweep has run since it was last read
+    GsPlan gsp;
+    GsEdge* gs_edge;
+    unsigned* gs_ticket;
+    unsigned gs_n;
+    int* gs_err;
+    bool gs_unread;
     cudaGraphExec_t gs_exec;
     long gs_launches;          // kernels in the captured GS graph
     // per-class launch counts and optional CUDA-event timing (aturan_profile)
@@ -131,6 +140,19 @@ int cuda_check(aturan_ctx* c, cudaError_t e, const char* what){
 
 #define CK(call) do { int rc_ = cuda_check(ctx, (call), #call); if(rc_) return rc_; } while(0)
 #define CK_LAUNCH(what) do { int rc_ = cuda_check(ctx, cudaGetLastError(), what); if(rc_) return rc_; } while(0)
+
+// Whether every bounded wait of the GS sweeps since the last call ended in time (gs_wave_kernel): read
+// where a caller waits for the stream or takes p_dyn. Synchronizes when there is something to read.
+int gs_waits_held(aturan_ctx* ctx){
+    if(!ctx->gs_unread) return ATURAN_OK;
+    int e = 0;
+    CK(cudaMemcpyAsync(&e, ctx->gs_err, sizeof e, cudaMemcpyDeviceToHost, ctx->st));
+    CK(cudaStreamSynchronize(ctx->st));
+    ctx->gs_unread = false;
+    if(!e) return ATURAN_OK;
+    CK(cudaMemsetAsync(ctx->gs_err, 0, sizeof e, ctx->st));
+    return fail(ctx, ATURAN_E_CUDA, "GS sweep: a wait between bands ran out; p_dyn is not valid");
+}
 
 size_t round_up(size_t x, size_t a){ return (x + a - 1) / a * a; }
 
@@ -438,6 +460,31 @@ int run_gs(aturan_ctx* ctx){
     const Grid g = ctx->g;
     const size_t fs = g.fstride;
     S* proj = reinterpret_cast<S*>(ctx->proj);
+    const S* form = proj;
+    auto pre = [&](cudaStream_t st){
+        launch_gs_pre(g, grp<S>(proj, 3, fs), grp<S>(proj, 4, fs), grp<S>(proj, 5, fs),
+                      grp<S>(proj, 0, fs), grp<S>(proj, 1, fs), grp<S>(proj, 2, fs), ctx->pdyn, ctx->gsw,
+                      ctx->pc, ctx->scratch, st);
+    };
+    if(ctx->gsp.nb > 0){
+        // the launch's ticket base and tag are host counters: a captured launch must not be replayed
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        CK(cudaStreamIsCapturing(ctx->st, &cap));
+        if(cap != cudaStreamCaptureStatusNone)
+            return fail(ctx, ATURAN_E_UNSUPPORTED, "the GS sweep cannot be captured into a graph");
+        Region reg(ctx, ATURAN_K_GS, 6);
+        pre(ctx->st);
+        CK_LAUNCH("GS source");
+        unsigned tag = ctx->gs_n + 1;
+        if(launch_gs_wave(form, g, ctx->pdyn, ctx->scratch, ctx->gsw, ctx->gsp, ctx->gs_edge, ctx->gs_ticket,
+                          ctx->gs_n * (unsigned)ctx->gsp.nb, tag ? tag : 1u, ctx->gs_err, ctx->st) < 0)
+            return cuda_check(ctx, cudaGetLastError(), "GS sweep") ? ATURAN_E_CUDA : fail(ctx, ATURAN_E_CUDA, "GS sweep");
+        ctx->gs_n++;
+        ctx->gs_unread = true;
+        launch_pdyn_bcs(g, ctx->pdyn, ctx->st);
+        CK_LAUNCH("GS sweep");
+        return ATURAN_OK;
+    }
     if(!ctx->gs_exec){
         // The hyperplane sweep is (im-2)+(jm-2)+(km-2)-1 dependent launches; capture the whole
         // call once per context and replay it.
@@ -445,14 +492,10 @@ int run_gs(aturan_ctx* ctx){
         CK(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
         cudaGraph_t graph;
         CK(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
-        launch_gs_pre(g, grp<S>(proj, 3, fs), grp<S>(proj, 4, fs), grp<S>(proj, 5, fs),
-                      grp<S>(proj, 0, fs), grp<S>(proj, 1, fs), grp<S>(proj, 2, fs), ctx->pdyn, ctx->gsw,
-                      ctx->pc, ctx->scratch, cs);
+        pre(cs);
         const int s_lo = 2, s_hi = (g.im - 2) + (g.jm - 2) + (g.km - 2);
-        ctx->gs_launches = 1 + (ctx->pc.press_incr ? 1 : 0) + (s_hi - s_lo + 1) + 3;
-        for(int s = s_lo; s <= s_hi; s++)
-            launch_gs_plane(g, ctx->pdyn, ctx->scratch, grp<S>(proj, 3, fs), grp<S>(proj, 4, fs),
-                            grp<S>(proj, 5, fs), ctx->gsw, ctx->pc, s, cs);
+        ctx->gs_launches = 2 + (s_hi - s_lo + 1) + 3;
+        for(int s = s_lo; s <= s_hi; s++) launch_gs_plane(form, g, ctx->pdyn, ctx->scratch, ctx->gsw, s, cs);
         launch_pdyn_bcs(g, ctx->pdyn, cs);
         cudaError_t e1 = cudaGetLastError();
         cudaError_t e2 = cudaStreamEndCapture(cs, &graph);
@@ -1031,6 +1074,8 @@ int aturan_ctx_create(const aturan_params* p, aturan_ctx** out){
     for(int n = 0; n < 6; n++) add((size_t)(sNM + 1) * sJ * 8);        // mode factorisations (Lc, Lc^T)
     for(int n = 0; n < 6; n++) add(nij * 8);                           // line factorisations (Lc, Lc^T)
     add(fs * 4); add(fs * 4);
+    ctx->gsp = gs_plan(g);
+    add(gs_edge_bytes(ctx->gsp)); add(4); add(4);
     if(ctx->mixed) add(2 * fs * 4);                                    // the temperature pair's low parts
     ctx->mem_bytes = bytes;
     // the stage kernels address every buffer of the allocation by 32-bit element offsets
@@ -1104,6 +1149,9 @@ int aturan_ctx_create(const aturan_params* p, aturan_ctx** out){
     ctx->mluT_idn = carve<double>(cur, (size_t)(sNM + 1) * sJ);
     ctx->lluT_a = carve<double>(cur, nij); ctx->lluT_cf = carve<double>(cur, nij); ctx->lluT_idn = carve<double>(cur, nij);
     ctx->r32 = carve<float>(cur, fs); ctx->e32 = carve<float>(cur, fs);
+    ctx->gs_edge = reinterpret_cast<GsEdge*>(carve<char>(cur, gs_edge_bytes(ctx->gsp)));
+    ctx->gs_ticket = carve<unsigned>(cur, 1);
+    ctx->gs_err = carve<int>(cur, 1);
     ctx->tlo = ctx->mixed ? carve<float>(cur, 2 * fs) : nullptr;
     ctx->host_part.resize(2 * ctx->sor_nblk);
 
@@ -1437,6 +1485,7 @@ static int xfer(aturan_ctx* ctx, int field, void* other, bool up, bool other_is_
         CK_LAUNCH("layout out");
         if(!other_is_device) CK(cudaMemcpyAsync(other, ctx->stage64, n * 8, cudaMemcpyDeviceToHost, ctx->st));
         CK(cudaStreamSynchronize(ctx->st));
+        if(field == ATURAN_P_DYN) return gs_waits_held(ctx);
     }
     return ATURAN_OK;
 }
@@ -1452,6 +1501,8 @@ static int xfer_many(aturan_ctx* ctx, int n, const int* fields, void* const* ptr
         if(fields[q] < 0 || fields[q] >= ATURAN_NFIELDS) return fail(ctx, ATURAN_E_INVALID, "field id out of range");
         if(!ptrs[q]) return fail(ctx, ATURAN_E_INVALID, "null buffer");
     }
+    bool takes_pdyn = false;
+    for(int q = 0; q < n && !up; q++) takes_pdyn |= fields[q] == ATURAN_P_DYN;
     const Grid& g = ctx->g;
     const size_t rows = (size_t)g.im * g.jm, nval = rows * g.km;
     auto pack = [&](int field, const double* src, double* tgt) -> int {
@@ -1476,7 +1527,9 @@ static int xfer_many(aturan_ctx* ctx, int n, const int* fields, void* const* ptr
                               : pack(fields[q], nullptr, reinterpret_cast<double*>(ptrs[q]));
             if(rc) return rc;
         }
-        if(!up) CK(cudaStreamSynchronize(ctx->st));
+        if(up) return ATURAN_OK;
+        if(takes_pdyn && ctx->gs_unread) return gs_waits_held(ctx);
+        CK(cudaStreamSynchronize(ctx->st));
         return ATURAN_OK;
     }
     double* buf[2] = {ctx->stage64, ctx->scratch};
@@ -1504,7 +1557,7 @@ static int xfer_many(aturan_ctx* ctx, int n, const int* fields, void* const* ptr
     CK(cudaEventRecord(ctx->ev_join, ctx->st2));
     CK(cudaStreamWaitEvent(ctx->st, ctx->ev_join, 0));
     CK(cudaStreamSynchronize(ctx->st));
-    return ATURAN_OK;
+    return takes_pdyn ? gs_waits_held(ctx) : ATURAN_OK;
 }
 
 int aturan_upload(aturan_ctx* ctx, int field, const double* host){ return xfer(ctx, field, (void*)host, true, false); }
@@ -2143,7 +2196,7 @@ int aturan_profile_read(aturan_ctx* ctx, double* ms, long* launches, int nkinds)
 int aturan_sync(aturan_ctx* ctx){
     if(!ctx) return ATURAN_E_INVALID;
     CK(cudaStreamSynchronize(ctx->st));
-    return ATURAN_OK;
+    return gs_waits_held(ctx);
 }
 
 }  // extern "C"

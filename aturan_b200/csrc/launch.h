@@ -13,11 +13,13 @@ template <typename S> struct ChemArgs;
 template <typename S> struct TurbArgs;
 template <typename S> struct PrecipArgs;
 template <typename S> struct McaArgs;
-struct GSW; struct RBW; struct PressConst; struct PostPlan;
+struct GSW; struct RBW; struct PressConst; struct PostPlan; struct GsPlan; struct GsEdge;
 
 // launch_stage: one RK4 stage, the momentum + T launch and then the scalar launch on st; given a
 // side stream (and two events), the momentum launch runs on side beside the scalar launch on st
 // (the two read the stage input and write disjoint fields) and st waits for it.
+// launch_gs_plane, launch_gs_wave: FP64 in both forms; `form` (unused) selects the translation unit,
+// hence the contraction of the sweep's sums (none in the FP64 form).
 #define ATURAN_DECLARE_LAUNCHERS(S, C)                                                                     \
 void launch_stage(const StageArgs<S, C>& a, cudaStream_t st, cudaStream_t side = nullptr,                   \
                   cudaEvent_t ef = nullptr, cudaEvent_t ej = nullptr);                                     \
@@ -29,8 +31,10 @@ void launch_hydro(Grid g, const S* t, const S* ps, const S* v, const S* w, const
 void launch_satadj(const SatArgs<S>& a, cudaStream_t st);                                                  \
 void launch_gs_pre(Grid g, S* au, S* av, S* aw, const S* ru, const S* rv, const S* rw, const double* P,    \
                    const GSW* w, PressConst c, double* incr, cudaStream_t st);                             \
-void launch_gs_plane(Grid g, double* P, const double* incr, const S* au, const S* av, const S* aw,         \
-                     const GSW* w, PressConst c, int s, cudaStream_t st);                                   \
+void launch_gs_plane(const S* form, Grid g, double* P, const double* src, const GSW* w, int s,             \
+                     cudaStream_t st);                                                                     \
+int launch_gs_wave(const S* form, Grid g, double* P, const double* src, const GSW* w, const GsPlan& pl,    \
+                   GsEdge* edge, unsigned* ticket, unsigned base, unsigned tag, int* err, cudaStream_t st); \
 void launch_rb_prep(Grid g, S* au, S* av, S* aw, S* ru, S* rv, S* rw, int rigid_lid,                       \
                     const RBW* w, PressConst c, double* src, cudaStream_t st);                             \
 int launch_post(const PostArgs<S>& a, const PostPlan& pl, S* t, float* tlo, cudaStream_t st);               \

@@ -180,6 +180,22 @@ int launch_mca_impl(const McaArgs<S>& a, cudaStream_t st){
 // Hydrostatic integral: threads per column (ROWS) and resident blocks per SM (MINB), measured.
 template <typename S> struct HydCfg { static constexpr int ROWS = 8, MINB = 2; };
 template <> struct HydCfg<float> { static constexpr int ROWS = 16, MINB = 2; };
+// The GS sweep: gs_wave_kernel built for the plan's count of sweeping threads; 1, or -1 on an error.
+template <int NC>
+static int gs_wave_as(Grid g, double* P, const double* src, const GSW* w, const GsPlan& pl, GsEdge* edge, unsigned* ticket,
+                      unsigned base, unsigned tag, int* err, cudaStream_t st){
+    static const bool ok = cudaFuncSetAttribute(gs_wave_kernel<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                GS_SMEM_MAX) == cudaSuccess || (cudaGetLastError(), false);
+    if(!ok) return -1;
+    gs_wave_kernel<NC><<<pl.nb, gs_threads(pl), pl.smem, st>>>(g, P, src, w, pl, edge, ticket, base, tag, err);
+    return cudaPeekAtLastError() == cudaSuccess ? 1 : -1;
+}
+static int gs_wave_nc(Grid g, double* P, const double* src, const GSW* w, const GsPlan& pl, GsEdge* edge, unsigned* ticket,
+                      unsigned base, unsigned tag, int* err, cudaStream_t st){
+    if(pl.nc == 128) return gs_wave_as<128>(g, P, src, w, pl, edge, ticket, base, tag, err, st);
+    if(pl.nc == 256) return gs_wave_as<256>(g, P, src, w, pl, edge, ticket, base, tag, err, st);
+    return gs_wave_as<384>(g, P, src, w, pl, edge, ticket, base, tag, err, st);
+}
 }  // namespace aturan
 
 #define ATURAN_DEFINE_LAUNCHERS(S, C)                                                                     \
@@ -229,14 +245,17 @@ void launch_satadj(const SatArgs<S>& a, cudaStream_t st){                       
 void launch_gs_pre(Grid g, S* au, S* av, S* aw, const S* ru, const S* rv, const S* rw, const double* P,    \
                    const GSW* w, PressConst c, double* incr, cudaStream_t st){                             \
     gs_aux_bc_kernel<S><<<dim3((g.km - 1 + 127) / 128, g.jm - 2), 128, 0, st>>>(g, au, av, aw);           \
-    if(c.press_incr)                                                                                      \
-        gs_incr_kernel<S><<<dim3((g.km - 1 + 127) / 128, g.jm - 2, g.im - 2), 128, 0, st>>>(              \
-            g, ru, rv, rw, P, w, c, incr);                                                                \
+    const dim3 cells((g.km - 1 + 127) / 128, g.jm - 2, g.im - 2);                                         \
+    if(c.press_incr) gs_incr_kernel<S><<<cells, 128, 0, st>>>(g, ru, rv, rw, P, w, c, incr);              \
+    else gs_src_kernel<S><<<cells, 128, 0, st>>>(g, au, av, aw, w, c, incr);                              \
 }                                                                                                         \
-void launch_gs_plane(Grid g, double* P, const double* incr, const S* au, const S* av, const S* aw,         \
-                     const GSW* w, PressConst c, int s, cudaStream_t st){                                   \
+void launch_gs_plane(const S*, Grid g, double* P, const double* src, const GSW* w, int s, cudaStream_t st){ \
     const int n = (g.im - 2) * (g.jm - 2);                                                                \
-    gs_hyperplane_kernel<S><<<(n + 255) / 256, 256, 0, st>>>(g, P, incr, au, av, aw, w, c, s);            \
+    gs_hyperplane_kernel<<<(n + 255) / 256, 256, 0, st>>>(g, P, src, w, s);                               \
+}                                                                                                         \
+int launch_gs_wave(const S*, Grid g, double* P, const double* src, const GSW* w, const GsPlan& pl,         \
+                   GsEdge* edge, unsigned* ticket, unsigned base, unsigned tag, int* err, cudaStream_t st){ \
+    return gs_wave_nc(g, P, src, w, pl, edge, ticket, base, tag, err, st);                                \
 }                                                                                                         \
 void launch_rb_prep(Grid g, S* au, S* av, S* aw, S* ru, S* rv, S* rw, int rigid_lid,                       \
                     const RBW* w, PressConst c, double* src, cudaStream_t st){                             \
