@@ -940,7 +940,7 @@ template <typename S>
 int run_mca(aturan_ctx* ctx){
     const Grid& g = ctx->g;
     const aturan_params& p = ctx->p;
-    if(mca_warp_bytes(g.im) > MCA_SMEM_MAX) return fail(ctx, ATURAN_E_UNSUPPORTED, "column too deep for the shared memory");
+    if(mca_col_bytes(g.im) > MCA_SMEM_MAX) return fail(ctx, ATURAN_E_UNSUPPORTED, "column too deep for the shared memory");
     int nl = 0;
     if(!ctx->mca_H_ready){
         // the cp table's running integral, formed once; ready only once its kernel has launched
@@ -975,6 +975,18 @@ int run_mca(aturan_ctx* ctx){
     a.nh4sh = X + (size_t)ATURAN_NH4SH * fs;
     a.ps = reinterpret_cast<const S*>(ctx->pstat);
     a.rho = reinterpret_cast<const S*>(ctx->forc) + (size_t)(ATURAN_RHO_MIX - ATURAN_NUE) * fs;
+    // the work fields lie in the RK4 stage buffers (free outside a step), as many to each as it holds:
+    // 12 FP64 fields, then the flags; 19 fields of the storage type each, so 9 + 3 in the mixed form
+    {
+        double* f[12];
+        const int in0 = (int)(19 * fs * sizeof(S) / (fs * sizeof(double)));
+        for(int n = 0; n < 12; n++)
+            f[n] = n < in0 ? reinterpret_cast<double*>(ctx->ybuf[0]) + n * fs : reinterpret_cast<double*>(ctx->ybuf[1]) + (n - in0) * fs;
+        a.hL = f[0]; a.qr = f[1]; a.w = f[2]; a.Teq = f[3];
+        for(int n = 0; n < MCA_NG; n++){ a.qt[n] = f[4 + n]; a.ceq[n] = f[8 + n]; }
+        a.flag = reinterpret_cast<unsigned char*>(reinterpret_cast<double*>(ctx->ybuf[1]) + 4 * fs);
+        a.next = reinterpret_cast<unsigned*>(ctx->counters + 6);
+    }
     Region reg(ctx, ATURAN_K_MCA, 0);
     const int n = launch_mca(a, ctx->st);
     if(n < 0) return fail(ctx, ATURAN_E_UNSUPPORTED, "mca: the column's shared memory");
@@ -2069,7 +2081,7 @@ int aturan_iteration(aturan_ctx* ctx, const aturan_iter_params* ip, int iter_n){
                           ip->turb.buoy != 0 || ip->turb.abl_taper != 0))
         return fail(ctx, ATURAN_E_UNSUPPORTED, "turbulence: only the default knobs are implemented");
     const bool mca = ip->mca_stride > 0 && iter_n % ip->mca_stride == 0;
-    if(ip->mca_stride > 0 && mca_warp_bytes(ctx->g.im) > MCA_SMEM_MAX)
+    if(ip->mca_stride > 0 && mca_col_bytes(ctx->g.im) > MCA_SMEM_MAX)
         return fail(ctx, ATURAN_E_UNSUPPORTED, "moist convective adjustment: column too deep for the shared memory");
     int rc;
     if(iter_n % 2 == 0){

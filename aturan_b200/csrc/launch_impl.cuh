@@ -1,6 +1,7 @@
 // Definitions of the launch wrappers declared in launch.h, instantiated per storage/compute type
 // by the translation unit that includes this file (fp64.cu, mixed.cu).
 #pragma once
+#include <algorithm>
 #include "rk4.cuh"
 #include "satadj.cuh"
 #include "pressure.cuh"
@@ -158,24 +159,40 @@ int launch_precip_impl(const PrecipArgs<S>& a, cudaStream_t st){
     precip_kernel<S><<<dim3((a.g.km + 31) / 32, a.g.jm), 128, 0, st>>>(a);
     return 1;
 }
-// The moist convective adjustment (mca.cuh): one warp per column, W warps per block, W = 4 halved
-// until the block's slices fit the shared memory; returns the launches, or -1 if one column's slice
-// does not fit.
-template <typename S>
-int launch_mca_impl(const McaArgs<S>& a, cudaStream_t st){
-    const size_t per = mca_warp_bytes(a.g.im);
-    int W = 4;
-    while(W > 1 && (size_t)W * per > MCA_SMEM_MAX) W /= 2;
-    if((size_t)W * per > MCA_SMEM_MAX) return -1;
-    const size_t sm = (size_t)W * per;
-    if(sm > 48 * 1024 &&
-       cudaFuncSetAttribute(mca_warp_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) != cudaSuccess){
+// The moist convective adjustment (mca.cuh); returns the launches, or -1 if a warp's columns do not fit
+// the shared memory. Lanes per column of the growth: 4 where there are columns enough to fill the chip
+// with them, else a warp per column.
+template <typename S, int G>
+int launch_mca_grow(const McaArgs<S>& a, cudaStream_t st){
+    const size_t sm = (32 / G) * mca_col_bytes(a.g.im);
+    if(sm > MCA_SMEM_MAX) return -1;
+    auto kern = mca_grow_kernel<S, G>;
+    if(sm > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) != cudaSuccess){
         cudaGetLastError();
         return -1;
     }
-    const long cols = (long)a.g.jm * a.g.km;
-    mca_warp_kernel<S><<<(unsigned)((cols + W - 1) / W), dim3(32, W), sm, st>>>(a);
+    int per_sm = 0;
+    if(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32, sm) != cudaSuccess || per_sm < 1){
+        cudaGetLastError();
+        return -1;
+    }
+    const long cols = (long)a.g.jm * a.g.km, blocks = (cols + 32 / G - 1) / (32 / G);
+    kern<<<(unsigned)std::min(blocks, (long)148 * per_sm), 32, sm, st>>>(a);
     return 1;
+}
+template <typename S>
+int launch_mca_impl(const McaArgs<S>& a, cudaStream_t st){
+    const Grid& g = a.g;
+    if(mca_col_bytes(g.im) > MCA_SMEM_MAX) return -1;
+    const dim3 b((g.km + 127) / 128, g.jm);
+    if(cudaMemsetAsync(a.next, 0, sizeof(unsigned), st) != cudaSuccess) return -1;
+    mca_prep_kernel<S><<<dim3(b.x, b.y, g.im), 128, 0, st>>>(a);
+    mca_test_kernel<S><<<dim3(b.x, b.y, g.im - 3), 128, 0, st>>>(a);
+    const bool small = (long)g.jm * g.km < MCA_SMALL_COLUMNS || 8 * mca_col_bytes(g.im) > MCA_SMEM_MAX;
+    const int n = small ? launch_mca_grow<S, 32>(a, st) : launch_mca_grow<S, 4>(a, st);
+    if(n < 0) return -1;
+    mca_finish_kernel<S><<<dim3(b.x, b.y, g.im - 2), 128, 0, st>>>(a);
+    return 4;
 }
 // Hydrostatic integral: threads per column (ROWS) and resident blocks per SM (MINB), measured.
 template <typename S> struct HydCfg { static constexpr int ROWS = 8, MINB = 2; };

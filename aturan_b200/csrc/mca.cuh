@@ -5,33 +5,44 @@
 // list H2O, NH3, H2S (its liquid set for both phases), CH4 and the NH4SH tracer of
 // cUranusModel.cpp:1276-1290.
 //
-// Every (j, k) column is independent. One warp takes one column and keeps its state in its own
-// slice of shared memory (16 values and 4 flags per level, two parcel slots): the lanes load,
-// convert and write back the levels in parallel, and run in parallel everything of a sweep that
-// does not depend on what the sweep has done before it:
-//   * at the start of each sweep every pair test (i, i+1) is evaluated, one pair per lane; while
-//     the sweep walks up the column a pair is re-tested only if one of its two cells has been
-//     mixed in this sweep, which is exactly when its inputs differ from the start's (the
-//     reference's first sweep makes the same reuse with its cached test of untouched pairs); the
-//     re-test's two equilibria (the parcel, the upper cell's own) are solved on two lanes at once;
-//   * a segment's mass-weighted means are summed by lane 0 in the reference's order; then one
-//     round of equilibria settles each of its cells on its own lane and, on further lanes, solves
-//     what the two growth tests (below and above) need, since none of those solves reads another's
-//     result (the lower neighbour lifted to the segment's bottom level, the mixed top cell lifted
-//     to the level above, that level's own equilibrium); the tests' decisions follow.
-// Each solve is a cell's equilibrium by Illinois regula falsi, so the arithmetic is FP64 whatever
-// the storage (FP32 storage in the mixed form is widened, T read as its FP32 pair). The solve, the
-// decision, the energy balance and the enthalpy inverse are out-of-line functions, and every round
-// reaches the solve through one call site: inlined at each call site the kernel's code outgrew the
-// instruction cache and most issue slots went unused for want of an instruction.
-// Every loop is bounded: 60 regula-falsi steps, 30 Newton steps of the enthalpy inverse, 64
-// sweeps, and a segment grows by one level per step within the column.
+// Every (j, k) column is independent, and within a column the reference's sweep is a serial chain of
+// equilibrium solves (Illinois regula falsi on the energy balance, FP64 whatever the storage: FP32
+// storage in the mixed form is widened, T read as its FP32 pair). Four launches take out of that
+// chain everything that is not part of it:
+//   mca_prep_kernel    per cell: liquid-water static energy, total mixing ratios, weight;
+//   mca_test_kernel    per pair (i, i+1): the upper cell's own equilibrium, the parcel's, the pair
+//                      test: all of a sweep's tests at its start, one thread each;
+//   mca_grow_kernel    per column with an unstable pair: the segments' growth, G lanes per column,
+//                      32 / G columns per warp, a column taken from a counter when one is finished;
+//   mca_finish_kernel  per mixed cell: its equilibrium at the final means, the write-back.
+// What makes this the reference's sweep:
+//   * A growth step reads only the equilibrium of the segment's lowest cell (the test below) and of
+//     the cell above it (unmixed, so the one of the start), and two parcels: three solves on three
+//     lanes at once. The other cells' equilibria are overwritten by the next step, so they are formed
+//     once, at the end. A solve can fail only on a non-finite energy (with cp(T); without, on a
+//     non-positive temperature, first at the top cell), which each step checks for the whole segment.
+//   * A segment stops growing when both its edge pairs test stable, so the reference's re-test of its
+//     upper edge is that same test again: the walk continues above it.
+//   * After one sweep every pair is stable: pairs inside a segment hold equal values, so the parcel
+//     and the upper cell's equilibrium are one solve and their difference is exactly zero; a segment's
+//     edge pairs were tested with the values they still have; every other pair was stable at the start
+//     and has not changed. The reference's further sweep finds nothing, so there is none here.
+// Measured at 41x181x361 (mixed, synthetic state): 6.0 ms -- prep 0.14, tests 1.38, growth 3.95, finish
+// 0.55 -- against 44.7 ms for one warp per column running the whole sweep with every settle and a
+// verifying sweep; 1.28 against 8.1 ms at 37x83x167, 0.63 against 0.88 ms at 21x37x73. Same bits.
+// The growth chain is what is left of the serial part: bound by the latency of its solves on small
+// grids, by FP64 issue on large ones. G = 4 keeps three of four lanes busy; with few columns a warp
+// per column (G = 32) has the shorter chain, as no other column of the warp delays it.
+// Every loop is bounded: 60 regula-falsi steps, 30 Newton steps of the enthalpy inverse, and a
+// segment grows by at least one level per step within the column.
 #pragma once
 #include "common.cuh"
 
 namespace aturan {
 
 constexpr int MCA_NG = 4;
+// Below as many columns as the chip holds groups of warps for, a warp per column in the growth.
+constexpr long MCA_SMALL_COLUMNS = 148 * 64;
 constexpr double CP_T_LO_D = 5.0, CP_T_HI_D = 1500.0, CP_DT_D = 0.5;   // CpH2.h:13
 
 struct McaGas { double ep, lv, ls, t_0, C, L0, R, del_alf, del_bet, C_i, L0_i, del_alf_i, del_bet_i; };
@@ -53,6 +64,11 @@ struct McaArgs {
     S* sp[MCA_NG][3];                // vapour, cloud, ice
     S* nh4sh;
     const S *ps, *rho;
+    // work fields in the padded layout: energy, NH4SH ratio, weight (0: the column is left alone), total
+    // ratios, the upper cells' own equilibria (Teq = 0: the solve failed) and their condensates
+    double *hL, *qr, *w, *qt[MCA_NG], *Teq, *ceq[MCA_NG];
+    unsigned char* flag;             // per cell: 1 the pair (i, i+1) is unstable at the start; 2 the cell was mixed
+    unsigned* next;                  // columns handed out to mca_grow_kernel's groups
 };
 
 __device__ __forceinline__ double mca_mx(double a, double b){ return (a < b) ? b : a; }   // std::max
@@ -63,6 +79,7 @@ static __device__ double mca_cp_h2(const McaConst& A, double T){
     const double Tc = T < CP_T_LO_D ? CP_T_LO_D : T;
     const double x = ((Tc > CP_T_HI_D ? CP_T_HI_D : Tc) - CP_T_LO_D) / CP_DT_D;
     int i = (int)x; if(i > CP_TABLE_N - 2) i = CP_TABLE_N - 2;
+    if(i < 0) i = 0;                                 // a NaN's index (the value stays NaN through f)
     const double f = x - i;
     return A.cp_tab[i] + f * (A.cp_tab[i + 1] - A.cp_tab[i]);
 }
@@ -73,6 +90,7 @@ static __device__ double mca_enth_h2(const McaConst& A, double T){
     if(T >= CP_T_HI_D) return A.H_tab[n - 1] + A.cp_tab[n - 1] * (T - CP_T_HI_D);
     const double x = (T - CP_T_LO_D) / CP_DT_D;
     int i = (int)x; if(i > n - 2) i = n - 2;
+    if(i < 0) i = 0;
     const double f = x - i;
     return A.H_tab[i] + CP_DT_D * f * (A.cp_tab[i] + 0.5 * f * (A.cp_tab[i + 1] - A.cp_tab[i]));
 }
@@ -103,286 +121,363 @@ static __device__ __noinline__ double mca_enth_inv(const McaConst& A, double h, 
 // ATPhys.h:49-53 (the saturation pressure) and ConvectiveAdjustment.h:437-453 without the phase
 // split; lg = log(T), the same value for every gas at one T, formed once by the caller
 __device__ __forceinline__ double mca_qsat(const McaGas& s, double T, double lg, double pr){
-    const double E = (T >= s.t_0) ? exp(s.C + (-s.L0 / T + s.del_alf * lg + s.del_bet * T) / (1e-3 * s.R))
-                                  : exp(s.C_i + (-s.L0_i / T + s.del_alf_i * lg + s.del_bet_i * T) / (1e-3 * s.R));
+    const bool liq = T >= s.t_0;                     // one expression for both sets: the lanes' phases differ
+    const double C = liq ? s.C : s.C_i, L0 = liq ? s.L0 : s.L0_i;
+    const double al = liq ? s.del_alf : s.del_alf_i, be = liq ? s.del_bet : s.del_bet_i;
+    const double E = exp(C + (-L0 / T + al * lg + be * T) / (1e-3 * s.R));
     const double q = s.ep * E / pr;
     return isfinite(q) ? q : 0.0;
 }
 __device__ __forceinline__ double mca_lat(const McaGas& s, double T){ return T >= s.t_0 ? s.lv : s.ls; }
 
-static __device__ __noinline__ double mca_fof(const McaConst& A, double TT, double hL, const double* qt, double pr, double z){
-    double f = mca_enth(A, TT) + A.grav * z - hL;
-    const double lg = log(TT);
-    for(int g = 0; g < MCA_NG; g++) f -= mca_lat(A.G[g], TT) * mca_mx(0.0, qt[g] - mca_qsat(A.G[g], TT, lg, pr));
-    return f;
+// Level height as the model stores it (float).
+__device__ __forceinline__ double mca_z(const McaConst& A, int i){ return (double)((float)i * A.hz) * 1.0e3; }
+__device__ __forceinline__ double mca_rho(const McaConst& A, double r_){     // rho_at, cUranusModel.h:526-531
+    if(!A.local_rho) return A.r_mix;
+    return (r_ > 0.0 && isfinite(r_)) ? r_ : A.r_mix;
 }
 
-// :455-488, the equilibrium of (hL, qt) at (p, z): Illinois regula falsi on the energy balance
-static __device__ __noinline__ bool mca_equil(const McaConst& A, double hL, const double* qt, double pr, double z, double& T, double* cond){
+// :455-488, the equilibrium of (hL, qt) at (p, z): Illinois regula falsi on the energy balance. The
+// balance is evaluated at one place in the code -- at the dry temperature T_lo (stage 0), the upper
+// bracket (stage 1), then the regula-falsi points -- so that lanes at different stages run together,
+// and the values at the returned T are kept rather than formed again.
+static __device__ __forceinline__ bool mca_equil(const McaConst& A, double hL, const double (&qt)[MCA_NG], double pr, double z,
+                                                 double& T, double (&cond)[MCA_NG]){
     const double cp = A.cp_mix, tol_T = 1.0e-10;
     const double T_lo = A.cp_dyn ? mca_enth_inv(A, hL - A.grav * z, 0.0) : (hL - A.grav * z) / cp;
     if(!(T_lo > 0.0) || !(pr > 0.0)) return false;
-    bool any = false;
-    const double lg_lo = log(T_lo);
-    for(int g = 0; g < MCA_NG; g++) if(qt[g] > mca_qsat(A.G[g], T_lo, lg_lo, pr)){ any = true; break; }
-    if(!any){ T = T_lo; for(int g = 0; g < MCA_NG; g++) cond[g] = 0.0; return true; }
-    double span = 0.0;
-    for(int g = 0; g < MCA_NG; g++) span += mca_mx(A.G[g].lv, A.G[g].ls) * mca_mx(0.0, qt[g]);
-    double a = T_lo, b = A.cp_dyn ? mca_enth_inv(A, mca_enth(A, T_lo) + span, T_lo) + 1.0e-9 : T_lo + span / cp + 1.0e-9;
-    double fa = mca_fof(A, a, hL, qt, pr, z), fb = mca_fof(A, b, hL, qt, pr, z);
+    double a = T_lo, b = T_lo, fa = 0.0, fb = 0.0, x = T_lo;
     int side = 0;
-    for(int it = 0; it < 60 && b - a > tol_T; it++){
-        double c = (fb - fa != 0.0) ? b - fb * (b - a) / (fb - fa) : 0.5 * (a + b);
-        if(!(c > a && c < b)) c = 0.5 * (a + b);
-        const double fc = mca_fof(A, c, hL, qt, pr, z);
-        if(fc < 0.0){ a = c; fa = fc; if(side == -1) fb *= 0.5; side = -1; }
-        else        { b = c; fb = fc; if(side == +1) fa *= 0.5; side = +1; }
-        if(fabs(fc) <= cp * tol_T){ a = b = c; break; }
+    for(int n = -2; ; n++){                          // n = it of the reference's loop from 0 on
+        const double e = mca_enth(A, x);
+        const double lg = log(x);
+        double f = e + A.grav * z - hL;
+        double d[MCA_NG];
+        bool any = false;
+#pragma unroll
+        for(int g = 0; g < MCA_NG; g++){
+            const double q = mca_qsat(A.G[g], x, lg, pr);
+            any |= qt[g] > q;
+            d[g] = mca_mx(0.0, qt[g] - q);
+            f -= mca_lat(A.G[g], x) * d[g];
+        }
+        bool keep = true;                            // x is the upper bracket: its condensates are the result's
+        bool stop = false;
+        if(n == -2){
+            if(!any){ T = T_lo; for(int g = 0; g < MCA_NG; g++) cond[g] = 0.0; return true; }
+            fa = f;
+            double span = 0.0;
+#pragma unroll
+            for(int g = 0; g < MCA_NG; g++) span += mca_mx(A.G[g].lv, A.G[g].ls) * mca_mx(0.0, qt[g]);
+            b = A.cp_dyn ? mca_enth_inv(A, e + span, T_lo) + 1.0e-9 : T_lo + span / cp + 1.0e-9;
+            x = b;
+            continue;
+        }
+        if(n == -1) fb = f;
+        else {
+            if(f < 0.0){ a = x; fa = f; if(side == -1) fb *= 0.5; side = -1; keep = false; }
+            else       { b = x; fb = f; if(side == +1) fa *= 0.5; side = +1; }
+            if(fabs(f) <= cp * tol_T){ a = b = x; keep = stop = true; }
+        }
+        if(keep){
+#pragma unroll
+            for(int g = 0; g < MCA_NG; g++) cond[g] = d[g];
+        }
+        if(stop || !(n + 1 < 60 && b - a > tol_T)) break;
+        x = (fb - fa != 0.0) ? b - fb * (b - a) / (fb - fa) : 0.5 * (a + b);
+        if(!(x > a && x < b)) x = 0.5 * (a + b);
     }
     T = b;
-    const double lg_b = log(T);
-    for(int g = 0; g < MCA_NG; g++) cond[g] = mca_mx(0.0, qt[g] - mca_qsat(A.G[g], T, lg_b, pr));
     return true;
 }
-
-// One column's state in its warp's slice of shared memory (levels 0..im-1, i0..i1 used).
-struct McaCol {
-    double *T, *p, *z, *rho, *w, *hL, *qr, *Teq;   // im each
-    double *qt, *ceq;                              // im * MCA_NG each
-    double *par;                                   // two parcel results: T, condensate[4], solved
-    unsigned char *touched, *eq_ok, *mod, *U;      // im each: mixed ever, equilibrium cached,
-                                                   // mixed in this sweep, the pair test of the sweep's start
-};
-constexpr int MCA_PAR = 6;                         // doubles per parcel slot
-// Bytes of one warp's slice for a column of im levels; a block's slices share at most MCA_SMEM_MAX.
-constexpr size_t MCA_SMEM_MAX = 227 * 1024;
-__host__ __device__ inline size_t mca_warp_bytes(int im){
-    return (size_t)(16 * im + 2 * MCA_PAR) * sizeof(double) + (((size_t)4 * im + 7) / 8) * 8;
-}
-__device__ inline McaCol mca_col(char* base, int im){
-    McaCol C;
-    double* d = reinterpret_cast<double*>(base);
-    C.T = d; C.p = d + im; C.z = d + 2 * im; C.rho = d + 3 * im; C.w = d + 4 * im; C.hL = d + 5 * im;
-    C.qr = d + 6 * im; C.Teq = d + 7 * im; C.qt = d + 8 * im; C.ceq = d + 12 * im; C.par = d + 16 * im;
-    unsigned char* f = reinterpret_cast<unsigned char*>(d + 16 * im + 2 * MCA_PAR);
-    C.touched = f; C.eq_ok = f + im; C.mod = f + 2 * im; C.U = f + 3 * im;
-    return C;
-}
-
-__device__ __forceinline__ double mca_trE(const McaConst& A, const McaCol& C, int i){ double e = 0.0; e += A.L_tr * C.qr[i]; return e; }
+__device__ __forceinline__ double mca_trE(const McaConst& A, double qr){ double e = 0.0; e += A.L_tr * qr; return e; }
 
 // :613-624, Ledoux virtual temperature with condensate loading; NH4SH is a condensed tracer
-static __device__ double mca_tv(const McaConst& A, const McaCol& C, double TT, const double* v_, const double* cnd, int i_tr){
+static __device__ __forceinline__ double mca_tv(const McaConst& A, double TT, const double (&v_)[MCA_NG], const double (&cnd)[MCA_NG], double qr){
     double f = 1.0;
+#pragma unroll
     for(int g = 0; g < MCA_NG; g++){ f += v_[g] * (1.0 / A.G[g].ep - 1.0); f -= cnd[g]; }
-    f -= C.qr[i_tr];
+    f -= qr;
     return TT * f;
 }
-
-// The equilibrium of cell a's state (hL, qt, NH4SH) at level b's pressure and height: the parcel
-// of a pair test (a below b), or a cell's own (a = b).
-__device__ __forceinline__ bool mca_solve_at(const McaConst& A, const McaCol& C, int a, int b, double& T, double* c){
-    return mca_equil(A, C.hL[a] + mca_trE(A, C, a), &C.qt[a * MCA_NG], C.p[b], C.z[b], T, c);
-}
-
-// :627-644, the test of the pair (a, b = a+1) once both equilibria are known: the parcel (cell a at
-// b's level: Tp, pc) against cell b's cached equilibrium.
-static __device__ __noinline__ bool mca_decide(const McaConst& A, const McaCol& C, double Tp, const double* pc, int a, int b){
+// :627-644, the test of a pair: the parcel (the lower cell's qt_a, qr_a at the upper cell's level: Tp, pc)
+// against the upper cell (qt_b, qr_b, its own equilibrium Tb, ec).
+static __device__ __forceinline__ bool mca_decide(const McaConst& A, double Tp, const double (&pc)[MCA_NG], const double (&qta)[MCA_NG], double qra,
+                                                  double Tb, const double (&ec)[MCA_NG], const double (&qtb)[MCA_NG], double qrb){
     const double tol_K = 1.0e-7;
-    double pv[MCA_NG], ec[MCA_NG], ev[MCA_NG];
-    const double Tb = C.Teq[b];
-    for(int g = 0; g < MCA_NG; g++) ec[g] = C.ceq[b * MCA_NG + g];
-    for(int g = 0; g < MCA_NG; g++){ pv[g] = C.qt[a * MCA_NG + g] - pc[g]; ev[g] = C.qt[b * MCA_NG + g] - ec[g]; }
-    const double dTv = mca_tv(A, C, Tp, pv, pc, a) - mca_tv(A, C, Tb, ev, ec, b);
+    double pv[MCA_NG], ev[MCA_NG];
+#pragma unroll
+    for(int g = 0; g < MCA_NG; g++){ pv[g] = qta[g] - pc[g]; ev[g] = qtb[g] - ec[g]; }
+    const double dTv = mca_tv(A, Tp, pv, pc, qra) - mca_tv(A, Tb, ev, ec, qrb);
     return dTv > tol_K;
 }
 
-// The whole test of the pair (a, b) on one lane: the parcel, b's equilibrium if not cached (written
-// by this lane only: each cell is the upper cell of one pair), the decision.
-static __device__ __noinline__ bool mca_unstable(const McaConst& A, McaCol& C, int a, int b){
-    double Tp, pc[MCA_NG];
-    if(!mca_solve_at(A, C, a, b, Tp, pc)) return false;
-    if(!C.eq_ok[b]){
-        if(!mca_solve_at(A, C, b, b, C.Teq[b], &C.ceq[b * MCA_NG])) return false;
-        C.eq_ok[b] = 1;
-    }
-    return mca_decide(A, C, Tp, pc, a, b);
-}
-
-// One round of equilibria across the warp, task t on lane t mod 32, every solve through one call
-// site so that the lanes run it together. Tasks 0 .. nset-1 settle the segment cells lo .. lo+nset-1
-// at their own levels (:645-661: T, the cached equilibrium, touched); the parcel tasks (cell ca
-// lifted to level lb, result in parcel slot s) and the own-equilibrium task (cell own, if not
-// cached) follow. Returns false on the lanes whose settle failed.
-__device__ __forceinline__ bool mca_round(const McaConst& A, McaCol& C, int lane, int lo, int nset,
-                                          int ca0, int lb0, int ca1, int lb1, int own){
-    const int ntask = nset + 3;
-    bool sok = true;
-    for(int t = lane; t < ntask; t += 32){
-        int ca, lb, slot = -1;
-        if(t < nset){ ca = lb = lo + t; }
-        else if(t == nset){ if(ca0 < 0) continue; ca = ca0; lb = lb0; slot = 0; }
-        else if(t == nset + 1){ if(ca1 < 0) continue; ca = ca1; lb = lb1; slot = 1; }
-        else { if(own < 0 || C.eq_ok[own]) continue; ca = lb = own; }
-        double* To = slot < 0 ? &C.Teq[lb] : &C.par[slot * MCA_PAR];
-        double* co = slot < 0 ? &C.ceq[lb * MCA_NG] : &C.par[slot * MCA_PAR + 1];
-        const bool ok = mca_solve_at(A, C, ca, lb, *To, co);
-        if(slot >= 0) C.par[slot * MCA_PAR + 5] = ok ? 1.0 : 0.0;
-        else if(ok){ C.eq_ok[lb] = 1; if(t < nset){ C.T[lb] = C.Teq[lb]; C.touched[lb] = 1; } }
-        else if(t < nset) sok = false;
-    }
-    return sok;
-}
-// The decision of a pair whose parcel is in slot s and whose upper cell's equilibrium is cached.
-__device__ __forceinline__ bool mca_slot_unstable(const McaConst& A, const McaCol& C, int s, int a, int b){
-    return C.par[s * MCA_PAR + 5] != 0.0 && C.eq_ok[b] && mca_decide(A, C, C.par[s * MCA_PAR], &C.par[s * MCA_PAR + 1], a, b);
-}
-
-// One warp per (j, k) column (blockDim = (32, W)), k over all km stored meridians as the reference
-// loops; the warp's slice of dynamic shared memory holds the column. The arguments stay in the
-// constant bank (__grid_constant__): the out-of-line helpers take the constants by reference, which
-// otherwise copies the whole argument block to every thread's stack and reads it from there. Six
-// resident blocks per SM (80 registers, the sweep's bookkeeping partly spilled to L1) measured 7 %
-// faster than four at 128 registers.
+// The arguments stay in the constant bank (__grid_constant__): the out-of-line enthalpy inverse takes the
+// constants by reference, which otherwise copies the whole argument block to every thread's stack.
 template <typename S>
-__global__ void __launch_bounds__(128, 6) mca_warp_kernel(const __grid_constant__ McaArgs<S> a){
+__global__ void __launch_bounds__(128) mca_prep_kernel(const __grid_constant__ McaArgs<S> a){
+    const Grid& g = a.g;
+    const McaConst& A = a.c;
+    const int k = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, i = blockIdx.z;
+    if(k >= g.km) return;
+    const size_t o = gidx(g, i, j, k);
+    const int i0 = 1, i1 = g.im - 2;
+    a.flag[o] = 0;
+    if(i < i0 || i > i1) return;
+    const double T = t_ld(a.t, a.tlo, o) * A.t_ref, p = (double)a.ps[o];
+    const double rho = mca_rho(A, A.local_rho ? (double)a.rho[o] : 0.0), z = mca_z(A, i);
+    bool ok = (T > 0.0) && (p > 0.0) && (rho > 0.0) && isfinite(T + p + rho);
+    const double lo = (i > i0) ? 0.5 * (mca_z(A, i - 1) + z) : mca_z(A, i0);
+    const double hi = (i < i1) ? 0.5 * (z + mca_z(A, i + 1)) : mca_z(A, i1);
+    const double w = rho * (hi - lo);
+    if(!(w > 0.0)) ok = false;
+    if(!ok){ a.w[o] = 0.0; return; }                 // its column is left alone: nothing else is read
+    double h = mca_enth(A, T) + A.grav * z;
+#pragma unroll
+    for(int q = 0; q < MCA_NG; q++){
+        const double qv = mca_mx(0.0, (double)a.sp[q][0][o]) / rho;
+        const double qc = mca_mx(0.0, (double)a.sp[q][1][o]) / rho;
+        const double qi = mca_mx(0.0, (double)a.sp[q][2][o]) / rho;
+        a.qt[q][o] = qv + qc + qi;
+        h -= A.G[q].lv * qc + A.G[q].ls * qi;
+    }
+    const double qr = (double)a.nh4sh[o] / rho;
+    h -= A.L_tr * qr;
+    a.qr[o] = qr;
+    a.hL[o] = h;
+    a.w[o] = w;
+}
+
+// Thread (i, j, k): cell i + 1's own equilibrium and the test of the pair (i, i + 1), i = 1 .. im-3.
+template <typename S>
+__global__ void __launch_bounds__(128) mca_test_kernel(const __grid_constant__ McaArgs<S> a){
+    const Grid& g = a.g;
+    const McaConst& A = a.c;
+    const int k = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, i = 1 + blockIdx.z;
+    if(k >= g.km) return;
+    const size_t o = gidx(g, i, j, k), ob = o + (size_t)g.jm * g.kp;
+    if(!(a.w[o] > 0.0) || !(a.w[ob] > 0.0)) return;  // a column that is left alone
+    double qa[MCA_NG], qb[MCA_NG];
+#pragma unroll
+    for(int q = 0; q < MCA_NG; q++){ qa[q] = a.qt[q][o]; qb[q] = a.qt[q][ob]; }
+    const double qra = a.qr[o], qrb = a.qr[ob];
+    const double ha = a.hL[o] + mca_trE(A, qra), hb = a.hL[ob] + mca_trE(A, qrb);
+    const double pr = (double)a.ps[ob], z = mca_z(A, i + 1);
+    double Tp = 0.0, pc[MCA_NG] = {0.0, 0.0, 0.0, 0.0}, Tb = 0.0, ec[MCA_NG] = {0.0, 0.0, 0.0, 0.0};
+    bool okp = false, okb = false;
+#pragma unroll 1
+    for(int s = 0; s < 2; s++){                      // the upper cell, then the parcel: one call site
+        double x[MCA_NG], T = 0.0, c[MCA_NG] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+        for(int q = 0; q < MCA_NG; q++) x[q] = s ? qa[q] : qb[q];
+        const bool ok = mca_equil(A, s ? ha : hb, x, pr, z, T, c);
+        if(s){ okp = ok; Tp = T; } else { okb = ok; Tb = T; }
+#pragma unroll
+        for(int q = 0; q < MCA_NG; q++){ if(s) pc[q] = c[q]; else ec[q] = c[q]; }
+    }
+    a.Teq[ob] = okb ? Tb : 0.0;
+#pragma unroll
+    for(int q = 0; q < MCA_NG; q++) a.ceq[q][ob] = ec[q];
+    a.flag[o] = okp && okb && mca_decide(A, Tp, pc, qa, qra, Tb, ec, qb, qrb) ? 1 : 0;
+}
+
+// One column's state in its group's slice of shared memory, and its bytes (7 doubles and a flag per level).
+struct McaCol { double *hL, *qr, *w, *qt; unsigned char* flag; };
+constexpr size_t MCA_SMEM_MAX = 227 * 1024;
+__host__ __device__ inline size_t mca_col_bytes(int im){ return (size_t)7 * im * sizeof(double) + ((size_t)im + 7) / 8 * 8; }
+
+// Blocks of one warp, G lanes per column. A group walks up its column from unstable pair to unstable
+// pair; every turn of the loop is one growth step of each group's segment, its three solves on three
+// lanes through one call site.
+template <typename S, int G>
+__global__ void __launch_bounds__(32) mca_grow_kernel(const __grid_constant__ McaArgs<S> a){
     extern __shared__ __align__(16) char mca_smem[];
     const Grid& g = a.g;
     const McaConst& A = a.c;
-    const unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x;
-    const long col = (long)blockIdx.x * blockDim.y + threadIdx.y;
-    if(col >= (long)g.jm * g.km) return;                     // a whole warp
-    const int j = (int)(col / g.km), k = (int)(col % g.km);
+    const int lane = threadIdx.x, gl = lane % G, grp = lane / G;
+    const unsigned gm = G == 32 ? 0xffffffffu : ((1u << (G & 31)) - 1u) << (grp * G);
     const int im = g.im, i0 = 1, i1 = im - 2;
-    if(i1 - i0 < 1) return;
-    McaCol C = mca_col(mca_smem + threadIdx.y * mca_warp_bytes(im), im);
-    const size_t pl = (size_t)g.jm * g.kp, o0 = gidx(g, 0, j, k);
-
-    bool ok = true;
-    for(int i = i0 + lane; i <= i1; i += 32){
-        const size_t o = o0 + (size_t)i * pl;
-        C.T[i] = t_ld(a.t, a.tlo, o) * A.t_ref;
-        C.p[i] = (double)a.ps[o];
-        C.z[i] = (double)((float)i * A.hz) * 1.0e3;
-        double rr = A.r_mix;                                // rho_at, cUranusModel.h:526-531
-        if(A.local_rho){ const double r_ = (double)a.rho[o]; rr = (r_ > 0.0 && isfinite(r_)) ? r_ : A.r_mix; }
-        C.rho[i] = rr;
-        if(!(C.T[i] > 0.0) || !(C.p[i] > 0.0) || !(C.rho[i] > 0.0) || !isfinite(C.T[i] + C.p[i] + C.rho[i])) ok = false;
+    const unsigned ncol = (unsigned)(g.jm * g.km);
+    const size_t pl = (size_t)g.jm * g.kp;
+    McaCol C;
+    {
+        double* d = reinterpret_cast<double*>(mca_smem + grp * mca_col_bytes(im));
+        C.hL = d; C.qr = d + im; C.w = d + 2 * im; C.qt = d + 3 * im;
+        C.flag = reinterpret_cast<unsigned char*>(d + 7 * im);
     }
-    if(!__all_sync(FULL, ok)) return;
-    __syncwarp();
-    for(int i = i0 + lane; i <= i1; i += 32){
-        const size_t o = o0 + (size_t)i * pl;
-        const double lo = (i > i0) ? 0.5 * (C.z[i - 1] + C.z[i]) : C.z[i0];
-        const double hi = (i < i1) ? 0.5 * (C.z[i] + C.z[i + 1]) : C.z[i1];
-        C.w[i] = C.rho[i] * (hi - lo);
-        if(!(C.w[i] > 0.0)) ok = false;
-        double h = mca_enth(A, C.T[i]) + A.grav * C.z[i];
-        for(int q = 0; q < MCA_NG; q++){
-            const int x = i * MCA_NG + q;
-            const double qv = mca_mx(0.0, (double)a.sp[q][0][o]) / C.rho[i];
-            const double qc = mca_mx(0.0, (double)a.sp[q][1][o]) / C.rho[i];
-            const double qi = mca_mx(0.0, (double)a.sp[q][2][o]) / C.rho[i];
-            C.qt[x] = qv + qc + qi;
-            h -= A.G[q].lv * qc + A.G[q].ls * qi;
+    bool active = false, done = false, have = false;     // a segment is growing; no column left; a column is loaded
+    int i = i0, lo = 0, hi = 0;
+    size_t o0 = 0;
+    while(true){
+        // a group without a segment: the next unstable pair of its column, or of the next column
+        while(!active && !done){
+            if(!have){
+                unsigned c = 0;
+                if(gl == 0) c = atomicAdd(a.next, 1u);
+                c = __shfl_sync(gm, c, 0, G);
+                if(c >= ncol){ done = true; break; }
+                const int j = (int)(c / (unsigned)g.km), k = (int)(c - (unsigned)j * g.km);
+                o0 = gidx(g, 0, j, k);
+                int un = 0, ok = 1;
+                for(int q = i0 + gl; q <= i1; q += G){
+                    const size_t o = o0 + (size_t)q * pl;
+                    const unsigned char f = a.flag[o];
+                    const double w = a.w[o];
+                    C.flag[q] = f; C.w[q] = w;
+                    un |= f;
+                    if(!(w > 0.0)) ok = 0;
+                }
+                un = __any_sync(gm, un);
+                ok = __all_sync(gm, ok);
+                if(!un) continue;
+                if(!ok){                                  // the column keeps its state
+                    for(int q = i0 + gl; q <= i1; q += G) a.flag[o0 + (size_t)q * pl] = 0;
+                    continue;
+                }
+                for(int q = i0 + gl; q <= i1; q += G){
+                    const size_t o = o0 + (size_t)q * pl;
+                    C.hL[q] = a.hL[o]; C.qr[q] = a.qr[o];
+#pragma unroll
+                    for(int s = 0; s < MCA_NG; s++) C.qt[q * MCA_NG + s] = a.qt[s][o];
+                }
+                __syncwarp(gm);
+                have = true;
+                i = i0;
+            }
+            // the first pair at or above i that was unstable at the start
+            while(i < i1){
+                const bool u = i + gl < i1 && C.flag[i + gl] == 1;
+                const unsigned m = __ballot_sync(gm, u) & gm;
+                if(m){ i += __ffs(m >> (grp * G)) - 1; break; }
+                i += G;
+            }
+            if(i < i1){ active = true; lo = i; hi = i + 1; break; }
+            // the column is finished: mixed cells' means and flags back
+            for(int q = i0 + gl; q <= i1; q += G){
+                const size_t o = o0 + (size_t)q * pl;
+                const bool mixed = C.flag[q] == 2;
+                a.flag[o] = mixed ? 2 : 0;
+                if(mixed){
+                    a.hL[o] = C.hL[q]; a.qr[o] = C.qr[q];
+#pragma unroll
+                    for(int s = 0; s < MCA_NG; s++) a.qt[s][o] = C.qt[q * MCA_NG + s];
+                }
+            }
+            __syncwarp(gm);
+            have = false;
         }
-        C.qr[i] = (double)a.nh4sh[o] / C.rho[i];
-        h -= A.L_tr * C.qr[i];
-        C.hL[i] = h;
-    }
-    for(int i = lane; i < im; i += 32){ C.touched[i] = 0; C.eq_ok[i] = 0; }
-    if(!__all_sync(FULL, ok)) return;
-    __syncwarp();
-
-    int passes = 0;
-    bool changed = true, fail = false;
-    long layers = 0;
-    while(changed && passes < 64 && !fail){
-        changed = false; passes++;
-        // every pair's test at the start of the sweep, one pair per lane
-        for(int i = i0 + lane; i < i1; i += 32) C.U[i] = mca_unstable(A, C, i, i + 1) ? 1 : 0;
-        for(int i = lane; i < im; i += 32) C.mod[i] = 0;
+        if(__all_sync(0xffffffffu, done)) return;
+        bool task = false, below = false, above = false;
+        int ca = lo, lb = lo;
+        if(active){
+            // the segment's mass-weighted means, each sum by one lane in the reference's order
+            double sw = 0.0, s0 = 0.0, s1 = 0.0;
+            if(gl < 4){
+                // lane 0: w and w hL; lanes 1, 2: two of w qt; lane 3: w qr
+                const double* x0 = gl == 0 ? C.hL : (gl == 3 ? C.qr : C.qt + (gl - 1) * 2);
+                const int st = gl == 0 || gl == 3 ? 1 : MCA_NG;
+                const double* x1 = st == 1 ? x0 : x0 + 1;
+                for(int q = lo; q <= hi; q++){
+                    const double w = C.w[q];
+                    sw += w;
+                    s0 += w * x0[q * st];
+                    s1 += w * x1[q * st];
+                }
+                s0 = s0 / sw;
+                s1 = s1 / sw;
+            }
+            const double m_h = __shfl_sync(gm, s0, 0, G), m_r = __shfl_sync(gm, s0, 3, G);
+            double m_q[MCA_NG];
+            m_q[0] = __shfl_sync(gm, s0, 1, G); m_q[1] = __shfl_sync(gm, s1, 1, G);
+            m_q[2] = __shfl_sync(gm, s0, 2, G); m_q[3] = __shfl_sync(gm, s1, 2, G);
+            for(int q = lo + gl; q <= hi; q += G){
+                C.hL[q] = m_h; C.qr[q] = m_r; C.flag[q] = 2;
+#pragma unroll
+                for(int s = 0; s < MCA_NG; s++) C.qt[q * MCA_NG + s] = m_q[s];
+            }
+            __syncwarp(gm);
+            // a settle of one of its cells would fail (mca_equil): the column keeps its state
+            const double h_top = m_h + mca_trE(A, m_r) - A.grav * mca_z(A, hi);
+            if(A.cp_dyn ? !isfinite(h_top) : !(h_top / A.cp_mix > 0.0)){
+                for(int q = i0 + gl; q <= i1; q += G) a.flag[o0 + (size_t)q * pl] = 0;
+                __syncwarp(gm);
+                active = have = false;
+            } else {
+                below = lo > i0; above = hi < i1;
+                if(gl == 0){ task = below; }                                       // cell lo's own equilibrium
+                else if(gl == 1){ task = below; ca = lo - 1; }                     // cell lo - 1 lifted to lo
+                else if(gl == 2){ task = above; ca = hi; lb = hi + 1; }            // the mixed cell hi lifted to hi + 1
+            }
+        }
         __syncwarp();
-        int i = i0;
-        while(i < i1 && !fail){
-            bool uns;
-            if(!C.mod[i] && !C.mod[i + 1]) uns = C.U[i] != 0;
-            else {
-                // re-test: the parcel (lane 0) and cell i+1's own equilibrium (lane 1) in one round
-                mca_round(A, C, lane, i, 0, i, i + 1, -1, -1, i + 1);
-                __syncwarp();
-                int u = 0;
-                if(lane == 0) u = mca_slot_unstable(A, C, 0, i, i + 1) ? 1 : 0;
-                u = __shfl_sync(FULL, u, 0);
-                uns = u != 0;
-                __syncwarp();
-            }
-            if(!uns){ i++; continue; }
-            int lo = i, hi = i + 1;
-            for(;;){
-                // the segment's mass-weighted means, summed in the reference's order
-                double m_h = 0.0, m_q[MCA_NG], m_r = 0.0;
-                if(lane == 0){
-                    double sw = 0.0, sh = 0.0, sq[MCA_NG] = {0.0, 0.0, 0.0, 0.0}, sr = 0.0;
-                    for(int q = lo; q <= hi; q++){
-                        sw += C.w[q]; sh += C.w[q] * C.hL[q];
-                        for(int s = 0; s < MCA_NG; s++) sq[s] += C.w[q] * C.qt[q * MCA_NG + s];
-                        sr += C.w[q] * C.qr[q];
-                    }
-                    m_h = sh / sw;
-                    for(int s = 0; s < MCA_NG; s++) m_q[s] = sq[s] / sw;
-                    m_r = sr / sw;
-                }
-                m_h = __shfl_sync(FULL, m_h, 0);
-                for(int s = 0; s < MCA_NG; s++) m_q[s] = __shfl_sync(FULL, lane == 0 ? m_q[s] : 0.0, 0);
-                m_r = __shfl_sync(FULL, m_r, 0);
-                for(int q = lo + lane; q <= hi; q += 32){
-                    C.hL[q] = m_h;
-                    for(int s = 0; s < MCA_NG; s++) C.qt[q * MCA_NG + s] = m_q[s];
-                    C.qr[q] = m_r;
-                    C.mod[q] = 1;
-                }
-                __syncwarp();
-                // one round: the segment's settles and the two growth tests' solves (cell lo-1
-                // lifted to level lo, the mixed cell hi lifted to level hi+1, cell hi+1's own),
-                // none of which depends on another; the decisions follow from the results
-                const bool below = lo > i0, above = hi < i1;
-                const bool sok = mca_round(A, C, lane, lo, hi - lo + 1, below ? lo - 1 : -1, lo,
-                                           above ? hi : -1, hi + 1, above ? hi + 1 : -1);
-                fail = !__all_sync(FULL, sok);
-                __syncwarp();
-                if(fail) break;
-                int gr = 0;
-                if(lane == 0 && below) gr = mca_slot_unstable(A, C, 0, lo - 1, lo) ? 1 : 0;
-                if(lane == 1 && above) gr = mca_slot_unstable(A, C, 1, hi, hi + 1) ? 2 : 0;
-                gr = __reduce_or_sync(FULL, (unsigned)gr);
-                __syncwarp();
-                if(gr & 1) lo--;
-                if(gr & 2) hi++;
-                if(!gr) break;
-            }
-            layers += hi - lo + 1;
-            changed = true;
-            i = hi;
+        double T = 0.0, c[MCA_NG] = {0.0, 0.0, 0.0, 0.0};
+        bool ok = false;
+        if(task){
+            double x[MCA_NG];
+#pragma unroll
+            for(int s = 0; s < MCA_NG; s++) x[s] = C.qt[ca * MCA_NG + s];
+            ok = mca_equil(A, C.hL[ca] + mca_trE(A, C.qr[ca]), x, (double)a.ps[o0 + (size_t)lb * pl], mca_z(A, lb), T, c);
         }
-    }
-    if(fail || layers == 0) return;                        // nothing written: the column keeps its state
-    for(int q = i0 + lane; q <= i1; q += 32){
-        if(!C.touched[q]) continue;
-        const size_t o = o0 + (size_t)q * pl;
-        t_st(a.t, a.tlo, o, C.T[q] / A.t_ref);
-        for(int s = 0; s < MCA_NG; s++){
-            const int x = q * MCA_NG + s;
-            const double ce = C.ceq[x];
-            const double qv = C.qt[x] - ce;
-            const bool liq = C.T[q] >= A.G[s].t_0;
-            a.sp[s][0][o] = (S)(qv * C.rho[q]);
-            a.sp[s][1][o] = (S)((liq ? ce : 0.0) * C.rho[q]);
-            a.sp[s][2][o] = (S)((liq ? 0.0 : ce) * C.rho[q]);
+        __syncwarp();
+        if(!active) continue;
+        // lane 0 tests the pair (lo - 1, lo) with lane 1's parcel and its own equilibrium, lane 2 the pair
+        // (hi, hi + 1) with its parcel and cell hi + 1's equilibrium of the start
+        double Tp = __shfl_sync(gm, T, 1, G), pc[MCA_NG];
+#pragma unroll
+        for(int s = 0; s < MCA_NG; s++) pc[s] = __shfl_sync(gm, c[s], 1, G);
+        bool okp = __shfl_sync(gm, (int)ok, 1, G) != 0;
+        bool grow = false;
+        if((gl == 0 && below) || (gl == 2 && above)){
+            double Tb = T, ec[MCA_NG], qa[MCA_NG], qb[MCA_NG];
+            int ia = lo - 1, ib = lo;
+            bool okb = ok;
+#pragma unroll
+            for(int s = 0; s < MCA_NG; s++) ec[s] = c[s];
+            if(gl == 2){
+                ia = hi; ib = hi + 1;
+                const size_t ob = o0 + (size_t)ib * pl;
+                Tp = T; okp = ok;
+                Tb = a.Teq[ob]; okb = Tb > 0.0;
+#pragma unroll
+                for(int s = 0; s < MCA_NG; s++){ pc[s] = c[s]; ec[s] = a.ceq[s][ob]; }
+            }
+#pragma unroll
+            for(int s = 0; s < MCA_NG; s++){ qa[s] = C.qt[ia * MCA_NG + s]; qb[s] = C.qt[ib * MCA_NG + s]; }
+            grow = okp && okb && mca_decide(A, Tp, pc, qa, C.qr[ia], Tb, ec, qb, C.qr[ib]);
         }
-        a.nh4sh[o] = (S)(C.qr[q] * C.rho[q]);
+        const unsigned gr = __ballot_sync(gm, grow) >> (grp * G);
+        if(gr & 1u) lo--;
+        if(gr & 4u) hi++;
+        if(!(gr & 5u)){ active = false; i = hi + 1; }
+        __syncwarp(gm);
     }
+}
+
+// Per mixed cell: its equilibrium at the final means and the write-back (:645-661, :800-849).
+template <typename S>
+__global__ void __launch_bounds__(128) mca_finish_kernel(const __grid_constant__ McaArgs<S> a){
+    const Grid& g = a.g;
+    const McaConst& A = a.c;
+    const int k = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, i = 1 + blockIdx.z;
+    if(k >= g.km) return;
+    const size_t o = gidx(g, i, j, k);
+    if(a.flag[o] != 2) return;
+    double qt[MCA_NG], ce[MCA_NG], T = 0.0;
+#pragma unroll
+    for(int s = 0; s < MCA_NG; s++) qt[s] = a.qt[s][o];
+    const double qr = a.qr[o];
+    if(!mca_equil(A, a.hL[o] + mca_trE(A, qr), qt, (double)a.ps[o], mca_z(A, i), T, ce)) return;
+    const double rho = mca_rho(A, A.local_rho ? (double)a.rho[o] : 0.0);
+    t_st(a.t, a.tlo, o, T / A.t_ref);
+#pragma unroll
+    for(int s = 0; s < MCA_NG; s++){
+        const double qv = qt[s] - ce[s];
+        const bool liq = T >= A.G[s].t_0;
+        a.sp[s][0][o] = (S)(qv * rho);
+        a.sp[s][1][o] = (S)((liq ? ce[s] : 0.0) * rho);
+        a.sp[s][2][o] = (S)((liq ? 0.0 : ce[s]) * rho);
+    }
+    a.nh4sh[o] = (S)(qr * rho);
 }
 
 // CpH2.h:66-75: the running integral of the cp table, in the table's order (one thread).
