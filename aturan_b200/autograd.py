@@ -37,16 +37,20 @@ class DryStepper:
         ctx = self.ctx
         xs = [x.detach().contiguous() for x in xs]
         torch.cuda.synchronize()
-        for n, t in self.saved.items():
-            ctx.upload_device(n, t.data_ptr())
-        for n, x in zip(DRY, xs):              # the state and its start-of-step copy
-            ctx.upload_device(n, x.data_ptr())
-            ctx.upload_device(n + "n", x.data_ptr())
+        # the state and its start-of-step copy
+        self._put([*self.saved.items(), *zip(DRY, xs), *((n + "n", x) for n, x in zip(DRY, xs))])
         ctx.rk4_step()
         self.n_forward += 1
-        out = [torch.empty(self.shape, dtype=torch.float64, device="cuda") for _ in DRY]
-        for n, o in zip(DRY, out):
-            ctx.download_device(n, o.data_ptr())
+        return self._take(DRY)
+
+    def _put(self, fields):
+        """(name, tensor) pairs into the context, in one call."""
+        self.ctx.upload_many([n for n, _ in fields], [t.data_ptr() for _, t in fields], on_device=True)
+
+    def _take(self, names):
+        """The context's fields as new tensors, in one call (waits for the step)."""
+        out = [torch.empty(self.shape, dtype=torch.float64, device="cuda") for _ in names]
+        self.ctx.download_many(list(names), [o.data_ptr() for o in out], on_device=True)
         return out
 
     def backward(self, ybar):
@@ -108,21 +112,13 @@ class DryFullStepper(DryStepper):
         torch.cuda.synchronize()
         ctx.set_heating(heat.data_ptr() if heat is not None else None)
         self.heated = heat is not None
-        for n, t in self.saved.items():
-            ctx.upload_device(n, t.data_ptr())
-        ctx.upload_device("p_dyn", self.zero.data_ptr())
-        for n, x in zip(DRY, xs):
-            ctx.upload_device(n, x.data_ptr())
-            ctx.upload_device(n + "n", x.data_ptr())
-        for n, a in zip(AUX, aux):
-            ctx.upload_device(n, a.data_ptr())
+        self._put([*self.saved.items(), ("p_dyn", self.zero), *zip(DRY, xs), *((n + "n", x) for n, x in zip(DRY, xs)),
+                   *zip(AUX, aux)])
         kind, omega, ms, tol = self.press
         ctx.pressure(kind, omega=omega, max_sweeps=ms, tol=tol)
         ctx.rk4_step()
         self.n_forward += 1
-        out = [torch.empty(self.shape, dtype=torch.float64, device="cuda") for _ in DRY + AUX]
-        for n, o in zip(DRY + AUX, out):
-            ctx.download_device(n, o.data_ptr())
+        out = self._take(DRY + AUX)
         return out[:4], out[4:]
 
     def backward(self, ybar, auxbar):
@@ -194,15 +190,7 @@ class MoistFullStepper(DryFullStepper):
         torch.cuda.synchronize()
         ctx.set_heating(heat.data_ptr() if heat is not None else None)
         self.heated = heat is not None
-        for n, t in self.saved.items():
-            ctx.upload_device(n, t.data_ptr())
-        for n, t in self.others.items():
-            ctx.upload_device(n, t.data_ptr())
-        ctx.upload_device("p_dyn", self.zero.data_ptr())
-        for n, x in zip(MOIST, xs):
-            ctx.upload_device(n, x.data_ptr())
-        for n, a in zip(AUX, aux):
-            ctx.upload_device(n, a.data_ptr())
+        self._put([*self.saved.items(), *self.others.items(), ("p_dyn", self.zero), *zip(MOIST, xs), *zip(AUX, aux)])
         ctx.restore_ncopies(1.0)               # every start-of-step copy is the step's input
         kind, omega, ms, tol = self.press
         ctx.pressure(kind, omega=omega, max_sweeps=ms, tol=tol)
@@ -210,9 +198,7 @@ class MoistFullStepper(DryFullStepper):
         ctx.sync_ncopies()                     # the adjusted scalars' copies (RK_SCALAR_SYNC)
         ctx.rk4_step()
         self.n_forward += 1
-        out = [torch.empty(self.shape, dtype=torch.float64, device="cuda") for _ in MOIST + AUX]
-        for n, o in zip(MOIST + AUX, out):
-            ctx.download_device(n, o.data_ptr())
+        out = self._take(MOIST + AUX)
         return out[:16], out[16:]
 
     def backward(self, ybar, auxbar):

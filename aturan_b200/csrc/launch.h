@@ -60,14 +60,19 @@ void launch_rb_colour(Grid g, double* P, const double* src, const RBW* w, int co
 
 // Layout conversions for the mixed-precision context (FP64 exchange <-> FP32 storage).
 void launch_f64_to_f32(const double* in, float* out, size_t n, cudaStream_t st);
-void launch_pack_in_f64(const double* in, double* out, int km, int kp, size_t rows, cudaStream_t st);
-void launch_pack_in_f32(const double* in, float* out, int km, int kp, size_t rows, cudaStream_t st);
-void launch_pack_out_f64(const double* in, double* out, int km, int kp, size_t rows, cudaStream_t st);
-void launch_pack_out_f32(const float* in, double* out, int km, int kp, size_t rows, cudaStream_t st);
+// Contiguous FP64 exchange buffers <-> padded fields, up to PACK_MAX of them in one launch.
+constexpr int PACK_MAX = 64;
+enum PackKind : unsigned char { PACK_F64, PACK_F32, PACK_PAIR };
+struct PackBatch {
+    const double* flat[PACK_MAX];     // [rows][km] FP64 (written when packing out)
+    void* dev[PACK_MAX];              // the padded field
+    float* lo[PACK_MAX];              // PACK_PAIR: the low parts of the temperature pair
+    PackKind kind[PACK_MAX];
+    unsigned n, div_m;                // values per field; e / km = e div_m >> div_s
+    int km, kp, div_s;
+};
+void launch_pack(PackBatch& p, int nf, int km, int kp, size_t rows, bool in, cudaStream_t st);
 void launch_f32_to_f64(const float* in, double* out, size_t n, cudaStream_t st);
-// The mixed form's temperature pair (common.cuh): FP64 exchange <-> (hi, lo) FP32 storage.
-void launch_pack_in_pair(const double* in, float* hi, float* lo, int km, int kp, size_t rows, cudaStream_t st);
-void launch_pack_out_pair(const float* hi, const float* lo, double* out, int km, int kp, size_t rows, cudaStream_t st);
 void launch_scale_copy_pair(const float* hi, const float* lo, float* ohi, float* olo, size_t n, double coeff, cudaStream_t st);
 
 }  // namespace aturan
