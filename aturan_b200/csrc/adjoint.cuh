@@ -10,10 +10,13 @@
 //   Xbar_s = J_s^T kbar_s (+ p_hydro part), ybar += Xbar_s, kbar_{s-1} = dt/6 w_{s-1} g + c_{s-1} Xbar_s,
 // then the hydrostatic integral's and the level means' adjoints add into ybar (T, v, w).
 //
-// J_s^T is a scatter of every interior cell's local partial derivatives onto its 7-point stencil.
-// It runs as gather, without atomics and in a fixed order: adj_local_kernel writes, per cell and
-// per field, the seven contributions the cell sends to its stencil points (ADJ_SLOTS arrays), and
-// adj_gather_kernel sums, per cell, the seven it receives from the cells whose stencils contain it.
+// J_s^T is a scatter of every interior cell's local partial derivatives onto its 7-point stencil. It
+// runs as gather, without atomics and in a fixed order: what a cell sends along one direction is a
+// product of its tendency adjoints and of values at the cell alone (its wind, viscosity and metric),
+// so adj_stage_kernel re-forms, for each cell, what its six neighbours send it; only the centre's own
+// part needs the stage input's differences. One launch per stage, no intermediate fields. Written out
+// as contributions per stencil point (38 fields dry, 122 moist, written by one launch and read by the
+// next) the same sums took 3.3x the memory traffic.
 // The partial derivatives are those of the forward's formulas (RHS_Uran_Turb.cpp:92-788), derived
 // term by term; cp(T) is the piecewise-linear table, differentiated within its interval (a kink
 // convention: the derivative of the interval the value falls in).
@@ -25,31 +28,29 @@
 namespace aturan {
 
 constexpr int ADJ_NF = 4;                          // t, u, v, w (state fields 0..3)
-constexpr int ADJ_SLOT_PH = 7 * ADJ_NF;            // p_hydro tp, tm, pe, pw
-constexpr int ADJ_SLOT_PD = ADJ_SLOT_PH + 4;       // p_dyn rp, rm, tp, tm, pe, pw
-constexpr int ADJ_SLOTS = ADJ_SLOT_PD + 6;         // per field rp, rm, tp, tm, pe, pw, c; then p_hydro, p_dyn
 // The moist form: the twelve condensable species (state fields 4..15, ATURAN_CH4 .. ATURAN_NH3_ICE)
-// join the dry four, their seven slots each after the dry layout.
+// join the dry four.
 constexpr int ADJ_NF_MOIST = 16;
-constexpr int ADJ_NSP = ADJ_NF_MOIST - ADJ_NF;
-constexpr int ADJ_SLOTS_MOIST = ADJ_SLOTS + 7 * ADJ_NSP;
-__host__ __device__ constexpr size_t adj_slot_base(int q){
-    return q < ADJ_NF ? (size_t)q * 7 : (size_t)ADJ_SLOTS + (size_t)(q - ADJ_NF) * 7;
-}
 
 struct AdjArgs {
     Grid g;
-    const double* X;            // stage input, field q (0..3) at X + q * fstride
+    const double* X;            // stage input, field q at X + q * fstride
     const double* X0;           // the step's input (boundary rows of every stage input)
-    const double* kbar;         // adjoint of the stage's tendencies, field q at kbar + q * fstride
+    const double* Xprev;        // the previous stage's input, or null at stage 0
+    const double* kbar;         // adjoint of the stage's tendencies, field q at kbar + q * fstride (0 off the interior)
+    const double* pe;           // ce_sp cp_mix / cp(T) kbar_t: the p_dyn gradients' factor (0 off the interior)
+    double* kbar_out;           // the previous stage's kbar and pe
+    double* pe_out;
     const double* auxbar;       // stage 3 only, else null: adjoint of aux_u, aux_v, aux_w (the tendencies
-                                // of u, v, w without the p_dyn gradient, RHS_Uran_Turb.cpp:1020-1022)
+                                // of u, v, w without the p_dyn gradient, RHS_Uran_Turb.cpp:1020-1022), 0 off the interior
     const double* pdyn;
-    const double* forc;         // forcing group (nue at offset 0)
+    const double* nt;           // the eddy viscosity as the tendencies use it (adj_nue)
     const GeoIJ<double>* geo;
     const double* cp_tab;
     RhsConst<double> k;
-    double* slot;               // ADJ_SLOTS fields
+    const double* g0;
+    double *ybar, *phbar, *pdbar;
+    double w_prev, c_prev;      // kbar_{s-1} = w_prev g0 + c_prev Xbar_s
     double* hacc;               // null, or the T tendencies' adjoint summed over the stages (heating)
 };
 
@@ -71,192 +72,217 @@ __device__ __forceinline__ void cp_lapse_d(const RhsConst<double>& k, const doub
     else        { *cp = k.cp_mix + k.cp_rh2 * (ch - k.cp_h2_const);               *dcp = k.cp_rh2 * dch; }
 }
 
-// Adjoints of one field's six differences -> the seven stencil values it was formed from.
-struct G6 { double d1r, d2r, d1t, d2t, d1p, d2p; };
-
-__device__ __forceinline__ void put7(double* slot, size_t fs, size_t o, int field, const G6& g, double dc,
-                                     const RhsConst<double>& k){
-    double* S = slot + (size_t)field * 7 * fs + o;
-    S[0 * fs] =  g.d1r * k.inv_2dr   + g.d2r * k.inv_dr2;      // to (i+1)
-    S[1 * fs] = -g.d1r * k.inv_2dr   + g.d2r * k.inv_dr2;      // to (i-1)
-    S[2 * fs] =  g.d1t * k.inv_2dthe + g.d2t * k.inv_dthe2;    // to (j+1)
-    S[3 * fs] = -g.d1t * k.inv_2dthe + g.d2t * k.inv_dthe2;    // to (j-1)
-    S[4 * fs] =  g.d1p * k.inv_2dphi + g.d2p * k.inv_dphi2;    // to (k+1)
-    S[5 * fs] = -g.d1p * k.inv_2dphi + g.d2p * k.inv_dphi2;    // to (k-1)
-    S[6 * fs] = dc - 2.0 * (g.d2r * k.inv_dr2 + g.d2t * k.inv_dthe2 + g.d2p * k.inv_dphi2);
+// cp(T) factor of the pressure work at T (nondimensional): cp_mix / cp(T), 1 without it.
+__device__ __forceinline__ double adj_cpf(const RhsConst<double>& K, const double* tab, double t){
+    if(!(K.cp_dyn && t > 0.0)) return 1.0;
+    double cp, dcp;
+    cp_lapse_d(K, tab, t * K.t_ref, &cp, &dcp);
+    return K.cp_mix / cp;
 }
+// The eddy viscosity the tendencies use, from the stored one.
+__device__ __forceinline__ double adj_nue(const RhsConst<double>& K, double nue_c){
+    return (K.turb_coupling != 0.0 && isfinite(nue_c)) ? K.turb_coupling * cmax(0.0, nue_c) : 0.0;
+}
+// The weights of one (i, j) row with which its cells send along r, theta and phi: of the transport (r1, t1,
+// p1, times the wind), of the first-order (t2; r2, for u twice) and second-order (t3, p3, inv_dr2) parts of
+// the diffusion, and of the metric cross terms (t4; p4, p5).
+struct AdjRow { double r2, t1, t2, t3, t4, p1, p3, p4, p5; };
 
-// Per interior cell: the local partial derivatives of rhs_t, rhs_u, rhs_v, rhs_w times the
-// tendencies' adjoints, as the contributions to each stencil point (RHS_Uran_Turb.cpp:92-788).
-__global__ void __launch_bounds__(128) adj_local_kernel(const AdjArgs a){
+// One reverse stage of the NF fields (RHS_Uran_Turb.cpp:92-850): per cell (every row, every distinct
+// meridian; the seam copy k = km-1 is read by no stencil and receives nothing) the sum of what the cells
+// whose stencils contain it send; added into ybar, phbar and pdbar; and the previous stage's kbar and pe on
+// the interior. A neighbour off the interior sends nothing: its weights are zero and the cell's own place is
+// read instead, so that every load is unconditional and issued before the first use (branches made each
+// neighbour's loads wait for the one before). A cell sends its tendency adjoint times
+//   transport: -wind * (r1, t1 or p1);  diffusion: D * (first- and second-order weights of its row),
+// the same weight for every field but its D (and u's own radial term), so a neighbour costs one weight per
+// D and one multiply-add per field. The rows' weights are formed once per block in shared memory.
+// Bound by the latency of its ~85 loads per cell at the registers they hold, then by their L2 traffic: it
+// reads the stage input, kbar, g0, nue, p_dyn and pe, and updates ybar, phbar and pdbar, ~33 words per cell
+// dry and ~105 moist. At 41x91x181: 103 us a stage dry and 254 moist at 4 and 3 resident blocks (128 and
+// 168 registers; 115 and 283 at one block more or less), against 108 and 374 as the two or three launches
+// that wrote and gathered the contributions.
+template <int NF>
+__global__ void __launch_bounds__(128, NF == ADJ_NF ? 4 : 3) adj_stage_kernel(const __grid_constant__ AdjArgs a){
     const Grid& g = a.g;
-    const int k = blockIdx.x * 32 + threadIdx.x;
-    const int j = 1 + blockIdx.y * 4 + threadIdx.y;
-    const int i = 1 + blockIdx.z;
-    if(k > g.km - 2 || j > g.jm - 2 || i > g.im - 2) return;
     const RhsConst<double>& K = a.k;
-    const GeoIJ<double> geo = a.geo[i * g.jm + j];
-    Nbr<double> nb;
-    nb.fs  = g.fstride;
-    nb.o   = gidx(g, i, j, k);
-    nb.oim = nb.o - (size_t)g.jm * g.kp; nb.oip = nb.o + (size_t)g.jm * g.kp;
-    nb.ojm = nb.o - g.kp;                nb.ojp = nb.o + g.kp;
-    nb.okw = nb.o - k + phi_wrap(k - 1, g.km);
-    nb.oke = nb.o - k + phi_wrap(k + 1, g.km);
-    nb.X   = a.X;
-    nb.xim = (i == 1) ? a.X0 : a.X;
-    nb.xip = (i == g.im - 2) ? a.X0 : a.X;
-    nb.xjm = (j == 1) ? a.X0 : a.X;
-    nb.xjp = (j == g.jm - 2) ? a.X0 : a.X;
-    const size_t o = nb.o, fs = g.fstride;
-
-    const D6<double> T = diff6(K, load7<double, double>(nb, 0));
-    const D6<double> U = diff6(K, load7<double, double>(nb, 1));
-    const D6<double> V = diff6(K, load7<double, double>(nb, 2));
-    const D6<double> W = diff6(K, load7<double, double>(nb, 3));
+    __shared__ AdjRow rows[14];          // of this block's four j: (i, j0 - 1 .. j0 + 4), then (i - 1, j), then (i + 1, j)
+    const int tj = threadIdx.y, j0 = blockIdx.y * 4, i = blockIdx.z;
+    {
+        const int r = tj * 32 + threadIdx.x;
+        if(r < 14){
+            const int ri = r < 6 ? i : (r < 10 ? i - 1 : i + 1), rj = r < 6 ? j0 - 1 + r : j0 + (r - 6) % 4;
+            const GeoIJ<double>& G = a.geo[min(max(ri, 0), g.im - 1) * g.jm + min(max(rj, 0), g.jm - 1)];
+            AdjRow w;
+            w.r2 = G.two_inv_rm * K.inv_2dr;
+            w.t1 = G.inv_rm * K.inv_2dthe; w.t2 = G.costhe_inv_rm2sinthe * K.inv_2dthe;
+            w.t3 = G.inv_rm2 * K.inv_dthe2; w.t4 = 2.0 * G.inv_rm2 * K.inv_2dthe;
+            w.p1 = G.inv_rmsinthe * K.inv_2dphi; w.p3 = G.inv_rm2sinthe2 * K.inv_dphi2;
+            w.p4 = 2.0 * G.inv_rm2sinthe * K.inv_2dphi; w.p5 = 2.0 * G.costhe * G.inv_rm2sinthe2 * K.inv_2dphi;
+            rows[r] = w;
+        }
+        __syncthreads();
+    }
+    const int k = blockIdx.x * 32 + threadIdx.x;
+    const int j = j0 + tj;
+    if(k > g.km - 2 || j > g.jm - 1) return;
+    // 32-bit offsets: a field has < 2^31 values and the tape's groups are reached field by field
+    const int fs = (int)g.fstride, si = g.jm * g.kp, sj = g.kp;
+    const int o = (int)gidx(g, i, j, k);
+    const bool ini = i >= 1 && i <= g.im - 2, inj = j >= 1 && j <= g.jm - 2;
+    const bool in = ini && inj;
+    const bool nb[6] = {inj && i >= 2, inj && i <= g.im - 3, ini && j >= 2, ini && j <= g.jm - 3, in, in};
+    const int on[6] = {nb[0] ? o - si : o, nb[1] ? o + si : o, nb[2] ? o - sj : o, nb[3] ? o + sj : o,
+                       o - k + phi_wrap(k - 1, g.km), o - k + phi_wrap(k + 1, g.km)};
+    // the stencil's own places (boundary rows from the step's input)
+    const int oc[4] = {in ? o - si : o, in ? o + si : o, in ? o - sj : o, in ? o + sj : o};
+    const double* const kb[ADJ_NF] = {a.kbar, a.kbar + (size_t)fs, a.kbar + 2 * (size_t)fs, a.kbar + 3 * (size_t)fs};
+    const double* const xsrc[4] = {i == 1 ? a.X0 : a.X, i == g.im - 2 ? a.X0 : a.X, j == 1 ? a.X0 : a.X, j == g.jm - 2 ? a.X0 : a.X};
+    double at[7], au[7], av[7], aw[7], a0[6], wn[6], pe[6], nt[7];
+#pragma unroll
+    for(int d = 0; d < 7; d++){
+        const int q = d < 6 ? on[d] : o;
+        at[d] = __ldg(kb[0] + q); au[d] = __ldg(kb[1] + q); av[d] = __ldg(kb[2] + q); aw[d] = __ldg(kb[3] + q);
+        nt[d] = __ldg(a.nt + q);
+        if(d < 6){
+            wn[d] = __ldg(a.X + (size_t)(1 + d / 2) * fs + q);
+            pe[d] = __ldg(a.pe + q);
+            a0[d] = d < 2 ? au[d] : (d < 4 ? av[d] : aw[d]);
+        }
+    }
+    auto stencil = [&](int q) -> R7<double> {
+        const size_t f = (size_t)q * fs;
+        R7<double> r;
+        r.c  = __ldg(a.X + f + o);
+        r.rm = __ldg(xsrc[0] + f + oc[0]); r.rp = __ldg(xsrc[1] + f + oc[1]);
+        r.tm = __ldg(xsrc[2] + f + oc[2]); r.tp = __ldg(xsrc[3] + f + oc[3]);
+        r.pw = __ldg(a.X + f + on[4]);     r.pe = __ldg(a.X + f + on[5]);
+        return r;
+    };
+    const R7<double> rT = stencil(0), rU = stencil(1), rV = stencil(2), rW = stencil(3);
     const double* P = a.pdyn;
-    const double dpdr   = (ld(P + nb.oip) - ld(P + nb.oim)) * K.inv_2dr;
-    const double dpdthe = (ld(P + nb.ojp) - ld(P + nb.ojm)) * K.inv_2dthe;
-    const double dpdphi = (ld(P + nb.oke) - ld(P + nb.okw)) * K.inv_2dphi;
-    const double nue_c = ld(a.forc + o);
-    const double nue_t = (K.turb_coupling != 0.0 && isfinite(nue_c)) ? K.turb_coupling * cmax(0.0, nue_c) : 0.0;
-    const double nue_t_s = nue_t / 0.9;
-    const double at = a.kbar[0 * fs + o];
-    if(a.hacc) a.hacc[o] += at;                 // rhs_t += heat_scale H(j,k) (aturan_set_heating)
-    const double au0 = a.kbar[1 * fs + o], av0 = a.kbar[2 * fs + o], aw0 = a.kbar[3 * fs + o];
-    // aux = the tendency without the p_dyn gradient: its adjoint joins the tendency's in every
-    // partial except those in p_dyn
-    const double au = au0 + (a.auxbar ? a.auxbar[0 * fs + o] : 0.0);
-    const double av = av0 + (a.auxbar ? a.auxbar[1 * fs + o] : 0.0);
-    const double aw = aw0 + (a.auxbar ? a.auxbar[2 * fs + o] : 0.0);
-
-    const double u = U.c, v = V.c, w = W.c;
-    const double inv_rm = geo.inv_rm, inv_rm2 = geo.inv_rm2, inv_rs = geo.inv_rmsinthe;
-    const double inv_rm2s = geo.inv_rm2sinthe, inv_rm2s2 = geo.inv_rm2sinthe2, cir = geo.costhe_inv_rm2sinthe;
-    const double costhe = geo.costhe, cot = geo.cotanthe, tir = geo.two_inv_rm;
-    const double D = 1.0 / K.re_eff + nue_t, Dt = 1.0 / K.re_pr + nue_t_s;
-
-    // pressure work and its cp(T) factor
-    double cpf = 1.0, dcpf = 0.0;
-    if(K.cp_dyn && T.c > 0.0){
-        double cp, dcp;
-        cp_lapse_d(K, a.cp_tab, T.c * K.t_ref, &cp, &dcp);
-        cpf = K.cp_mix / cp;
-        dcpf = -K.cp_mix / (cp * cp) * dcp * K.t_ref;
+    const double p_im = __ldg(P + oc[0]), p_ip = __ldg(P + oc[1]), p_jm = __ldg(P + oc[2]), p_jp = __ldg(P + oc[3]);
+    const double p_kw = __ldg(P + on[4]), p_ke = __ldg(P + on[5]);
+    if(a.auxbar){                                       // the aux adjoint joins every partial but those in p_dyn
+#pragma unroll
+        for(int d = 0; d < 7; d++){
+            const int q = d < 6 ? on[d] : o;
+            au[d] += __ldg(a.auxbar + q); av[d] += __ldg(a.auxbar + (size_t)fs + q); aw[d] += __ldg(a.auxbar + 2 * (size_t)fs + q);
+        }
     }
-    const double P0 = K.ce_sp * (u * dpdr + v * inv_rm * dpdthe + w * inv_rs * dpdphi);
-
-    // direct (centre) partials of the four tendencies
-    const double du = au * (-U.d1r + 2.0 * inv_rm2 * D - geo.sponge)
-                    + av * (-V.d1r - v * inv_rm)
-                    + aw * (-W.d1r - w * inv_rm - K.cor_sc * K.p2om * geo.sinthe_bf)
-                    + at * (K.ce_sp * dpdr * cpf - T.d1r);
-    const double dv = au * (-inv_rm * U.d1t)
-                    + av * (-inv_rm * V.d1t - u * inv_rm - geo.v_metric * D)
-                    + aw * (-inv_rm * W.d1t - w * cot * inv_rm - K.cor_sc * K.p2om * costhe)
-                    + at * (K.ce_sp * inv_rm * dpdthe * cpf - inv_rm * T.d1t);
-    const double dw = au * (-inv_rs * U.d1p - K.cor_rad_f * K.m2om * geo.sinthe_bf)
-                    + av * (-inv_rs * V.d1p + 2.0 * w * cot * inv_rm - K.cor_sc * K.m2om * costhe)
-                    + aw * (-inv_rs * W.d1p - (u + v * cot) * inv_rm - geo.v_metric * D)
-                    + at * (K.ce_sp * inv_rs * dpdphi * cpf - inv_rs * T.d1p);
-    const double dT = at * P0 * dcpf;
-
-    G6 gT, gU, gV, gW;
-    gT.d1r = at * (-u + tir * Dt);            gT.d2r = at * Dt;
-    gT.d1t = at * (-v * inv_rm + cir * Dt);   gT.d2t = at * inv_rm2 * Dt;
-    gT.d1p = at * (-w * inv_rs);              gT.d2p = at * inv_rm2s2 * Dt;
-
-    gU.d1r = au * (-u + 4.0 * inv_rm * D);    gU.d2r = au * D;
-    gU.d1t = au * (-v * inv_rm + cir * D) + av * (2.0 * inv_rm2 * D);
-    gU.d2t = au * inv_rm2 * D;
-    gU.d1p = au * (-w * inv_rs) + aw * (2.0 * inv_rm2s * D);
-    gU.d2p = au * inv_rm2s2 * D;
-
-    gV.d1r = av * (-u + tir * D);             gV.d2r = av * D;
-    gV.d1t = av * (-v * inv_rm + cir * D);    gV.d2t = av * inv_rm2 * D;
-    gV.d1p = av * (-w * inv_rs) + aw * (2.0 * costhe * inv_rm2s2 * D);
-    gV.d2p = av * inv_rm2s2 * D;
-
-    gW.d1r = aw * (-u + tir * D);             gW.d2r = aw * D;
-    gW.d1t = aw * (-v * inv_rm + cir * D);    gW.d2t = aw * inv_rm2 * D;
-    gW.d1p = aw * (-w * inv_rs) - av * (2.0 * costhe * inv_rm2s2 * D);
-    gW.d2p = aw * inv_rm2s2 * D;
-
-    put7(a.slot, fs, o, 0, gT, dT, K);
-    put7(a.slot, fs, o, 1, gU, du, K);
-    put7(a.slot, fs, o, 2, gV, dv, K);
-    put7(a.slot, fs, o, 3, gW, dw, K);
-    // p_hydro: rhs_v -= (ph[j+1] - ph[j-1]) inv_2dthe inv_rm, rhs_w -= (ph[k+1] - ph[k-1]) inv_2dphi inv_rs
-    double* S = a.slot + (size_t)ADJ_SLOT_PH * fs + o;
-    S[0 * fs] = -av * K.inv_2dthe * inv_rm;   // to (j+1)
-    S[1 * fs] =  av * K.inv_2dthe * inv_rm;   // to (j-1)
-    S[2 * fs] = -aw * K.inv_2dphi * inv_rs;   // to (k+1)
-    S[3 * fs] =  aw * K.inv_2dphi * inv_rs;   // to (k-1)
-    // p_dyn: rhs_u -= dpdr scale_p, rhs_v -= dpdthe scale_p inv_rm, rhs_w -= dpdphi scale_p inv_rs,
-    // rhs_t += ce_sp (u dpdr + v inv_rm dpdthe + w inv_rs dpdphi) cpf (aux carries none of it)
-    const double gdr = -K.scale_p * au0 + K.ce_sp * u * cpf * at;
-    const double gdt = -K.scale_p * inv_rm * av0 + K.ce_sp * v * inv_rm * cpf * at;
-    const double gdp = -K.scale_p * inv_rs * aw0 + K.ce_sp * w * inv_rs * cpf * at;
-    double* Q = a.slot + (size_t)ADJ_SLOT_PD * fs + o;
-    Q[0 * fs] =  gdr * K.inv_2dr;             // to (i+1)
-    Q[1 * fs] = -gdr * K.inv_2dr;             // to (i-1)
-    Q[2 * fs] =  gdt * K.inv_2dthe;           // to (j+1)
-    Q[3 * fs] = -gdt * K.inv_2dthe;           // to (j-1)
-    Q[4 * fs] =  gdp * K.inv_2dphi;           // to (k+1)
-    Q[5 * fs] = -gdp * K.inv_2dphi;           // to (k-1)
-}
-
-// The twelve condensable species' tendencies (RHS_Uran_Turb.cpp:790-850, scalar_rhs in rk4.cuh):
-// rhs_q = -(u d1r + v/r d1t + w/(r sin) d1p)(q) + D_q lap(q) + forcing, D_q = 1/(Sc_g Re) + nue_t/0.9,
-// the forcing (precipitation sources, mass fluxes) held fixed. Per interior cell and species: the
-// seven stencil contributions into the species' slots, and the transport's partials in u, v, w
-// added to the centre slots of u, v, w that adj_local_kernel wrote (same cell, same thread, the
-// next launch on the stream). a.X, a.X0, a.kbar hold ADJ_NF_MOIST fields.
-__global__ void __launch_bounds__(128) adj_species_local_kernel(const AdjArgs a){
-    const Grid& g = a.g;
-    const int k = blockIdx.x * 32 + threadIdx.x;
-    const int j = 1 + blockIdx.y * 4 + threadIdx.y;
-    const int i = 1 + blockIdx.z;
-    if(k > g.km - 2 || j > g.jm - 2 || i > g.im - 2) return;
-    const RhsConst<double>& K = a.k;
-    const GeoIJ<double> geo = a.geo[i * g.jm + j];
-    Nbr<double> nb;
-    nb.fs  = g.fstride;
-    nb.o   = gidx(g, i, j, k);
-    nb.oim = nb.o - (size_t)g.jm * g.kp; nb.oip = nb.o + (size_t)g.jm * g.kp;
-    nb.ojm = nb.o - g.kp;                nb.ojp = nb.o + g.kp;
-    nb.okw = nb.o - k + phi_wrap(k - 1, g.km);
-    nb.oke = nb.o - k + phi_wrap(k + 1, g.km);
-    nb.X   = a.X;
-    nb.xim = (i == 1) ? a.X0 : a.X;
-    nb.xip = (i == g.im - 2) ? a.X0 : a.X;
-    nb.xjm = (j == 1) ? a.X0 : a.X;
-    nb.xjp = (j == g.jm - 2) ? a.X0 : a.X;
-    const size_t o = nb.o, fs = g.fstride;
-    const double u = a.X[1 * fs + o], v = a.X[2 * fs + o], w = a.X[3 * fs + o];
-    const double nue_c = ld(a.forc + o);
-    const double nue_t = (K.turb_coupling != 0.0 && isfinite(nue_c)) ? K.turb_coupling * cmax(0.0, nue_c) : 0.0;
-    const double nue_t_s = nue_t / 0.9;
-    const double inv_rm = geo.inv_rm, inv_rm2 = geo.inv_rm2, inv_rs = geo.inv_rmsinthe;
-    const double inv_rm2s2 = geo.inv_rm2sinthe2, cir = geo.costhe_inv_rm2sinthe, tir = geo.two_inv_rm;
-    double du = 0.0, dv = 0.0, dw = 0.0;
-    for(int n = 0; n < ADJ_NSP; n++){
-        const int q = ADJ_NF + n;
-        const D6<double> Q = diff6(K, load7<double, double>(nb, q));
-        const double aq = a.kbar[(size_t)q * fs + o];
-        const double Dq = K.inv_sc_re[n / 3] + nue_t_s;
-        G6 gq;
-        gq.d1r = aq * (-u + tir * Dq);           gq.d2r = aq * Dq;
-        gq.d1t = aq * (-v * inv_rm + cir * Dq);  gq.d2t = aq * inv_rm2 * Dq;
-        gq.d1p = aq * (-w * inv_rs);             gq.d2p = aq * inv_rm2s2 * Dq;
-        put7(a.slot + (size_t)ADJ_SLOTS * fs, fs, o, n, gq, 0.0, K);
-        du -= aq * Q.d1r;
-        dv -= aq * inv_rm * Q.d1t;
-        dw -= aq * inv_rs * Q.d1p;
+    const double ire = K.inv_re_eff, irp = K.inv_re_pr, i09 = 1.0 / 0.9;
+    double xt = 0.0, xu = 0.0, xv = 0.0, xw = 0.0, h = 0.0, pd = 0.0;
+    double lap = 0.0, inv_rm = 0.0, inv_rs = 0.0;
+    if(in){                                             // the centre's own part
+        const GeoIJ<double>& geo = a.geo[i * g.jm + j];
+        const AdjRow& R = rows[1 + tj];
+        const D6<double> T = diff6(K, rT), U = diff6(K, rU), V = diff6(K, rV), W = diff6(K, rW);
+        const double u = U.c, v = V.c, w = W.c, t0 = T.c;
+        inv_rm = geo.inv_rm; inv_rs = geo.inv_rmsinthe;
+        const double dpdr = (p_ip - p_im) * K.inv_2dr, dpdthe = (p_jp - p_jm) * K.inv_2dthe * inv_rm, dpdphi = (p_ke - p_kw) * K.inv_2dphi * inv_rs;
+        const double costhe = geo.costhe, cot = geo.cotanthe, c_t = at[6], c_u = au[6], c_v = av[6], c_w = aw[6];
+        const double D = ire + nt[6], Dt = irp + nt[6] * i09, vm = geo.v_metric * D;
+        if(a.hacc) a.hacc[o] += c_t;                    // rhs_t += heat_scale H(j,k) (aturan_set_heating)
+        // pressure work and its cp(T) factor
+        double cpf = 1.0, dcpf = 0.0;
+        if(K.cp_dyn && t0 > 0.0){
+            double cp, dcp;
+            cp_lapse_d(K, a.cp_tab, t0 * K.t_ref, &cp, &dcp);
+            cpf = K.cp_mix / cp;
+            dcpf = -cpf / cp * dcp * K.t_ref;
+        }
+        const double P0 = K.ce_sp * (u * dpdr + v * dpdthe + w * dpdphi), cec = K.ce_sp * cpf;
+        const double ut = inv_rm * U.d1t, vt = inv_rm * V.d1t, wt = inv_rm * W.d1t, tt = inv_rm * T.d1t;
+        const double up = inv_rs * U.d1p, vp = inv_rs * V.d1p, wp = inv_rs * W.d1p, tp = inv_rs * T.d1p;
+        lap = 2.0 * (K.inv_dr2 + R.t3 + R.p3);
+        xu = c_u * (-U.d1r + D * (2.0 * geo.inv_rm2 - lap) - geo.sponge)
+           + c_v * (-V.d1r - v * inv_rm)
+           + c_w * (-W.d1r - w * inv_rm - K.cor_sc * K.p2om * geo.sinthe_bf)
+           + c_t * (cec * dpdr - T.d1r);
+        xv = c_u * -ut
+           + c_v * (-vt - u * inv_rm - vm - D * lap)
+           + c_w * (-wt - w * cot * inv_rm - K.cor_sc * K.p2om * costhe)
+           + c_t * (cec * dpdthe - tt);
+        xw = c_u * (-up - K.cor_rad_f * K.m2om * geo.sinthe_bf)
+           + c_v * (-vp + 2.0 * w * cot * inv_rm - K.cor_sc * K.m2om * costhe)
+           + c_w * (-wp - (u + v * cot) * inv_rm - vm - D * lap)
+           + c_t * (cec * dpdphi - tp);
+        xt = c_t * (P0 * dcpf - Dt * lap);
     }
-    a.slot[(1 * 7 + 6) * fs + o] += du;
-    a.slot[(2 * 7 + 6) * fs + o] += dv;
-    a.slot[(3 * 7 + 6) * fs + o] += dw;
+    double cw[6], cd[6];                                // transport and diffusion weights of the neighbours
+#pragma unroll
+    for(int d = 0; d < 6; d++){
+        const AdjRow& R = rows[d == 0 ? 6 + tj : (d == 1 ? 10 + tj : (d == 2 ? tj : (d == 3 ? 2 + tj : 1 + tj)))];
+        const double sg = (d & 1) ? -1.0 : 1.0;         // the first differences' sign: + from the lower neighbour
+        const double m = nb[d] ? 1.0 : 0.0;
+        const double D = ire + nt[d], Dt = irp + nt[d] * i09;
+        const double c = m * sg * (d < 2 ? K.inv_2dr : (d < 4 ? R.t1 : R.p1));
+        cw[d] = -wn[d] * c;
+        cd[d] = d < 2 ? m * (sg * R.r2 + K.inv_dr2) : (d < 4 ? m * (sg * R.t2 + R.t3) : m * R.p3);
+        const double WT = cw[d] + Dt * cd[d], WD = cw[d] + D * cd[d];
+        xt += at[d] * WT; xv += av[d] * WD; xw += aw[d] * WD;
+        if(d < 2) xu += au[d] * (WD + D * (m * sg * R.r2));
+        else {
+            xu += au[d] * WD;
+            if(d < 4){ xu += av[d] * (m * sg * R.t4 * D); h -= av[d] * c; }
+            else {
+                const double c5 = m * sg * R.p5 * D;
+                xu += aw[d] * (m * sg * R.p4 * D); xv += aw[d] * c5; xw -= av[d] * c5;
+                h -= aw[d] * c;
+            }
+        }
+        pd += (wn[d] * pe[d] - K.scale_p * a0[d]) * c;
+    }
+    if(NF == ADJ_NF_MOIST){
+        // The twelve condensable species (:790-850, scalar_rhs in rk4.cuh): rhs_q = -(u d1r + v/r d1t +
+        // w/(r sin) d1p)(q) + D_q lap(q) + forcing, D_q = 1/(Sc_g Re) + nue_t/0.9, the forcing held fixed.
+        double bw[6];
+#pragma unroll
+        for(int d = 0; d < 6; d++) bw[d] = cw[d] + (nt[d] * i09) * cd[d];
+        const double b0 = -(nt[6] * i09) * lap;
+#pragma unroll 1
+        for(int gi = 0; gi < (NF - ADJ_NF) / 3; gi++){
+            const double isc = K.inv_sc_re[gi];
+            double W[6];
+#pragma unroll
+            for(int d = 0; d < 6; d++) W[d] = bw[d] + isc * cd[d];
+            const double W0 = b0 - isc * lap;
+#pragma unroll
+            for(int n = 0; n < 3; n++){
+                const size_t f = (size_t)(ADJ_NF + 3 * gi + n) * fs;
+                const double* kq = a.kbar + f;
+                double an[6];
+#pragma unroll
+                for(int d = 0; d < 6; d++) an[d] = __ldg(kq + on[d]);
+                const R7<double> rq = stencil(ADJ_NF + 3 * gi + n);
+                const double aq = __ldg(kq + o), yb = a.ybar[f + o], g0 = __ldg(a.g0 + f + o);
+                double x = aq * W0;
+                // inv_rm and inv_rs are 0 off the interior, where aq is 0 too
+                xu -= aq * ((rq.rp - rq.rm) * K.inv_2dr);
+                xv -= aq * inv_rm * ((rq.tp - rq.tm) * K.inv_2dthe);
+                xw -= aq * inv_rs * ((rq.pe - rq.pw) * K.inv_2dphi);
+#pragma unroll
+                for(int d = 0; d < 6; d++) x += an[d] * W[d];
+                a.ybar[f + o] = yb + x;
+                if(in && a.Xprev) a.kbar_out[f + o] = a.w_prev * g0 + a.c_prev * x;
+            }
+        }
+    }
+    const double x[ADJ_NF] = {xt, xu, xv, xw};
+#pragma unroll
+    for(int q = 0; q < ADJ_NF; q++) a.ybar[(size_t)q * fs + o] += x[q];
+    a.phbar[o] += h;
+    a.pdbar[o] += pd;
+    if(in && a.Xprev){
+        double kt = 0.0;
+#pragma unroll
+        for(int q = 0; q < ADJ_NF; q++){
+            const double kn = a.w_prev * a.g0[(size_t)q * fs + o] + a.c_prev * x[q];
+            if(q == 0) kt = kn;
+            a.kbar_out[(size_t)q * fs + o] = kn;
+        }
+        a.pe_out[o] = K.ce_sp * adj_cpf(K, a.cp_tab, ld(a.Xprev + o)) * kt;
+    }
 }
 
 // ---- the saturation adjustment's implicit adjoint ----
@@ -444,54 +470,12 @@ __global__ void __launch_bounds__(128) adj_satadj_kernel(Grid g, const double* p
     ybar[q] = Tb * t_ref;
 }
 
-// Per cell (every row, every meridian; the seam copy k = km-1 is read by no stencil and receives
-// nothing): the sum of what the cells whose stencils contain it sent, in a fixed order. Adds the
-// result into ybar and phbar; for s > 0 also forms the previous stage's kbar on the interior.
-__global__ void __launch_bounds__(128) adj_gather_kernel(Grid g, const double* slot, double* ybar, double* phbar,
-                                                         double* pdbar, const double* g0, double* kbar, double w_prev,
-                                                         double c_prev, int has_prev, int nf){
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y;
-    const int i = blockIdx.z;
-    if(k >= g.km - 1) return;
-    const size_t fs = g.fstride, si = (size_t)g.jm * g.kp, sj = g.kp;
-    const size_t o = gidx(g, i, j, k);
-    const size_t okw = o - k + phi_wrap(k - 1, g.km), oke = o - k + phi_wrap(k + 1, g.km);
-    const bool interior = i >= 1 && i <= g.im - 2 && j >= 1 && j <= g.jm - 2;
-    for(int q = 0; q < nf; q++){
-        const double* S = slot + adj_slot_base(q) * fs;
-        double x = S[6 * fs + o];
-        if(i >= 1)        x += S[0 * fs + o - si];
-        if(i <= g.im - 2) x += S[1 * fs + o + si];
-        if(j >= 1)        x += S[2 * fs + o - sj];
-        if(j <= g.jm - 2) x += S[3 * fs + o + sj];
-        x += S[4 * fs + okw];
-        x += S[5 * fs + oke];
-        ybar[q * fs + o] += x;
-        if(has_prev && interior) kbar[q * fs + o] = w_prev * g0[q * fs + o] + c_prev * x;
-    }
-    const double* S = slot + (size_t)ADJ_SLOT_PH * fs;
-    double h = 0.0;
-    if(j >= 1)        h += S[0 * fs + o - sj];
-    if(j <= g.jm - 2) h += S[1 * fs + o + sj];
-    h += S[2 * fs + okw];
-    h += S[3 * fs + oke];
-    phbar[o] += h;
-    const double* Q = slot + (size_t)ADJ_SLOT_PD * fs;
-    double pd = 0.0;
-    if(i >= 1)        pd += Q[0 * fs + o - si];
-    if(i <= g.im - 2) pd += Q[1 * fs + o + si];
-    if(j >= 1)        pd += Q[2 * fs + o - sj];
-    if(j <= g.jm - 2) pd += Q[3 * fs + o + sj];
-    pd += Q[4 * fs + okw];
-    pd += Q[5 * fs + oke];
-    pdbar[o] += pd;
-}
-
 // The final update's adjoint: g = ybar' (times 0 where T' was clamped), ybar = g, kbar_3 =
-// dt/6 w_3 g on the interior. ybar_in is the caller's adjoint of the step's output.
+// dt/6 w_3 g on the interior. ybar_in is the caller's adjoint of the step's output; pe of stage 3 is
+// formed from its input t3, nt from nue.
 __global__ void adj_init_kernel(Grid g, const double* ybar_in, const double* t_out, double t_min, double t_max,
-                                double w3, double* g0, double* ybar, double* kbar, double* phbar, double* pdbar, int nf){
+                                double w3, double* g0, double* ybar, double* kbar, double* phbar, double* pdbar, int nf,
+                                RhsConst<double> K, const double* cp_tab, const double* t3, const double* nue, double* pe, double* nt){
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y;
     const int i = blockIdx.z;
@@ -499,15 +483,18 @@ __global__ void adj_init_kernel(Grid g, const double* ybar_in, const double* t_o
     const size_t fs = g.fstride;
     const size_t o = gidx(g, i, j, k);
     const bool interior = i >= 1 && i <= g.im - 2 && j >= 1 && j <= g.jm - 2 && k <= g.km - 2;
+#pragma unroll 4
     for(int q = 0; q < nf; q++){
         double v = ybar_in[q * fs + o];
         if(q == 0 && interior && !(t_out[o] > t_min && t_out[o] < t_max)) v = 0.0;
         g0[q * fs + o] = interior ? v : 0.0;
         ybar[q * fs + o] = v;
         kbar[q * fs + o] = interior ? w3 * v : 0.0;
+        if(q == 0) pe[o] = interior ? K.ce_sp * adj_cpf(K, cp_tab, t3[o]) * (w3 * v) : 0.0;
     }
     phbar[o] = 0.0;
     pdbar[o] = 0.0;
+    nt[o] = adj_nue(K, nue[o]);
 }
 
 // Hydrostatic integral's adjoint, per column (RungeKutta_Uran_Turb.cpp:62-177): p_hydro(i) =
@@ -515,49 +502,69 @@ __global__ void adj_init_kernel(Grid g, const double* ybar_in, const double* t_o
 // follow filter advances, else 1). Fbar(m) = dr/2 (S(m+1) + [m >= 1] S(m)), S the suffix sums of
 // phbar. Adds the met part into vbar, wbar and the local buoy part into Tbar; leaves, per cell,
 // the contribution to its level mean's adjoint in rbar.
+//
+// A block owns 32 consecutive columns. All its threads bring a chunk of phbar (top down) into shared
+// memory, one warp turns it into suffix sums in order (only those adds are serial), all threads do the
+// per-cell work. One thread per column walking the levels, the divisions in its chain, left 65 blocks
+// for the chip at 41x91x181 and took 151 us.
+constexpr int ADJ_HCH = 48;                        // levels per chunk
 __global__ void __launch_bounds__(256) adj_hydro_kernel(Grid g, const double* t, const double* ps, const double* v,
                                                         const double* w, const double* ref, const double* rm_i,
                                                         const double* cor_j, const double* phbar, double* ybar,
                                                         double* rbar, HydroConst h){
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if(c >= g.jm * g.km) return;
-    const int j = c / g.km, k = c - j * g.km;
+    __shared__ double sS[ADJ_HCH + 1][32];         // S(m) of the chunk's levels; the last row S of the level above it
+    const int tx = threadIdx.x, ty = threadIdx.y;
+    const int c = blockIdx.x * 32 + tx;
+    const bool col = c < g.jm * g.km;
+    const int j = col ? c / g.km : 0, k = col ? c - j * g.km : 0;
     const size_t fs = g.fstride;
     const double cB = h.follow_on ? 1.0 - 1.0 / h.follow_tau : 1.0;
     const double cor = cor_j[j];
-    double S_next = 0.0;                           // S(m+1)
-    for(int m = g.im - 1; m >= 0; m--){
-        const size_t o = gidx(g, m, j, k);
-        const double Sm = S_next + phbar[o];
-        const double Fb = 0.5 * h.dr * (S_next + (m >= 1 ? Sm : 0.0));
-        S_next = Sm;
-        const double vv = v[o], ww = w[o];
-        ybar[2 * fs + o] += Fb * 2.0 * vv / rm_i[m];
-        ybar[3 * fs + o] += Fb * (2.0 * ww / rm_i[m] + cor);
-        const double T = t[o];
-        double rb = 0.0;
-        if(T > 0.0){
-            const double b = h.g * ps[o] / (h.rR * T * h.t_ref);
-            const double f = h.m_nd_rel_b * (b - ref[m]) / ref[m];
-            if(isfinite(f)){
-                const double FbB = cB * Fb;
-                ybar[o] += FbB * h.m_nd_rel_b / ref[m] * (-b / T);
-                rb = FbB * (-h.m_nd_rel_b * b / (ref[m] * ref[m]));
-            }
+    double S = 0.0;                                // the serial lane's running suffix sum
+    for(int m1 = g.im; m1 > 0; m1 -= ADJ_HCH){     // levels m0 .. m1 - 1
+        const int m0 = max(0, m1 - ADJ_HCH), n = m1 - m0;
+        for(int r = ty; r < n; r += 8) sS[r][tx] = col ? phbar[gidx(g, m0 + r, j, k)] : 0.0;
+        __syncthreads();
+        if(ty == 0){
+            sS[n][tx] = S;
+            for(int r = n - 1; r >= 0; r--){ S += sS[r][tx]; sS[r][tx] = S; }
         }
-        rbar[o] = rb;
+        __syncthreads();
+        if(col)
+            for(int r = ty; r < n; r += 8){
+                const int m = m0 + r;
+                const size_t o = gidx(g, m, j, k);
+                const double Fb = 0.5 * h.dr * (sS[r + 1][tx] + (m >= 1 ? sS[r][tx] : 0.0));
+                const double vv = v[o], ww = w[o], T = t[o], p = ps[o];
+                const double yv = ybar[2 * fs + o], yw = ybar[3 * fs + o], yt = ybar[o];
+                ybar[2 * fs + o] = yv + Fb * 2.0 * vv / rm_i[m];
+                ybar[3 * fs + o] = yw + Fb * (2.0 * ww / rm_i[m] + cor);
+                double rb = 0.0;
+                if(T > 0.0){
+                    const double b = h.g * p / (h.rR * T * h.t_ref);
+                    const double f = h.m_nd_rel_b * (b - ref[m]) / ref[m];
+                    if(isfinite(f)){
+                        const double FbB = cB * Fb;
+                        ybar[o] = yt + FbB * h.m_nd_rel_b / ref[m] * (-b / T);
+                        rb = FbB * (-h.m_nd_rel_b * b / (ref[m] * ref[m]));
+                    }
+                }
+                rbar[o] = rb;
+            }
+        __syncthreads();
     }
 }
 
-// Level mean's adjoint (RungeKutta_Uran_Turb.cpp:18-37): per level, Rbar = sum rbar and the
-// weight sum W over the valid cells, in a fixed tree order; then per valid cell
-// Tbar += Rbar / W * wsin_j * db/dT, db/dT = -b / T.
+// Level mean's adjoint (RungeKutta_Uran_Turb.cpp:18-37): per level, Rbar = sum rbar and the weight sum W
+// over the valid cells, in a fixed tree order (ADJ_LB blocks per level, their partials added in block
+// order by the apply kernel); then per valid cell Tbar += Rbar / W * wsin_j * db/dT, db/dT = -b / T.
+constexpr int ADJ_LB = 16;
 __global__ void __launch_bounds__(256) adj_level_sum_kernel(Grid g, const double* t, const double* ps,
                                                             const double* wsin, const double* rbar,
                                                             HydroConst h, double* lev){
-    const int m = blockIdx.x;
+    const int m = blockIdx.y;
     double s = 0.0, ws = 0.0;
-    for(int c = threadIdx.x; c < g.jm * g.km; c += blockDim.x){
+    for(int c = blockIdx.x * 256 + threadIdx.x; c < g.jm * g.km; c += ADJ_LB * 256){
         const int j = c / g.km, k = c - j * g.km;
         const size_t o = gidx(g, m, j, k);
         const double T = t[o];
@@ -574,21 +581,24 @@ __global__ void __launch_bounds__(256) adj_level_sum_kernel(Grid g, const double
         if(threadIdx.x < st){ ss[threadIdx.x] += ss[threadIdx.x + st]; sw[threadIdx.x] += sw[threadIdx.x + st]; }
         __syncthreads();
     }
-    if(threadIdx.x == 0){ lev[2 * m] = ss[0]; lev[2 * m + 1] = sw[0]; }
+    if(threadIdx.x == 0){ double* q = lev + 2 * ((size_t)m * ADJ_LB + blockIdx.x); q[0] = ss[0]; q[1] = sw[0]; }
 }
 
-__global__ void adj_level_apply_kernel(Grid g, const double* t, const double* ps, const double* wsin,
-                                       const double* lev, HydroConst h, double* ybar){
+__global__ void __launch_bounds__(128) adj_level_apply_kernel(Grid g, const double* t, const double* ps, const double* wsin,
+                                                              const double* lev, HydroConst h, double* ybar){
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y;
     const int m = blockIdx.z;
+    double R = 0.0, W = 0.0;
+#pragma unroll
+    for(int b = 0; b < ADJ_LB; b++){ R += __ldg(lev + 2 * (m * ADJ_LB + b)); W += __ldg(lev + 2 * (m * ADJ_LB + b) + 1); }
     if(k >= g.km) return;
     const size_t o = gidx(g, m, j, k);
     const double T = t[o];
-    if(!(T > 0.0) || !(lev[2 * m + 1] > 0.0)) return;
+    if(!(T > 0.0) || !(W > 0.0)) return;
     const double b = h.g * ps[o] / (h.rR * T * h.t_ref);
     if(!isfinite(b)) return;
-    ybar[o] += lev[2 * m] / lev[2 * m + 1] * wsin[j] * (-b / T);
+    ybar[o] += R / W * wsin[j] * (-b / T);
 }
 
 // The heating field's adjoint: heat_scale times the T tendencies' adjoint summed over the stages and

@@ -86,7 +86,7 @@ struct aturan_ctx {
     // and the adjoint's work arrays; null when the tape is off
     double* tape;
     bool tape_valid;           // a taped RK4 step has run since the tape was switched on
-    double *tX, *tTout, *tPd, *tSrc, *tref, *aslot, *aybar, *akbar, *ag0, *aphbar, *arbar, *apdbar, *aaux, *alev;
+    double *tX, *tTout, *tPd, *tSrc, *tref, *aybar, *akbar, *akbar2, *ape, *ag0, *aphbar, *arbar, *apdbar, *aaux, *alev;
     bool tape_p_valid;         // a taped RB_SOR / RB_LINE pressure call has run since the tape was switched on
     double* ahacc;             // the T tendencies' adjoint summed over the stages (heating gradient)
     int tape_nf;               // fields taped per stage: ADJ_NF (dry) or ADJ_NF_MOIST (aturan_tape(ctx, 2))
@@ -1610,15 +1610,14 @@ int aturan_tape(aturan_ctx* ctx, int on){
     const Grid& g = ctx->g;
     const size_t fs = g.fstride;
     const int NT = want;
-    const size_t nslot = NT == ADJ_NF ? ADJ_SLOTS : ADJ_SLOTS_MOIST;
-    // stage inputs 4 x NT, T output, p_dyn, pressure source, slots, ybar NT, kbar NT, g0 NT, phbar,
-    // rbar, pdbar, aux adjoint 3, heating accumulator, the moist tape's adjustment input NT; level
-    // means + sums
-    const size_t nf = 4 * NT + 3 + nslot + 3 * NT + 3 + 3 + 1 + (NT == ADJ_NF ? 0 : NT);
-    const size_t bytes = (nf * fs + 3 * (size_t)g.im) * sizeof(double);
+    // stage inputs 4 x NT, T output, p_dyn, pressure source, ybar NT, two kbar NT and pe (a stage reads one
+    // and writes the other), the eddy viscosity, g0 NT, phbar, rbar, pdbar, aux adjoint 3, heating accumulator, the moist tape's
+    // adjustment input NT; level means + sums
+    const size_t nf = 4 * NT + 3 + 3 * NT + 3 + NT + 3 + 3 + 1 + (NT == ADJ_NF ? 0 : NT);
+    const size_t bytes = (nf * fs + (1 + 2 * ADJ_LB) * (size_t)g.im) * sizeof(double);
     void* mem = nullptr;
     if(cudaMalloc(&mem, bytes) != cudaSuccess){ cudaGetLastError(); return fail(ctx, ATURAN_E_NOMEM, "tape allocation"); }
-    CK(cudaMemsetAsync(mem, 0, bytes, ctx->st));      // slots stay zero outside the interior
+    CK(cudaMemsetAsync(mem, 0, bytes, ctx->st));      // kbar, pe and the aux adjoint stay zero off the interior
     double* cur = reinterpret_cast<double*>(mem);
     auto take = [&](size_t n){ double* r = cur; cur += n; return r; };
     ctx->tape = reinterpret_cast<double*>(mem);
@@ -1627,9 +1626,10 @@ int aturan_tape(aturan_ctx* ctx, int on){
     ctx->tTout = take(fs);
     ctx->tPd = take(fs);
     ctx->tSrc = take(fs);
-    ctx->aslot = take(nslot * fs);
     ctx->aybar = take(NT * fs);
     ctx->akbar = take(NT * fs);
+    ctx->akbar2 = take(NT * fs);
+    ctx->ape = take(3 * fs);
     ctx->ag0 = take(NT * fs);
     ctx->aphbar = take(fs);
     ctx->arbar = take(fs);
@@ -1638,7 +1638,7 @@ int aturan_tape(aturan_ctx* ctx, int on){
     ctx->ahacc = take(fs);
     ctx->tPre = NT == ADJ_NF ? nullptr : take(NT * fs);
     ctx->tref = take(g.im);
-    ctx->alev = take(2 * g.im);
+    ctx->alev = take(2 * ADJ_LB * g.im);
     ctx->tape_valid = false;
     ctx->tape_p_valid = false;
     ctx->tape_sat_pending = false;
@@ -1678,40 +1678,44 @@ int rk4_adjoint_impl(aturan_ctx* ctx, int nf, const double* const* ybar, const d
     const double t_min = K.t_min, t_max = K.t_max;
     const dim3 gc((g.km + 127) / 128, g.jm, g.im);
     adj_init_kernel<<<gc, 128, 0, ctx->st>>>(g, ctx->ag0, ctx->tTout, t_min, t_max, dt / 6.0 * 1.0,
-                                             ctx->ag0, ctx->aybar, ctx->akbar, ctx->aphbar, ctx->apdbar, nf);
+                                             ctx->ag0, ctx->aybar, ctx->akbar, ctx->aphbar, ctx->apdbar, nf, K,
+                                             reinterpret_cast<const double*>(ctx->cp_tab), ctx->tX + (size_t)3 * nf * fs,
+                                             reinterpret_cast<const double*>(ctx->forc), ctx->ape, ctx->ape + 2 * fs);
     CK_LAUNCH("adjoint init"); nl++;
     AdjArgs a;
     a.g = g;
     a.X0 = ctx->tX;
-    a.kbar = ctx->akbar;
     a.pdyn = ctx->tPd;                                  // p_dyn as the taped step read it
-    a.forc = reinterpret_cast<const double*>(ctx->forc);
+    a.nt = ctx->ape + 2 * fs;
     a.geo = reinterpret_cast<const GeoIJ<double>*>(ctx->geo);
     a.cp_tab = reinterpret_cast<const double*>(ctx->cp_tab);
     a.k = K;
-    a.slot = ctx->aslot;
+    a.g0 = ctx->ag0;
+    a.ybar = ctx->aybar; a.phbar = ctx->aphbar; a.pdbar = ctx->apdbar;
     a.hacc = heatbar ? ctx->ahacc : nullptr;
     if(heatbar) CK(cudaMemsetAsync(ctx->ahacc, 0, fs * 8, ctx->st));
-    const dim3 gs((g.km - 1 + 31) / 32, (g.jm - 2 + 3) / 4, g.im - 2);
-    const dim3 gg((g.km - 1 + 127) / 128, g.jm, g.im);
+    const dim3 gs((g.km - 1 + 31) / 32, (g.jm + 3) / 4, g.im);
+    // each stage reads one kbar and pe and writes the others
+    double* kb[2] = {ctx->akbar, ctx->akbar2};
+    double* pe[2] = {ctx->ape, ctx->ape + fs};
     for(int stage = 3; stage >= 0; stage--){
+        const int prev = stage - 1, r = (3 - stage) & 1;
         a.X = ctx->tX + (size_t)stage * nf * fs;
+        a.Xprev = prev >= 0 ? ctx->tX + (size_t)prev * nf * fs : nullptr;
+        a.kbar = kb[r]; a.pe = pe[r];
+        a.kbar_out = kb[1 - r]; a.pe_out = pe[1 - r];
         a.auxbar = (stage == 3 && auxbar) ? ctx->aaux : nullptr;   // aux is stage 3's output
-        adj_local_kernel<<<gs, dim3(32, 4), 0, ctx->st>>>(a);
-        nl++;
-        if(nf == ADJ_NF_MOIST){ adj_species_local_kernel<<<gs, dim3(32, 4), 0, ctx->st>>>(a); nl++; }
-        const int prev = stage - 1;
-        const double w_prev = prev >= 0 ? dt / 6.0 * ((prev == 0 || prev == 3) ? 1.0 : 2.0) : 0.0;
-        const double c_prev = prev >= 0 ? ((prev == 0 || prev == 1) ? 0.5 * dt : (prev == 2 ? dt : 0.0)) : 0.0;
-        adj_gather_kernel<<<gg, 128, 0, ctx->st>>>(g, ctx->aslot, ctx->aybar, ctx->aphbar, ctx->apdbar, ctx->ag0,
-                                                  ctx->akbar, w_prev, c_prev, prev >= 0 ? 1 : 0, nf);
+        a.w_prev = prev >= 0 ? dt / 6.0 * ((prev == 0 || prev == 3) ? 1.0 : 2.0) : 0.0;
+        a.c_prev = prev >= 0 ? ((prev == 0 || prev == 1) ? 0.5 * dt : (prev == 2 ? dt : 0.0)) : 0.0;
+        if(nf == ADJ_NF_MOIST) adj_stage_kernel<ADJ_NF_MOIST><<<gs, dim3(32, 4), 0, ctx->st>>>(a);
+        else adj_stage_kernel<ADJ_NF><<<gs, dim3(32, 4), 0, ctx->st>>>(a);
         CK_LAUNCH("adjoint stage"); nl++;
     }
     const double* t0 = ctx->tX;
-    adj_hydro_kernel<<<(g.jm * g.km + 255) / 256, 256, 0, ctx->st>>>(
+    adj_hydro_kernel<<<(g.jm * g.km + 31) / 32, dim3(32, 8), 0, ctx->st>>>(
         g, t0, reinterpret_cast<const double*>(ctx->pstat), t0 + 2 * fs, t0 + 3 * fs, ctx->tref, ctx->rm_i, ctx->cor_j,
         ctx->aphbar, ctx->aybar, ctx->arbar, ctx->hc);
-    adj_level_sum_kernel<<<g.im, 256, 0, ctx->st>>>(g, t0, reinterpret_cast<const double*>(ctx->pstat), ctx->wsin,
+    adj_level_sum_kernel<<<dim3(ADJ_LB, g.im), 256, 0, ctx->st>>>(g, t0, reinterpret_cast<const double*>(ctx->pstat), ctx->wsin,
                                                    ctx->arbar, ctx->hc, ctx->alev);
     adj_level_apply_kernel<<<gc, 128, 0, ctx->st>>>(g, t0, reinterpret_cast<const double*>(ctx->pstat), ctx->wsin,
                                                     ctx->alev, ctx->hc, ctx->aybar);
