@@ -237,8 +237,8 @@ void launch_buoy(Grid g, const S* t, const S* ps, const double* wsin, HydroConst
     if(exact){                                                                                            \
         buoy_terms_kernel<S><<<dim3(bx.nbx, g.im), BX_CH, 0, st>>>(g, t, ps, wsin, h, bx.terms, bx.bpart, bx.nbx); \
         buoy_predict_kernel<<<g.im, 256, 0, st>>>(bx.nbx, bx.bpart, bx.bexp);                               \
-        buoy_units_kernel<<<dim3(bx.nbx, g.im), BX_CH, 0, st>>>(g, bx.nbx, bx.terms, bx.bexp, bx.bunits);  \
-        buoy_serial_pass_kernel<<<g.im, 32, 0, st>>>(g, bx.nbx, bx.terms, bx.bexp, bx.bunits, ref);         \
+        buoy_units_kernel<<<dim3((bx.nbx + 7) / 8, g.im), 256, 0, st>>>(g, bx.nbx, bx.terms, bx.bexp, bx.bunits);  \
+        buoy_serial_pass_kernel<<<g.im, 64, 0, st>>>(g, bx.nbx, bx.terms, bx.bpart, bx.bexp, bx.bunits, ref); \
         return;                                                                                           \
     }                                                                                                     \
     buoy_partial_kernel<S><<<dim3(nblk, g.im), 256, 0, st>>>(g, t, ps, wsin, h, part_sum, part_w, nblk); \

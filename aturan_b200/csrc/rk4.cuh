@@ -830,11 +830,12 @@ static __global__ void buoy_finish_kernel(int im, int nblk, const double* part_s
 //     predicts the binade each chunk's running sum stays in, if one;
 //   pass 3 (buoy_units_kernel, one block per chunk): (I_0, I_1) of every predicted chunk, by an
 //     ordered tree over its terms' own actions;
-//   pass 4 (buoy_serial_pass_kernel, one warp per level): the chunks in order, each applied in O(1)
-//     when s lies in the predicted binade and the result stays below its top, and term by term
-//     otherwise (the first chunks, where s is small, and the ~9 where s crosses a power of two).
-// Every O(1) step is checked exactly, so the prediction only decides speed. A level with a
-// negative term (not monotone) runs all its chunks term by term.
+//   pass 4 (buoy_serial_pass_kernel, one warp per level and sum): the chunks in order, up to 32 at a
+//     time by a scan of their actions while s lies in the predicted binade and the result stays
+//     below its top, and otherwise (the first chunks, where s is small, and the ~9 where s crosses a
+//     power of two) 32 terms at a time by a scan of the terms' actions, broken where s crosses.
+// Every such step is checked exactly, so the prediction only decides speed. A chunk with a negative
+// term (not monotone; the sine of the last colatitude can round below 0) is added term by term.
 // Both sums (w b and w) go this way; the mean is s / w as in the reference.
 constexpr int BX_CH = 256;
 
@@ -874,21 +875,17 @@ __global__ void __launch_bounds__(BX_CH) buoy_terms_kernel(Grid g, const S* t, c
 
 // pass 2: the approximate prefix of the chunk sums (a block scan over tiles of 256 chunks) and the
 // predicted binade of each chunk's running sum (INT_MIN: not predicted to stay in one binade, or
-// the level has a negative term), one block per level.
+// the chunk has a negative term), one block per level.
 static __global__ void __launch_bounds__(256) buoy_predict_kernel(int nbx, const double* bpart, int* bexp){
     const int lev = blockIdx.x;
     const double* bp = bpart + 3 * (size_t)lev * nbx;
     int* E = bexp + 2 * (size_t)lev * nbx;
     __shared__ double scb[256], scw[256];
-    __shared__ int negl;
-    if(threadIdx.x == 0) negl = 0;
-    __syncthreads();
-    for(int b = threadIdx.x; b < nbx; b += 256) if(bp[3 * b + 2] != 0.0) negl = 1;
-    __syncthreads();
     double carry_b = 0.0, carry_w = 0.0;
     for(int b0 = 0; b0 < nbx; b0 += 256){
         const int b = b0 + threadIdx.x;
         const double vb = (b < nbx) ? bp[3 * b] : 0.0, vw = (b < nbx) ? bp[3 * b + 1] : 0.0;
+        const bool neg = b < nbx && bp[3 * b + 2] != 0.0;
         scb[threadIdx.x] = vb; scw[threadIdx.x] = vw;
         __syncthreads();
         for(int off = 1; off < 256; off <<= 1){
@@ -904,7 +901,7 @@ static __global__ void __launch_bounds__(256) buoy_predict_kernel(int nbx, const
             const double ew_lo = (pw_end - vw) * (1.0 - 1e-9), ew_hi = pw_end * (1.0 + 1e-9);
             // binades whose unit and scale are normal powers of two: -970 <= e <= 1000
             auto pred = [&](double lo, double hi) -> int {
-                if(negl || !(lo > 0.0)) return INT_MIN;
+                if(neg || !(lo > 0.0)) return INT_MIN;
                 const int e = ilogb(lo);
                 return (e == ilogb(hi) && e >= -970 && e <= 1000) ? e : INT_MIN;
             };
@@ -940,134 +937,148 @@ __device__ __forceinline__ longlong2 units_then(longlong2 A, longlong2 B){
     return C;
 }
 
-// pass 3: each chunk's action (units for an even and an odd start) in its predicted binade, by an
-// ordered tree over its terms, one block per chunk; the same for the weights.
-static __global__ void __launch_bounds__(BX_CH) buoy_units_kernel(Grid g, int nbx, const double* terms, const int* bexp,
-                                                                  long long* bunits){
-    const int lev = blockIdx.y, b = blockIdx.x;
+// An action's inclusive scan over the lanes, in order.
+__device__ __forceinline__ longlong2 units_scan(longlong2 v, int lane){
+#pragma unroll
+    for(int off = 1; off < 32; off <<= 1){
+        longlong2 p;
+        p.x = __shfl_up_sync(0xffffffffu, v.x, off);
+        p.y = __shfl_up_sync(0xffffffffu, v.y, off);
+        if(lane >= off) v = units_then(p, v);
+    }
+    return v;
+}
+// The binade of a running sum, INT_MIN where its unit and scale are not normal powers of two.
+__device__ __forceinline__ int sum_binade(double s){
+    if(!(s > 0.0)) return INT_MIN;
+    const int e = ilogb(s);
+    return (e >= -970 && e <= 1000) ? e : INT_MIN;
+}
+// pass 3: each chunk's action (units for an even and an odd start) in its predicted binade, a warp per
+// chunk: each lane composes BX_PL consecutive terms, an ordered scan composes the lanes; the same for the
+// weights. (A block per chunk with the ordered tree over single terms in shared memory: 41 us.)
+constexpr int BX_PL = BX_CH / 32;
+static __global__ void __launch_bounds__(256) buoy_units_kernel(Grid g, int nbx, const double* terms, const int* bexp,
+                                                                long long* bunits){
+    const int lev = blockIdx.y, lane = threadIdx.x & 31, b = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if(b >= nbx) return;                                 // a whole warp
     const int ncell = g.jm * g.km;
-    const int c = b * BX_CH + threadIdx.x;
     const int* E = bexp + 2 * ((size_t)lev * nbx + b);
-    const double* xb = terms + (size_t)lev * 2 * ncell;
-    __shared__ longlong2 ub[BX_CH], uw[BX_CH];
-    const int eb = E[0], ew = E[1];
-    const longlong2 zero = make_longlong2(0, 0);
-    ub[threadIdx.x] = (eb != INT_MIN && c < ncell) ? term_units(xb[c], eb) : zero;
-    uw[threadIdx.x] = (ew != INT_MIN && c < ncell) ? term_units(xb[ncell + c], ew) : zero;
-    __syncthreads();
-    for(int st = 1; st < BX_CH; st <<= 1){               // ordered: (t, t + st) into t
-        if((threadIdx.x & (2 * st - 1)) == 0){
-            ub[threadIdx.x] = units_then(ub[threadIdx.x], ub[threadIdx.x + st]);
-            uw[threadIdx.x] = units_then(uw[threadIdx.x], uw[threadIdx.x + st]);
+    long long* U = bunits + 4 * ((size_t)lev * nbx + b);
+#pragma unroll
+    for(int q = 0; q < 2; q++){
+        const double* x = terms + (size_t)lev * 2 * ncell + (size_t)q * ncell;
+        const int e = E[q];
+        if(e == INT_MIN) continue;                       // its units are not read
+        double v[BX_PL];
+#pragma unroll
+        for(int u = 0; u < BX_PL; u++){ const int r = b * BX_CH + lane * BX_PL + u; v[u] = r < ncell ? x[r] : 0.0; }
+        longlong2 A = make_longlong2(0, 0);
+#pragma unroll
+        for(int u = 0; u < BX_PL; u++) A = units_then(A, term_units(v[u], e));
+        A = units_scan(A, lane);
+        if(lane == 31){ U[2 * q] = A.x; U[2 * q + 1] = A.y; }
+    }
+}
+
+// pass 4.
+// s plus the warp's BX_CH terms v >= 0 (BX_PL consecutive ones per lane), in order, each addition rounded
+// as the serial sum's: each lane composes its terms' actions in s's binade, a scan over the lanes applies
+// them up to the lane that takes s out of the binade, and that lane's terms are added as they are.
+__device__ __forceinline__ double sum_terms(double s, const double (&v)[BX_PL], int lane){
+    constexpr long long TOP = 1LL << 53;
+    bool any = false;
+#pragma unroll
+    for(int u = 0; u < BX_PL; u++) any |= v[u] != 0.0;
+    int p = 0;                                         // lanes below p are in
+    while(p < 32){
+        const int e = sum_binade(s);
+        long long before = 0;                          // the sum in units before lane c
+        int c;
+        if(e == INT_MIN){                              // s = 0 or out of range: the next lane that changes it
+            const unsigned m = __ballot_sync(0xffffffffu, lane >= p && any);
+            if(!m) break;
+            c = __ffs(m) - 1;
+        } else {
+            longlong2 A = make_longlong2(0, 0);
+            if(lane >= p){
+                const double top = pow2(e + 1);
+#pragma unroll
+                for(int u = 0; u < BX_PL; u++){
+                    // a term of at least a whole binade crosses by itself (its units may not fit)
+                    longlong2 B = make_longlong2(TOP, TOP);
+                    if(v[u] < top) B = term_units(v[u], e);
+                    A = units_then(A, B);
+                }
+            }
+            A = units_scan(A, lane);
+            const long long si = (long long)(s * pow2(52 - e));        // exact integer
+            const long long tot = si + ((si & 1) ? A.y : A.x);
+            const unsigned m = __ballot_sync(0xffffffffu, tot >= TOP);
+            if(!m){ s = (double)__shfl_sync(0xffffffffu, tot, 31) * pow2(e - 52); break; }
+            c = __ffs(m) - 1;
+            before = c > 0 ? __shfl_sync(0xffffffffu, tot, c > 0 ? c - 1 : 0) : si;
+            s = (double)before * pow2(e - 52);
         }
-        __syncthreads();
+        double t[BX_PL];
+#pragma unroll
+        for(int u = 0; u < BX_PL; u++) t[u] = __shfl_sync(0xffffffffu, v[u], c);
+#pragma unroll
+        for(int u = 0; u < BX_PL; u++) s += t[u];
+        p = c + 1;
     }
-    if(threadIdx.x == 0){
-        long long* U = bunits + 4 * ((size_t)lev * nbx + b);
-        U[0] = ub[0].x; U[1] = ub[0].y; U[2] = uw[0].x; U[3] = uw[0].y;
-    }
+    return s;
 }
 
-// pass 4: the chunks in order, one warp per level. Lane 0 applies a chunk in O(1) when s lies in
-// its predicted binade and the result stays below the binade's top; otherwise the warp stages the
-// chunk's terms in shared memory and lane 0 adds them one by one. Between O(1) chunks of one binade
-// the running sum stays an integer count of units (si), so the dependent chain is one integer add.
-struct RunSum {
-    double s;        // the running sum, when !in_units
-    long long si;    // s / 2^(e-52), when in_units
-    int e;
-    bool in_units;
-};
-__device__ __forceinline__ void run_to_double(RunSum& r){
-    if(r.in_units){ r.s = (double)r.si * pow2(r.e - 52); r.in_units = false; }    // exact
-}
-__device__ __forceinline__ bool chunk_fast(RunSum& r, int e, const long long* I){
-    if(e == INT_MIN){ run_to_double(r); return false; }
-    if(!(r.in_units && r.e == e)){
-        run_to_double(r);
-        const double lo = pow2(e);
-        if(!(r.s >= lo && r.s < 2.0 * lo)) return false;
-        r.si = (long long)(r.s * pow2(52 - e));        // exact integer
-        r.e = e;
-        r.in_units = true;
-    }
-    const long long ni = r.si + I[r.si & 1];
-    if(ni >= (1LL << 53)){ run_to_double(r); return false; }
-    r.si = ni;
-    return true;
-}
-
-static __global__ void __launch_bounds__(32) buoy_serial_pass_kernel(Grid g, int nbx, const double* terms, const int* bexp,
-                                                                     const long long* bunits, double* ref){
-    constexpr int TILE = 256;                          // chunks whose binades and units are staged at once
-    const int lev = blockIdx.x, lane = threadIdx.x;
+// Block (level): warp 0 the terms' sum, warp 1 the weights'. 41x181x361: 66 us, against 151 with lane 0 of one warp
+// applying the chunks and the terms one by one for both sums; at 41x91x181, whose last sine is negative,
+// 54 against 249 us (every chunk went term by term).
+static __global__ void __launch_bounds__(64) buoy_serial_pass_kernel(Grid g, int nbx, const double* terms, const double* bpart,
+                                                                     const int* bexp, const long long* bunits, double* ref){
+    const int lev = blockIdx.x, lane = threadIdx.x & 31, c = threadIdx.x >> 5;
     const int ncell = g.jm * g.km;
-    const double* xs[2] = {terms + (size_t)lev * 2 * ncell, terms + (size_t)lev * 2 * ncell + ncell};
-    const int* E = bexp + 2 * (size_t)lev * nbx;
-    const long long* U = bunits + 4 * (size_t)lev * nbx;
-    __shared__ int se[2 * TILE];
-    __shared__ long long su[4 * TILE];
-    // the terms of chunks taken term by term, [chunk parity][chain]: a chunk predicted to need it
-    // is copied in (cp.async) while the chunk before it is applied
-    __shared__ double stg[2][2][BX_CH];
-    RunSum rs{0.0, 0, 0, false}, rw{0.0, 0, 0, false};   // lane 0's
-    for(int b0 = 0; b0 < nbx; b0 += TILE){
-        const int nt = min(TILE, nbx - b0);
-        for(int q = lane; q < 2 * nt; q += 32) se[q] = E[2 * b0 + q];
-        for(int q = lane; q < 4 * nt; q += 32) su[q] = U[4 * (size_t)b0 + q];
-        __syncwarp();
-        int staged = 0;                                // chains whose chunk bt is copied in: bit c
-        for(int bt = 0; bt < nt; bt++){
-            const int b = b0 + bt;
-            const int n = min(BX_CH, ncell - b * BX_CH);
-            // copy in the next chunk's terms for each chain predicted to take it term by term
-            int next = 0;
-            if(bt + 1 < nt){
-                const int b1 = b + 1, n1 = min(BX_CH, ncell - b1 * BX_CH);
-                for(int c = 0; c < 2; c++){
-                    if(se[2 * (bt + 1) + c] != INT_MIN) continue;
-                    next |= 1 << c;
-                    const double* x = xs[c] + (size_t)b1 * BX_CH;
-                    for(int q = lane; q < n1; q += 32) cp_async_n<8>(&stg[b1 & 1][c][q], x + q);
-                }
-            }
-            cp_async_commit();                         // one group per chunk, possibly empty
-            int ok = 0;
-            if(lane == 0){                             // the two chains' O(1) steps side by side
-                const bool okb = chunk_fast(rs, se[2 * bt], su + 4 * bt);
-                const bool okw = chunk_fast(rw, se[2 * bt + 1], su + 4 * bt + 2);
-                ok = (okb ? 1 : 0) | (okw ? 2 : 0);
-            }
-            ok = __shfl_sync(0xffffffffu, ok, 0);
-            // the chains that failed their O(1) step, term by term (RunSum in double form); the
-            // two chains are named, not selected through a reference, so they stay in registers
-            auto by_terms = [&](RunSum& r, int c){
-                if(!(staged & (1 << c))){               // not predicted: copy now
-                    const double* x = xs[c] + (size_t)b * BX_CH;
-                    for(int q = lane; q < n; q += 32) stg[b & 1][c][q] = x[q];
-                }
-                __syncwarp();
-                if(lane == 0){
-                    const double* t = stg[b & 1][c];
-                    double acc = r.s;
-#pragma unroll 8
-                    for(int q = 0; q < n; q++) acc += t[q];
-                    r.s = acc;
-                }
-                __syncwarp();
-            };
-            if((ok & 3) != 3) cp_async_wait<1>();     // chunk b's copies (all but the newest group)
-            if(!(ok & 1)) by_terms(rs, 0);
-            if(!(ok & 2)) by_terms(rw, 1);
-            staged = next;
+    const double* x = terms + (size_t)lev * 2 * ncell + (size_t)c * ncell;
+    const int* E = bexp + 2 * (size_t)lev * nbx + c;
+    const long long* U = bunits + 4 * (size_t)lev * nbx + 2 * c;
+    const double* neg = bpart + 3 * (size_t)lev * nbx + 2;
+    __shared__ double stg[2][BX_CH];
+    double s = 0.0;
+    int b = 0;
+    while(b < nbx){
+        // the chunks from b on whose predicted binade is s's, applied together up to the binade's top
+        const int q = b + lane;
+        const int e = sum_binade(s);
+        const bool same = q < nbx && e != INT_MIN && E[2 * min(q, nbx - 1)] == e;
+        const unsigned ms = __ballot_sync(0xffffffffu, same);
+        if(ms & 1u){
+            longlong2 A = make_longlong2(0, 0);
+            if(same){ A.x = U[4 * (size_t)q]; A.y = U[4 * (size_t)q + 1]; }
+            A = units_scan(A, lane);
+            const long long si = (long long)(s * pow2(52 - e));
+            const long long tot = si + ((si & 1) ? A.y : A.x);
+            const unsigned mo = __ballot_sync(0xffffffffu, same && tot < (1LL << 53));
+            const int n = mo == 0xffffffffu ? 32 : __ffs(~mo) - 1;           // leading lanes that hold
+            if(n > 0){ s = (double)__shfl_sync(0xffffffffu, tot, n - 1) * pow2(e - 52); b += n; continue; }
         }
-        cp_async_wait<0>();
-        __syncwarp();
+        // chunk b by its terms, loaded together
+        const int n = min(BX_CH, ncell - b * BX_CH);
+        double v[BX_PL];
+#pragma unroll
+        for(int u = 0; u < BX_PL; u++){ const int r = lane * BX_PL + u; v[u] = r < n ? x[(size_t)b * BX_CH + r] : 0.0; }
+        if(neg[3 * (size_t)b] != 0.0){
+#pragma unroll
+            for(int u = 0; u < BX_PL; u++) stg[c][lane * BX_PL + u] = v[u];
+            __syncwarp();
+#pragma unroll 8
+            for(int r = 0; r < BX_CH; r++) s += stg[c][r];        // every lane alike; past the end zeros
+            __syncwarp();
+        } else s = sum_terms(s, v, lane);
+        b++;
     }
-    if(lane == 0){
-        run_to_double(rs); run_to_double(rw);
-        ref[lev] = (rw.s > 0.0) ? rs.s / rw.s : 0.0;
-    }
+    __shared__ double sum[2];
+    if(lane == 0) sum[c] = s;
+    __syncthreads();
+    if(threadIdx.x == 0) ref[lev] = (sum[1] > 0.0) ? sum[0] / sum[1] : 0.0;
 }
 
 // ---- RungeKutta_Uran_Turb.cpp:62-177: per column (j, k) -- every column, the seam copy and the
