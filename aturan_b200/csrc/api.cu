@@ -81,7 +81,9 @@ struct aturan_ctx {
     double last_resid;
     int sor_nblk;
     int sor_pm;                // Fourier modes per block of the column correction's tridiagonal solves
-    std::vector<double> host_part;
+    SorCheck* sor_check;
+    cudaStream_t st_check = nullptr;   // reads the solve's checks
+    cudaEvent_t ev_check[2] = {nullptr, nullptr};
     // adjoint tape (aturan_tape): stage inputs of t, u, v, w, the step's T output and level means,
     // and the adjoint's work arrays; null when the tape is off
     double* tape;
@@ -549,26 +551,31 @@ int run_rb(aturan_ctx* ctx, int sweeps, double omega){
 
 // ---- RB_SOR: the shared solver's equation to a relative L2 residual (sor.cuh) ----
 
-// Residual of P against src: relative L2 norm (host sum of the block partials, fixed order).
-// TR: of the transposed operator. shift: apply the source's compatibility shift in this pass
-// (after sor_compat with apply = false).
+// Residual of P against src as check `slot` of a solve (slot < 0: its column sums only). TR: of the
+// transposed operator. shift: apply the source's compatibility shift in this pass (after sor_compat
+// with apply = false).
 template <typename T, bool TR = false>
-int sor_residual(aturan_ctx* ctx, const T* P, const T* src, bool want_col, double* rel, double* abs_rr,
+int sor_residual(aturan_ctx* ctx, const T* P, const T* src, bool want_col, int slot, double tol, bool first,
                  bool fill32 = false, const double* shift = nullptr){
     const Grid g = ctx->g;
     double* src_w = nullptr;
     if constexpr(std::is_same<T, double>::value) src_w = shift ? const_cast<double*>(src) : nullptr;
     sor_colsum_kernel<T, TR><<<dim3((g.km - 1 + 31) / 32, g.jm - 2), dim3(32, 8), 0, ctx->st>>>(
-        g, P, src, ctx->rbw, ctx->sor_colR, ctx->sor_part, want_col ? 1 : 0,
+        g, P, src, ctx->rbw, ctx->sor_colR, ctx->sor_part, want_col ? 1 : 0, SorCheckArg{ctx->sor_check, slot, first, tol},
         fill32 ? ctx->r32 : nullptr, fill32 ? ctx->e32 : nullptr, src_w, src_w ? shift : nullptr);
     CK_LAUNCH("residual");
-    if(!rel) return ATURAN_OK;                                 // column sums only: no host round trip
-    CK(cudaMemcpyAsync(ctx->host_part.data(), ctx->sor_part, 2 * ctx->sor_nblk * 8, cudaMemcpyDeviceToHost, ctx->st));
-    CK(cudaStreamSynchronize(ctx->st));
-    double rr = 0.0, ss = 0.0;
-    for(int n = 0; n < ctx->sor_nblk; n++){ rr += ctx->host_part[2 * n]; ss += ctx->host_part[2 * n + 1]; }
-    if(abs_rr) *abs_rr = std::sqrt(rr);
-    *rel = ss > 0.0 ? std::sqrt(rr / ss) : std::sqrt(rr);
+    if(slot >= 0) CK(cudaEventRecord(ctx->ev_check[slot], ctx->st));
+    return ATURAN_OK;
+}
+
+// The answer of check `slot`, read on a stream of its own: what was enqueued after the check keeps
+// the solve's stream busy meanwhile.
+int sor_answer(aturan_ctx* ctx, int slot, double* rel){
+    SorCheck c;
+    CK(cudaStreamWaitEvent(ctx->st_check, ctx->ev_check[slot], 0));
+    CK(cudaMemcpyAsync(&c, ctx->sor_check, sizeof c, cudaMemcpyDeviceToHost, ctx->st_check));
+    CK(cudaStreamSynchronize(ctx->st_check));
+    *rel = rel_residual(c.rr[slot], c.ss[slot]);
     return ATURAN_OK;
 }
 
@@ -594,7 +601,8 @@ int sor_correct(aturan_ctx* ctx, T* P){
     sor_gemm_kernel<<<gi, 256, 0, ctx->st>>>(c.J, c.N, c.NM + 1, MatRef{ctx->sor_Ac, 1, c.J}, MatRef{ctx->sor_ct, c.N, 1},
                                             MatRef{ctx->sor_As, 1, c.J}, MatRef{ctx->sor_st, c.N, 1},
                                             1.0, ctx->sor_q, nullptr, c.N, 1, kci, sz_q);
-    sor_add_kernel<T, TR><<<dim3((c.N + 127) / 128, g.jm - 2), 128, 0, ctx->st>>>(g, ctx->sor_q, P, SOR_KSPLIT, sz_q);
+    sor_add_kernel<T, TR><<<dim3((c.N + 127) / 128, g.jm - 2), 128, 0, ctx->st>>>(g, ctx->sor_q, P, SOR_KSPLIT, sz_q,
+                                                                                  &ctx->sor_check->stop);
     CK_LAUNCH("column-uniform correction");
     return ATURAN_OK;
 }
@@ -613,20 +621,32 @@ bool line_smem_attr(){
 }
 
 // One relaxation sweep (both colours) of the folded operator (TR: its transpose): point
-// (line = false) or radial line.
+// (line = false) or radial line. chained: the launch before is a point pass of the same solve, so
+// this one may start beside it (sor_colour_kernel says what it does before it waits).
 template <typename T, bool TR = false>
-void sor_sweep(aturan_ctx* ctx, T* E, const T* R, double omega, bool line){
+int sor_sweep(aturan_ctx* ctx, T* E, const T* R, double omega, bool line, bool chained){
     const Grid g = ctx->g;
+    const int* stop = &ctx->sor_check->stop;
     if(line && line_smem<T>(g) > 48 * 1024) line_smem_attr<T, TR>();
     for(int colour = 0; colour < 2; colour++){
-        if(line)
+        if(line){
             sor_line_kernel<T, TR><<<dim3((g.km / 2 + LINE_COLS - 1) / LINE_COLS, g.jm - 2), 256, line_smem<T>(g), ctx->st>>>(
                 g, E, R, ctx->rbw, TR ? ctx->lluT_a : ctx->llu_a, TR ? ctx->lluT_cf : ctx->llu_cf,
-                TR ? ctx->lluT_idn : ctx->llu_idn, colour, omega);
-        else
-            sor_colour_kernel<T, TR><<<dim3((g.km / 2 + 127) / 128, g.jm - 2, g.im - 2), 128, 0, ctx->st>>>(
-                g, E, R, ctx->rbw, colour, omega);
+                TR ? ctx->lluT_idn : ctx->llu_idn, colour, omega, stop);
+            continue;
+        }
+        cudaLaunchAttribute at;
+        at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at.val.programmaticStreamSerializationAllowed = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((g.km / 2 * (g.jm - 2) + COLOUR_NT - 1) / COLOUR_NT, (g.im - 2 + COLOUR_CH - 1) / COLOUR_CH);
+        cfg.blockDim = dim3(COLOUR_NT);
+        cfg.stream = ctx->st;
+        cfg.attrs = &at;
+        cfg.numAttrs = chained || colour == 1 ? 1 : 0;
+        CK(cudaLaunchKernelEx(&cfg, sor_colour_kernel<T, TR>, g, E, R, (const RBW*)ctx->rbw, colour, omega, stop));
     }
+    return ATURAN_OK;
 }
 
 int sor_check_sizes(aturan_ctx* ctx, double omega, bool line){
@@ -659,24 +679,54 @@ const double* sor_compat(aturan_ctx* ctx, double* src, bool transposed, bool app
     return shift;
 }
 
-// FP64 red-black solve of Lc P = src (TR: Lc^T P = src) on the interior from the given P, src
-// compatible. Returns ATURAN_OK at tol, ATURAN_NOT_CONVERGED at the cap; counts launches into nl.
-template <bool TR>
-int solve_fp64(aturan_ctx* ctx, double* P, const double* src, double omega, int max_sweeps, double tol, bool line,
-               int* sweeps_done, double* resid, long& nl, const double* shift = nullptr){
-    const int check_every = sor_check_every(line), every = sor_correct_every(line);
+// The loop of a solve: check (the relative residual of P) and iterate (sweeps s .. next, returning
+// next) until a check meets tol or max_sweeps are done. The sweeps after a check, and the check
+// after those, are enqueued before that check's answer is read; once a check has met tol they do
+// nothing (SorCheck), so sweeps and results are those of a loop that waits each time.
+// Returns ATURAN_OK at tol, ATURAN_NOT_CONVERGED at the cap.
+template <typename Check, typename Iterate>
+int solve_loop(aturan_ctx* ctx, int max_sweeps, double tol, int* sweeps_done, double* resid, Check check, Iterate iterate){
     double r = 0.0;
     int s = 0;
-    int rc = sor_residual<double, TR>(ctx, P, src, true, &r, nullptr, false, shift); if(rc) return rc; nl++;
-    while(s < max_sweeps && !(r <= tol)){
-        if(s % every == 0){ rc = sor_correct<double, TR>(ctx, P); if(rc) return rc; nl += 4; }
-        for(int n = 0; n < check_every && s < max_sweeps; n++, s++){ sor_sweep<double, TR>(ctx, P, src, omega, line); nl += 2; }
-        CK_LAUNCH("SOR sweeps");
-        rc = sor_residual<double, TR>(ctx, P, src, s % every == 0, &r, nullptr); if(rc) return rc; nl++;
+    int rc = check(0, 0); if(rc) return rc;
+    for(int n = 0;; n++){
+        int next = s;
+        const bool more = s < max_sweeps;
+        if(more){
+            rc = iterate(s, &next); if(rc) return rc;
+            rc = check((n + 1) & 1, next); if(rc) return rc;
+        }
+        rc = sor_answer(ctx, n & 1, &r); if(rc) return rc;
+        if(r <= tol || !more) break;
+        s = next;
     }
     if(sweeps_done) *sweeps_done = s;
     if(resid) *resid = r;
     return r <= tol ? ATURAN_OK : ATURAN_NOT_CONVERGED;
+}
+
+// FP64 red-black solve of Lc P = src (TR: Lc^T P = src) on the interior from the given P, src
+// compatible. Counts launches into nl.
+template <bool TR>
+int solve_fp64(aturan_ctx* ctx, double* P, const double* src, double omega, int max_sweeps, double tol, bool line,
+               int* sweeps_done, double* resid, long& nl, const double* shift = nullptr){
+    const int check_every = sor_check_every(line), every = sor_correct_every(line);
+    return solve_loop(ctx, max_sweeps, tol, sweeps_done, resid,
+        [&](int slot, int s){
+            nl++;
+            return sor_residual<double, TR>(ctx, P, src, s % every == 0, slot, tol, s == 0, false, s == 0 ? shift : nullptr);
+        },
+        [&](int s, int* next){
+            int rc;
+            if(s % every == 0){ rc = sor_correct<double, TR>(ctx, P); if(rc) return rc; nl += 4; }
+            for(int n = 0; n < check_every && s < max_sweeps; n++, s++){
+                rc = sor_sweep<double, TR>(ctx, P, src, omega, line, n > 0); if(rc) return rc;
+                nl += 2;
+            }
+            CK_LAUNCH("SOR sweeps");
+            *next = s;
+            return (int)ATURAN_OK;
+        });
 }
 
 // The mixed form of the same solve: FP64 iterative refinement around FP32 correction solves,
@@ -690,33 +740,35 @@ int solve_mixed(aturan_ctx* ctx, double* P, const double* src, double omega, int
     // FP32 sweeps per refinement step: for line SOR 2 (measured at 41x181x361, warm: two
     // refinement steps of 2 reach 3e-8 against 6 sweeps with 3 per step, 0.53 vs 0.59 ms)
     const int inner = line ? 2 : 48;
-    double r = 0.0;
-    int s = 0;
     // Each FP64 residual also leaves r in FP32, e = 0 and the column sums of r: what the next
     // correction solve starts from (one pass over p and src per refinement step).
-    int rc = sor_residual<double, TR>(ctx, P, src, true, &r, nullptr, true, shift); if(rc) return rc; nl++;
-    while(s < max_sweeps && !(r <= tol)){
-        for(int n = 0; n < inner && s < max_sweeps; n++, s++){
-            // the correction on the same cadence as the FP64 solve (once per `every` sweeps,
-            // counted over the whole solve): after the first one the column-uniform error is
-            // gone and a later refinement step's correction changes nothing (measured: same
-            // sweep count, 0.14 ms less at 41x181x361); with e = 0 its column sums are r's
-            if(s % every == 0){
-                if(n != 0){ rc = sor_residual<float, TR>(ctx, ctx->e32, ctx->r32, true, nullptr, nullptr); if(rc) return rc; nl++; }
-                rc = sor_correct<float, TR>(ctx, ctx->e32); if(rc) return rc;
-                nl += 4;
+    return solve_loop(ctx, max_sweeps, tol, sweeps_done, resid,
+        [&](int slot, int s){
+            nl++;
+            return sor_residual<double, TR>(ctx, P, src, true, slot, tol, s == 0, true, s == 0 ? shift : nullptr);
+        },
+        [&](int s, int* next){
+            int rc;
+            for(int n = 0; n < inner && s < max_sweeps; n++, s++){
+                // the correction on the same cadence as the FP64 solve (once per `every` sweeps,
+                // counted over the whole solve): after the first one the column-uniform error is
+                // gone and a later refinement step's correction changes nothing (measured: same
+                // sweep count, 0.14 ms less at 41x181x361); with e = 0 its column sums are r's
+                const bool correct = s % every == 0;
+                if(correct){
+                    if(n != 0){ rc = sor_residual<float, TR>(ctx, ctx->e32, ctx->r32, true, -1, 0.0, false); if(rc) return rc; nl++; }
+                    rc = sor_correct<float, TR>(ctx, ctx->e32); if(rc) return rc;
+                    nl += 4;
+                }
+                rc = sor_sweep<float, TR>(ctx, ctx->e32, ctx->r32, omega, line, n > 0 && !correct); if(rc) return rc;
+                nl += 2;
             }
-            sor_sweep<float, TR>(ctx, ctx->e32, ctx->r32, omega, line);
-            nl += 2;
-        }
-        sor_axpy_kernel<<<148 * 8, 256, 0, ctx->st>>>(fs, P, ctx->e32);
-        CK_LAUNCH("SOR refinement");
-        nl++;
-        rc = sor_residual<double, TR>(ctx, P, src, true, &r, nullptr, true); if(rc) return rc; nl++;
-    }
-    if(sweeps_done) *sweeps_done = s;
-    if(resid) *resid = r;
-    return r <= tol ? ATURAN_OK : ATURAN_NOT_CONVERGED;
+            sor_axpy_kernel<<<148 * 8, 256, 0, ctx->st>>>(fs, P, ctx->e32, &ctx->sor_check->stop);
+            CK_LAUNCH("SOR refinement");
+            nl++;
+            *next = s;
+            return (int)ATURAN_OK;
+        });
 }
 
 template <typename S>
@@ -1100,7 +1152,7 @@ int aturan_ctx_create(const aturan_params* p, aturan_ctx** out){
     for(int n = 0; n < 6; n++) add(nij * 8);                           // line factorisations (Lc, Lc^T)
     add(fs * 4); add(fs * 4);
     ctx->gsp = gs_plan(g);
-    add(gs_edge_bytes(ctx->gsp)); add(4); add(4);
+    add(gs_edge_bytes(ctx->gsp)); add(4); add(4); add(sizeof(SorCheck));
     if(ctx->mixed) add(2 * fs * 4);                                    // the temperature pair's low parts
     ctx->mem_bytes = bytes;
     // the stage kernels address every buffer of the allocation by 32-bit element offsets
@@ -1116,9 +1168,12 @@ int aturan_ctx_create(const aturan_params* p, aturan_ctx** out){
     if(cudaStreamCreateWithPriority(&ctx->st2, cudaStreamNonBlocking, prio_lo) != cudaSuccess){
         cudaStreamDestroy(ctx->st); delete ctx; return ATURAN_E_CUDA;
     }
+    if(cudaStreamCreateWithPriority(&ctx->st_check, cudaStreamNonBlocking, prio_hi) != cudaSuccess){
+        cudaStreamDestroy(ctx->st2); cudaStreamDestroy(ctx->st); delete ctx; return ATURAN_E_CUDA;
+    }
     {
-        cudaEvent_t* evs[6] = {&ctx->ev_fork, &ctx->ev_join, &ctx->ev_xcopy[0], &ctx->ev_xcopy[1],
-                               &ctx->ev_xpack[0], &ctx->ev_xpack[1]};
+        cudaEvent_t* evs[8] = {&ctx->ev_fork, &ctx->ev_join, &ctx->ev_xcopy[0], &ctx->ev_xcopy[1],
+                               &ctx->ev_xpack[0], &ctx->ev_xpack[1], &ctx->ev_check[0], &ctx->ev_check[1]};
         for(cudaEvent_t* e : evs){
             if(cudaEventCreateWithFlags(e, cudaEventDisableTiming) != cudaSuccess){
                 cudaGetLastError();
@@ -1177,8 +1232,8 @@ int aturan_ctx_create(const aturan_params* p, aturan_ctx** out){
     ctx->gs_edge = reinterpret_cast<GsEdge*>(carve<char>(cur, gs_edge_bytes(ctx->gsp)));
     ctx->gs_ticket = carve<unsigned>(cur, 1);
     ctx->gs_err = carve<int>(cur, 1);
+    ctx->sor_check = carve<SorCheck>(cur, 1);
     ctx->tlo = ctx->mixed ? carve<float>(cur, 2 * fs) : nullptr;
-    ctx->host_part.resize(2 * ctx->sor_nblk);
 
     // zero everything once: padding columns and unused planes read as 0, never as garbage
     if(cudaMemsetAsync(ctx->mem, 0, bytes, ctx->st) != cudaSuccess){ aturan_ctx_destroy(ctx); return ATURAN_E_CUDA; }
@@ -1469,7 +1524,9 @@ int aturan_ctx_destroy(aturan_ctx* ctx){
     for(int b = 0; b < 2; b++){
         if(ctx->ev_xcopy[b]) cudaEventDestroy(ctx->ev_xcopy[b]);
         if(ctx->ev_xpack[b]) cudaEventDestroy(ctx->ev_xpack[b]);
+        if(ctx->ev_check[b]) cudaEventDestroy(ctx->ev_check[b]);
     }
+    if(ctx->st_check) cudaStreamDestroy(ctx->st_check);
     if(ctx->st2) cudaStreamDestroy(ctx->st2);
     if(ctx->st) cudaStreamDestroy(ctx->st);
     delete ctx;
