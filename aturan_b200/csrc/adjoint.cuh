@@ -104,6 +104,7 @@ struct AdjRow { double r2, t1, t2, t3, t4, p1, p3, p4, p5; };
 // that wrote and gathered the contributions.
 template <int NF>
 __global__ void __launch_bounds__(128, NF == ADJ_NF ? 4 : 3) adj_stage_kernel(const __grid_constant__ AdjArgs a){
+    chain_wait();
     const Grid& g = a.g;
     const RhsConst<double>& K = a.k;
     __shared__ AdjRow rows[14];          // of this block's four j: (i, j0 - 1 .. j0 + 4), then (i - 1, j), then (i + 1, j)
@@ -405,6 +406,7 @@ __device__ void sat_entry_adj(const GasConst& G, double hc, const SatEntry& e, d
 // before it. pre: the taped state before the adjustment; post: after it (ADJ_NF_MOIST fields each).
 __global__ void __launch_bounds__(128) adj_satadj_kernel(Grid g, const double* pre, const double* post, const double* ps,
                                                          const double* rho_mix, SatConst K, double* ybar){
+    chain_wait();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y, i = blockIdx.z;
     if(k >= g.km) return;
@@ -476,6 +478,7 @@ __global__ void __launch_bounds__(128) adj_satadj_kernel(Grid g, const double* p
 __global__ void adj_init_kernel(Grid g, const double* ybar_in, const double* t_out, double t_min, double t_max,
                                 double w3, double* g0, double* ybar, double* kbar, double* phbar, double* pdbar, int nf,
                                 RhsConst<double> K, const double* cp_tab, const double* t3, const double* nue, double* pe, double* nt){
+    chain_wait();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y;
     const int i = blockIdx.z;
@@ -512,6 +515,7 @@ __global__ void __launch_bounds__(256) adj_hydro_kernel(Grid g, const double* t,
                                                         const double* w, const double* ref, const double* rm_i,
                                                         const double* cor_j, const double* phbar, double* ybar,
                                                         double* rbar, HydroConst h){
+    chain_wait();
     __shared__ double sS[ADJ_HCH + 1][32];         // S(m) of the chunk's levels; the last row S of the level above it
     const int tx = threadIdx.x, ty = threadIdx.y;
     const int c = blockIdx.x * 32 + tx;
@@ -562,6 +566,7 @@ constexpr int ADJ_LB = 16;
 __global__ void __launch_bounds__(256) adj_level_sum_kernel(Grid g, const double* t, const double* ps,
                                                             const double* wsin, const double* rbar,
                                                             HydroConst h, double* lev){
+    chain_wait();
     const int m = blockIdx.y;
     double s = 0.0, ws = 0.0;
     for(int c = blockIdx.x * 256 + threadIdx.x; c < g.jm * g.km; c += ADJ_LB * 256){
@@ -586,6 +591,7 @@ __global__ void __launch_bounds__(256) adj_level_sum_kernel(Grid g, const double
 
 __global__ void __launch_bounds__(128) adj_level_apply_kernel(Grid g, const double* t, const double* ps, const double* wsin,
                                                               const double* lev, HydroConst h, double* ybar){
+    chain_wait();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y;
     const int m = blockIdx.z;
@@ -604,6 +610,7 @@ __global__ void __launch_bounds__(128) adj_level_apply_kernel(Grid g, const doub
 // The heating field's adjoint: heat_scale times the T tendencies' adjoint summed over the stages and
 // the interior levels, per (j,k); 0 on the polar rows and the seam column, which no stage reads.
 __global__ void adj_heat_reduce_kernel(Grid g, const double* hacc, double scale, double* out){
+    chain_wait();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if(c >= g.jm * g.km) return;
     const int j = c / g.km, k = c - j * g.km;
@@ -618,6 +625,7 @@ __global__ void adj_heat_reduce_kernel(Grid g, const double* hacc, double scale,
 
 // F^T in reverse order of launch_pdyn_bcs: seam copy, theta folds (every level), radial folds.
 __global__ void adj_pbc_p_kernel(Grid g, double* B){
+    chain_wait();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if(c >= g.im * g.jm) return;
     const int i = c / g.jm, j = c - i * g.jm;
@@ -625,6 +633,7 @@ __global__ void adj_pbc_p_kernel(Grid g, double* B){
     B[gidx(g, i, j, g.km - 1)] = 0.0;
 }
 __global__ void adj_pbc_t_kernel(Grid g, double* B){
+    chain_wait();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int i = blockIdx.y;
     if(k >= g.km) return;
@@ -634,6 +643,7 @@ __global__ void adj_pbc_t_kernel(Grid g, double* B){
     B[gidx(g, i, g.jm - 2, k)] += C43 * bn; B[gidx(g, i, g.jm - 3, k)] -= C13 * bn;
 }
 __global__ void adj_pbc_r_kernel(Grid g, double* B){
+    chain_wait();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y;
     if(k >= g.km) return;
@@ -649,6 +659,7 @@ __global__ void adj_pbc_r_kernel(Grid g, double* B){
 // clamped source.
 __global__ void adj_compat_mask_kernel(Grid g, const double* lam, const double* mean, double ratio,
                                        const double* src_fwd, const RBW* w, double* sbar){
+    chain_wait();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = 1 + blockIdx.y;
     const int i = 1 + blockIdx.z;
@@ -666,6 +677,7 @@ __global__ void adj_compat_mask_kernel(Grid g, const double* lam, const double* 
 // or cubically extrapolated from the interior, and av = 0 on the polar rows (Pressure_Uran.cpp:30-146).
 __global__ void adj_div_kernel(Grid g, const double* sbar, const RBW* w, PressConst c, int rigid_lid,
                                double* aub, double* avb, double* awb){
+    chain_wait();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y;
     const int i = blockIdx.z;

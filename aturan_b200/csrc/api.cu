@@ -553,14 +553,14 @@ int run_rb(aturan_ctx* ctx, int sweeps, double omega){
 
 // Residual of P against src as check `slot` of a solve (slot < 0: its column sums only). TR: of the
 // transposed operator. shift: apply the source's compatibility shift in this pass (after sor_compat
-// with apply = false).
+// with apply = false). after_point: the launch before is a point pass.
 template <typename T, bool TR = false>
 int sor_residual(aturan_ctx* ctx, const T* P, const T* src, bool want_col, int slot, double tol, bool first,
-                 bool fill32 = false, const double* shift = nullptr){
+                 bool after_point, bool fill32 = false, const double* shift = nullptr){
     const Grid g = ctx->g;
     double* src_w = nullptr;
     if constexpr(std::is_same<T, double>::value) src_w = shift ? const_cast<double*>(src) : nullptr;
-    sor_colsum_kernel<T, TR><<<dim3((g.km - 1 + 31) / 32, g.jm - 2), dim3(32, 8), 0, ctx->st>>>(
+    chain_if(!after_point, sor_colsum_kernel<T, TR>, dim3((g.km - 1 + 31) / 32, g.jm - 2), dim3(32, 8), 0, ctx->st, 
         g, P, src, ctx->rbw, ctx->sor_colR, ctx->sor_part, want_col ? 1 : 0, SorCheckArg{ctx->sor_check, slot, first, tol},
         fill32 ? ctx->r32 : nullptr, fill32 ? ctx->e32 : nullptr, src_w, src_w ? shift : nullptr);
     CK_LAUNCH("residual");
@@ -589,19 +589,19 @@ int sor_correct(aturan_ctx* ctx, T* P){
     const long sz_ac = (long)(c.NM + 1) * c.J, sz_q = (long)c.J * c.N;
     const int kcf = ((c.N + SOR_KSPLIT - 1) / SOR_KSPLIT + 31) / 32 * 32;
     const dim3 gf((c.NM + 1 + 31) / 32, (c.J + 31) / 32, SOR_KSPLIT);
-    sor_gemm_kernel<<<gf, 256, 0, ctx->st>>>(c.J, c.NM + 1, c.N, R, MatRef{ctx->sor_ctT, c.NM + 1, 1},
+    chain(sor_gemm_kernel, gf, 256, 0, ctx->st, c.J, c.NM + 1, c.N, R, MatRef{ctx->sor_ctT, c.NM + 1, 1},
                                             R, MatRef{ctx->sor_stT, c.NM + 1, 1}, 1.0 / c.A2y,
                                             ctx->sor_Ac, ctx->sor_As, 1, c.J, kcf, sz_ac);
     ModeLU lu = TR ? ModeLU{ctx->mluT_a, ctx->mluT_cf, ctx->mluT_idn} : ModeLU{ctx->mlu_a, ctx->mlu_cf, ctx->mlu_idn};
     const int pm = ctx->sor_pm;
-    sor_tridiag_kernel<<<(c.NM + 1 + pm - 1) / pm, 128, (size_t)8 * c.J * (5 * pm + 4), ctx->st>>>(
+    chain(sor_tridiag_kernel, (c.NM + 1 + pm - 1) / pm, 128, (size_t)8 * c.J * (5 * pm + 4), ctx->st, 
         c, lu, ctx->sor_Ac, ctx->sor_As, pm, TR ? 1 : 0, SOR_KSPLIT, sz_ac);
     const int kci = ((c.NM + 1 + SOR_KSPLIT - 1) / SOR_KSPLIT + 31) / 32 * 32;
     const dim3 gi((c.N + 31) / 32, (c.J + 31) / 32, SOR_KSPLIT);
-    sor_gemm_kernel<<<gi, 256, 0, ctx->st>>>(c.J, c.N, c.NM + 1, MatRef{ctx->sor_Ac, 1, c.J}, MatRef{ctx->sor_ct, c.N, 1},
+    chain(sor_gemm_kernel, gi, 256, 0, ctx->st, c.J, c.N, c.NM + 1, MatRef{ctx->sor_Ac, 1, c.J}, MatRef{ctx->sor_ct, c.N, 1},
                                             MatRef{ctx->sor_As, 1, c.J}, MatRef{ctx->sor_st, c.N, 1},
                                             1.0, ctx->sor_q, nullptr, c.N, 1, kci, sz_q);
-    sor_add_kernel<T, TR><<<dim3((c.N + 127) / 128, g.jm - 2), 128, 0, ctx->st>>>(g, ctx->sor_q, P, SOR_KSPLIT, sz_q,
+    chain(sor_add_kernel<T, TR>, dim3((c.N + 127) / 128, g.jm - 2), 128, 0, ctx->st, g, ctx->sor_q, P, SOR_KSPLIT, sz_q,
                                                                                   &ctx->sor_check->stop);
     CK_LAUNCH("column-uniform correction");
     return ATURAN_OK;
@@ -621,8 +621,8 @@ bool line_smem_attr(){
 }
 
 // One relaxation sweep (both colours) of the folded operator (TR: its transpose): point
-// (line = false) or radial line. chained: the launch before is a point pass of the same solve, so
-// this one may start beside it (sor_colour_kernel says what it does before it waits).
+// (line = false) or radial line. chained: the launch before is a point pass of the same solve, so that
+// a point pass may read what none writes before it waits for it (sor_colour_kernel).
 template <typename T, bool TR = false>
 int sor_sweep(aturan_ctx* ctx, T* E, const T* R, double omega, bool line, bool chained){
     const Grid g = ctx->g;
@@ -630,21 +630,13 @@ int sor_sweep(aturan_ctx* ctx, T* E, const T* R, double omega, bool line, bool c
     if(line && line_smem<T>(g) > 48 * 1024) line_smem_attr<T, TR>();
     for(int colour = 0; colour < 2; colour++){
         if(line){
-            sor_line_kernel<T, TR><<<dim3((g.km / 2 + LINE_COLS - 1) / LINE_COLS, g.jm - 2), 256, line_smem<T>(g), ctx->st>>>(
+            chain(sor_line_kernel<T, TR>, dim3((g.km / 2 + LINE_COLS - 1) / LINE_COLS, g.jm - 2), 256, line_smem<T>(g), ctx->st, 
                 g, E, R, ctx->rbw, TR ? ctx->lluT_a : ctx->llu_a, TR ? ctx->lluT_cf : ctx->llu_cf,
                 TR ? ctx->lluT_idn : ctx->llu_idn, colour, omega, stop);
             continue;
         }
-        cudaLaunchAttribute at;
-        at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        at.val.programmaticStreamSerializationAllowed = 1;
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((g.km / 2 * (g.jm - 2) + COLOUR_NT - 1) / COLOUR_NT, (g.im - 2 + COLOUR_CH - 1) / COLOUR_CH);
-        cfg.blockDim = dim3(COLOUR_NT);
-        cfg.stream = ctx->st;
-        cfg.attrs = &at;
-        cfg.numAttrs = chained || colour == 1 ? 1 : 0;
-        CK(cudaLaunchKernelEx(&cfg, sor_colour_kernel<T, TR>, g, E, R, (const RBW*)ctx->rbw, colour, omega, stop));
+        const dim3 grid((g.km / 2 * (g.jm - 2) + COLOUR_NT - 1) / COLOUR_NT, (g.im - 2 + COLOUR_CH - 1) / COLOUR_CH);
+        chain_if(chained || colour == 1, sor_colour_kernel<T, TR>, grid, COLOUR_NT, 0, ctx->st, g, E, R, ctx->rbw, colour, omega, stop);
     }
     return ATURAN_OK;
 }
@@ -673,9 +665,9 @@ const double* sor_compat(aturan_ctx* ctx, double* src, bool transposed, bool app
     const int ny = ((g.jm - 2) * (g.km - 1) + 255) / 256;
     // past the residual pass's block partials: the first residual reads it while writing those
     double* shift = ctx->sor_part + 2 * ctx->sor_nblk;
-    sor_ysum_kernel<<<ny, 256, 0, ctx->st>>>(g, src, ctx->sor_part, transposed ? 1 : 0);
-    sor_shift_finish_kernel<<<1, 256, 0, ctx->st>>>(ctx->sor_part, ny, shift);
-    if(apply) sor_shift_kernel<<<148 * 4, 256, 0, ctx->st>>>(g, src, shift);
+    chain(sor_ysum_kernel, ny, 256, 0, ctx->st, g, src, ctx->sor_part, transposed ? 1 : 0);
+    chain(sor_shift_finish_kernel, 1, 256, 0, ctx->st, ctx->sor_part, ny, shift);
+    if(apply) chain(sor_shift_kernel, 148 * 4, 256, 0, ctx->st, g, src, shift);
     return shift;
 }
 
@@ -714,7 +706,7 @@ int solve_fp64(aturan_ctx* ctx, double* P, const double* src, double omega, int 
     return solve_loop(ctx, max_sweeps, tol, sweeps_done, resid,
         [&](int slot, int s){
             nl++;
-            return sor_residual<double, TR>(ctx, P, src, s % every == 0, slot, tol, s == 0, false, s == 0 ? shift : nullptr);
+            return sor_residual<double, TR>(ctx, P, src, s % every == 0, slot, tol, s == 0, !line && s > 0, false, s == 0 ? shift : nullptr);
         },
         [&](int s, int* next){
             int rc;
@@ -745,7 +737,7 @@ int solve_mixed(aturan_ctx* ctx, double* P, const double* src, double omega, int
     return solve_loop(ctx, max_sweeps, tol, sweeps_done, resid,
         [&](int slot, int s){
             nl++;
-            return sor_residual<double, TR>(ctx, P, src, true, slot, tol, s == 0, true, s == 0 ? shift : nullptr);
+            return sor_residual<double, TR>(ctx, P, src, true, slot, tol, s == 0, false, true, s == 0 ? shift : nullptr);
         },
         [&](int s, int* next){
             int rc;
@@ -756,14 +748,14 @@ int solve_mixed(aturan_ctx* ctx, double* P, const double* src, double omega, int
                 // sweep count, 0.14 ms less at 41x181x361); with e = 0 its column sums are r's
                 const bool correct = s % every == 0;
                 if(correct){
-                    if(n != 0){ rc = sor_residual<float, TR>(ctx, ctx->e32, ctx->r32, true, -1, 0.0, false); if(rc) return rc; nl++; }
+                    if(n != 0){ rc = sor_residual<float, TR>(ctx, ctx->e32, ctx->r32, true, -1, 0.0, false, !line); if(rc) return rc; nl++; }
                     rc = sor_correct<float, TR>(ctx, ctx->e32); if(rc) return rc;
                     nl += 4;
                 }
                 rc = sor_sweep<float, TR>(ctx, ctx->e32, ctx->r32, omega, line, n > 0 && !correct); if(rc) return rc;
                 nl += 2;
             }
-            sor_axpy_kernel<<<148 * 8, 256, 0, ctx->st>>>(fs, P, ctx->e32, &ctx->sor_check->stop);
+            chain_if(line, sor_axpy_kernel, 148 * 8, 256, 0, ctx->st, fs, P, ctx->e32, &ctx->sor_check->stop);
             CK_LAUNCH("SOR refinement");
             nl++;
             *next = s;
@@ -1734,7 +1726,7 @@ int rk4_adjoint_impl(aturan_ctx* ctx, int nf, const double* const* ybar, const d
     const RhsConst<double>& K = ctx->k64;
     const double t_min = K.t_min, t_max = K.t_max;
     const dim3 gc((g.km + 127) / 128, g.jm, g.im);
-    adj_init_kernel<<<gc, 128, 0, ctx->st>>>(g, ctx->ag0, ctx->tTout, t_min, t_max, dt / 6.0 * 1.0,
+    chain(adj_init_kernel, gc, 128, 0, ctx->st, g, ctx->ag0, ctx->tTout, t_min, t_max, dt / 6.0 * 1.0,
                                              ctx->ag0, ctx->aybar, ctx->akbar, ctx->aphbar, ctx->apdbar, nf, K,
                                              reinterpret_cast<const double*>(ctx->cp_tab), ctx->tX + (size_t)3 * nf * fs,
                                              reinterpret_cast<const double*>(ctx->forc), ctx->ape, ctx->ape + 2 * fs);
@@ -1764,21 +1756,21 @@ int rk4_adjoint_impl(aturan_ctx* ctx, int nf, const double* const* ybar, const d
         a.auxbar = (stage == 3 && auxbar) ? ctx->aaux : nullptr;   // aux is stage 3's output
         a.w_prev = prev >= 0 ? dt / 6.0 * ((prev == 0 || prev == 3) ? 1.0 : 2.0) : 0.0;
         a.c_prev = prev >= 0 ? ((prev == 0 || prev == 1) ? 0.5 * dt : (prev == 2 ? dt : 0.0)) : 0.0;
-        if(nf == ADJ_NF_MOIST) adj_stage_kernel<ADJ_NF_MOIST><<<gs, dim3(32, 4), 0, ctx->st>>>(a);
-        else adj_stage_kernel<ADJ_NF><<<gs, dim3(32, 4), 0, ctx->st>>>(a);
+        if(nf == ADJ_NF_MOIST) chain(adj_stage_kernel<ADJ_NF_MOIST>, gs, dim3(32, 4), 0, ctx->st, a);
+        else chain(adj_stage_kernel<ADJ_NF>, gs, dim3(32, 4), 0, ctx->st, a);
         CK_LAUNCH("adjoint stage"); nl++;
     }
     const double* t0 = ctx->tX;
-    adj_hydro_kernel<<<(g.jm * g.km + 31) / 32, dim3(32, 8), 0, ctx->st>>>(
+    chain(adj_hydro_kernel, (g.jm * g.km + 31) / 32, dim3(32, 8), 0, ctx->st, 
         g, t0, reinterpret_cast<const double*>(ctx->pstat), t0 + 2 * fs, t0 + 3 * fs, ctx->tref, ctx->rm_i, ctx->cor_j,
         ctx->aphbar, ctx->aybar, ctx->arbar, ctx->hc);
-    adj_level_sum_kernel<<<dim3(ADJ_LB, g.im), 256, 0, ctx->st>>>(g, t0, reinterpret_cast<const double*>(ctx->pstat), ctx->wsin,
+    chain(adj_level_sum_kernel, dim3(ADJ_LB, g.im), 256, 0, ctx->st, g, t0, reinterpret_cast<const double*>(ctx->pstat), ctx->wsin,
                                                    ctx->arbar, ctx->hc, ctx->alev);
-    adj_level_apply_kernel<<<gc, 128, 0, ctx->st>>>(g, t0, reinterpret_cast<const double*>(ctx->pstat), ctx->wsin,
+    chain(adj_level_apply_kernel, gc, 128, 0, ctx->st, g, t0, reinterpret_cast<const double*>(ctx->pstat), ctx->wsin,
                                                     ctx->alev, ctx->hc, ctx->aybar);
     CK_LAUNCH("adjoint hydrostatic"); nl += 3;
     if(nf == ADJ_NF_MOIST && ctx->tape_sat_valid){     // the step's adjustment, before its RK4
-        adj_satadj_kernel<<<gc, 128, 0, ctx->st>>>(g, ctx->tPre, ctx->tX, reinterpret_cast<const double*>(ctx->pstat),
+        chain(adj_satadj_kernel, gc, 128, 0, ctx->st, g, ctx->tPre, ctx->tX, reinterpret_cast<const double*>(ctx->pstat),
                                                    reinterpret_cast<const double*>(ctx->forc) + (size_t)(ATURAN_RHO_MIX - ATURAN_NUE) * fs,
                                                    ctx->sc, ctx->aybar);
         CK_LAUNCH("adjoint saturation adjustment"); nl++;
@@ -1787,7 +1779,7 @@ int rk4_adjoint_impl(aturan_ctx* ctx, int nf, const double* const* ybar, const d
     CK(pack_doubles(g, nf, xbar, ctx->aybar, fs, false, ctx->st));
     if(pbar) CK(pack_doubles(g, 1, &pbar, ctx->apdbar, fs, false, ctx->st));
     if(heatbar){
-        adj_heat_reduce_kernel<<<(g.jm * g.km + 255) / 256, 256, 0, ctx->st>>>(g, ctx->ahacc, K.heat_scale, heatbar);
+        chain(adj_heat_reduce_kernel, (g.jm * g.km + 255) / 256, 256, 0, ctx->st, g, ctx->ahacc, K.heat_scale, heatbar);
         CK_LAUNCH("heating adjoint");
     }
     CK(cudaStreamSynchronize(ctx->st));
@@ -1848,9 +1840,9 @@ int aturan_pressure_adjoint(aturan_ctx* ctx, int kind, double omega, int max_swe
     CK(cudaMemsetAsync(B, 0, 3 * fs * 8, ctx->st));
     CK(pack_doubles(g, 1, &pbar, B, fs, true, ctx->st));
     // the boundary passes' adjoint, in reverse order
-    adj_pbc_p_kernel<<<(g.im * g.jm + 255) / 256, 256, 0, ctx->st>>>(g, B);
-    adj_pbc_t_kernel<<<dim3((g.km + 127) / 128, g.im), 128, 0, ctx->st>>>(g, B);
-    adj_pbc_r_kernel<<<dim3((g.km + 127) / 128, g.jm), 128, 0, ctx->st>>>(g, B);
+    chain(adj_pbc_p_kernel, (g.im * g.jm + 255) / 256, 256, 0, ctx->st, g, B);
+    chain(adj_pbc_t_kernel, dim3((g.km + 127) / 128, g.im), 128, 0, ctx->st, g, B);
+    chain(adj_pbc_r_kernel, dim3((g.km + 127) / 128, g.jm), 128, 0, ctx->st, g, B);
     sor_compat(ctx, B, true);               // zero-mean (it is, up to rounding, when p_dyn enters by differences)
     CK_LAUNCH("pressure adjoint: boundary passes");
     nl += 6;
@@ -1859,14 +1851,14 @@ int aturan_pressure_adjoint(aturan_ctx* ctx, int kind, double omega, int max_swe
     const int status = solve_fp64<true>(ctx, lam, B, omega, max_sweeps, tol, line, &s, &r, nl);
     if(status < 0) return status;
     const int ny = ((g.jm - 2) * (g.km - 1) + 255) / 256;
-    sor_ysum_kernel<<<ny, 256, 0, ctx->st>>>(g, lam, ctx->sor_part, 1);
-    sor_shift_finish_kernel<<<1, 256, 0, ctx->st>>>(ctx->sor_part, ny, ctx->sor_part + 2 * ny);
+    chain(sor_ysum_kernel, ny, 256, 0, ctx->st, g, lam, ctx->sor_part, 1);
+    chain(sor_shift_finish_kernel, 1, 256, 0, ctx->st, ctx->sor_part, ny, ctx->sor_part + 2 * ny);
     const double n_int = (double)(g.im - 2) * (g.jm - 2) * (g.km - 1);
     const double sum_w = (double)(g.im - 1) * (g.jm - 1) * (g.km - 1);   // sum of y_i y_j over the interior
-    adj_compat_mask_kernel<<<dim3((g.km - 1 + 127) / 128, g.jm - 2, g.im - 2), 128, 0, ctx->st>>>(
+    chain(adj_compat_mask_kernel, dim3((g.km - 1 + 127) / 128, g.jm - 2, g.im - 2), 128, 0, ctx->st, 
         g, lam, ctx->sor_part + 2 * ny, n_int / sum_w, ctx->tSrc, ctx->rbw, sbar);
     double* aub = ctx->ag0;
-    adj_div_kernel<<<dim3((g.km + 127) / 128, g.jm, g.im), 128, 0, ctx->st>>>(
+    chain(adj_div_kernel, dim3((g.km + 127) / 128, g.jm, g.im), 128, 0, ctx->st, 
         g, sbar, ctx->rbw, ctx->pc, ctx->p.rigid_lid, aub, aub + fs, aub + 2 * fs);
     CK_LAUNCH("pressure adjoint: source");
     nl += 4;

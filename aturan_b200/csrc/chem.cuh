@@ -124,6 +124,7 @@ __device__ __forceinline__ void nh4sh_bisect(double& lo, double& hi, double stop
 // ChemistryUran.h:140-177 per cell, :210-275 over every cell; counts formed / decomposed cells.
 template <typename S>
 __global__ void __launch_bounds__(128) nh4sh_eq_kernel(ChemArgs<S> a){
+    chain_wait();
     const Grid& g = a.g;
     const int k = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, i = blockIdx.z;
     int formed = 0, decomposed = 0;
@@ -218,6 +219,7 @@ __device__ __forceinline__ double chem_lapv(const Chem7& x, double rm, double rm
 // store (a store could alias a later load as far as the compiler knows).
 template <typename S>
 __global__ void __launch_bounds__(128) chem_diff_kernel(ChemArgs<S> a){
+    chain_wait();
     const Grid& g = a.g;
     const int k = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, i = blockIdx.z;
     if(k >= g.km) return;
@@ -288,6 +290,7 @@ __device__ __forceinline__ double chem_superbee(double r){
 // the Superbee correction fluxlim_nh4sh (FluxLimiter.h:89-186).
 template <typename S>
 __global__ void __launch_bounds__(128) chem_limit_kernel(ChemArgs<S> a){
+    chain_wait();
     const Grid& g = a.g;
     const ChemConst& c = a.c;
     const int k_first = c.per ? 0 : 1;

@@ -17,11 +17,12 @@ namespace aturan {
 ATURAN_DEFINE_LAUNCHERS(double, double)
 
 __global__ void scale_copy_f64_kernel(const double* in, double* out, size_t n, double coeff){
+    chain_wait();
     for(size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < n; t += (size_t)gridDim.x * blockDim.x)
         out[t] = coeff * in[t];
 }
 void launch_scale_copy_f64(const double* in, double* out, size_t n, double coeff, cudaStream_t st){
-    scale_copy_f64_kernel<<<148 * 8, 256, 0, st>>>(in, out, n, coeff);
+    chain(scale_copy_f64_kernel, 148 * 8, 256, 0, st, in, out, n, coeff);
 }
 
 void launch_mca_H(const double* cp_tab, double* H, cudaStream_t st){
@@ -33,13 +34,13 @@ int launch_filter_f64(const Grid& g, double* x, bool ai, bool aj, bool ak, doubl
 }
 
 void launch_pdyn_bcs(Grid g, double* P, cudaStream_t st){
-    pdyn_bc_r_kernel<<<dim3((g.km + 127) / 128, g.jm), 128, 0, st>>>(g, P);
-    pdyn_bc_t_kernel<<<dim3((g.km + 127) / 128, g.im), 128, 0, st>>>(g, P);
-    pdyn_bc_p_kernel<<<(g.im * g.jm + 255) / 256, 256, 0, st>>>(g, P);
+    chain(pdyn_bc_r_kernel, dim3((g.km + 127) / 128, g.jm), 128, 0, st, g, P);
+    chain(pdyn_bc_t_kernel, dim3((g.km + 127) / 128, g.im), 128, 0, st, g, P);
+    chain(pdyn_bc_p_kernel, (g.im * g.jm + 255) / 256, 256, 0, st, g, P);
 }
 
 void launch_rb_colour(Grid g, double* P, const double* src, const RBW* w, int colour, double omega, cudaStream_t st){
     const int half = g.km / 2;
-    rb_colour_kernel<<<dim3((half + 127) / 128, g.jm - 2, g.im - 2), 128, 0, st>>>(g, P, src, w, colour, omega);
+    chain(rb_colour_kernel, dim3((half + 127) / 128, g.jm - 2, g.im - 2), 128, 0, st, g, P, src, w, colour, omega);
 }
 }  // namespace aturan

@@ -48,19 +48,19 @@ void launch_scalars(const StageArgs<S, C>& a, dim3 grid2, cudaStream_t st){
         static const bool attr = (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, sm) == cudaSuccess)
                                  || (cudaGetLastError(), false);
         (void)attr;
-        kern<<<grid2, dim3(32, 4), sm, st>>>(a);
+        chain(kern, grid2, dim3(32, 4), sm, st, a);
     } else {
-        rk_scalar_pair_kernel<S, C, StageCfg<S>::PD, StageCfg<S>::MINB2><<<grid2, dim3(32, 4), 0, st>>>(a);
+        chain(rk_scalar_pair_kernel<S, C, StageCfg<S>::PD, StageCfg<S>::MINB2>, grid2, dim3(32, 4), 0, st, a);
     }
 }
 template <typename S, typename C>
 void launch_momentum(const StageArgs<S, C>& a, dim3 grid2, cudaStream_t st){
     if constexpr(StageCfg<S>::MP > 0){
-        rk_stage_pair_kernel<S, C, StageCfg<S>::MP><<<grid2, dim3(32, 4), 0, st>>>(a);
+        chain(rk_stage_pair_kernel<S, C, StageCfg<S>::MP>, grid2, dim3(32, 4), 0, st, a);
     } else {
         const Grid& g = a.g;
         const dim3 grid((g.km - 1 + 31) / 32, (g.jm - 2 + 3) / 4, g.im - 2);
-        rk_stage_kernel<S, C, StageCfg<S>::MINB1><<<grid, dim3(32, 4), 0, st>>>(a);
+        chain(rk_stage_kernel<S, C, StageCfg<S>::MINB1>, grid, dim3(32, 4), 0, st, a);
     }
 }
 // damp_wiggles (lib/Utils.cpp:224-317) on x along the axes selected, k then j then i; lo: the low
@@ -80,11 +80,11 @@ int launch_filter(const Grid& g, S* x, float* lo, bool ai, bool aj, bool ak, dou
         static const bool big = (cudaFuncSetAttribute(post_filter_k_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                       8192 * (int)sizeof(double)) == cudaSuccess) || (cudaGetLastError(), false);
         (void)big;
-        post_filter_k_kernel<S><<<(rows + R - 1) / R, dim3(32, R), sm, st>>>(g, x, lo, coeff, phi_periodic && g.km > 2, rows);
+        chain(post_filter_k_kernel<S>, (rows + R - 1) / R, dim3(32, R), sm, st, g, x, lo, coeff, phi_periodic && g.km > 2, rows);
         n++;
     }
-    if(aj){ post_filter_j_kernel<S><<<dim3(cols_k.x, g.im), 128, 0, st>>>(g, x, lo, coeff); n++; }
-    if(ai){ post_filter_i_kernel<S><<<dim3(cols_k.x, g.jm), 128, 0, st>>>(g, x, lo, coeff); n++; }
+    if(aj){ chain(post_filter_j_kernel<S>, dim3(cols_k.x, g.im), 128, 0, st, g, x, lo, coeff); n++; }
+    if(ai){ chain(post_filter_i_kernel<S>, dim3(cols_k.x, g.jm), 128, 0, st, g, x, lo, coeff); n++; }
     return n;
 }
 // damp_wiggles on x along all three axes in one fused pass into the scratch field y, copied back
@@ -93,7 +93,7 @@ template <typename S>
 int launch_filter3(const Grid& g, S* x, S* y, double strength, int phi_periodic, cudaStream_t st){
     const double coeff = strength * 0.25;                 // lib/Utils.cpp:232
     const dim3 grid((g.km + FT_K - 1) / FT_K, (g.jm + FT_J - 1) / FT_J, (g.im + FT_I - 1) / FT_I);
-    post_filter3_kernel<S><<<grid, dim3(32, 8), 0, st>>>(g, x, y, coeff, phi_periodic && g.km > 2);
+    chain(post_filter3_kernel<S>, grid, dim3(32, 8), 0, st, g, x, y, coeff, phi_periodic && g.km > 2);
     cudaMemcpyAsync(x, y, g.fstride * sizeof(S), cudaMemcpyDeviceToDevice, st);
     return 1;
 }
@@ -110,13 +110,13 @@ int launch_post_impl(const PostArgs<S>& a, const PostPlan& pl, S* t, float* tlo,
     if(pl.damp_t_vert != 0.0) filt(t, tlo, true, false, false, pl.damp_t_vert);
     if(pl.vel_shapiro != 0.0){ filt(a.u, nullptr, true, true, true, pl.vel_shapiro); filt(a.v, nullptr, true, true, true, pl.vel_shapiro);
                                filt(a.w, nullptr, true, true, true, pl.vel_shapiro); }
-    post_bc_radius_kernel<S><<<dim3(cols_k.x, g.jm, POST_NRAD), 128, 0, st>>>(a);
-    post_bc_theta_kernel<S><<<dim3(cols_k.x, g.im, POST_NTHZ + POST_NTHX), 128, 0, st>>>(a);
-    post_bc_phi_kernel<S><<<dim3((g.im * g.jm + 127) / 128, POST_NPHI), 128, 0, st>>>(a);
+    chain(post_bc_radius_kernel<S>, dim3(cols_k.x, g.jm, POST_NRAD), 128, 0, st, a);
+    chain(post_bc_theta_kernel<S>, dim3(cols_k.x, g.im, POST_NTHZ + POST_NTHX), 128, 0, st, a);
+    chain(post_bc_phi_kernel<S>, dim3((g.im * g.jm + 127) / 128, POST_NPHI), 128, 0, st, a);
     n += 3;
     if(pl.species_clamp){
-        post_clamp_kernel<S><<<dim3(pl.nb, POST_NSP), POST_CLAMP_NT, 0, st>>>(a, pl.part);
-        post_clamp_finish_kernel<<<POST_NSP, POST_CLAMP_NT, 0, st>>>(pl.part, pl.nb, pl.out);
+        chain(post_clamp_kernel<S>, dim3(pl.nb, POST_NSP), POST_CLAMP_NT, 0, st, a, pl.part);
+        chain(post_clamp_finish_kernel, POST_NSP, POST_CLAMP_NT, 0, st, pl.part, pl.nb, pl.out);
         n += 2;
     }
     return n;
@@ -128,14 +128,14 @@ int launch_chem_impl(const ChemArgs<S>& a, int what, cudaStream_t st){
     const Grid& g = a.g;
     const dim3 cols((g.km + 127) / 128, g.jm, g.im);
     int n = 0;
-    if(what & 1){ nh4sh_eq_kernel<S><<<cols, 128, 0, st>>>(a); n++; }
+    if(what & 1){ chain(nh4sh_eq_kernel<S>, cols, 128, 0, st, a); n++; }
     if(what & 2){
-        chem_diff_kernel<S><<<cols, 128, 0, st>>>(a);
+        chain(chem_diff_kernel<S>, cols, 128, 0, st, a);
         n++;
         S* f1[4] = {a.df_h2s, a.df_nh3, a.df_nh4sh, a.tmf};
         for(S* x : f1) n += launch_filter3<S>(g, x, a.scratch, 1.0, a.c.per, st);
         const int kn = g.km - 1 - (a.c.per ? 0 : 1);
-        chem_limit_kernel<S><<<dim3((kn + 127) / 128, g.jm - 2, g.im - 2), 128, 0, st>>>(a);
+        chain(chem_limit_kernel<S>, dim3((kn + 127) / 128, g.jm - 2, g.im - 2), 128, 0, st, a);
         n++;
         S* f2[4] = {a.mf_h2s, a.mf_nh3, a.mf_nh4sh, a.fl};
         for(S* x : f2) n += launch_filter3<S>(g, x, a.scratch, 1.0, a.c.per, st);
@@ -147,16 +147,16 @@ template <typename S>
 int launch_turb_impl(const TurbArgs<S>& a, cudaStream_t st){
     const Grid& g = a.g;
     const int kn = g.km - 1 - (a.c.per ? 0 : 1);
-    turb_sources_kernel<S><<<dim3((kn + 127) / 128, g.jm - 2, g.im - 2), 128, 0, st>>>(a);
-    turb_column_kernel<S><<<dim3((g.km + 127) / 128, g.jm), 128, 0, st>>>(a);
+    chain(turb_sources_kernel<S>, dim3((kn + 127) / 128, g.jm - 2, g.im - 2), 128, 0, st, a);
+    chain(turb_column_kernel<S>, dim3((g.km + 127) / 128, g.jm), 128, 0, st, a);
     const long nedge = (a.c.per ? (long)(g.im - 1) * (g.jm - 2) : 0) + (long)(g.jm - 2) * g.km + (long)g.im * g.km;
-    turb_edges_kernel<S><<<(unsigned)((nedge + 127) / 128), 128, 0, st>>>(a);
+    chain(turb_edges_kernel<S>, (unsigned)((nedge + 127) / 128), 128, 0, st, a);
     return 3;
 }
 // The precipitation (precip.cuh): one thread per column; returns the number of launches.
 template <typename S>
 int launch_precip_impl(const PrecipArgs<S>& a, cudaStream_t st){
-    precip_kernel<S><<<dim3((a.g.km + 31) / 32, a.g.jm), 128, 0, st>>>(a);
+    chain(precip_kernel<S>, dim3((a.g.km + 31) / 32, a.g.jm), 128, 0, st, a);
     return 1;
 }
 // The moist convective adjustment (mca.cuh); returns the launches, or -1 if a warp's columns do not fit
@@ -177,7 +177,7 @@ int launch_mca_grow(const McaArgs<S>& a, cudaStream_t st){
         return -1;
     }
     const long cols = (long)a.g.jm * a.g.km, blocks = (cols + 32 / G - 1) / (32 / G);
-    kern<<<(unsigned)std::min(blocks, (long)148 * per_sm), 32, sm, st>>>(a);
+    chain(kern, (unsigned)std::min(blocks, (long)148 * per_sm), 32, sm, st, a);
     return 1;
 }
 template <typename S>
@@ -186,12 +186,12 @@ int launch_mca_impl(const McaArgs<S>& a, cudaStream_t st){
     if(mca_col_bytes(g.im) > MCA_SMEM_MAX) return -1;
     const dim3 b((g.km + 127) / 128, g.jm);
     if(cudaMemsetAsync(a.next, 0, sizeof(unsigned), st) != cudaSuccess) return -1;
-    mca_prep_kernel<S><<<dim3(b.x, b.y, g.im), 128, 0, st>>>(a);
-    mca_test_kernel<S><<<dim3(b.x, b.y, g.im - 3), 128, 0, st>>>(a);
+    chain(mca_prep_kernel<S>, dim3(b.x, b.y, g.im), 128, 0, st, a);
+    chain(mca_test_kernel<S>, dim3(b.x, b.y, g.im - 3), 128, 0, st, a);
     const bool small = (long)g.jm * g.km < MCA_SMALL_COLUMNS || 8 * mca_col_bytes(g.im) > MCA_SMEM_MAX;
     const int n = small ? launch_mca_grow<S, 32>(a, st) : launch_mca_grow<S, 4>(a, st);
     if(n < 0) return -1;
-    mca_finish_kernel<S><<<dim3(b.x, b.y, g.im - 2), 128, 0, st>>>(a);
+    chain(mca_finish_kernel<S>, dim3(b.x, b.y, g.im - 2), 128, 0, st, a);
     return 4;
 }
 // Hydrostatic integral: threads per column (ROWS) and resident blocks per SM (MINB), measured.
@@ -204,7 +204,7 @@ static int gs_wave_as(Grid g, double* P, const double* src, const GSW* w, const 
     static const bool ok = cudaFuncSetAttribute(gs_wave_kernel<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                 GS_SMEM_MAX) == cudaSuccess || (cudaGetLastError(), false);
     if(!ok) return -1;
-    gs_wave_kernel<NC><<<pl.nb, gs_threads(pl), pl.smem, st>>>(g, P, src, w, pl, edge, ticket, base, tag, err);
+    chain(gs_wave_kernel<NC>, pl.nb, gs_threads(pl), pl.smem, st, g, P, src, w, pl, edge, ticket, base, tag, err);
     return cudaPeekAtLastError() == cudaSuccess ? 1 : -1;
 }
 static int gs_wave_nc(Grid g, double* P, const double* src, const GSW* w, const GsPlan& pl, GsEdge* edge, unsigned* ticket,
@@ -235,21 +235,21 @@ void launch_stage(const StageArgs<S, C>& a, cudaStream_t st, cudaStream_t side, 
 void launch_buoy(Grid g, const S* t, const S* ps, const double* wsin, HydroConst h, double* part_sum,     \
                  double* part_w, int nblk, double* ref, int exact, const BuoyScratch& bx, cudaStream_t st){ \
     if(exact){                                                                                            \
-        buoy_terms_kernel<S><<<dim3(bx.nbx, g.im), BX_CH, 0, st>>>(g, t, ps, wsin, h, bx.terms, bx.bpart, bx.nbx); \
-        buoy_predict_kernel<<<g.im, 256, 0, st>>>(bx.nbx, bx.bpart, bx.bexp);                               \
-        buoy_units_kernel<<<dim3((bx.nbx + 7) / 8, g.im), 256, 0, st>>>(g, bx.nbx, bx.terms, bx.bexp, bx.bunits);  \
-        buoy_serial_pass_kernel<<<g.im, 64, 0, st>>>(g, bx.nbx, bx.terms, bx.bpart, bx.bexp, bx.bunits, ref); \
+        chain(buoy_terms_kernel<S>, dim3(bx.nbx, g.im), BX_CH, 0, st, g, t, ps, wsin, h, bx.terms, bx.bpart, bx.nbx); \
+        chain(buoy_predict_kernel, g.im, 256, 0, st, bx.nbx, bx.bpart, bx.bexp);                               \
+        chain(buoy_units_kernel, dim3((bx.nbx + 7) / 8, g.im), 256, 0, st, g, bx.nbx, bx.terms, bx.bexp, bx.bunits);  \
+        chain(buoy_serial_pass_kernel, g.im, 64, 0, st, g, bx.nbx, bx.terms, bx.bpart, bx.bexp, bx.bunits, ref); \
         return;                                                                                           \
     }                                                                                                     \
-    buoy_partial_kernel<S><<<dim3(nblk, g.im), 256, 0, st>>>(g, t, ps, wsin, h, part_sum, part_w, nblk); \
-    buoy_finish_kernel<<<(g.im + 63) / 64, 64, 0, st>>>(g.im, nblk, part_sum, part_w, ref);               \
+    chain(buoy_partial_kernel<S>, dim3(nblk, g.im), 256, 0, st, g, t, ps, wsin, h, part_sum, part_w, nblk); \
+    chain(buoy_finish_kernel, (g.im + 63) / 64, 64, 0, st, g.im, nblk, part_sum, part_w, ref);               \
 }                                                                                                         \
 void launch_hydro(Grid g, const S* t, const S* ps, const S* v, const S* w, const double* ref,              \
                   const double* rm_i, const double* cor_j, const double* pbaro, const double* pb0,         \
                   double* pbf, double* ph, HydroConst h, int advance, cudaStream_t st){                    \
     const int n = g.jm * g.km;                                                                            \
     constexpr int R = HydCfg<S>::ROWS;                                                                    \
-    hydro_kernel<S, R, HydCfg<S>::MINB><<<(n + 31) / 32, dim3(32, R), 0, st>>>(g, t, ps, v, w, ref, rm_i,   \
+    chain(hydro_kernel<S, R, HydCfg<S>::MINB>, (n + 31) / 32, dim3(32, R), 0, st, g, t, ps, v, w, ref, rm_i,   \
                                                                   cor_j, pbaro, pb0, pbf, ph, h, advance); \
 }                                                                                                         \
 void launch_satadj(const SatArgs<S>& a, cudaStream_t st){                                                  \
@@ -257,14 +257,14 @@ void launch_satadj(const SatArgs<S>& a, cudaStream_t st){                       
     static const bool carve = (prefer_max_shared(satadj_kernel<S, NT>), true);                            \
     (void)carve;                                                                                          \
     dim3 grid((a.g.km + NT - 1) / NT, a.g.jm, a.g.im);                                                    \
-    satadj_kernel<S, NT><<<grid, NT, 0, st>>>(a);                                                         \
+    chain(satadj_kernel<S, NT>, grid, NT, 0, st, a);                                                         \
 }                                                                                                         \
 void launch_gs_pre(Grid g, S* au, S* av, S* aw, const S* ru, const S* rv, const S* rw, const double* P,    \
                    const GSW* w, PressConst c, double* incr, cudaStream_t st){                             \
-    gs_aux_bc_kernel<S><<<dim3((g.km - 1 + 127) / 128, g.jm - 2), 128, 0, st>>>(g, au, av, aw);           \
+    chain(gs_aux_bc_kernel<S>, dim3((g.km - 1 + 127) / 128, g.jm - 2), 128, 0, st, g, au, av, aw);           \
     const dim3 cells((g.km - 1 + 127) / 128, g.jm - 2, g.im - 2);                                         \
-    if(c.press_incr) gs_incr_kernel<S><<<cells, 128, 0, st>>>(g, ru, rv, rw, P, w, c, incr);              \
-    else gs_src_kernel<S><<<cells, 128, 0, st>>>(g, au, av, aw, w, c, incr);                              \
+    if(c.press_incr) chain(gs_incr_kernel<S>, cells, 128, 0, st, g, ru, rv, rw, P, w, c, incr);              \
+    else chain(gs_src_kernel<S>, cells, 128, 0, st, g, au, av, aw, w, c, incr);                              \
 }                                                                                                         \
 void launch_gs_plane(const S*, Grid g, double* P, const double* src, const GSW* w, int s, cudaStream_t st){ \
     const int n = (g.im - 2) * (g.jm - 2);                                                                \
@@ -276,10 +276,10 @@ int launch_gs_wave(const S*, Grid g, double* P, const double* src, const GSW* w,
 }                                                                                                         \
 void launch_rb_prep(Grid g, S* au, S* av, S* aw, S* ru, S* rv, S* rw, int rigid_lid,                       \
                     const RBW* w, PressConst c, double* src, cudaStream_t st){                             \
-    prep_rt_kernel<S><<<dim3((g.km - 1 + 127) / 128, (g.jm - 2) + (g.im - 2)), 128, 0, st>>>(             \
+    chain(prep_rt_kernel<S>, dim3((g.km - 1 + 127) / 128, (g.jm - 2) + (g.im - 2)), 128, 0, st,              \
         g, au, av, aw, ru, rv, rw, rigid_lid);                                                            \
-    prep_seam_kernel<S><<<(g.im * g.jm + 255) / 256, 256, 0, st>>>(g, au, av, aw, ru, rv, rw);            \
-    rb_src_kernel<S><<<dim3((g.km - 1 + 127) / 128, g.jm - 2, g.im - 2), 128, 0, st>>>(                   \
+    chain(prep_seam_kernel<S>, (g.im * g.jm + 255) / 256, 256, 0, st, g, au, av, aw, ru, rv, rw);            \
+    chain(rb_src_kernel<S>, dim3((g.km - 1 + 127) / 128, g.jm - 2, g.im - 2), 128, 0, st,                    \
         g, au, av, aw, w, c, src);                                                                        \
 }                                                                                                         \
 int launch_post(const PostArgs<S>& a, const PostPlan& pl, S* t, float* tlo, cudaStream_t st){              \

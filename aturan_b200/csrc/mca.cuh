@@ -216,6 +216,7 @@ static __device__ __forceinline__ bool mca_decide(const McaConst& A, double Tp, 
 // constants by reference, which otherwise copies the whole argument block to every thread's stack.
 template <typename S>
 __global__ void __launch_bounds__(128) mca_prep_kernel(const __grid_constant__ McaArgs<S> a){
+    chain_wait();
     const Grid& g = a.g;
     const McaConst& A = a.c;
     const int k = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, i = blockIdx.z;
@@ -251,6 +252,7 @@ __global__ void __launch_bounds__(128) mca_prep_kernel(const __grid_constant__ M
 // Thread (i, j, k): cell i + 1's own equilibrium and the test of the pair (i, i + 1), i = 1 .. im-3.
 template <typename S>
 __global__ void __launch_bounds__(128) mca_test_kernel(const __grid_constant__ McaArgs<S> a){
+    chain_wait();
     const Grid& g = a.g;
     const McaConst& A = a.c;
     const int k = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, i = 1 + blockIdx.z;
@@ -291,6 +293,7 @@ __host__ __device__ inline size_t mca_col_bytes(int im){ return (size_t)7 * im *
 // lanes through one call site.
 template <typename S, int G>
 __global__ void __launch_bounds__(32) mca_grow_kernel(const __grid_constant__ McaArgs<S> a){
+    chain_wait();
     extern __shared__ __align__(16) char mca_smem[];
     const Grid& g = a.g;
     const McaConst& A = a.c;
@@ -456,6 +459,7 @@ __global__ void __launch_bounds__(32) mca_grow_kernel(const __grid_constant__ Mc
 // Per mixed cell: its equilibrium at the final means and the write-back (:645-661, :800-849).
 template <typename S>
 __global__ void __launch_bounds__(128) mca_finish_kernel(const __grid_constant__ McaArgs<S> a){
+    chain_wait();
     const Grid& g = a.g;
     const McaConst& A = a.c;
     const int k = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, i = 1 + blockIdx.z;

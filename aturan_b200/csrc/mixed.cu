@@ -12,19 +12,22 @@ namespace aturan {
 ATURAN_DEFINE_LAUNCHERS(float, float)
 
 __global__ void f64_to_f32_kernel(const double* in, float* out, size_t n){
+    chain_wait();
     for(size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < n; t += (size_t)gridDim.x * blockDim.x)
         out[t] = (float)in[t];
 }
 __global__ void f32_to_f64_kernel(const float* in, double* out, size_t n){
+    chain_wait();
     for(size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < n; t += (size_t)gridDim.x * blockDim.x)
         out[t] = (double)in[t];
 }
 __global__ void scale_copy_f32_kernel(const float* in, float* out, size_t n, double coeff){
+    chain_wait();
     for(size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < n; t += (size_t)gridDim.x * blockDim.x)
         out[t] = (float)(coeff * (double)in[t]);
 }
 void launch_scale_copy_f32(const float* in, float* out, size_t n, double coeff, cudaStream_t st){
-    scale_copy_f32_kernel<<<148 * 8, 256, 0, st>>>(in, out, n, coeff);
+    chain(scale_copy_f32_kernel, 148 * 8, 256, 0, st, in, out, n, coeff);
 }
 
 // Contiguous [im][jm][km] FP64 <-> padded [im][jm][kp] fields, the layout change and (FP32 fields, the
@@ -37,6 +40,7 @@ void launch_scale_copy_f32(const float* in, float* out, size_t n, double coeff, 
 constexpr int PACK_NT = 256, PACK_U = 8;
 template <bool IN>
 __global__ void __launch_bounds__(PACK_NT) pack_kernel(const __grid_constant__ PackBatch p){
+    chain_wait();
     const int f = blockIdx.y;
     const unsigned base = blockIdx.x * (PACK_NT * PACK_U) + threadIdx.x;
     const double* const cin = p.flat[f];
@@ -82,21 +86,22 @@ void launch_pack(PackBatch& p, int nf, int km, int kp, size_t rows, bool in, cud
     p.div_s = 31 + s;                                          // exact for e < 2^31: m = ceil(2^(31 + s) / km) < 2^32
     p.div_m = (unsigned)(((1ull << (31 + s)) + km - 1) / km);
     const dim3 grid((p.n + PACK_NT * PACK_U - 1) / (PACK_NT * PACK_U), nf);
-    if(in) pack_kernel<true><<<grid, PACK_NT, 0, st>>>(p);
-    else   pack_kernel<false><<<grid, PACK_NT, 0, st>>>(p);
+    if(in) chain(pack_kernel<true>, grid, PACK_NT, 0, st, p);
+    else   chain(pack_kernel<false>, grid, PACK_NT, 0, st, p);
 }
 __global__ void scale_copy_pair_kernel(const float* hi, const float* lo, float* ohi, float* olo, size_t n, double coeff){
+    chain_wait();
     for(size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < n; t += (size_t)gridDim.x * blockDim.x)
         t_st(ohi, olo, t, coeff * t_ld(hi, lo, t));
 }
 void launch_scale_copy_pair(const float* hi, const float* lo, float* ohi, float* olo, size_t n, double coeff, cudaStream_t st){
-    scale_copy_pair_kernel<<<148 * 8, 256, 0, st>>>(hi, lo, ohi, olo, n, coeff);
+    chain(scale_copy_pair_kernel, 148 * 8, 256, 0, st, hi, lo, ohi, olo, n, coeff);
 }
 
 void launch_f64_to_f32(const double* in, float* out, size_t n, cudaStream_t st){
-    f64_to_f32_kernel<<<148 * 8, 256, 0, st>>>(in, out, n);
+    chain(f64_to_f32_kernel, 148 * 8, 256, 0, st, in, out, n);
 }
 void launch_f32_to_f64(const float* in, double* out, size_t n, cudaStream_t st){
-    f32_to_f64_kernel<<<148 * 8, 256, 0, st>>>(in, out, n);
+    chain(f32_to_f64_kernel, 148 * 8, 256, 0, st, in, out, n);
 }
 }  // namespace aturan

@@ -58,6 +58,7 @@ __device__ __forceinline__ double post_max0(double x){ return (0.0 < x) ? x : 0.
 // the mixed form's temperature pair when x is its t (common.cuh), else null.
 template <typename S>
 __global__ void __launch_bounds__(128) post_filter_k_kernel(Grid g, S* x, float* lo, double coeff, int seam, int rows){
+    chain_wait();
     extern __shared__ double sm[];
     const int r = blockIdx.x * blockDim.y + threadIdx.y;
     if(r >= rows) return;                          // a whole warp: only warp-level syncs below
@@ -90,6 +91,7 @@ __device__ __forceinline__ void post_walk(S* x0, float* lo0, size_t st, int n, d
 }
 template <typename S>
 __global__ void __launch_bounds__(128) post_filter_j_kernel(Grid g, S* x, float* lo, double coeff){
+    chain_wait();
     const int k = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y;
     if(k >= g.km) return;
     const size_t o = gidx(g, i, 0, k);
@@ -97,6 +99,7 @@ __global__ void __launch_bounds__(128) post_filter_j_kernel(Grid g, S* x, float*
 }
 template <typename S>
 __global__ void __launch_bounds__(128) post_filter_i_kernel(Grid g, S* x, float* lo, double coeff){
+    chain_wait();
     const int k = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y;
     if(k >= g.km) return;
     const size_t o = gidx(g, 0, j, k);
@@ -116,6 +119,7 @@ __global__ void __launch_bounds__(128) post_filter_i_kernel(Grid g, S* x, float*
 constexpr int FT_K = 32, FT_J = 8, FT_I = 4;
 template <typename S>
 __global__ void __launch_bounds__(256) post_filter3_kernel(Grid g, const S* __restrict__ x, S* __restrict__ y, double coeff, int seam){
+    chain_wait();
     __shared__ double YK[FT_I + 2][FT_J + 2][FT_K];
     __shared__ double YJ[FT_I + 2][FT_J][FT_K];
     const int tk = threadIdx.x, ty = threadIdx.y;              // 32 x 8
@@ -167,6 +171,7 @@ __global__ void __launch_bounds__(256) post_filter3_kernel(Grid g, const S* __re
 // reads and writes only its own field's column, so the fields run side by side.
 template <typename S>
 __global__ void __launch_bounds__(128) post_bc_radius_kernel(PostArgs<S> a){
+    chain_wait();
     const Grid& g = a.g;
     const int k = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, n = blockIdx.z;
     if(k >= g.km) return;
@@ -231,6 +236,7 @@ __global__ void __launch_bounds__(128) post_bc_radius_kernel(PostArgs<S> a){
 // 0..POST_NTHZ-1 are zeroed at the poles, the others extrapolated. ----
 template <typename S>
 __global__ void __launch_bounds__(128) post_bc_theta_kernel(PostArgs<S> a){
+    chain_wait();
     const Grid& g = a.g;
     const int k = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y, n = blockIdx.z;
     if(k >= g.km) return;
@@ -259,6 +265,7 @@ __global__ void __launch_bounds__(128) post_bc_theta_kernel(PostArgs<S> a){
 // of one field ----
 template <typename S>
 __global__ void __launch_bounds__(128) post_bc_phi_kernel(PostArgs<S> a){
+    chain_wait();
     const Grid& g = a.g;
     const int r = blockIdx.x * blockDim.x + threadIdx.x;      // row (i, j)
     if(r >= g.im * g.jm) return;
@@ -306,6 +313,7 @@ __device__ __forceinline__ void post_clamp_one(S* R, int k, int km, double x, do
 
 template <typename S>
 __global__ void __launch_bounds__(POST_CLAMP_NT) post_clamp_kernel(PostArgs<S> a, double* part){
+    chain_wait();
     using V = typename Vec16<S>::T;
     constexpr int NV = Vec16<S>::N, U = 4;
     const Grid& g = a.g;
@@ -346,6 +354,7 @@ __global__ void __launch_bounds__(POST_CLAMP_NT) post_clamp_kernel(PostArgs<S> a
 
 // One block per species: thread t adds partials t, t + 256, ... in order, then a fixed tree.
 static __global__ void __launch_bounds__(POST_CLAMP_NT) post_clamp_finish_kernel(const double* part, int nb, double* out){
+    chain_wait();
     const int n = blockIdx.x;
     double s = 0.0, c = 0.0;
     for(int b = threadIdx.x; b < nb; b += POST_CLAMP_NT){ s += part[2 * ((size_t)n * nb + b)]; c += part[2 * ((size_t)n * nb + b) + 1]; }

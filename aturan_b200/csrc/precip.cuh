@@ -45,6 +45,7 @@ __device__ __forceinline__ double pr_min(double a, double b){ return (b < a) ? b
 // Lane 4c + n of a warp: species n of the warp's column c (k = 8 * warp + c of the block's 32).
 template <typename S>
 __global__ void __launch_bounds__(128) precip_kernel(const __grid_constant__ PrecipArgs<S> a){
+    chain_wait();
     const Grid& g = a.g;
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31, n = lane & 3;

@@ -42,6 +42,7 @@ struct PressConst {
 // ---- PressureSolverUran.h:70-81: aux radial planes ----
 template <typename S>
 __global__ void gs_aux_bc_kernel(Grid g, S* au, S* av, S* aw){
+    chain_wait();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = 1 + blockIdx.y;
     if(k > g.km - 2 || j > g.jm - 2) return;
@@ -58,6 +59,7 @@ __global__ void gs_aux_bc_kernel(Grid g, S* au, S* av, S* aw){
 template <typename S>
 __global__ void gs_incr_kernel(Grid g, const S* ru, const S* rv, const S* rw, const double* P,
                                const GSW* w, PressConst c, double* incr){
+    chain_wait();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = 1 + blockIdx.y;
     const int i = 1 + blockIdx.z;
@@ -85,6 +87,7 @@ __global__ void gs_incr_kernel(Grid g, const S* ru, const S* rv, const S* rw, co
 // before the sweep (it reads no pressure).
 template <typename S>
 __global__ void gs_src_kernel(Grid g, const S* au, const S* av, const S* aw, const GSW* w, PressConst c, double* src){
+    chain_wait();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = 1 + blockIdx.y;
     const int i = 1 + blockIdx.z;
@@ -164,6 +167,7 @@ template <int NC>
 static __global__ void __launch_bounds__(768, 1) gs_wave_kernel(Grid g, double* P, const double* src, const GSW* w,
                                                                 GsPlan pl, GsEdge* edge, unsigned* ticket, unsigned base,
                                                                 unsigned tag, int* err){
+    chain_wait();
     extern __shared__ __align__(16) double gs_sm[];
     const int ipad = pl.ipad, B = pl.B;
     double* ringP = gs_sm;                                    // [B + 1][ipad][GSR]
@@ -414,6 +418,7 @@ static __global__ void __launch_bounds__(256) gs_hyperplane_kernel(Grid g, doubl
 // the polar rows over every (i,k), then the seam copy (PressureSolverUran.h:213-244,
 // PressureSolver.h:718-746) ----
 static __global__ void pdyn_bc_r_kernel(Grid g, double* P){
+    chain_wait();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y;
     if(k >= g.km) return;
@@ -421,6 +426,7 @@ static __global__ void pdyn_bc_r_kernel(Grid g, double* P){
     P[gidx(g, g.im - 1, j, k)] = C43 * P[gidx(g, g.im - 2, j, k)] - C13 * P[gidx(g, g.im - 3, j, k)];
 }
 static __global__ void pdyn_bc_t_kernel(Grid g, double* P){
+    chain_wait();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int i = blockIdx.y;
     if(k >= g.km) return;
@@ -428,6 +434,7 @@ static __global__ void pdyn_bc_t_kernel(Grid g, double* P){
     P[gidx(g, i, g.jm - 1, k)] = C43 * P[gidx(g, i, g.jm - 2, k)] - C13 * P[gidx(g, i, g.jm - 3, k)];
 }
 static __global__ void pdyn_bc_p_kernel(Grid g, double* P){
+    chain_wait();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if(c >= g.im * g.jm) return;
     const int i = c / g.jm, j = c - i * g.jm;
@@ -439,6 +446,7 @@ static __global__ void pdyn_bc_p_kernel(Grid g, double* P){
 // run in one launch; the seam copy follows. ----
 template <typename S>
 __global__ void prep_rt_kernel(Grid g, S* au, S* av, S* aw, S* ru, S* rv, S* rw, int rigid_lid){
+    chain_wait();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y;                       // y < jm-2: radial pass row j = y+1, else polar pass level
     if(k > g.km - 2) return;
@@ -471,6 +479,7 @@ __global__ void prep_rt_kernel(Grid g, S* au, S* av, S* aw, S* ru, S* rv, S* rw,
 }
 template <typename S>
 __global__ void prep_seam_kernel(Grid g, S* au, S* av, S* aw, S* ru, S* rv, S* rw){
+    chain_wait();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if(c >= g.im * g.jm) return;
     const int i = c / g.jm, j = c - i * g.jm;
@@ -482,6 +491,7 @@ __global__ void prep_seam_kernel(Grid g, S* au, S* av, S* aw, S* ru, S* rv, S* r
 template <typename S>
 __global__ void rb_src_kernel(Grid g, const S* au, const S* av, const S* aw, const RBW* w,
                               PressConst c, double* src){
+    chain_wait();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = 1 + blockIdx.y;
     const int i = 1 + blockIdx.z;
@@ -502,6 +512,7 @@ __global__ void rb_src_kernel(Grid g, const S* au, const S* av, const S* aw, con
 // reference's update p = (acc - src) / den; other omega over-relax it (RB_SOR). ----
 static __global__ void __launch_bounds__(256) rb_colour_kernel(Grid g, double* P, const double* src, const RBW* w,
                                                         int colour, double omega){
+    chain_wait();
     const int half = g.km / 2;                       // km-1 even: each row holds half of each colour
     const int k2 = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = 1 + blockIdx.y;

@@ -469,6 +469,7 @@ __device__ __forceinline__ void stage_update2(const StageArgs<S, C>& a, S* W, co
 // arithmetic per cell, in the same order, as rk_stage_kernel<..., 2, ...>.
 template <typename S, typename C, int PD, int MINB>
 __global__ void __launch_bounds__(128, MINB) rk_scalar_pair_kernel(const StageArgs<S, C> a){
+    chain_wait();
     const Grid& g = a.g;
     const int k = 2 * (blockIdx.x * 32 + threadIdx.x);
     const int j = 1 + blockIdx.y * 4 + threadIdx.y;
@@ -586,6 +587,7 @@ __device__ __forceinline__ void take_scalar2(ScalarIn2<C>& in, const AsyncSlot<S
 
 template <typename S, typename C, int D, int MINB>
 __global__ void __launch_bounds__(128, MINB) rk_scalar_async_kernel(const StageArgs<S, C> a){
+    chain_wait();
     extern __shared__ __align__(16) unsigned char ring_raw[];
     AsyncSlot<S>* ring = reinterpret_cast<AsyncSlot<S>*>(ring_raw);
     const Grid& g = a.g;
@@ -644,6 +646,7 @@ __global__ void __launch_bounds__(128, MINB) rk_scalar_async_kernel(const StageA
 // of the cell are issued before its first store. MINB is the launch bound on resident blocks per SM.
 template <typename S, typename C, int MINB>
 __global__ void __launch_bounds__(128, MINB) rk_stage_kernel(const StageArgs<S, C> a){
+    chain_wait();
     const Grid& g = a.g;
     const int k = blockIdx.x * 32 + threadIdx.x;
     const int j = 1 + blockIdx.y * 4 + threadIdx.y;
@@ -736,6 +739,7 @@ __device__ __forceinline__ void load_momentum2(MomIn<C>& A, MomIn<C>& B, const S
 // and store instructions and address arithmetic per cell. Grid as the scalar launch's.
 template <typename S, typename C, int MINB>
 __global__ void __launch_bounds__(128, MINB) rk_stage_pair_kernel(const StageArgs<S, C> a){
+    chain_wait();
     const Grid& g = a.g;
     const int k = 2 * (blockIdx.x * 32 + threadIdx.x);
     const int j = 1 + blockIdx.y * 4 + threadIdx.y;
@@ -784,6 +788,7 @@ __global__ void __launch_bounds__(128, MINB) rk_stage_pair_kernel(const StageArg
 template <typename S>
 __global__ void __launch_bounds__(256) buoy_partial_kernel(Grid g, const S* t, const S* ps, const double* wsin,
                                                            HydroConst h, double* part_sum, double* part_w, int nblk){
+    chain_wait();
     const int lev = blockIdx.y;
     const int ncell = g.jm * g.km;
     double s = 0.0, w = 0.0;
@@ -809,6 +814,7 @@ __global__ void __launch_bounds__(256) buoy_partial_kernel(Grid g, const S* t, c
 }
 
 static __global__ void buoy_finish_kernel(int im, int nblk, const double* part_sum, const double* part_w, double* ref){
+    chain_wait();
     const int lev = blockIdx.x * blockDim.x + threadIdx.x;
     if(lev >= im) return;
     double s = 0.0, w = 0.0;
@@ -842,6 +848,7 @@ constexpr int BX_CH = 256;
 template <typename S>
 __global__ void __launch_bounds__(BX_CH) buoy_terms_kernel(Grid g, const S* t, const S* ps, const double* wsin,
                                                           HydroConst h, double* terms, double* bpart, int nbx){
+    chain_wait();
     const int lev = blockIdx.y;
     const int ncell = g.jm * g.km;
     const int c = blockIdx.x * BX_CH + threadIdx.x;
@@ -877,6 +884,7 @@ __global__ void __launch_bounds__(BX_CH) buoy_terms_kernel(Grid g, const S* t, c
 // predicted binade of each chunk's running sum (INT_MIN: not predicted to stay in one binade, or
 // the chunk has a negative term), one block per level.
 static __global__ void __launch_bounds__(256) buoy_predict_kernel(int nbx, const double* bpart, int* bexp){
+    chain_wait();
     const int lev = blockIdx.x;
     const double* bp = bpart + 3 * (size_t)lev * nbx;
     int* E = bexp + 2 * (size_t)lev * nbx;
@@ -960,6 +968,7 @@ __device__ __forceinline__ int sum_binade(double s){
 constexpr int BX_PL = BX_CH / 32;
 static __global__ void __launch_bounds__(256) buoy_units_kernel(Grid g, int nbx, const double* terms, const int* bexp,
                                                                 long long* bunits){
+    chain_wait();
     const int lev = blockIdx.y, lane = threadIdx.x & 31, b = blockIdx.x * 8 + (threadIdx.x >> 5);
     if(b >= nbx) return;                                 // a whole warp
     const int ncell = g.jm * g.km;
@@ -1035,6 +1044,7 @@ __device__ __forceinline__ double sum_terms(double s, const double (&v)[BX_PL], 
 // 54 against 249 us (every chunk went term by term).
 static __global__ void __launch_bounds__(64) buoy_serial_pass_kernel(Grid g, int nbx, const double* terms, const double* bpart,
                                                                      const int* bexp, const long long* bunits, double* ref){
+    chain_wait();
     const int lev = blockIdx.x, lane = threadIdx.x & 31, c = threadIdx.x >> 5;
     const int ncell = g.jm * g.km;
     const double* x = terms + (size_t)lev * 2 * ncell + (size_t)c * ncell;
@@ -1102,6 +1112,7 @@ __global__ void __launch_bounds__(32 * ROWS, MINB) hydro_kernel(Grid g, const S*
                                                     const double* __restrict__ cor_j, const double* __restrict__ pbaro,
                                                     const double* __restrict__ pb0, double* __restrict__ pbf,
                                                     double* __restrict__ ph, HydroConst h, int advance){
+    chain_wait();
     constexpr int HYD_PER = HYD_CH / ROWS;
     static_assert(HYD_CH % ROWS == 0, "a chunk splits evenly over the rows");
     __shared__ double sm[HYD_CH][32], sb[HYD_CH][32];

@@ -96,6 +96,7 @@ __device__ __forceinline__ double qsat(const GasConst& G, bool ice, double rho_c
 // (measured: 6 % faster than half as many).
 template <typename S, int NT>
 __global__ void __launch_bounds__(NT, 1024 / NT) satadj_kernel(const SatArgs<S> a){
+    chain_wait();
     constexpr bool FAST = sizeof(S) == 4;            // the mixed form
     const Grid& g = a.g;
     const int k = blockIdx.x * blockDim.x + threadIdx.x;

@@ -127,6 +127,7 @@ __global__ void __launch_bounds__(256) sor_colsum_kernel(Grid g, const T* P, con
                                                          double* colR, double* part, int want_col, SorCheckArg chk,
                                                          float* r32 = nullptr, float* e32 = nullptr,
                                                          double* src_w = nullptr, const double* shift = nullptr){
+    chain_wait();
     if(!chk.first && chk.c->stop) return;
     const int N = g.km - 1;
     const int k = blockIdx.x * 32 + threadIdx.x;
@@ -236,6 +237,7 @@ __device__ __forceinline__ void gemm_stage(double (*t)[33], const MatRef& A, int
 __global__ void __launch_bounds__(256) sor_gemm_kernel(int M, int Nn, int K, MatRef A1, MatRef B1, MatRef A2,
                                                        MatRef B2, double scale, double* C1, double* C2,
                                                        long crs, long ccs, int kc, long cz){
+    chain_wait();
     __shared__ double sa1[32][33], sb1[32][33], sa2[32][33], sb2[32][33];   // sa[r][k], sb[c][k]
     const int r0 = blockIdx.y * 32, c0 = blockIdx.x * 32;
     const int kb = blockIdx.z * kc, ke = min(K, kb + kc);
@@ -289,6 +291,7 @@ __global__ void __launch_bounds__(256) sor_gemm_kernel(int M, int Nn, int K, Mat
 // 8 J (5 pm + 4) bytes.
 __global__ void __launch_bounds__(128) sor_tridiag_kernel(SorConst s, ModeLU lu, double* Ac, double* As, int pm,
                                                           int tr, int nsplit, long split_stride){
+    chain_wait();
     extern __shared__ double sm[];
     const int J = s.J, np = 2 * pm, ldr = np + 1, ldf = pm + 1;
     double* sd = sm;                                     // [J][ldr]
@@ -359,6 +362,7 @@ __global__ void __launch_bounds__(128) sor_tridiag_kernel(SorConst s, ModeLU lu,
 // (TR: y_i q, the trial functions of the transposed system's correction.)
 template <typename T, bool TR = false>
 __global__ void __launch_bounds__(128) sor_add_kernel(Grid g, const double* qbuf, T* P, int nsplit, long split_stride, const int* stop){
+    chain_wait();
     if(*stop) return;
     const int N = g.km - 1;
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -439,7 +443,7 @@ __global__ void __launch_bounds__(COLOUR_NT, COLOUR_MB) sor_colour_kernel(Grid g
         rr[q] = (double)__ldg(R + o[q]);
     }
     const bool done = *stop != 0;
-    cudaGridDependencySynchronize();
+    chain_wait();
     cudaTriggerProgrammaticLaunchCompletion();
     if(done) return;
     // where a neighbour is folded, the other one's address (TR, of weight 0: the cell's own), so that
@@ -496,6 +500,7 @@ template <> struct LineArith<float> { using A = double; static constexpr int LV 
 template <typename T, bool TR = false>
 __global__ void __launch_bounds__(256, 4) sor_line_kernel(Grid g, T* P, const T* R, const RBW* w, const double* la,
                                                        const double* lcf, const double* lidn, int colour, double omega, const int* stop){
+    chain_wait();
     if(*stop) return;
     using A = typename LineArith<T>::A;
     constexpr int LINE_LV = LineArith<T>::LV;
@@ -618,6 +623,7 @@ __global__ void __launch_bounds__(256, 4) sor_line_kernel(Grid g, T* P, const T*
 // Compatibility: per-block partial sums of y_i y_j src and y_i y_j over the interior (plain: of
 // src and 1, the transposed operator's left null vector being the constant).
 __global__ void __launch_bounds__(256) sor_ysum_kernel(Grid g, const double* src, double* part, int plain){
+    chain_wait();
     const int J = g.jm - 2, N = g.km - 1;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     double a = 0.0, b = 0.0;
@@ -642,6 +648,7 @@ __global__ void __launch_bounds__(256) sor_ysum_kernel(Grid g, const double* src
 
 // The shift = sum(y y src) / sum(y y) from the partials, in a fixed tree order (one block).
 __global__ void __launch_bounds__(256) sor_shift_finish_kernel(const double* part, int nblk, double* shift){
+    chain_wait();
     __shared__ double sa[256], sb[256];
     double a = 0.0, b = 0.0;
     for(int n = threadIdx.x; n < nblk; n += 256){ a += part[2 * n]; b += part[2 * n + 1]; }
@@ -656,6 +663,7 @@ __global__ void __launch_bounds__(256) sor_shift_finish_kernel(const double* par
 
 // src -= shift on the interior (the shift is read from device memory: no host round trip).
 __global__ void sor_shift_kernel(Grid g, double* src, const double* shift_p){
+    chain_wait();
     const double shift = *shift_p;
     const int J = g.jm - 2, N = g.km - 1;
     for(int c = blockIdx.x * blockDim.x + threadIdx.x; c < J * N; c += gridDim.x * blockDim.x){
@@ -667,6 +675,7 @@ __global__ void sor_shift_kernel(Grid g, double* src, const double* shift_p){
 // Mixed form: p += e over every cell (e is zero on the boundary rows and the seam column, which no
 // correction solve writes).
 __global__ void sor_axpy_kernel(size_t n, double* P, const float* e, const int* stop){
+    chain_wait();
     if(*stop) return;
     for(size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < n; t += (size_t)gridDim.x * blockDim.x)
         P[t] += (double)e[t];

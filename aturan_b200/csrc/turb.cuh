@@ -50,6 +50,7 @@ __device__ __forceinline__ double turb_blend(double inner, double outer, double 
 
 template <typename S>
 __global__ void __launch_bounds__(128) turb_sources_kernel(TurbArgs<S> a){
+    chain_wait();
     const Grid& g = a.g;
     const TurbConst& c = a.c;
     const int kf = c.per ? 0 : 1;
@@ -163,6 +164,7 @@ __global__ void __launch_bounds__(128) turb_sources_kernel(TurbArgs<S> a){
 // i = 0 (:414-419), clamp_nue on every level (:565-589).
 template <typename S>
 __global__ void __launch_bounds__(128) turb_column_kernel(TurbArgs<S> a){
+    chain_wait();
     const Grid& g = a.g;
     const TurbConst& c = a.c;
     const int k = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y;
@@ -206,6 +208,7 @@ __global__ void __launch_bounds__(128) turb_column_kernel(TurbArgs<S> a){
 // cells off the lid and pole rows, the lid row, the pole pairs.
 template <typename S>
 __global__ void __launch_bounds__(128) turb_edges_kernel(TurbArgs<S> a){
+    chain_wait();
     const Grid& g = a.g;
     const int im = g.im, jm = g.jm, km = g.km;
     const long nseam = a.c.per ? (long)(im - 1) * (jm - 2) : 0;
