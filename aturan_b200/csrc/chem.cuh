@@ -9,7 +9,7 @@
 // is two 7-point stencil passes over the interior (the diffusive tendencies and the thermal mass
 // flux; then the mass rates and the Superbee limiter) with the filters between and after them;
 // every pass streams a few planes of the state and is bound by HBM; each filter is one fused pass
-// over the three axes (post.cuh, post_filter3_kernel) and a copy back. Arithmetic is FP64 on the
+// over the three axes, four fields to a launch (post.cuh, post_filter3_kernel). Arithmetic is FP64 on the
 // stored values (FP32 storage in the mixed form is widened, computed in FP64 and rounded back), in
 // the reference's operand order; the per-level and per-latitude factors (radius, metric radius,
 // sin and cos of the colatitude) come from a host table made with the host's libm, so the FP64
@@ -45,7 +45,7 @@ struct ChemArgs {
     ChemTab tab;
     ChemConst c;
     unsigned long long* counts;                       // [formed, decomposed]
-    S* scratch;                                       // one field the fused filters write before the copy back
+    S* scratch;                                       // FT_N fields: the unfiltered values the fused filters read
 };
 
 __device__ __forceinline__ double chem_max(double a, double b){ return (a < b) ? b : a; }   // std::max
@@ -62,6 +62,12 @@ __device__ __forceinline__ double nh4sh_f(double x, double T0, double heat, doub
     const double T = T0 + heat * x, RT = 8314.46 * T;
     return (a - x) * (b - x) * RT * RT - nh4sh_kp(T);
 }
+// f(0) from K0 = K_p(T0): nh4sh_f's operations at x = 0 (heat 0 is 0, or NaN where heat is not
+// finite, and then so is f).
+__device__ __forceinline__ double nh4sh_f0(double T0, double heat, double a, double b, double K0){
+    const double T = T0 + heat * 0.0, RT = 8314.46 * T;
+    return (a - 0.0) * (b - 0.0) * RT * RT - K0;
+}
 __device__ __forceinline__ double nh4sh_df(double x, double T0, double heat, double a, double b, double& f){
     const double R = 8314.46, T = T0 + heat * x, RT = R * T;
     const double P = (a - x) * (b - x), K = exp10(14.82 - 4705.0 / T) * 101325.0 * 101325.0;
@@ -74,14 +80,18 @@ __device__ __forceinline__ double nh4sh_df(double x, double T0, double heat, dou
 // decreasing on the bracket (the formation heat moves T by millikelvin, against (a-x)(b-x) going
 // from ab to 0), so at a midpoint farther than `band` from the root r its sign is that of r - xm;
 // r comes from safeguarded Newton (a step that leaves the bracket is replaced by its midpoint),
-// and f itself is evaluated, as the reference does, at the ~4 midpoints inside the band instead
-// of at all ~50. The final bracket is checked with f at both ends; a bracket that does not hold
+// and f itself is evaluated, as the reference does, at the ~3 midpoints inside the band instead
+// of at all ~50 (41 x 181 x 361, FP64-bound: 960 us with 14 Newton steps a cell and the evaluations
+// at each lane's own step, 438 so). The final bracket is checked with f at both ends; a bracket that does not hold
 // (no single root, or Newton astray) is bisected again with f at every midpoint.
 __device__ __forceinline__ void nh4sh_bisect(double& lo, double& hi, double stop, double T0, double heat,
                                              double a, double b, double x0){
     const double lo0 = lo, hi0 = hi;
-    // Newton estimate of the root
-    double r = (x0 > lo && x0 < hi) ? x0 : 0.5 * (lo + hi);
+    // Newton estimate of the root. A step below stop / 4 is the last (its own error is its square),
+    // whether or not it stays inside the bracket: a root within an ulp of min(a, b) starts at hi, and
+    // bisecting back into the bracket would cost it ~25 steps. Asking for 1e-3 stop, below an ulp of
+    // r, kept it stepping to and fro (14 evaluations of f and f' per cell; 2 so).
+    double r = (x0 >= lo && x0 <= hi) ? x0 : 0.5 * (lo + hi);
     {
         double l = lo, h = hi;
         for(int it = 0; it < 60; it++){
@@ -89,19 +99,30 @@ __device__ __forceinline__ void nh4sh_bisect(double& lo, double& hi, double stop
             const double d = nh4sh_df(r, T0, heat, a, b, f);
             if(f > 0.0) l = r; else h = r;
             double rn = (d != 0.0 && isfinite(d)) ? r - f / d : 0.5 * (l + h);
-            if(!(rn > l && rn < h)) rn = 0.5 * (l + h);
-            const bool done = fabs(rn - r) <= 1.0e-3 * stop || h - l <= 1.0e-3 * stop;
+            const bool done = fabs(rn - r) <= 0.25 * stop || h - l <= 0.25 * stop;
+            if(!done && !(rn > l && rn < h)) rn = 0.5 * (l + h);
             r = rn;
             if(done) break;
         }
     }
-    // Newton leaves r within 1e-3 stop of the root; the computed sign of f is unreliable only within
-    // rounding of it (relative ~1e-16 of the bracket, stop being 1e-15 of it), so 8 stop is ample
-    const double band = 8.0 * stop;
+    // With u = a - x, v = b - x, the computed sign of f is unreliable within its rounding, ~8e-16 K_p,
+    // of the root: 8e-16 uv / (u + v) <= 8e-16 min(u, v) in x, below stop; r adds a quarter of that.
+    const double band = 4.0 * stop;
     // whether the sign of f at each end was evaluated (the initial ends' signs are the caller's
     // tests: f(lo) > 0, and f(hi) <= 0 at x = 0 or x = min(a, b), where f = -K_p) or inferred
     bool lo_ev = true, hi_ev = true;
-    for(int it = 0; it < 80; it++){
+    // first the midpoints outside the band, which need no f and take the same few instructions in
+    // every lane; the evaluations, from the first midpoint inside it on, then run side by side
+    // instead of each lane's at its own step
+    int it = 0;
+    for(; it < 80; it++){
+        const double xm = 0.5 * (lo + hi);
+        const bool pos = xm < r - band;
+        if(!pos && !(xm > r + band)) break;
+        if(pos){ lo = xm; lo_ev = false; } else { hi = xm; hi_ev = false; }
+        if(hi - lo <= stop){ it = 80; break; }
+    }
+    for(; it < 80; it++){
         const double xm = 0.5 * (lo + hi);
         bool pos, ev = false;
         if(xm < r - band) pos = true;
@@ -140,20 +161,23 @@ __global__ void __launch_bounds__(128) nh4sh_eq_kernel(ChemArgs<S> a){
             const double B = chem_max(0.0, hs) / c.m_h2s;
             const double Sx = chem_max(0.0, ns) / c.m_nh4sh;
             const double heat = c.L_f * c.m_nh4sh / (c.cp_mix * rho);
-            const double f0 = nh4sh_f(0.0, T0, heat, A, B);
+            const double K0 = nh4sh_kp(T0);
+            const double f0 = nh4sh_f0(T0, heat, A, B, K0);
             double lo = 0.0, hi = 0.0, x0 = 0.0;
             bool go = true;
             if(f0 > 0.0){
                 lo = 0.0; hi = chem_min(A, B);
-                // the fixed-T root (ChemistryUran.h:199-208's cancellation-free form) starts Newton
-                const double RT = 8314.46 * T0;
-                const double K = nh4sh_kp(T0) / (RT * RT), d = A - B;
-                x0 = (A * B > K) ? 2.0 * (A * B - K) / ((A + B) + sqrt(d * d + 4.0 * K)) : 0.0;
             } else if(Sx > 0.0){
                 if(nh4sh_f(-Sx, T0, heat, A, B) <= 0.0){ lo = hi = -Sx; }
-                else { lo = -Sx; hi = 0.0; x0 = -0.5 * Sx; }
+                else { lo = -Sx; hi = 0.0; }
             } else go = false;
             if(go){
+                if(hi > lo){
+                    // the fixed-T root (ChemistryUran.h:199-208's cancellation-free form) starts Newton
+                    const double RT = 8314.46 * T0;
+                    const double K = K0 / (RT * RT), d = A - B;
+                    x0 = 2.0 * (A * B - K) / ((A + B) + sqrt(d * d + 4.0 * K));
+                }
                 if(hi > lo) nh4sh_bisect(lo, hi, 1.0e-15 * chem_max(A, chem_max(B, Sx)), T0, heat, A, B, x0);
                 const double x = (f0 > 0.0) ? lo : hi;
                 if(x != 0.0){
@@ -229,7 +253,11 @@ __global__ void __launch_bounds__(128) chem_diff_kernel(ChemArgs<S> a){
     const double rho = (double)a.ps[q] * 1e5 / (c.R_mix * t0 * c.t_ref);
     const int k_first = c.per ? 0 : 1;
     if(i < 1 || i > g.im - 2 || j < 1 || j > g.jm - 2 || k < k_first || k > g.km - 2){
+        // what the filter reads off the interior: the fields as they are
+        const S f0 = a.df_h2s[q], f1 = a.df_nh3[q], f2 = a.df_nh4sh[q], f3 = a.tmf[q];
         a.rho_mix[q] = (S)rho;
+        S* const y = a.scratch + q;
+        y[0] = f0; y[g.fstride] = f1; y[2 * g.fstride] = f2; y[3 * g.fstride] = f3;
         return;
     }
     const size_t pl = (size_t)g.jm * g.kp, kp = (size_t)g.kp;
@@ -275,10 +303,8 @@ __global__ void __launch_bounds__(128) chem_diff_kernel(ChemArgs<S> a){
     const double dfn = c.D_nh3 * chem_lapv(N, rml, rmsl, cl, c);
     const double dfx = c.D_nh4sh * chem_lapv(X, rml, rmsl, cl, c);
     a.rho_mix[q] = (S)rho;
-    a.tmf[q] = (S)tmf;
-    a.df_h2s[q] = (S)dfh;
-    a.df_nh3[q] = (S)dfn;
-    a.df_nh4sh[q] = (S)dfx;
+    S* const y = a.scratch + q;
+    y[0] = (S)dfh; y[g.fstride] = (S)dfn; y[2 * g.fstride] = (S)dfx; y[3 * g.fstride] = (S)tmf;
 }
 
 // FluxLimiter.h:68-70
@@ -294,9 +320,16 @@ __global__ void __launch_bounds__(128) chem_limit_kernel(ChemArgs<S> a){
     const Grid& g = a.g;
     const ChemConst& c = a.c;
     const int k_first = c.per ? 0 : 1;
-    const int k = k_first + blockIdx.x * blockDim.x + threadIdx.x, j = 1 + blockIdx.y, i = 1 + blockIdx.z;
-    if(k > g.km - 2) return;
-    const size_t o = gidx(g, i, j, k), pl = (size_t)g.jm * g.kp, kp = (size_t)g.kp;
+    const int k = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, i = blockIdx.z;
+    if(k >= g.km) return;
+    const size_t o = gidx(g, i, j, k);
+    S* const y = a.scratch + o;
+    if(i < 1 || i > g.im - 2 || j < 1 || j > g.jm - 2 || k < k_first || k > g.km - 2){
+        const S f0 = a.mf_h2s[o], f1 = a.mf_nh3[o], f2 = a.mf_nh4sh[o], f3 = a.fl[o];
+        y[0] = f0; y[g.fstride] = f1; y[2 * g.fstride] = f2; y[3 * g.fstride] = f3;
+        return;
+    }
+    const size_t pl = (size_t)g.jm * g.kp, kp = (size_t)g.kp;
     // every load of the cell before its first store (a store could alias a later load as far as
     // the compiler knows); the far upwind values loaded whether or not the flow's sign reads them
     const double dh = (double)a.df_h2s[o], dn = (double)a.df_nh3[o], dx = (double)a.df_nh4sh[o];
@@ -333,10 +366,10 @@ __global__ void __launch_bounds__(128) chem_limit_kernel(ChemArgs<S> a){
         const double r = (ww >= 0.0) ? db / denom : (x_p2 - q_pp) / denom;
         corr += (1.0 - chem_superbee(r)) * fabs(ww) * inv_rmsinthe * (df - db) / (2.0 * c.dphi);
     }
-    a.mf_h2s[o] = (S)(0.0 + c.dsign * dh);
-    a.mf_nh3[o] = (S)(0.0 + c.dsign * dn);
-    a.mf_nh4sh[o] = (S)(0.0 + c.dsign * dx);
-    a.fl[o] = (S)corr;
+    y[0] = (S)(0.0 + c.dsign * dh);
+    y[g.fstride] = (S)(0.0 + c.dsign * dn);
+    y[2 * g.fstride] = (S)(0.0 + c.dsign * dx);
+    y[3 * g.fstride] = (S)corr;
 }
 
 }  // namespace aturan

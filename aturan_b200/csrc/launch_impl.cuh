@@ -87,14 +87,16 @@ int launch_filter(const Grid& g, S* x, float* lo, bool ai, bool aj, bool ak, dou
     if(ai){ chain(post_filter_i_kernel<S>, dim3(cols_k.x, g.jm), 128, 0, st, g, x, lo, coeff); n++; }
     return n;
 }
-// damp_wiggles on x along all three axes in one fused pass into the scratch field y, copied back
-// over x (post_filter3_kernel); returns the launches.
+// damp_wiggles along all three axes of FT_N fields in one fused pass, the fields' unfiltered values in
+// scratch (post_filter3_kernel); returns the launches.
 template <typename S>
-int launch_filter3(const Grid& g, S* x, S* y, double strength, int phi_periodic, cudaStream_t st){
+int launch_filter3(const Grid& g, const S* scratch, S* const (&y)[FT_N], double strength, int phi_periodic, cudaStream_t st){
     const double coeff = strength * 0.25;                 // lib/Utils.cpp:232
-    const dim3 grid((g.km + FT_K - 1) / FT_K, (g.jm + FT_J - 1) / FT_J, (g.im + FT_I - 1) / FT_I);
-    chain(post_filter3_kernel<S>, grid, dim3(32, 8), 0, st, g, x, y, coeff, phi_periodic && g.km > 2);
-    cudaMemcpyAsync(x, y, g.fstride * sizeof(S), cudaMemcpyDeviceToDevice, st);
+    const int ni = (g.im + FT_I - 1) / FT_I;
+    const dim3 grid((g.km + FT_K - 1) / FT_K, (g.jm + FT_J - 1) / FT_J, ni * FT_N);
+    Filter3<S> f;
+    for(int n = 0; n < FT_N; n++){ f.x[n] = scratch + n * g.fstride; f.y[n] = y[n]; }
+    chain(post_filter3_kernel<S>, grid, dim3(32, 8), 0, st, g, f, ni, coeff, phi_periodic && g.km > 2);
     return 1;
 }
 // The passes after RK4 in the reference's order; returns the number of launches.
@@ -132,13 +134,12 @@ int launch_chem_impl(const ChemArgs<S>& a, int what, cudaStream_t st){
     if(what & 2){
         chain(chem_diff_kernel<S>, cols, 128, 0, st, a);
         n++;
-        S* f1[4] = {a.df_h2s, a.df_nh3, a.df_nh4sh, a.tmf};
-        for(S* x : f1) n += launch_filter3<S>(g, x, a.scratch, 1.0, a.c.per, st);
-        const int kn = g.km - 1 - (a.c.per ? 0 : 1);
-        chain(chem_limit_kernel<S>, dim3((kn + 127) / 128, g.jm - 2, g.im - 2), 128, 0, st, a);
+        S* const f1[FT_N] = {a.df_h2s, a.df_nh3, a.df_nh4sh, a.tmf};
+        n += launch_filter3<S>(g, a.scratch, f1, 1.0, a.c.per, st);
+        chain(chem_limit_kernel<S>, cols, 128, 0, st, a);
         n++;
-        S* f2[4] = {a.mf_h2s, a.mf_nh3, a.mf_nh4sh, a.fl};
-        for(S* x : f2) n += launch_filter3<S>(g, x, a.scratch, 1.0, a.c.per, st);
+        S* const f2[FT_N] = {a.mf_h2s, a.mf_nh3, a.mf_nh4sh, a.fl};
+        n += launch_filter3<S>(g, a.scratch, f2, 1.0, a.c.per, st);
     }
     return n;
 }
