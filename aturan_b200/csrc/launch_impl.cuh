@@ -92,11 +92,11 @@ int launch_filter(const Grid& g, S* x, float* lo, bool ai, bool aj, bool ak, dou
 template <typename S>
 int launch_filter3(const Grid& g, const S* scratch, S* const (&y)[FT_N], double strength, int phi_periodic, cudaStream_t st){
     const double coeff = strength * 0.25;                 // lib/Utils.cpp:232
-    const int ni = (g.im + FT_I - 1) / FT_I;
+    const int li = filter3_levels(g.km, g.jm, g.im), ni = (g.im + li - 1) / li;
     const dim3 grid((g.km + FT_K - 1) / FT_K, (g.jm + FT_J - 1) / FT_J, ni * FT_N);
     Filter3<S> f;
     for(int n = 0; n < FT_N; n++){ f.x[n] = scratch + n * g.fstride; f.y[n] = y[n]; }
-    chain(post_filter3_kernel<S>, grid, dim3(32, 8), 0, st, g, f, ni, coeff, phi_periodic && g.km > 2);
+    chain(post_filter3_kernel<S>, grid, dim3(32, 8), 0, st, g, f, ni, li, coeff, phi_periodic && g.km > 2);
     return 1;
 }
 // The passes after RK4 in the reference's order; returns the number of launches.

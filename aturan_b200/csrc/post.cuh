@@ -120,54 +120,69 @@ __global__ void __launch_bounds__(128) post_filter_i_kernel(Grid g, S* x, float*
 // and eight copies back of 10 us at 41 x 181 x 361 (FP64).
 constexpr int FT_N = 4;
 template <typename S> struct Filter3 { const S* x[FT_N]; S* y[FT_N]; };
-constexpr int FT_K = 32, FT_J = 8, FT_I = 4;
+//
+// A block takes FT_K meridians x FT_J rows and walks up li levels: the k pass of a level's rows
+// (and the halo row on each side) goes to shared memory, double-buffered so that a level costs one
+// barrier; the thread of a column forms the j pass from it and keeps the last three levels' j passes
+// in registers for the i pass. The next level is in flight in registers meanwhile (two or four ahead
+// cost warps and were slower). Four FP64 fields of 41 x 181 x 361: 83 us with tiles of 4 levels staged
+// whole, 58 so (172 MB: 26 us).
+//
+// A block takes FT_K meridians x FT_J rows and walks up li levels: the k pass of a level's rows
+// (and the halo row on each side) goes to shared memory, double-buffered so that a level costs one
+// barrier; the thread of a column forms the j pass from it and keeps the last three levels' j passes
+// in registers for the i pass. The next level is in flight in registers meanwhile (two or four ahead
+// cost warps and were slower). Four FP64 fields of 41 x 181 x 361: 83 us with tiles of 4 levels staged
+// whole, 58 so (172 MB: 26 us).
+// li: 21 levels a block, so that the halo levels cost a tenth, while that still makes a wave of blocks
+// (58 us there, 66 with 7 levels), else 7 (21 x 37 x 73: 5.6 us against 10).
+constexpr int FT_K = 32, FT_J = 8;
+inline int filter3_levels(int km, int jm, int im){
+    const long cols = (long)((km + FT_K - 1) / FT_K) * ((jm + FT_J - 1) / FT_J) * FT_N;
+    return cols * ((im + 20) / 21) >= 148 * 8 ? 21 : 7;
+}
 template <typename S>
-__global__ void __launch_bounds__(256) post_filter3_kernel(Grid g, const __grid_constant__ Filter3<S> f, int ni, double coeff, int seam){
+__global__ void __launch_bounds__(FT_K * FT_J) post_filter3_kernel(Grid g, const __grid_constant__ Filter3<S> f, int ni, int li, double coeff, int seam){
     chain_wait();
+    __shared__ double YK[2][FT_J + 2][FT_K];
     const int n = blockIdx.z / ni;
     const S* __restrict__ x = f.x[n];
-    S* __restrict__ y = f.y[n];
-    __shared__ double YK[FT_I + 2][FT_J + 2][FT_K];
-    __shared__ double YJ[FT_I + 2][FT_J][FT_K];
     const int tk = threadIdx.x, ty = threadIdx.y;              // 32 x 8
-    const int k = blockIdx.x * FT_K + tk, j0 = blockIdx.y * FT_J, i0 = (blockIdx.z - n * ni) * FT_I;
+    const int k = blockIdx.x * FT_K + tk, j = blockIdx.y * FT_J + ty, i0 = (blockIdx.z - n * ni) * li;
     const int km = g.km;
-    const bool kin = k < km;
-    // the k pass's own index and neighbours (damp_wiggles, lib/Utils.cpp:250-265)
-    int kc = k, km1 = 0, kp1 = 0;
-    if(kin){
-        if(seam && k == km - 1) kc = 0;
-        km1 = seam ? (kc == 0 ? km - 2 : kc - 1) : (kc - 1 + km) % km;
-        kp1 = seam ? (kc == km - 2 ? 0 : kc + 1) : (kc + 1) % km;
-    }
-    for(int r = ty; r < (FT_I + 2) * (FT_J + 2); r += 8){
-        const int ii = r / (FT_J + 2), jj = r % (FT_J + 2);
-        const int i = min(max(i0 - 1 + ii, 0), g.im - 1), j = min(max(j0 - 1 + jj, 0), g.jm - 1);
-        double v = 0.0;
-        if(kin){
-            const S* row = x + gidx(g, i, j, 0);
-            const double c = (double)__ldg(row + kc);
-            v = c + coeff * ((double)__ldg(row + km1) - 2.0 * c + (double)__ldg(row + kp1));
-        }
-        YK[ii][jj][tk] = v;
-    }
-    __syncthreads();
-    for(int r = ty; r < (FT_I + 2) * FT_J; r += 8){
-        const int ii = r / FT_J, jj = r % FT_J;
-        const int j = j0 + jj;
-        // j - 1 and j + 1 clamped to the poles: the halo rows hold the clamped rows already
-        const double c = YK[ii][jj + 1][tk];
-        YJ[ii][jj][tk] = c + coeff * (YK[ii][jj][tk] - 2.0 * c + YK[ii][jj + 2][tk]);
-        (void)j;
-    }
-    __syncthreads();
-    if(!kin) return;
-    for(int r = ty; r < FT_I * FT_J; r += 8){
-        const int ii = r / FT_J, jj = r % FT_J;
-        const int i = i0 + ii, j = j0 + jj;
-        if(i >= g.im || j >= g.jm) continue;
-        const double c = YJ[ii + 1][jj][tk];
-        y[gidx(g, i, j, k)] = (S)(c + coeff * (YJ[ii][jj][tk] - 2.0 * c + YJ[ii + 2][jj][tk]));
+    const int i1 = min(i0 + li, g.im);
+    // the k pass's own index and neighbours (damp_wiggles, lib/Utils.cpp:250-265); off the row, those of
+    // its first cell
+    const int kq = k < km ? k : 0;
+    const int kc = seam && kq == km - 1 ? 0 : kq;
+    const int km1 = seam ? (kc == 0 ? km - 2 : kc - 1) : (kc - 1 + km) % km;
+    const int kp1 = seam ? (kc == km - 2 ? 0 : kc + 1) : (kc + 1) % km;
+    // this thread's rows: its own, and for the first and last row of the block the halo row
+    const size_t pl = (size_t)g.jm * g.kp;
+    const bool edge = ty == 0 || ty == FT_J - 1;
+    const S* const row = x + (size_t)min(j, g.jm - 1) * g.kp;
+    const S* const halo = x + (size_t)min(max(ty == 0 ? j - 1 : j + 1, 0), g.jm - 1) * g.kp;
+    const int slot = ty == 0 ? 0 : FT_J + 1;
+    S* const y = f.y[n] + (size_t)min(j, g.jm - 1) * g.kp + k;
+    const bool on = k < km && j < g.jm;
+    S c, w, e, hc = S(0), hw = S(0), he = S(0);
+    auto fetch = [&](int i){
+        const size_t o = (size_t)min(max(i, 0), g.im - 1) * pl;
+        c = __ldg(row + o + kc); w = __ldg(row + o + km1); e = __ldg(row + o + kp1);
+        if(edge){ hc = __ldg(halo + o + kc); hw = __ldg(halo + o + km1); he = __ldg(halo + o + kp1); }
+    };
+    double ym = 0.0, y0 = 0.0;                                  // j passes of levels i - 2 and i - 1
+    fetch(i0 - 1);
+    for(int i = i0 - 1; i <= i1; i++){
+        double (*b)[FT_K] = YK[i & 1];
+        b[ty + 1][tk] = (double)c + coeff * ((double)w - 2.0 * (double)c + (double)e);
+        if(edge) b[slot][tk] = (double)hc + coeff * ((double)hw - 2.0 * (double)hc + (double)he);
+        if(i < i1) fetch(i + 1);
+        __syncthreads();
+        const double v = b[ty + 1][tk];
+        const double yp = v + coeff * (b[ty][tk] - 2.0 * v + b[ty + 2][tk]);
+        if(on && i > i0) y[(size_t)(i - 1) * pl] = (S)(y0 + coeff * (ym - 2.0 * y0 + yp));
+        ym = y0; y0 = yp;
     }
 }
 
