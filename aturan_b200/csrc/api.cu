@@ -1018,12 +1018,14 @@ int run_mca(aturan_ctx* ctx){
     const size_t fs = g.fstride;
     for(int n = 0; n < MCA_NG; n++){
         const aturan_gas& s = p.gas[order[n]];
-        c.G[n] = McaGas{ s.ep, s.lv, s.ls, s.t_0, s.C, s.L0, s.R, s.del_alf, s.del_bet, s.C_i, s.L0_i, s.del_alf_i, s.del_bet_i };
+        c.G[n] = McaGas{ s.ep, s.lv, s.ls, s.t_0, s.C, s.L0, s.R, s.del_alf, s.del_bet, s.C_i, s.L0_i, s.del_alf_i, s.del_bet_i,
+                         1e-3 * s.R, 1.0 / (1e-3 * s.R), 1.0 / s.ep - 1.0 };
         for(int q = 0; q < 3; q++) a.sp[n][q] = X + (size_t)(fv[n] + q) * fs;
     }
     c.L_tr = p.nh4sh_sync ? 4705.0 * std::log(10.0) * 8314.46 / 51.1114 : 0.0;   // ChemistryUran.h:132
     c.t_ref = p.t_ref; c.grav = p.g; c.cp_mix = p.cp_mix; c.r_mix = p.r_mix; c.cp_h2 = p.cp_h2;
     c.r_h2 = p.r_h2; c.r_he = p.r_he; c.r_ch4 = p.r_ch4; c.cp_he = p.cp_he; c.cp_ch4 = p.cp_ch4;
+    c.k_h2 = p.r_h2 / p.r_mix; c.den = p.r_h2 + p.r_he + p.r_ch4; c.yden = 1.0 / c.den;
     c.hz = (float)(p.L_atm / (g.im - 1));                      // cUranusModel.h:1205-1208
     c.cp_dyn = p.cp_dyn; c.cp_mode = p.cp_h2_mode; c.cp_gas = p.cp_gas; c.local_rho = p.local_rho;
     c.cp_tab = ctx->cp_tab64; c.H_tab = ctx->mca_H;

@@ -13,6 +13,18 @@
 
 namespace aturan {
 
+// a / d by the reciprocal y = 1 / d that the caller holds (itself a division's result), correctly
+// rounded, the same bits as the division: after one correction the quotient is faithful, and the
+// remainder of a faithful quotient is exact, so the second rounds as the division does (Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor", 1990). For a, d and
+// a / d well inside the normal range (or a = +0); elsewhere the last bit, or an infinity, may differ.
+// Five multiply-adds without a branch, against ~10, a reciprocal estimate and a branch for a division.
+__host__ __device__ __forceinline__ double div_by(double a, double d, double y){
+    double q = a * y;
+    q = fma(fma(-q, d, a), y, q);
+    return fma(fma(-q, d, a), y, q);
+}
+
 // Launches of one stream follow one another by programmatic stream serialisation: the next kernel's
 // blocks are placed once the last block of the kernel before has exited, beside the flush of its
 // writes and the launch's own latency, and every kernel waits (chain_wait, its first statement) until

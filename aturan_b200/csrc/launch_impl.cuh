@@ -161,8 +161,8 @@ int launch_precip_impl(const PrecipArgs<S>& a, cudaStream_t st){
     return 1;
 }
 // The moist convective adjustment (mca.cuh); returns the launches, or -1 if a warp's columns do not fit
-// the shared memory. Lanes per column of the growth: 4 where there are columns enough to fill the chip
-// with them, else a warp per column.
+// the shared memory. Lanes per column of the growth: 4 where the columns fill the chip's resident warps
+// so, 8 below that (MCA_SMALL_COLUMNS).
 template <typename S, int G>
 int launch_mca_grow(const McaArgs<S>& a, cudaStream_t st){
     const size_t sm = (32 / G) * mca_col_bytes(a.g.im);
@@ -189,8 +189,8 @@ int launch_mca_impl(const McaArgs<S>& a, cudaStream_t st){
     if(cudaMemsetAsync(a.next, 0, sizeof(unsigned), st) != cudaSuccess) return -1;
     chain(mca_prep_kernel<S>, dim3(b.x, b.y, g.im), 128, 0, st, a);
     chain(mca_test_kernel<S>, dim3(b.x, b.y, g.im - 3), 128, 0, st, a);
-    const bool small = (long)g.jm * g.km < MCA_SMALL_COLUMNS || 8 * mca_col_bytes(g.im) > MCA_SMEM_MAX;
-    const int n = small ? launch_mca_grow<S, 32>(a, st) : launch_mca_grow<S, 4>(a, st);
+    const bool small = (long)g.jm * g.km <= MCA_SMALL_COLUMNS;
+    const int n = small ? launch_mca_grow<S, 8>(a, st) : launch_mca_grow<S, 4>(a, st);
     if(n < 0) return -1;
     chain(mca_finish_kernel<S>, dim3(b.x, b.y, g.im - 2), 128, 0, st, a);
     return 4;

@@ -27,12 +27,15 @@
 //     and the upper cell's equilibrium are one solve and their difference is exactly zero; a segment's
 //     edge pairs were tested with the values they still have; every other pair was stable at the start
 //     and has not changed. The reference's further sweep finds nothing, so there is none here.
-// Measured at 41x181x361 (mixed, synthetic state): 6.0 ms -- prep 0.14, tests 1.38, growth 3.95, finish
-// 0.55 -- against 44.7 ms for one warp per column running the whole sweep with every settle and a
-// verifying sweep; 1.28 against 8.1 ms at 37x83x167, 0.63 against 0.88 ms at 21x37x73. Same bits.
+// Measured at 41x181x361 (mixed, synthetic state): 4.3 ms -- prep 0.14, tests 1.18, growth 2.50, finish
+// 0.46 -- against 44.7 ms for one warp per column running the whole sweep with every settle and a
+// verifying sweep; 1.1 against 8.1 ms at 37x83x167, 0.34 against 0.88 ms at 21x37x73. Same bits. (With
+// every quotient a division and a column's whole state in shared memory: 6.0, 1.28 and 0.63 ms.)
 // The growth chain is what is left of the serial part: bound by the latency of its solves on small
-// grids, by FP64 issue on large ones. G = 4 keeps three of four lanes busy; with few columns a warp
-// per column (G = 32) has the shorter chain, as no other column of the warp delays it.
+// grids, by that and FP64 issue on large ones, so it takes as many warps an SM as 128 registers allow
+// (16; the state in shared memory left room for 12). G = 4 keeps three of four lanes busy; few columns
+// take more lanes each, the chain of a warp being that of its slowest column (21x37x73: 0.25 ms with
+// G = 8, 0.30 with 4, 0.27 with 16, 0.45 with 32; 37x83x167: 0.61 with 4, 1.07 with 8).
 // Every loop is bounded: 60 regula-falsi steps, 30 Newton steps of the enthalpy inverse, and a
 // segment grows by at least one level per step within the column.
 #pragma once
@@ -41,15 +44,17 @@
 namespace aturan {
 
 constexpr int MCA_NG = 4;
-// Below as many columns as the chip holds groups of warps for, a warp per column in the growth.
+// Up to as many columns as the chip holds at once with 8 lanes each in the growth (16 warps an SM).
 constexpr long MCA_SMALL_COLUMNS = 148 * 64;
 constexpr double CP_T_LO_D = 5.0, CP_T_HI_D = 1500.0, CP_DT_D = 0.5;   // CpH2.h:13
 
-struct McaGas { double ep, lv, ls, t_0, C, L0, R, del_alf, del_bet, C_i, L0_i, del_alf_i, del_bet_i; };
+struct McaGas { double ep, lv, ls, t_0, C, L0, R, del_alf, del_bet, C_i, L0_i, del_alf_i, del_bet_i;
+                double rd, yrd, tv; };   // 1e-3 R and its reciprocal; 1 / ep - 1
 
 struct McaConst {
     McaGas G[MCA_NG];                // H2O, NH3, H2S, CH4
     double L_tr, t_ref, grav, cp_mix, r_mix, cp_h2, r_h2, r_he, r_ch4, cp_he, cp_ch4;
+    double k_h2, den, yden;          // r_h2 / r_mix; r_h2 + r_he + r_ch4 and its reciprocal
     float hz;                        // level spacing [km] as the model stores it (float)
     int cp_dyn, cp_mode, cp_gas, local_rho;
     const double *cp_tab, *H_tab;    // H2 cp table and its running integral (CpH2.h:66-75)
@@ -97,14 +102,14 @@ static __device__ double mca_enth_h2(const McaConst& A, double T){
 static __device__ double mca_cp(const McaConst& A, double T){
     if(!A.cp_dyn) return A.cp_mix;
     const double ch = mca_cp_h2(A, T);
-    if(A.cp_gas) return (A.r_h2 * ch + A.r_he * A.cp_he + A.r_ch4 * A.cp_ch4) / (A.r_h2 + A.r_he + A.r_ch4);
-    return A.cp_mix + (A.r_h2 / A.r_mix) * (ch - A.cp_h2);
+    if(A.cp_gas) return div_by(A.r_h2 * ch + A.r_he * A.cp_he + A.r_ch4 * A.cp_ch4, A.den, A.yden);
+    return A.cp_mix + A.k_h2 * (ch - A.cp_h2);
 }
 static __device__ double mca_enth(const McaConst& A, double T){
     if(!A.cp_dyn) return A.cp_mix * T;
     const double hh = mca_enth_h2(A, T);
-    if(A.cp_gas) return (A.r_h2 * hh + (A.r_he * A.cp_he + A.r_ch4 * A.cp_ch4) * T) / (A.r_h2 + A.r_he + A.r_ch4);
-    return (A.cp_mix - (A.r_h2 / A.r_mix) * A.cp_h2) * T + (A.r_h2 / A.r_mix) * hh;
+    if(A.cp_gas) return div_by(A.r_h2 * hh + (A.r_he * A.cp_he + A.r_ch4 * A.cp_ch4) * T, A.den, A.yden);
+    return (A.cp_mix - A.k_h2 * A.cp_h2) * T + A.k_h2 * hh;
 }
 static __device__ __noinline__ double mca_enth_inv(const McaConst& A, double h, double T0){
     if(!A.cp_dyn) return h / A.cp_mix;
@@ -119,13 +124,16 @@ static __device__ __noinline__ double mca_enth_inv(const McaConst& A, double h, 
 }
 
 // ATPhys.h:49-53 (the saturation pressure) and ConvectiveAdjustment.h:437-453 without the phase
-// split; lg = log(T), the same value for every gas at one T, formed once by the caller
-__device__ __forceinline__ double mca_qsat(const McaGas& s, double T, double lg, double pr){
+// split; lg = log(T), yT = 1 / T, ypr = 1 / pr, the same for every gas at one T, formed once by the
+// caller. Its three quotients a gas, and those by constants elsewhere, are products with reciprocals
+// (div_by): the divisions' bits, and the four gases' chains run side by side instead of one after the
+// other's branches. Where E leaves the normal range q is 0 or far below what qt holds.
+__device__ __forceinline__ double mca_qsat(const McaGas& s, double T, double lg, double yT, double pr, double ypr){
     const bool liq = T >= s.t_0;                     // one expression for both sets: the lanes' phases differ
     const double C = liq ? s.C : s.C_i, L0 = liq ? s.L0 : s.L0_i;
     const double al = liq ? s.del_alf : s.del_alf_i, be = liq ? s.del_bet : s.del_bet_i;
-    const double E = exp(C + (-L0 / T + al * lg + be * T) / (1e-3 * s.R));
-    const double q = s.ep * E / pr;
+    const double E = exp(C + div_by(div_by(-L0, T, yT) + al * lg + be * T, s.rd, s.yrd));
+    const double q = div_by(s.ep * E, pr, ypr);
     return isfinite(q) ? q : 0.0;
 }
 __device__ __forceinline__ double mca_lat(const McaGas& s, double T){ return T >= s.t_0 ? s.lv : s.ls; }
@@ -148,15 +156,16 @@ static __device__ __forceinline__ bool mca_equil(const McaConst& A, double hL, c
     if(!(T_lo > 0.0) || !(pr > 0.0)) return false;
     double a = T_lo, b = T_lo, fa = 0.0, fb = 0.0, x = T_lo;
     int side = 0;
+    const double ypr = 1.0 / pr;
     for(int n = -2; ; n++){                          // n = it of the reference's loop from 0 on
         const double e = mca_enth(A, x);
-        const double lg = log(x);
+        const double lg = log(x), yT = 1.0 / x;
         double f = e + A.grav * z - hL;
         double d[MCA_NG];
         bool any = false;
 #pragma unroll
         for(int g = 0; g < MCA_NG; g++){
-            const double q = mca_qsat(A.G[g], x, lg, pr);
+            const double q = mca_qsat(A.G[g], x, lg, yT, pr, ypr);
             any |= qt[g] > q;
             d[g] = mca_mx(0.0, qt[g] - q);
             f -= mca_lat(A.G[g], x) * d[g];
@@ -196,7 +205,7 @@ __device__ __forceinline__ double mca_trE(const McaConst& A, double qr){ double 
 static __device__ __forceinline__ double mca_tv(const McaConst& A, double TT, const double (&v_)[MCA_NG], const double (&cnd)[MCA_NG], double qr){
     double f = 1.0;
 #pragma unroll
-    for(int g = 0; g < MCA_NG; g++){ f += v_[g] * (1.0 / A.G[g].ep - 1.0); f -= cnd[g]; }
+    for(int g = 0; g < MCA_NG; g++){ f += v_[g] * A.G[g].tv; f -= cnd[g]; }
     f -= qr;
     return TT * f;
 }
@@ -251,7 +260,7 @@ __global__ void __launch_bounds__(128) mca_prep_kernel(const __grid_constant__ M
 
 // Thread (i, j, k): cell i + 1's own equilibrium and the test of the pair (i, i + 1), i = 1 .. im-3.
 template <typename S>
-__global__ void __launch_bounds__(128) mca_test_kernel(const __grid_constant__ McaArgs<S> a){
+__global__ void __launch_bounds__(128, 4) mca_test_kernel(const __grid_constant__ McaArgs<S> a){
     chain_wait();
     const Grid& g = a.g;
     const McaConst& A = a.c;
@@ -283,33 +292,38 @@ __global__ void __launch_bounds__(128) mca_test_kernel(const __grid_constant__ M
     a.flag[o] = okp && okb && mca_decide(A, Tp, pc, qa, qra, Tb, ec, qb, qrb) ? 1 : 0;
 }
 
-// One column's state in its group's slice of shared memory, and its bytes (7 doubles and a flag per level).
-struct McaCol { double *hL, *qr, *w, *qt; unsigned char* flag; };
+// What a group keeps of its column in shared memory, and its bytes: the weights and a flag per level.
+struct McaCol { double* w; unsigned char* flag; };
 constexpr size_t MCA_SMEM_MAX = 227 * 1024;
-__host__ __device__ inline size_t mca_col_bytes(int im){ return (size_t)7 * im * sizeof(double) + ((size_t)im + 7) / 8 * 8; }
+__host__ __device__ inline size_t mca_col_bytes(int im){ return (size_t)im * sizeof(double) + ((size_t)im + 7) / 8 * 8; }
 
-// Blocks of one warp, G lanes per column. A group walks up its column from unstable pair to unstable
+// Blocks of one warp, G (4 to 16) lanes per column. A group walks up its column from unstable pair to unstable
 // pair; every turn of the loop is one growth step of each group's segment, its three solves on three
-// lanes through one call site.
+// lanes through one call site. The cells of a growing segment all hold its means, which stay in
+// registers until it has stopped growing and go to the work fields then; of the other cells a step
+// reads only those next to the segment, from the work fields. So shared memory holds no more than the
+// weights (the column's whole state there left room for 12 warps an SM, and the solves are latency).
 template <typename S, int G>
-__global__ void __launch_bounds__(32) mca_grow_kernel(const __grid_constant__ McaArgs<S> a){
+__global__ void __launch_bounds__(32, 16) mca_grow_kernel(const __grid_constant__ McaArgs<S> a){
     chain_wait();
     extern __shared__ __align__(16) char mca_smem[];
     const Grid& g = a.g;
     const McaConst& A = a.c;
     const int lane = threadIdx.x, gl = lane % G, grp = lane / G;
-    const unsigned gm = G == 32 ? 0xffffffffu : ((1u << (G & 31)) - 1u) << (grp * G);
+    const unsigned gm = ((1u << G) - 1u) << (grp * G);
     const int im = g.im, i0 = 1, i1 = im - 2;
     const unsigned ncol = (unsigned)(g.jm * g.km);
     const size_t pl = (size_t)g.jm * g.kp;
     McaCol C;
-    {
-        double* d = reinterpret_cast<double*>(mca_smem + grp * mca_col_bytes(im));
-        C.hL = d; C.qr = d + im; C.w = d + 2 * im; C.qt = d + 3 * im;
-        C.flag = reinterpret_cast<unsigned char*>(d + 7 * im);
-    }
+    C.w = reinterpret_cast<double*>(mca_smem + grp * mca_col_bytes(im));
+    C.flag = reinterpret_cast<unsigned char*>(C.w + im);
+    // the sums a lane forms: lane 0 w and w hL; lanes 1, 2 two of w qt; lane 3 w qr
+    const double* const x0 = gl == 0 ? a.hL : gl == 1 ? a.qt[0] : gl == 2 ? a.qt[2] : a.qr;
+    const double* const x1 = gl == 1 ? a.qt[1] : gl == 2 ? a.qt[3] : x0;
     bool active = false, done = false, have = false;     // a segment is growing; no column left; a column is loaded
     int i = i0, lo = 0, hi = 0;
+    int ml = 0, mh = -1;                                 // the cells that hold the means s0, s1 of the last step
+    double s0 = 0.0, s1 = 0.0;
     size_t o0 = 0;
     while(true){
         // a group without a segment: the next unstable pair of its column, or of the next column
@@ -337,12 +351,6 @@ __global__ void __launch_bounds__(32) mca_grow_kernel(const __grid_constant__ Mc
                     for(int q = i0 + gl; q <= i1; q += G) a.flag[o0 + (size_t)q * pl] = 0;
                     continue;
                 }
-                for(int q = i0 + gl; q <= i1; q += G){
-                    const size_t o = o0 + (size_t)q * pl;
-                    C.hL[q] = a.hL[o]; C.qr[q] = a.qr[o];
-#pragma unroll
-                    for(int s = 0; s < MCA_NG; s++) C.qt[q * MCA_NG + s] = a.qt[s][o];
-                }
                 __syncwarp(gm);
                 have = true;
                 i = i0;
@@ -354,51 +362,39 @@ __global__ void __launch_bounds__(32) mca_grow_kernel(const __grid_constant__ Mc
                 if(m){ i += __ffs(m >> (grp * G)) - 1; break; }
                 i += G;
             }
-            if(i < i1){ active = true; lo = i; hi = i + 1; break; }
-            // the column is finished: mixed cells' means and flags back
-            for(int q = i0 + gl; q <= i1; q += G){
-                const size_t o = o0 + (size_t)q * pl;
-                const bool mixed = C.flag[q] == 2;
-                a.flag[o] = mixed ? 2 : 0;
-                if(mixed){
-                    a.hL[o] = C.hL[q]; a.qr[o] = C.qr[q];
-#pragma unroll
-                    for(int s = 0; s < MCA_NG; s++) a.qt[s][o] = C.qt[q * MCA_NG + s];
-                }
-            }
+            if(i < i1){ active = true; lo = i; hi = i + 1; ml = hi; mh = lo; break; }
+            // the column is finished: its flags back
+            for(int q = i0 + gl; q <= i1; q += G) a.flag[o0 + (size_t)q * pl] = C.flag[q] == 2 ? 2 : 0;
             __syncwarp(gm);
             have = false;
         }
         if(__all_sync(0xffffffffu, done)) return;
         bool task = false, below = false, above = false;
-        int ca = lo, lb = lo;
+        int lb = lo;
+        double m_h = 0.0, m_r = 0.0, m_q[MCA_NG] = {0.0, 0.0, 0.0, 0.0};
+        double h = 0.0, qr = 0.0, x[MCA_NG];             // the cell this lane solves for
         if(active){
-            // the segment's mass-weighted means, each sum by one lane in the reference's order
-            double sw = 0.0, s0 = 0.0, s1 = 0.0;
+            // the segment's mass-weighted means, each sum by one lane in the reference's order: the cell it
+            // grew to below, the cells that hold the last means, the cell it grew to above
             if(gl < 4){
-                // lane 0: w and w hL; lanes 1, 2: two of w qt; lane 3: w qr
-                const double* x0 = gl == 0 ? C.hL : (gl == 3 ? C.qr : C.qt + (gl - 1) * 2);
-                const int st = gl == 0 || gl == 3 ? 1 : MCA_NG;
-                const double* x1 = st == 1 ? x0 : x0 + 1;
+                const size_t ol = o0 + (size_t)lo * pl, oh = o0 + (size_t)hi * pl;
+                const double b0 = lo < ml ? x0[ol] : 0.0, b1 = lo < ml ? x1[ol] : 0.0;
+                const double e0 = hi > mh ? x0[oh] : 0.0, e1 = hi > mh ? x1[oh] : 0.0;
+                double sw = 0.0, t0 = 0.0, t1 = 0.0;
                 for(int q = lo; q <= hi; q++){
                     const double w = C.w[q];
+                    const double v0 = q < ml ? b0 : q > mh ? e0 : s0, v1 = q < ml ? b1 : q > mh ? e1 : s1;
                     sw += w;
-                    s0 += w * x0[q * st];
-                    s1 += w * x1[q * st];
+                    t0 += w * v0;
+                    t1 += w * v1;
                 }
-                s0 = s0 / sw;
-                s1 = s1 / sw;
+                s0 = t0 / sw;
+                s1 = t1 / sw;
             }
-            const double m_h = __shfl_sync(gm, s0, 0, G), m_r = __shfl_sync(gm, s0, 3, G);
-            double m_q[MCA_NG];
+            ml = lo; mh = hi;
+            m_h = __shfl_sync(gm, s0, 0, G); m_r = __shfl_sync(gm, s0, 3, G);
             m_q[0] = __shfl_sync(gm, s0, 1, G); m_q[1] = __shfl_sync(gm, s1, 1, G);
             m_q[2] = __shfl_sync(gm, s0, 2, G); m_q[3] = __shfl_sync(gm, s1, 2, G);
-            for(int q = lo + gl; q <= hi; q += G){
-                C.hL[q] = m_h; C.qr[q] = m_r; C.flag[q] = 2;
-#pragma unroll
-                for(int s = 0; s < MCA_NG; s++) C.qt[q * MCA_NG + s] = m_q[s];
-            }
-            __syncwarp(gm);
             // a settle of one of its cells would fail (mca_equil): the column keeps its state
             const double h_top = m_h + mca_trE(A, m_r) - A.grav * mca_z(A, hi);
             if(A.cp_dyn ? !isfinite(h_top) : !(h_top / A.cp_mix > 0.0)){
@@ -407,51 +403,65 @@ __global__ void __launch_bounds__(32) mca_grow_kernel(const __grid_constant__ Mc
                 active = have = false;
             } else {
                 below = lo > i0; above = hi < i1;
+                h = m_h; qr = m_r;
+#pragma unroll
+                for(int s = 0; s < MCA_NG; s++) x[s] = m_q[s];
                 if(gl == 0){ task = below; }                                       // cell lo's own equilibrium
-                else if(gl == 1){ task = below; ca = lo - 1; }                     // cell lo - 1 lifted to lo
-                else if(gl == 2){ task = above; ca = hi; lb = hi + 1; }            // the mixed cell hi lifted to hi + 1
+                else if(gl == 1){                                                  // cell lo - 1 lifted to lo
+                    task = below;
+                    if(below){
+                        const size_t oa = o0 + (size_t)(lo - 1) * pl;
+                        h = a.hL[oa]; qr = a.qr[oa];
+#pragma unroll
+                        for(int s = 0; s < MCA_NG; s++) x[s] = a.qt[s][oa];
+                    }
+                }
+                else if(gl == 2){ task = above; lb = hi + 1; }                     // the mixed cell hi lifted to hi + 1
             }
         }
         __syncwarp();
         double T = 0.0, c[MCA_NG] = {0.0, 0.0, 0.0, 0.0};
         bool ok = false;
-        if(task){
-            double x[MCA_NG];
-#pragma unroll
-            for(int s = 0; s < MCA_NG; s++) x[s] = C.qt[ca * MCA_NG + s];
-            ok = mca_equil(A, C.hL[ca] + mca_trE(A, C.qr[ca]), x, (double)a.ps[o0 + (size_t)lb * pl], mca_z(A, lb), T, c);
-        }
+        if(task) ok = mca_equil(A, h + mca_trE(A, qr), x, (double)a.ps[o0 + (size_t)lb * pl], mca_z(A, lb), T, c);
         __syncwarp();
         if(!active) continue;
         // lane 0 tests the pair (lo - 1, lo) with lane 1's parcel and its own equilibrium, lane 2 the pair
         // (hi, hi + 1) with its parcel and cell hi + 1's equilibrium of the start
-        double Tp = __shfl_sync(gm, T, 1, G), pc[MCA_NG];
+        double Tp = __shfl_sync(gm, T, 1, G), pc[MCA_NG], qa[MCA_NG], qb[MCA_NG];
 #pragma unroll
-        for(int s = 0; s < MCA_NG; s++) pc[s] = __shfl_sync(gm, c[s], 1, G);
+        for(int s = 0; s < MCA_NG; s++){ pc[s] = __shfl_sync(gm, c[s], 1, G); qa[s] = __shfl_sync(gm, x[s], 1, G); }
+        double ra = __shfl_sync(gm, qr, 1, G), rb = m_r;
         bool okp = __shfl_sync(gm, (int)ok, 1, G) != 0;
         bool grow = false;
         if((gl == 0 && below) || (gl == 2 && above)){
-            double Tb = T, ec[MCA_NG], qa[MCA_NG], qb[MCA_NG];
-            int ia = lo - 1, ib = lo;
+            double Tb = T, ec[MCA_NG];
             bool okb = ok;
 #pragma unroll
-            for(int s = 0; s < MCA_NG; s++) ec[s] = c[s];
+            for(int s = 0; s < MCA_NG; s++){ ec[s] = c[s]; qb[s] = m_q[s]; }
             if(gl == 2){
-                ia = hi; ib = hi + 1;
-                const size_t ob = o0 + (size_t)ib * pl;
+                const size_t ob = o0 + (size_t)(hi + 1) * pl;
                 Tp = T; okp = ok;
                 Tb = a.Teq[ob]; okb = Tb > 0.0;
+                ra = m_r; rb = a.qr[ob];
 #pragma unroll
-                for(int s = 0; s < MCA_NG; s++){ pc[s] = c[s]; ec[s] = a.ceq[s][ob]; }
+                for(int s = 0; s < MCA_NG; s++){ pc[s] = c[s]; ec[s] = a.ceq[s][ob]; qa[s] = m_q[s]; qb[s] = a.qt[s][ob]; }
             }
-#pragma unroll
-            for(int s = 0; s < MCA_NG; s++){ qa[s] = C.qt[ia * MCA_NG + s]; qb[s] = C.qt[ib * MCA_NG + s]; }
-            grow = okp && okb && mca_decide(A, Tp, pc, qa, C.qr[ia], Tb, ec, qb, C.qr[ib]);
+            grow = okp && okb && mca_decide(A, Tp, pc, qa, ra, Tb, ec, qb, rb);
         }
         const unsigned gr = __ballot_sync(gm, grow) >> (grp * G);
         if(gr & 1u) lo--;
         if(gr & 4u) hi++;
-        if(!(gr & 5u)){ active = false; i = hi + 1; }
+        if(!(gr & 5u)){
+            // the segment has stopped growing: its cells hold the means
+            for(int q = lo + gl; q <= hi; q += G){
+                const size_t o = o0 + (size_t)q * pl;
+                C.flag[q] = 2;
+                a.hL[o] = m_h; a.qr[o] = m_r;
+#pragma unroll
+                for(int s = 0; s < MCA_NG; s++) a.qt[s][o] = m_q[s];
+            }
+            active = false; i = hi + 1;
+        }
         __syncwarp(gm);
     }
 }
