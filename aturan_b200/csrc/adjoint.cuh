@@ -99,11 +99,13 @@ struct AdjRow { double r2, t1, t2, t3, t4, p1, p3, p4, p5; };
 // D and one multiply-add per field. The rows' weights are formed once per block in shared memory.
 // Bound by the latency of its ~85 loads per cell at the registers they hold, then by their L2 traffic: it
 // reads the stage input, kbar, g0, nue, p_dyn and pe, and updates ybar, phbar and pdbar, ~33 words per cell
-// dry and ~105 moist. At 41x91x181: 103 us a stage dry and 254 moist at 4 and 3 resident blocks (128 and
-// 168 registers; 115 and 283 at one block more or less), against 108 and 374 as the two or three launches
-// that wrote and gathered the contributions.
+// dry and ~105 moist. Whatever a cell adds to is loaded before its first store: a load behind a store
+// waits for it, and ten of them in a row cost more than the sums. At 41x91x181: 77 us a stage dry and 180
+// moist at 4 and 2 resident blocks (128 and 255 registers; 79 at 3 and 87 at 5 blocks dry, 203 at 3 moist),
+// against 108 and 374 as the two or three launches that wrote and gathered the contributions, and 103 and
+// 254 with those loads between the stores.
 template <int NF>
-__global__ void __launch_bounds__(128, NF == ADJ_NF ? 4 : 3) adj_stage_kernel(const __grid_constant__ AdjArgs a){
+__global__ void __launch_bounds__(128, NF == ADJ_NF ? 4 : 2) adj_stage_kernel(const __grid_constant__ AdjArgs a){
     chain_wait();
     const Grid& g = a.g;
     const RhsConst<double>& K = a.k;
@@ -248,41 +250,60 @@ __global__ void __launch_bounds__(128, NF == ADJ_NF ? 4 : 3) adj_stage_kernel(co
 #pragma unroll
             for(int d = 0; d < 6; d++) W[d] = bw[d] + isc * cd[d];
             const double W0 = b0 - isc * lap;
+            // every load of the gas's three fields before the first store, which the compiler must assume
+            // to alias them
+            double an[3][6], aq[3], yb[3], g0[3];
+            R7<double> rq[3];
 #pragma unroll
             for(int n = 0; n < 3; n++){
                 const size_t f = (size_t)(ADJ_NF + 3 * gi + n) * fs;
                 const double* kq = a.kbar + f;
-                double an[6];
 #pragma unroll
-                for(int d = 0; d < 6; d++) an[d] = __ldg(kq + on[d]);
-                const R7<double> rq = stencil(ADJ_NF + 3 * gi + n);
-                const double aq = __ldg(kq + o), yb = a.ybar[f + o], g0 = __ldg(a.g0 + f + o);
-                double x = aq * W0;
+                for(int d = 0; d < 6; d++) an[n][d] = __ldg(kq + on[d]);
+                rq[n] = stencil(ADJ_NF + 3 * gi + n);
+                aq[n] = __ldg(kq + o); yb[n] = a.ybar[f + o]; g0[n] = __ldg(a.g0 + f + o);
+            }
+#pragma unroll
+            for(int n = 0; n < 3; n++){
+                const size_t f = (size_t)(ADJ_NF + 3 * gi + n) * fs;
+                double x = aq[n] * W0;
                 // inv_rm and inv_rs are 0 off the interior, where aq is 0 too
-                xu -= aq * ((rq.rp - rq.rm) * K.inv_2dr);
-                xv -= aq * inv_rm * ((rq.tp - rq.tm) * K.inv_2dthe);
-                xw -= aq * inv_rs * ((rq.pe - rq.pw) * K.inv_2dphi);
+                xu -= aq[n] * ((rq[n].rp - rq[n].rm) * K.inv_2dr);
+                xv -= aq[n] * inv_rm * ((rq[n].tp - rq[n].tm) * K.inv_2dthe);
+                xw -= aq[n] * inv_rs * ((rq[n].pe - rq[n].pw) * K.inv_2dphi);
 #pragma unroll
-                for(int d = 0; d < 6; d++) x += an[d] * W[d];
-                a.ybar[f + o] = yb + x;
-                if(in && a.Xprev) a.kbar_out[f + o] = a.w_prev * g0 + a.c_prev * x;
+                for(int d = 0; d < 6; d++) x += an[n][d] * W[d];
+                a.ybar[f + o] = yb[n] + x;
+                if(in && a.Xprev) a.kbar_out[f + o] = a.w_prev * g0[n] + a.c_prev * x;
             }
         }
     }
+    // what the cell adds to, all of it loaded before the first store
     const double x[ADJ_NF] = {xt, xu, xv, xw};
+    const bool prev = in && a.Xprev;
+    double yb[ADJ_NF], gb[ADJ_NF] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
-    for(int q = 0; q < ADJ_NF; q++) a.ybar[(size_t)q * fs + o] += x[q];
-    a.phbar[o] += h;
-    a.pdbar[o] += pd;
-    if(in && a.Xprev){
+    for(int q = 0; q < ADJ_NF; q++) yb[q] = a.ybar[(size_t)q * fs + o];
+    const double ph = a.phbar[o], pdb = a.pdbar[o];
+    double tp = 0.0;
+    if(prev){
+#pragma unroll
+        for(int q = 0; q < ADJ_NF; q++) gb[q] = __ldg(a.g0 + (size_t)q * fs + o);
+        tp = __ldg(a.Xprev + o);
+    }
+#pragma unroll
+    for(int q = 0; q < ADJ_NF; q++) a.ybar[(size_t)q * fs + o] = yb[q] + x[q];
+    a.phbar[o] = ph + h;
+    a.pdbar[o] = pdb + pd;
+    if(prev){
         double kt = 0.0;
 #pragma unroll
         for(int q = 0; q < ADJ_NF; q++){
-            const double kn = a.w_prev * a.g0[(size_t)q * fs + o] + a.c_prev * x[q];
+            const double kn = a.w_prev * gb[q] + a.c_prev * x[q];
             if(q == 0) kt = kn;
             a.kbar_out[(size_t)q * fs + o] = kn;
         }
-        a.pe_out[o] = K.ce_sp * adj_cpf(K, a.cp_tab, ld(a.Xprev + o)) * kt;
+        a.pe_out[o] = K.ce_sp * adj_cpf(K, a.cp_tab, tp) * kt;
     }
 }
 
@@ -475,7 +496,7 @@ __global__ void __launch_bounds__(128) adj_satadj_kernel(Grid g, const double* p
 // The final update's adjoint: g = ybar' (times 0 where T' was clamped), ybar = g, kbar_3 =
 // dt/6 w_3 g on the interior. ybar_in is the caller's adjoint of the step's output; pe of stage 3 is
 // formed from its input t3, nt from nue.
-__global__ void adj_init_kernel(Grid g, const double* ybar_in, const double* t_out, double t_min, double t_max,
+__global__ void __launch_bounds__(128) adj_init_kernel(Grid g, const double* ybar_in, const double* t_out, double t_min, double t_max,
                                 double w3, double* g0, double* ybar, double* kbar, double* phbar, double* pdbar, int nf,
                                 RhsConst<double> K, const double* cp_tab, const double* t3, const double* nue, double* pe, double* nt){
     chain_wait();
@@ -486,18 +507,25 @@ __global__ void adj_init_kernel(Grid g, const double* ybar_in, const double* t_o
     const size_t fs = g.fstride;
     const size_t o = gidx(g, i, j, k);
     const bool interior = i >= 1 && i <= g.im - 2 && j >= 1 && j <= g.jm - 2 && k <= g.km - 2;
-#pragma unroll 4
-    for(int q = 0; q < nf; q++){
-        double v = ybar_in[q * fs + o];
-        if(q == 0 && interior && !(t_out[o] > t_min && t_out[o] < t_max)) v = 0.0;
-        g0[q * fs + o] = interior ? v : 0.0;
-        ybar[q * fs + o] = v;
-        kbar[q * fs + o] = interior ? w3 * v : 0.0;
-        if(q == 0) pe[o] = interior ? K.ce_sp * adj_cpf(K, cp_tab, t3[o]) * (w3 * v) : 0.0;
+    const double to = t_out[o], t3o = t3[o], nu = nue[o];
+    // four fields at a time (nf is 4 or 16), their loads before their stores
+    for(int q0 = 0; q0 < nf; q0 += 4){
+        double v[4];
+#pragma unroll
+        for(int c = 0; c < 4; c++) v[c] = ybar_in[(q0 + c) * fs + o];
+        if(q0 == 0 && interior && !(to > t_min && to < t_max)) v[0] = 0.0;
+#pragma unroll
+        for(int c = 0; c < 4; c++){
+            const size_t p = (q0 + c) * fs + o;
+            g0[p] = interior ? v[c] : 0.0;
+            ybar[p] = v[c];
+            kbar[p] = interior ? w3 * v[c] : 0.0;
+        }
+        if(q0 == 0) pe[o] = interior ? K.ce_sp * adj_cpf(K, cp_tab, t3o) * (w3 * v[0]) : 0.0;
     }
     phbar[o] = 0.0;
     pdbar[o] = 0.0;
-    nt[o] = adj_nue(K, nue[o]);
+    nt[o] = adj_nue(K, nu);
 }
 
 // Hydrostatic integral's adjoint, per column (RungeKutta_Uran_Turb.cpp:62-177): p_hydro(i) =
