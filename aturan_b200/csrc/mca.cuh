@@ -243,15 +243,21 @@ __global__ void __launch_bounds__(128) mca_prep_kernel(const __grid_constant__ M
     if(!(w > 0.0)) ok = false;
     if(!ok){ a.w[o] = 0.0; return; }                 // its column is left alone: nothing else is read
     double h = mca_enth(A, T) + A.grav * z;
+    // every load before the first store, which the compiler must assume to alias them
+    double x[MCA_NG][3];
+#pragma unroll
+    for(int q = 0; q < MCA_NG; q++)
+#pragma unroll
+        for(int n = 0; n < 3; n++) x[q][n] = (double)a.sp[q][n][o];
+    const double qr = (double)a.nh4sh[o] / rho;
 #pragma unroll
     for(int q = 0; q < MCA_NG; q++){
-        const double qv = mca_mx(0.0, (double)a.sp[q][0][o]) / rho;
-        const double qc = mca_mx(0.0, (double)a.sp[q][1][o]) / rho;
-        const double qi = mca_mx(0.0, (double)a.sp[q][2][o]) / rho;
+        const double qv = mca_mx(0.0, x[q][0]) / rho;
+        const double qc = mca_mx(0.0, x[q][1]) / rho;
+        const double qi = mca_mx(0.0, x[q][2]) / rho;
         a.qt[q][o] = qv + qc + qi;
         h -= A.G[q].lv * qc + A.G[q].ls * qi;
     }
-    const double qr = (double)a.nh4sh[o] / rho;
     h -= A.L_tr * qr;
     a.qr[o] = qr;
     a.hL[o] = h;
