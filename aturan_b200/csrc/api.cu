@@ -586,23 +586,23 @@ int sor_correct(aturan_ctx* ctx, T* P){
     const Grid g = ctx->g;
     const SorConst& c = ctx->sorc;
     const MatRef R{ctx->sor_colR, c.N, 1};                        // (jj, k)
+    const int* stop = &ctx->sor_check->stop;
     const long sz_ac = (long)(c.NM + 1) * c.J, sz_q = (long)c.J * c.N;
     const int kcf = ((c.N + SOR_KSPLIT - 1) / SOR_KSPLIT + 31) / 32 * 32;
     const dim3 gf((c.NM + 1 + 31) / 32, (c.J + 31) / 32, SOR_KSPLIT);
     chain(sor_gemm_kernel, gf, 256, 0, ctx->st, c.J, c.NM + 1, c.N, R, MatRef{ctx->sor_ctT, c.NM + 1, 1},
                                             R, MatRef{ctx->sor_stT, c.NM + 1, 1}, 1.0 / c.A2y,
-                                            ctx->sor_Ac, ctx->sor_As, 1, c.J, kcf, sz_ac);
+                                            ctx->sor_Ac, ctx->sor_As, 1, c.J, kcf, sz_ac, stop);
     ModeLU lu = TR ? ModeLU{ctx->mluT_a, ctx->mluT_cf, ctx->mluT_idn} : ModeLU{ctx->mlu_a, ctx->mlu_cf, ctx->mlu_idn};
     const int pm = ctx->sor_pm;
     chain(sor_tridiag_kernel, (c.NM + 1 + pm - 1) / pm, 128, (size_t)8 * c.J * (5 * pm + 4), ctx->st, 
-        c, lu, ctx->sor_Ac, ctx->sor_As, pm, TR ? 1 : 0, SOR_KSPLIT, sz_ac);
+        c, lu, ctx->sor_Ac, ctx->sor_As, pm, TR ? 1 : 0, SOR_KSPLIT, sz_ac, stop);
     const int kci = ((c.NM + 1 + SOR_KSPLIT - 1) / SOR_KSPLIT + 31) / 32 * 32;
     const dim3 gi((c.N + 31) / 32, (c.J + 31) / 32, SOR_KSPLIT);
     chain(sor_gemm_kernel, gi, 256, 0, ctx->st, c.J, c.N, c.NM + 1, MatRef{ctx->sor_Ac, 1, c.J}, MatRef{ctx->sor_ct, c.N, 1},
                                             MatRef{ctx->sor_As, 1, c.J}, MatRef{ctx->sor_st, c.N, 1},
-                                            1.0, ctx->sor_q, nullptr, c.N, 1, kci, sz_q);
-    chain(sor_add_kernel<T, TR>, dim3((c.N + 127) / 128, g.jm - 2), 128, 0, ctx->st, g, ctx->sor_q, P, SOR_KSPLIT, sz_q,
-                                                                                  &ctx->sor_check->stop);
+                                            1.0, ctx->sor_q, nullptr, c.N, 1, kci, sz_q, stop);
+    chain(sor_add_kernel<T, TR>, dim3((c.N + 127) / 128, g.jm - 2), 128, 0, ctx->st, g, ctx->sor_q, P, SOR_KSPLIT, sz_q, stop);
     CK_LAUNCH("column-uniform correction");
     return ATURAN_OK;
 }
@@ -671,25 +671,30 @@ const double* sor_compat(aturan_ctx* ctx, double* src, bool transposed, bool app
     return shift;
 }
 
-// The loop of a solve: check (the relative residual of P) and iterate (sweeps s .. next, returning
-// next) until a check meets tol or max_sweeps are done. The sweeps after a check, and the check
-// after those, are enqueued before that check's answer is read; once a check has met tol they do
-// nothing (SorCheck), so sweeps and results are those of a loop that waits each time.
+// The loop of a solve: check (the relative residual of P), correct (what precedes the sweeps) and sweep
+// (sweeps s .. next, returning next). What follows a check is enqueued before that check's answer is
+// read: the correction and, if `ahead`, the sweeps and the check after them (line relaxation, a few
+// launches; the 32 of point relaxation would be 60 us of empty launches at the end, and the
+// correction covers the answer's way). Once a check has met tol it all does nothing (SorCheck), so
+// sweeps and results are those of a loop that waits each time.
 // Returns ATURAN_OK at tol, ATURAN_NOT_CONVERGED at the cap.
-template <typename Check, typename Iterate>
-int solve_loop(aturan_ctx* ctx, int max_sweeps, double tol, int* sweeps_done, double* resid, Check check, Iterate iterate){
+template <typename Check, typename Correct, typename Sweep>
+int solve_loop(aturan_ctx* ctx, int max_sweeps, double tol, bool ahead, int* sweeps_done, double* resid, Check check,
+               Correct correct, Sweep sweep){
     double r = 0.0;
     int s = 0;
     int rc = check(0, 0); if(rc) return rc;
     for(int n = 0;; n++){
         int next = s;
         const bool more = s < max_sweeps;
+        auto go = [&]() -> int { const int e = sweep(s, &next); return e ? e : check((n + 1) & 1, next); };
         if(more){
-            rc = iterate(s, &next); if(rc) return rc;
-            rc = check((n + 1) & 1, next); if(rc) return rc;
+            rc = correct(s); if(rc) return rc;
+            if(ahead){ rc = go(); if(rc) return rc; }
         }
         rc = sor_answer(ctx, n & 1, &r); if(rc) return rc;
         if(r <= tol || !more) break;
+        if(!ahead){ rc = go(); if(rc) return rc; }
         s = next;
     }
     if(sweeps_done) *sweeps_done = s;
@@ -703,14 +708,18 @@ template <bool TR>
 int solve_fp64(aturan_ctx* ctx, double* P, const double* src, double omega, int max_sweeps, double tol, bool line,
                int* sweeps_done, double* resid, long& nl, const double* shift = nullptr){
     const int check_every = sor_check_every(line), every = sor_correct_every(line);
-    return solve_loop(ctx, max_sweeps, tol, sweeps_done, resid,
+    return solve_loop(ctx, max_sweeps, tol, line, sweeps_done, resid,
         [&](int slot, int s){
             nl++;
             return sor_residual<double, TR>(ctx, P, src, s % every == 0, slot, tol, s == 0, !line && s > 0, false, s == 0 ? shift : nullptr);
         },
+        [&](int s){
+            if(s % every) return (int)ATURAN_OK;
+            nl += 4;
+            return sor_correct<double, TR>(ctx, P);
+        },
         [&](int s, int* next){
             int rc;
-            if(s % every == 0){ rc = sor_correct<double, TR>(ctx, P); if(rc) return rc; nl += 4; }
             for(int n = 0; n < check_every && s < max_sweeps; n++, s++){
                 rc = sor_sweep<double, TR>(ctx, P, src, omega, line, n > 0); if(rc) return rc;
                 nl += 2;
@@ -734,10 +743,16 @@ int solve_mixed(aturan_ctx* ctx, double* P, const double* src, double omega, int
     const int inner = line ? 2 : 48;
     // Each FP64 residual also leaves r in FP32, e = 0 and the column sums of r: what the next
     // correction solve starts from (one pass over p and src per refinement step).
-    return solve_loop(ctx, max_sweeps, tol, sweeps_done, resid,
+    return solve_loop(ctx, max_sweeps, tol, line, sweeps_done, resid,
         [&](int slot, int s){
             nl++;
             return sor_residual<double, TR>(ctx, P, src, true, slot, tol, s == 0, false, true, s == 0 ? shift : nullptr);
+        },
+        [&](int s){
+            // with e = 0 the residual's column sums are the correction solve's own
+            if(s % every) return (int)ATURAN_OK;
+            nl += 4;
+            return sor_correct<float, TR>(ctx, ctx->e32);
         },
         [&](int s, int* next){
             int rc;
@@ -745,14 +760,14 @@ int solve_mixed(aturan_ctx* ctx, double* P, const double* src, double omega, int
                 // the correction on the same cadence as the FP64 solve (once per `every` sweeps,
                 // counted over the whole solve): after the first one the column-uniform error is
                 // gone and a later refinement step's correction changes nothing (measured: same
-                // sweep count, 0.14 ms less at 41x181x361); with e = 0 its column sums are r's
-                const bool correct = s % every == 0;
-                if(correct){
-                    if(n != 0){ rc = sor_residual<float, TR>(ctx, ctx->e32, ctx->r32, true, -1, 0.0, false, !line); if(rc) return rc; nl++; }
+                // sweep count, 0.14 ms less at 41x181x361)
+                const bool now = n != 0 && s % every == 0;
+                if(now){
+                    rc = sor_residual<float, TR>(ctx, ctx->e32, ctx->r32, true, -1, 0.0, false, !line); if(rc) return rc;
                     rc = sor_correct<float, TR>(ctx, ctx->e32); if(rc) return rc;
-                    nl += 4;
+                    nl += 5;
                 }
-                rc = sor_sweep<float, TR>(ctx, ctx->e32, ctx->r32, omega, line, n > 0 && !correct); if(rc) return rc;
+                rc = sor_sweep<float, TR>(ctx, ctx->e32, ctx->r32, omega, line, n > 0 && !now); if(rc) return rc;
                 nl += 2;
             }
             chain_if(line, sor_axpy_kernel, 148 * 8, 256, 0, ctx->st, fs, P, ctx->e32, &ctx->sor_check->stop);

@@ -236,8 +236,9 @@ __device__ __forceinline__ void gemm_stage(double (*t)[33], const MatRef& A, int
 // consumer (the tridiagonal kernel, the add kernel) sums the gridDim.z partials in order.
 __global__ void __launch_bounds__(256) sor_gemm_kernel(int M, int Nn, int K, MatRef A1, MatRef B1, MatRef A2,
                                                        MatRef B2, double scale, double* C1, double* C2,
-                                                       long crs, long ccs, int kc, long cz){
+                                                       long crs, long ccs, int kc, long cz, const int* stop){
     chain_wait();
+    if(*stop) return;
     __shared__ double sa1[32][33], sb1[32][33], sa2[32][33], sb2[32][33];   // sa[r][k], sb[c][k]
     const int r0 = blockIdx.y * 32, c0 = blockIdx.x * 32;
     const int kb = blockIdx.z * kc, ke = min(K, kb + kc);
@@ -287,11 +288,15 @@ __global__ void __launch_bounds__(256) sor_gemm_kernel(int M, int Nn, int K, Mat
 // A block takes pm modes (2 pm problems, problem t = 2 m + part): all of its threads stage the
 // right-hand sides (the sum of the transform's nsplit partials) into shared memory as [q][t] (row stride 2 pm + 1: conflict-free) and the
 // modes' factors as [q][m] (stride pm + 1); then one thread per problem runs the two dependent
-// recurrences on shared-memory latency, in place, and the block writes back. Shared memory:
+// recurrences, TRI_R rows at a time in registers with the next rows' loads issued before this group's
+// stores (row by row, each load waited for the store before it, which it may alias: 31 us a solve at
+// 41 x 181 x 361, 20 so); mode 0's sums are the first warp's. The block writes back. Shared memory:
 // 8 J (5 pm + 4) bytes.
+constexpr int TRI_R = 8;
 __global__ void __launch_bounds__(128) sor_tridiag_kernel(SorConst s, ModeLU lu, double* Ac, double* As, int pm,
-                                                          int tr, int nsplit, long split_stride){
+                                                          int tr, int nsplit, long split_stride, const int* stop){
     chain_wait();
+    if(*stop) return;
     extern __shared__ double sm[];
     const int J = s.J, np = 2 * pm, ldr = np + 1, ldf = pm + 1;
     double* sd = sm;                                     // [J][ldr]
@@ -316,6 +321,21 @@ __global__ void __launch_bounds__(128) sor_tridiag_kernel(SorConst s, ModeLU lu,
     __syncthreads();
     const int lt = threadIdx.x;
     const int lm = lt >> 1, part = lt & 1, m = m0 + lm;
+    // mode 0's column (problem 0) minus its mean by the weights ywt (plain: 1), by the first warp
+    auto demean = [&](bool plain){
+        double yr = 0.0;
+        for(int q = lt; q < J; q += 32) yr += (plain ? 1.0 : ywt(q, 0, J - 1)) * sd[q * ldr];
+#pragma unroll
+        for(int d = 16; d > 0; d >>= 1) yr += __shfl_xor_sync(0xffffffffu, yr, d);
+        const double sh = yr / (plain ? (double)J : (double)(J + 1));
+        for(int q = lt; q < J; q += 32) sd[q * ldr] -= sh;
+        __syncwarp();
+    };
+    if(m0 == 0 && lt < 32){                              // compatible with the left null vector; the pinned row
+        demean(tr != 0);
+        if(lt == 0) sd[0] = 0.0;
+        __syncwarp();
+    }
     if(lt < np && m < nmode){
         double* d = sd + lt;
         if(part == 1 && (m == 0 || 2 * m == s.N)){
@@ -324,27 +344,39 @@ __global__ void __launch_bounds__(128) sor_tridiag_kernel(SorConst s, ModeLU lu,
             const double* a = fa + lm;
             const double* cf = fc + lm;
             const double* idn = fi + lm;
-            if(m == 0){                                       // compatible with the left null vector
-                double yr = 0.0, ys = 0.0;
-                for(int q = 0; q < J; q++){ const double wq = tr ? 1.0 : ywt(q, 0, J - 1); yr += wq * d[q * ldr]; ys += wq; }
-                const double sh = yr / ys;
-                for(int q = 0; q < J; q++) d[q * ldr] -= sh;
-                d[0] = 0.0;                                   // the pinned row
+            // rows q0 .. q0 + TRI_R - 1 of the right-hand side and a factor (past the end: of the last row)
+            double dv[TRI_R], av[TRI_R], iv[TRI_R], y = 0.0;
+            auto load = [&](const double* f1, int q0, int step){
+#pragma unroll
+                for(int r = 0; r < TRI_R; r++){
+                    const int q = min(max(q0 + step * r, 0), J - 1);
+                    dv[r] = d[q * ldr]; av[r] = f1[q * ldf]; iv[r] = idn[q * ldf];
+                }
+            };
+            load(a, 0, 1);
+            for(int q0 = 0; q0 < J; q0 += TRI_R){
+                double x[TRI_R];
+#pragma unroll
+                for(int r = 0; r < TRI_R; r++){ x[r] = (dv[r] - av[r] * y) * iv[r]; if(q0 + r < J) y = x[r]; }
+                load(a, q0 + TRI_R, 1);
+#pragma unroll
+                for(int r = 0; r < TRI_R; r++) if(q0 + r < J) d[(q0 + r) * ldr] = x[r];
             }
-            double yp = 0.0;
-#pragma unroll 4
-            for(int q = 0; q < J; q++){ yp = (d[q * ldr] - a[q * ldf] * yp) * idn[q * ldf]; d[q * ldr] = yp; }
-            double x = d[(J - 1) * ldr];
-#pragma unroll 4
-            for(int q = J - 2; q >= 0; q--){ x = d[q * ldr] - cf[q * ldf] * x; d[q * ldr] = x; }
-            if(m == 0 && !tr){                                // the free constant: zero y-weighted mean
-                double yq = 0.0, ys = 0.0;
-                for(int q = 0; q < J; q++){ const double wq = ywt(q, 0, J - 1); yq += wq * d[q * ldr]; ys += wq; }
-                const double sh = yq / ys;
-                for(int q = 0; q < J; q++) d[q * ldr] -= sh;
+            // back: the last row's factor cf is not used (x there is y)
+            double xb = 0.0;
+            load(cf, J - 1, -1);
+            for(int q0 = J - 1; q0 >= 0; q0 -= TRI_R){
+                double x[TRI_R];
+#pragma unroll
+                for(int r = 0; r < TRI_R; r++){ x[r] = q0 - r == J - 1 ? dv[r] : dv[r] - av[r] * xb; xb = x[r]; }
+                load(cf, q0 - TRI_R, -1);
+#pragma unroll
+                for(int r = 0; r < TRI_R; r++) if(q0 - r >= 0) d[(q0 - r) * ldr] = x[r];
             }
         }
     }
+    __syncwarp();
+    if(m0 == 0 && lt < 32 && !tr) demean(false);         // the free constant: zero y-weighted mean
     __syncthreads();
     for(int idx = threadIdx.x; idx < pm * J; idx += blockDim.x){
         const int lm2 = idx / J, q = idx - lm2 * J;
