@@ -921,6 +921,9 @@ int run_chem(aturan_ctx* ctx, const aturan_chem_params* cp, int what, cudaStream
     c.cp_nh3 = cp->cp_nh3; c.cp_h2s = cp->cp_h2s; c.cp_nh4sh = cp->cp_nh4sh;
     c.k_nh3 = cp->k_nh3; c.k_h2s = cp->k_h2s; c.k_nh4sh = cp->k_nh4sh;
     c.dr = p.dr; c.dthe = p.dthe; c.dphi = p.dphi;
+    c.y2dr = 1.0 / (2.0 * c.dr); c.y2dthe = 1.0 / (2.0 * c.dthe); c.y2dphi = 1.0 / (2.0 * c.dphi);
+    c.ydr2 = 1.0 / (c.dr * c.dr); c.ydthe2 = 1.0 / (c.dthe * c.dthe); c.ydphi2 = 1.0 / (c.dphi * c.dphi);
+    c.k_cr = c.c_mix / c.r_mix;
     c.dsign = cp->difflux_plus ? 1.0 : -1.0;                                  // ChemistryUran.h:64-65
     c.sinthe_min = p.sinthe_min; c.floor = cp->polar_floor;
     c.per = cp->phi_periodic != 0;

@@ -25,6 +25,8 @@ struct ChemConst {
     double D_nh3, D_h2s, DT_nh3, DT_h2s, D_nh4sh, DT_nh4sh, c_mix;
     double cp_nh3, cp_h2s, cp_nh4sh, k_nh3, k_h2s, k_nh4sh;
     double dr, dthe, dphi, dsign;
+    double y2dr, y2dthe, y2dphi, ydr2, ydthe2, ydphi2;   // reciprocals of 2 d and d d
+    double k_cr;                                      // c_mix / r_mix
     double sinthe_min, floor;                         // the model's polar metric floor; ATPhys's divisor floor
     int per;                                          // the periodic phi seam
 };
@@ -116,11 +118,9 @@ __device__ __forceinline__ void nh4sh_bisect(double& lo, double& hi, double stop
     // instead of each lane's at its own step
     int it = 0;
     for(; it < 80; it++){
-        const double xm = 0.5 * (lo + hi);
-        const bool pos = xm < r - band;
-        if(!pos && !(xm > r + band)) break;
-        if(pos){ lo = xm; lo_ev = false; } else { hi = xm; hi_ev = false; }
-        if(hi - lo <= stop){ it = 80; break; }
+        const double xm = 0.5 * (lo + hi), dx = xm - r;       // (r lies in the bracket, or a quarter stop
+        if(!(fabs(dx) > band)) break;                         // off it: the bracket is still wider than stop)
+        if(dx < 0.0){ lo = xm; lo_ev = false; } else { hi = xm; hi_ev = false; }
     }
     for(; it < 80; it++){
         const double xm = 0.5 * (lo + hi);
@@ -218,48 +218,38 @@ __device__ __forceinline__ Chem7 chem_ld7(const S* x, size_t q, size_t pl, size_
     v.kp = (double)x[q + dke]; v.km = (double)x[q - dkw];
     return v;
 }
-// ChemistryUran.h:601-686 without SeaMount cells: the central first differences at the cell
-__device__ __forceinline__ void chem_d1v(const Chem7& x, const ChemConst& c, double& dr_, double& dt_, double& dp_){
-    dr_ = (x.ip - x.im) / (2.0 * c.dr);
-    dt_ = (x.jp - x.jm) / (2.0 * c.dthe);
-    dp_ = (x.kp - x.km) / (2.0 * c.dphi);
+// x / d: in the fast form by d's reciprocal y, the division's bits (div_by)
+template <bool FAST>
+__device__ __forceinline__ double chem_div(double x, double d, double y){
+    if constexpr(FAST) return div_by(x, d, y); else return x / d;
 }
-// ChemistryUran.h:576-598 (exp_rm = 1: coord_stretching is false)
-__device__ __forceinline__ double chem_lapv(const Chem7& x, double rm, double rmsinthe, double costhe, const ChemConst& c){
-    const double exp_rm = 1.0, exp_2_rm = exp_rm * exp_rm;
+// ChemistryUran.h:601-686 without SeaMount cells: the central first differences at the cell
+template <bool FAST>
+__device__ __forceinline__ void chem_d1v(const Chem7& x, const ChemConst& c, double& dr_, double& dt_, double& dp_){
+    dr_ = chem_div<FAST>(x.ip - x.im, 2.0 * c.dr, c.y2dr);
+    dt_ = chem_div<FAST>(x.jp - x.jm, 2.0 * c.dthe, c.y2dthe);
+    dp_ = chem_div<FAST>(x.kp - x.km, 2.0 * c.dphi, c.y2dphi);
+}
+// ChemistryUran.h:576-598 (exp_rm = 1: coord_stretching is false) with the row's factors: 2 / rm,
+// cos / (rm rmsinthe), rm rm and rmsinthe rmsinthe with their reciprocals; dr_, dt_: chem_d1v's
+struct ChemLap { double two_rm, ct, rm2, yrm2, rs2, yrs2; };
+template <bool FAST>
+__device__ __forceinline__ double chem_lapv(const Chem7& x, const ChemLap& L, double dcdr, double dcdthe, const ChemConst& c){
     const double v = x.c;
-    const double d2cdr2 = (x.ip - 2.0 * v + x.im) / (c.dr * c.dr) * exp_2_rm;
-    const double d2cdthe2 = (x.jp - 2.0 * v + x.jm) / (c.dthe * c.dthe);
-    const double d2cdphi2 = (x.kp - 2.0 * v + x.km) / (c.dphi * c.dphi);
-    const double dcdr = (x.ip - x.im) / (2.0 * c.dr) * exp_rm;
-    const double dcdthe = (x.jp - x.jm) / (2.0 * c.dthe);
-    return d2cdr2 + 2.0 / rm * dcdr + d2cdthe2 / (rm * rm) + costhe / (rm * rmsinthe) * dcdthe
-         + d2cdphi2 / (rmsinthe * rmsinthe);
+    const double d2cdr2 = chem_div<FAST>(x.ip - 2.0 * v + x.im, c.dr * c.dr, c.ydr2);
+    const double d2cdthe2 = chem_div<FAST>(x.jp - 2.0 * v + x.jm, c.dthe * c.dthe, c.ydthe2);
+    const double d2cdphi2 = chem_div<FAST>(x.kp - 2.0 * v + x.km, c.dphi * c.dphi, c.ydphi2);
+    return d2cdr2 + L.two_rm * dcdr + chem_div<FAST>(d2cdthe2, L.rm2, L.yrm2) + L.ct * dcdthe
+         + chem_div<FAST>(d2cdphi2, L.rs2, L.yrs2);
 }
 
-// rho_mix on every cell (ChemistryUran.h:312-320); on the interior the thermal mass flux and the
-// diffusive tendencies difflux_x = D_x lap(c_x) (passes 1 and 2, ChemistryUran.h:322-419, with
-// j_* formed at the cell where pass 2 reads them). Every load of a cell comes before its first
-// store (a store could alias a later load as far as the compiler knows).
-template <typename S>
-__global__ void __launch_bounds__(128) chem_diff_kernel(ChemArgs<S> a){
-    chain_wait();
+// On the interior the thermal mass flux and the diffusive tendencies difflux_x = D_x lap(c_x) (passes 1
+// and 2, ChemistryUran.h:322-419, with j_* formed at the cell where pass 2 reads them).
+struct ChemDiff { double h2s, nh3, nh4sh, tmf; };
+template <typename S, bool FAST>
+__device__ __forceinline__ ChemDiff chem_cell(const ChemArgs<S>& a, double t0, size_t q, int i, int j, int k){
     const Grid& g = a.g;
-    const int k = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, i = blockIdx.z;
-    if(k >= g.km) return;
     const ChemConst& c = a.c;
-    const size_t q = gidx(g, i, j, k);
-    const double t0 = t_ld(a.t, a.tlo, q);
-    const double rho = (double)a.ps[q] * 1e5 / (c.R_mix * t0 * c.t_ref);
-    const int k_first = c.per ? 0 : 1;
-    if(i < 1 || i > g.im - 2 || j < 1 || j > g.jm - 2 || k < k_first || k > g.km - 2){
-        // what the filter reads off the interior: the fields as they are
-        const S f0 = a.df_h2s[q], f1 = a.df_nh3[q], f2 = a.df_nh4sh[q], f3 = a.tmf[q];
-        a.rho_mix[q] = (S)rho;
-        S* const y = a.scratch + q;
-        y[0] = f0; y[g.fstride] = f1; y[2 * g.fstride] = f2; y[3 * g.fstride] = f3;
-        return;
-    }
     const size_t pl = (size_t)g.jm * g.kp, kp = (size_t)g.kp;
     int dkw, dke;
     chem_kn(k, g.km, c.per, dkw, dke);
@@ -276,35 +266,76 @@ __global__ void __launch_bounds__(128) chem_diff_kernel(ChemArgs<S> a){
     // pass 1's metric: the raw radius and max(sinthe_min, |sin|)
     const double rm = a.tab.rad[i];
     const double rmsinthe = rm * chem_max(c.sinthe_min, fabs(a.tab.sin[j]));
-    double dtdr, dtdthe, dtdphi;
-    chem_d1v(T, c, dtdr, dtdthe, dtdphi);
-    double hr, ht, hp, nr, nt, np, sr, stt, sp;
-    chem_d1v(H, c, hr, ht, hp);
-    chem_d1v(N, c, nr, nt, np);
-    chem_d1v(X, c, sr, stt, sp);
-    const double jT_nh3 = c.DT_nh3 / t0 * dtdr;
-    const double jT_h2s = c.DT_h2s / t0 * dtdr;
-    const double jT_nh4sh = c.DT_nh4sh / t0 * dtdr;
-    const double d_nh3 = nr + fabs(nt) / rm + np / rmsinthe;
-    const double d_h2s = hr + fabs(ht) / rm + hp / rmsinthe;
-    const double d_nh4sh = sr + fabs(stt) / rm + sp / rmsinthe;
-    const double j_nh3 = c.c_mix / c.r_mix * (c.m_nh3 * c.D_nh3 * d_nh3 - jT_nh3);
-    const double j_h2s = c.c_mix / c.r_mix * (c.m_h2s * c.D_h2s * d_h2s - jT_h2s);
-    const double j_nh4sh = c.c_mix / c.r_mix * (c.m_nh4sh * c.D_nh4sh * d_nh4sh - jT_nh4sh);
-    const double w0 = 0.0;                            // w_nh3, w_h2s, w_nh4sh in the equilibrium form
-    const double tmf = (j_nh3 * c.cp_nh3 + j_h2s * c.cp_h2s + j_nh4sh * c.cp_nh4sh)
-                       * (dtdr + fabs(dtdthe) / rm + dtdphi / rmsinthe)
-                       + t0 * (w0 * c.k_nh3 + w0 * c.k_h2s + w0 * c.k_nh4sh);
-    // the Laplacian's metric: the metric radius and max(sin, floor)
+    // the Laplacian's: the metric radius and max(sin, floor)
     const double rml = a.tab.rmm[i];
     const double rmsl = rml * chem_max(a.tab.sin[j], c.floor);
-    const double cl = a.tab.cos[j];
-    const double dfh = c.D_h2s * chem_lapv(H, rml, rmsl, cl, c);
-    const double dfn = c.D_nh3 * chem_lapv(N, rml, rmsl, cl, c);
-    const double dfx = c.D_nh4sh * chem_lapv(X, rml, rmsl, cl, c);
-    a.rho_mix[q] = (S)rho;
+    ChemLap L;
+    L.rm2 = rml * rml; L.rs2 = rmsl * rmsl;
+    L.two_rm = 2.0 / rml; L.ct = a.tab.cos[j] / (rml * rmsl);
+    double yrm = 0.0, yrs = 0.0, yt = 0.0;
+    L.yrm2 = L.yrs2 = 0.0;
+    if constexpr(FAST){ yrm = 1.0 / rm; yrs = 1.0 / rmsinthe; yt = 1.0 / t0; L.yrm2 = 1.0 / L.rm2; L.yrs2 = 1.0 / L.rs2; }
+    auto by_rm = [&](double x){ return chem_div<FAST>(x, rm, yrm); };
+    auto by_rs = [&](double x){ return chem_div<FAST>(x, rmsinthe, yrs); };
+    auto by_t = [&](double x){ return chem_div<FAST>(x, t0, yt); };
+    double dtdr, dtdthe, dtdphi;
+    chem_d1v<FAST>(T, c, dtdr, dtdthe, dtdphi);
+    double hr, ht, hp, nr, nt, np, sr, stt, sp;
+    chem_d1v<FAST>(H, c, hr, ht, hp);
+    chem_d1v<FAST>(N, c, nr, nt, np);
+    chem_d1v<FAST>(X, c, sr, stt, sp);
+    const double jT_nh3 = by_t(c.DT_nh3) * dtdr;
+    const double jT_h2s = by_t(c.DT_h2s) * dtdr;
+    const double jT_nh4sh = by_t(c.DT_nh4sh) * dtdr;
+    const double d_nh3 = nr + by_rm(fabs(nt)) + by_rs(np);
+    const double d_h2s = hr + by_rm(fabs(ht)) + by_rs(hp);
+    const double d_nh4sh = sr + by_rm(fabs(stt)) + by_rs(sp);
+    const double j_nh3 = c.k_cr * (c.m_nh3 * c.D_nh3 * d_nh3 - jT_nh3);
+    const double j_h2s = c.k_cr * (c.m_h2s * c.D_h2s * d_h2s - jT_h2s);
+    const double j_nh4sh = c.k_cr * (c.m_nh4sh * c.D_nh4sh * d_nh4sh - jT_nh4sh);
+    const double w0 = 0.0;                            // w_nh3, w_h2s, w_nh4sh in the equilibrium form
+    ChemDiff r;
+    r.tmf = (j_nh3 * c.cp_nh3 + j_h2s * c.cp_h2s + j_nh4sh * c.cp_nh4sh)
+            * (dtdr + by_rm(fabs(dtdthe)) + by_rs(dtdphi))
+            + t0 * (w0 * c.k_nh3 + w0 * c.k_h2s + w0 * c.k_nh4sh);
+    r.h2s = c.D_h2s * chem_lapv<FAST>(H, L, hr, ht, c);
+    r.nh3 = c.D_nh3 * chem_lapv<FAST>(N, L, nr, nt, c);
+    r.nh4sh = c.D_nh4sh * chem_lapv<FAST>(X, L, sr, stt, c);
+    return r;
+}
+template <typename S>
+__device__ __noinline__ ChemDiff chem_cell_plain(const ChemArgs<S>& a, double t0, size_t q, int i, int j, int k){
+    return chem_cell<S, false>(a, t0, q, i, j, k);
+}
+
+// rho_mix on every cell (ChemistryUran.h:312-320) and chem_cell on the interior, its 42 quotients by the
+// spacings, the row's metric and the temperature as products with their reciprocals (div_by: the same
+// bits; a cell whose result is not finite is formed again with divisions, which tell an infinity from a
+// NaN). Every load of a cell comes before its first store (a store could alias a later load as far as the
+// compiler knows). 41 x 181 x 361, FP64: 224 us with the divisions, bound by them; 110 so, at 5 blocks an SM (114 and 124 at 4 and 6).
+template <typename S>
+__global__ void __launch_bounds__(128, 5) chem_diff_kernel(const __grid_constant__ ChemArgs<S> a){
+    chain_wait();
+    const Grid& g = a.g;
+    const int k = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, i = blockIdx.z;
+    if(k >= g.km) return;
+    const ChemConst& c = a.c;
+    const size_t q = gidx(g, i, j, k);
+    const double t0 = t_ld(a.t, a.tlo, q);
+    const double rho = (double)a.ps[q] * 1e5 / (c.R_mix * t0 * c.t_ref);
+    const int k_first = c.per ? 0 : 1;
     S* const y = a.scratch + q;
-    y[0] = (S)dfh; y[g.fstride] = (S)dfn; y[2 * g.fstride] = (S)dfx; y[3 * g.fstride] = (S)tmf;
+    if(i < 1 || i > g.im - 2 || j < 1 || j > g.jm - 2 || k < k_first || k > g.km - 2){
+        // what the filter reads off the interior: the fields as they are
+        const S f0 = a.df_h2s[q], f1 = a.df_nh3[q], f2 = a.df_nh4sh[q], f3 = a.tmf[q];
+        a.rho_mix[q] = (S)rho;
+        y[0] = f0; y[g.fstride] = f1; y[2 * g.fstride] = f2; y[3 * g.fstride] = f3;
+        return;
+    }
+    ChemDiff r = chem_cell<S, true>(a, t0, q, i, j, k);
+    if(!isfinite(r.tmf + r.h2s + r.nh3 + r.nh4sh)) r = chem_cell_plain<S>(a, t0, q, i, j, k);
+    a.rho_mix[q] = (S)rho;
+    y[0] = (S)r.h2s; y[g.fstride] = (S)r.nh3; y[2 * g.fstride] = (S)r.nh4sh; y[3 * g.fstride] = (S)r.tmf;
 }
 
 // FluxLimiter.h:68-70
