@@ -553,14 +553,14 @@ int run_rb(aturan_ctx* ctx, int sweeps, double omega){
 
 // Residual of P against src as check `slot` of a solve (slot < 0: its column sums only). TR: of the
 // transposed operator. shift: apply the source's compatibility shift in this pass (after sor_compat
-// with apply = false). after_point: the launch before is a point pass.
+// with apply = false).
 template <typename T, bool TR = false>
 int sor_residual(aturan_ctx* ctx, const T* P, const T* src, bool want_col, int slot, double tol, bool first,
-                 bool after_point, bool fill32 = false, const double* shift = nullptr){
+                 bool fill32 = false, const double* shift = nullptr){
     const Grid g = ctx->g;
     double* src_w = nullptr;
     if constexpr(std::is_same<T, double>::value) src_w = shift ? const_cast<double*>(src) : nullptr;
-    chain_if(!after_point, sor_colsum_kernel<T, TR>, dim3((g.km - 1 + 31) / 32, g.jm - 2), dim3(32, 8), 0, ctx->st, 
+    chain(sor_colsum_kernel<T, TR>, dim3((g.km - 1 + 31) / 32, g.jm - 2), dim3(32, 8), 0, ctx->st, 
         g, P, src, ctx->rbw, ctx->sor_colR, ctx->sor_part, want_col ? 1 : 0, SorCheckArg{ctx->sor_check, slot, first, tol},
         fill32 ? ctx->r32 : nullptr, fill32 ? ctx->e32 : nullptr, src_w, src_w ? shift : nullptr);
     CK_LAUNCH("residual");
@@ -580,9 +580,10 @@ int sor_answer(aturan_ctx* ctx, int slot, double* rel){
 }
 
 // The column-uniform correction (TR: the transposed system's y-shaped one) from the column sums
-// left in sor_colR by the last residual.
+// left in sor_colR by the last residual. x2: the corrected iterate goes there in split form (point
+// sweeps follow); null: into P.
 template <typename T, bool TR = false>
-int sor_correct(aturan_ctx* ctx, T* P){
+int sor_correct(aturan_ctx* ctx, T* P, T* x2){
     const Grid g = ctx->g;
     const SorConst& c = ctx->sorc;
     const MatRef R{ctx->sor_colR, c.N, 1};                        // (jj, k)
@@ -602,7 +603,7 @@ int sor_correct(aturan_ctx* ctx, T* P){
     chain(sor_gemm_kernel, gi, 256, 0, ctx->st, c.J, c.N, c.NM + 1, MatRef{ctx->sor_Ac, 1, c.J}, MatRef{ctx->sor_ct, c.N, 1},
                                             MatRef{ctx->sor_As, 1, c.J}, MatRef{ctx->sor_st, c.N, 1},
                                             1.0, ctx->sor_q, nullptr, c.N, 1, kci, sz_q, stop);
-    chain(sor_add_kernel<T, TR>, dim3((c.N + 127) / 128, g.jm - 2), 128, 0, ctx->st, g, ctx->sor_q, P, SOR_KSPLIT, sz_q, stop);
+    chain(sor_add_kernel<T, TR>, dim3((c.N + 127) / 128, g.jm - 2), 128, 0, ctx->st, g, ctx->sor_q, P, x2, SOR_KSPLIT, sz_q, stop);
     CK_LAUNCH("column-uniform correction");
     return ATURAN_OK;
 }
@@ -620,9 +621,25 @@ bool line_smem_attr(){
     return ok;
 }
 
+// The point sweeps' work fields, free outside the RK4 step and the adjustment: the iterate and the
+// right-hand side split by colour (sor_colour_kernel).
+template <typename T>
+inline T* sor_x2(aturan_ctx* ctx){ return reinterpret_cast<T*>(ctx->ybuf[1]); }
+template <typename T>
+inline T* sor_r2(aturan_ctx* ctx){ return sor_x2<T>(ctx) + ctx->g.fstride; }
+// x into split form x2 (to) or back; the launch before a merge is a point pass (so this one is plain).
+template <typename T>
+int sor_split(aturan_ctx* ctx, T* x, T* x2, bool to){
+    const Grid g = ctx->g;
+    const dim3 grid((g.km - 1 + 127) / 128, g.jm - 2, (g.im - 2 + 7) / 8);
+    chain_if(to, sor_split_kernel<T>, grid, 128, 0, ctx->st, g, x, x2, to ? 1 : 0, &ctx->sor_check->stop);
+    CK_LAUNCH("colour split");
+    return ATURAN_OK;
+}
+
 // One relaxation sweep (both colours) of the folded operator (TR: its transpose): point
-// (line = false) or radial line. chained: the launch before is a point pass of the same solve, so that
-// a point pass may read what none writes before it waits for it (sor_colour_kernel).
+// (line = false; of the split fields) or radial line. chained: the launch before is a point pass of the
+// same solve, so that a point pass may read what none writes before it waits for it (sor_colour_kernel).
 template <typename T, bool TR = false>
 int sor_sweep(aturan_ctx* ctx, T* E, const T* R, double omega, bool line, bool chained){
     const Grid g = ctx->g;
@@ -635,8 +652,8 @@ int sor_sweep(aturan_ctx* ctx, T* E, const T* R, double omega, bool line, bool c
                 TR ? ctx->lluT_idn : ctx->llu_idn, colour, omega, stop);
             continue;
         }
-        const dim3 grid((g.km / 2 * (g.jm - 2) + COLOUR_NT - 1) / COLOUR_NT, (g.im - 2 + COLOUR_CH - 1) / COLOUR_CH);
-        chain_if(chained || colour == 1, sor_colour_kernel<T, TR>, grid, COLOUR_NT, 0, ctx->st, g, E, R, ctx->rbw, colour, omega, stop);
+        const dim3 grid(((g.km - 1) / 2 * (g.jm - 2) + COLOUR_NT - 1) / COLOUR_NT, (g.im - 2 + COLOUR_CH - 1) / COLOUR_CH);
+        chain_if(chained || colour == 1, sor_colour_kernel<T, TR>, grid, COLOUR_NT, 0, ctx->st, g, sor_x2<T>(ctx), sor_r2<T>(ctx), ctx->rbw, colour, omega, stop);
     }
     return ATURAN_OK;
 }
@@ -711,12 +728,13 @@ int solve_fp64(aturan_ctx* ctx, double* P, const double* src, double omega, int 
     return solve_loop(ctx, max_sweeps, tol, line, sweeps_done, resid,
         [&](int slot, int s){
             nl++;
-            return sor_residual<double, TR>(ctx, P, src, s % every == 0, slot, tol, s == 0, !line && s > 0, false, s == 0 ? shift : nullptr);
+            return sor_residual<double, TR>(ctx, P, src, s % every == 0, slot, tol, s == 0, false, s == 0 ? shift : nullptr);
         },
         [&](int s){
             if(s % every) return (int)ATURAN_OK;
             nl += 4;
-            return sor_correct<double, TR>(ctx, P);
+            if(!line && s == 0){ const int rc = sor_split(ctx, const_cast<double*>(src), sor_r2<double>(ctx), true); if(rc) return rc; nl++; }
+            return sor_correct<double, TR>(ctx, P, line ? nullptr : sor_x2<double>(ctx));
         },
         [&](int s, int* next){
             int rc;
@@ -725,6 +743,7 @@ int solve_fp64(aturan_ctx* ctx, double* P, const double* src, double omega, int 
                 nl += 2;
             }
             CK_LAUNCH("SOR sweeps");
+            if(!line){ rc = sor_split(ctx, P, sor_x2<double>(ctx), false); if(rc) return rc; nl++; }
             *next = s;
             return (int)ATURAN_OK;
         });
@@ -746,13 +765,14 @@ int solve_mixed(aturan_ctx* ctx, double* P, const double* src, double omega, int
     return solve_loop(ctx, max_sweeps, tol, line, sweeps_done, resid,
         [&](int slot, int s){
             nl++;
-            return sor_residual<double, TR>(ctx, P, src, true, slot, tol, s == 0, false, true, s == 0 ? shift : nullptr);
+            return sor_residual<double, TR>(ctx, P, src, true, slot, tol, s == 0, true, s == 0 ? shift : nullptr);
         },
         [&](int s){
             // with e = 0 the residual's column sums are the correction solve's own
             if(s % every) return (int)ATURAN_OK;
             nl += 4;
-            return sor_correct<float, TR>(ctx, ctx->e32);
+            if(!line){ const int rc = sor_split(ctx, ctx->r32, sor_r2<float>(ctx), true); if(rc) return rc; nl++; }
+            return sor_correct<float, TR>(ctx, ctx->e32, line ? nullptr : sor_x2<float>(ctx));
         },
         [&](int s, int* next){
             int rc;
@@ -763,14 +783,16 @@ int solve_mixed(aturan_ctx* ctx, double* P, const double* src, double omega, int
                 // sweep count, 0.14 ms less at 41x181x361)
                 const bool now = n != 0 && s % every == 0;
                 if(now){
-                    rc = sor_residual<float, TR>(ctx, ctx->e32, ctx->r32, true, -1, 0.0, false, !line); if(rc) return rc;
-                    rc = sor_correct<float, TR>(ctx, ctx->e32); if(rc) return rc;
+                    if(!line){ rc = sor_split(ctx, ctx->e32, sor_x2<float>(ctx), false); if(rc) return rc; nl++; }
+                    rc = sor_residual<float, TR>(ctx, ctx->e32, ctx->r32, true, -1, 0.0, false); if(rc) return rc;
+                    rc = sor_correct<float, TR>(ctx, ctx->e32, line ? nullptr : sor_x2<float>(ctx)); if(rc) return rc;
                     nl += 5;
                 }
                 rc = sor_sweep<float, TR>(ctx, ctx->e32, ctx->r32, omega, line, n > 0 && !now); if(rc) return rc;
                 nl += 2;
             }
-            chain_if(line, sor_axpy_kernel, 148 * 8, 256, 0, ctx->st, fs, P, ctx->e32, &ctx->sor_check->stop);
+            if(!line){ rc = sor_split(ctx, ctx->e32, sor_x2<float>(ctx), false); if(rc) return rc; nl++; }
+            chain(sor_axpy_kernel, 148 * 8, 256, 0, ctx->st, fs, P, ctx->e32, &ctx->sor_check->stop);
             CK_LAUNCH("SOR refinement");
             nl++;
             *next = s;

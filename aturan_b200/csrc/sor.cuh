@@ -390,12 +390,67 @@ __global__ void __launch_bounds__(128) sor_tridiag_kernel(SorConst s, ModeLU lu,
     }
 }
 
-// Onto every interior level of the column: P[i][j][k] += q(j,k).
-// (TR: y_i q, the trial functions of the transposed system's correction.)
-template <typename T, bool TR = false>
-__global__ void __launch_bounds__(128) sor_add_kernel(Grid g, const double* qbuf, T* P, int nsplit, long split_stride, const int* stop){
+// Red-black SOR colour pass of the folded operator, Lc e = r, for T = double (the FP64 solve) or
+// float (the correction solve of the mixed form: e and r in FP32, the row assembled in FP64 and
+// rounded once).
+//
+// The passes work on the iterate and the right-hand side split by colour (SplitIx): cell (i, j, k) of colour
+// (i + j + k) & 1 at half-meridian k / 2 of that colour's field. A pass then reads contiguous rows of one
+// colour for the neighbours and of the other for its own cells, half of what the interleaved rows made it
+// fetch. The correction that precedes every run of sweeps writes the split iterate, a merge behind the run
+// puts it back.
+//
+// A pass is a few us of work, so what bounds a sweep is also the time from one pass to the next: a pass of
+// 41 x 91 x 181 took 4.4 us and the next began 2 us later. The launches are chained (programmatic
+// stream serialisation): a block may be placed while the pass before it drains, reads what no pass
+// writes (weights, right-hand sides), forms the row's weights and the reciprocal of its diagonal,
+// and only then waits for that pass. It lets the next pass in after its own wait, so that at most
+// two passes share the chip. After the wait all loads of a thread's COLOUR_CH cells (levels i, i+1
+// of one half-meridian) are issued together, unconditionally: a folded neighbour has its address
+// and weight changed, not its load skipped. P is read by plain loads (the wait orders those, not the
+// read-only path). The quotient by the diagonal is the reciprocal's product corrected by its own
+// remainder (Markstein). Measured: a 256-sweep solve at 41 x 91 x 181 took 4.43 ms unchained, 2.80 chained
+// on interleaved rows and takes 2.37 with 2 cells a thread and 9 blocks an SM (1 cell, 16 blocks: 2.92;
+// 4 cells, 5 blocks: 2.58; 3 cells, 6 blocks: 2.64).
+struct SplitIx {
+    int hp, half;               // row pitch and meridians of a colour
+    size_t fsh;                 // elements of a colour
+    __device__ __forceinline__ explicit SplitIx(const Grid& g) : hp(g.kp / 2), half((g.km - 1) / 2), fsh(g.fstride / 2) {}
+    __device__ __forceinline__ size_t at(const Grid& g, int i, int j, int k) const {
+        return ((i + j + k) & 1) * fsh + ((size_t)i * g.jm + j) * hp + (k >> 1);
+    }
+};
+// The interior of x into split form (to = true) or back.
+template <typename T>
+__global__ void __launch_bounds__(128) sor_split_kernel(Grid g, T* x, T* x2, int to, const int* stop){
     chain_wait();
     if(*stop) return;
+    const SplitIx sx(g);
+    const int k = blockIdx.x * blockDim.x + threadIdx.x, j = 1 + blockIdx.y;
+    if(k >= g.km - 1) return;
+    constexpr int CH = 8;
+    for(int i0 = 1 + blockIdx.z * CH; i0 < min(g.im - 1, 1 + (int)(blockIdx.z + 1) * CH); i0 += CH){
+        T v[CH];
+#pragma unroll
+        for(int c = 0; c < CH; c++)
+            if(i0 + c < g.im - 1) v[c] = to ? x[gidx(g, i0 + c, j, k)] : x2[sx.at(g, i0 + c, j, k)];
+#pragma unroll
+        for(int c = 0; c < CH; c++)
+            if(i0 + c < g.im - 1){
+                if(to) x2[sx.at(g, i0 + c, j, k)] = v[c];
+                else x[gidx(g, i0 + c, j, k)] = v[c];
+            }
+    }
+}
+
+// Onto every interior level of the column: P[i][j][k] += q(j,k).
+// (TR: y_i q, the trial functions of the transposed system's correction.) Given x2, the sum goes there, in
+// split form, and P stays as it is.
+template <typename T, bool TR = false>
+__global__ void __launch_bounds__(128) sor_add_kernel(Grid g, const double* qbuf, T* P, T* x2, int nsplit, long split_stride, const int* stop){
+    chain_wait();
+    if(*stop) return;
+    const SplitIx sx(g);
     const int N = g.km - 1;
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = 1 + blockIdx.y;
@@ -411,48 +466,36 @@ __global__ void __launch_bounds__(128) sor_add_kernel(Grid g, const double* qbuf
 #pragma unroll
         for(int c = 0; c < CH; c++){
             const int i = i0 + c;
-            if(i < g.im - 1) P[gidx(g, i, j, k)] = (T)((double)v[c] + (TR ? ywt(i, 1, g.im - 2) * q : q));
+            if(i < g.im - 1){
+                T* const d = x2 ? x2 + sx.at(g, i, j, k) : P + gidx(g, i, j, k);
+                *d = (T)((double)v[c] + (TR ? ywt(i, 1, g.im - 2) * q : q));
+            }
         }
     }
 }
 
-// Red-black SOR colour pass of the folded operator, Lc e = r, for T = double (the FP64 solve) or
-// float (the correction solve of the mixed form: e and r in FP32, the row assembled in FP64 and
-// rounded once).
-//
-// A pass is a few us of work, so what bounds a sweep is the time from one pass to the next: a pass of
-// 41 x 91 x 181 took 4.4 us and the next began 2 us later. The launches are chained (programmatic
-// stream serialisation): a block may be placed while the pass before it drains, reads what no pass
-// writes (weights, right-hand sides), forms the row's weights and the reciprocal of its diagonal,
-// and only then waits for that pass. It lets the next pass in after its own wait, so that at most
-// two passes share the chip. After the wait all loads of a thread's COLOUR_CH cells (levels i, i+1
-// of one pair of meridians) are issued together, unconditionally: a folded neighbour has its address
-// and weight changed, not its load skipped. P is read by plain loads (the wait orders those, not the
-// read-only path). The quotient by the diagonal is the reciprocal's product corrected by its own
-// remainder (Markstein). Measured: a 256-sweep solve at 41 x 91 x 181 took 4.43 ms and takes 3.17
-// with 2 cells a thread and 9 blocks an SM (1 cell, 16 blocks: 3.19; 3 and 4 cells: 3.35).
 constexpr int COLOUR_CH = 2, COLOUR_NT = 128, COLOUR_MB = 9;
 template <typename T, bool TR = false>
-__global__ void __launch_bounds__(COLOUR_NT, COLOUR_MB) sor_colour_kernel(Grid g, T* E, const T* R, const RBW* w, int colour, double omega,
-                                                               const int* stop){
-    const int half = g.km / 2;
+__global__ void __launch_bounds__(COLOUR_NT, COLOUR_MB) sor_colour_kernel(Grid g, T* E2, const T* R2, const RBW* w, int colour, double omega,
+                                                                          const int* stop){
+    const SplitIx sx(g);
     const int c = blockIdx.x * COLOUR_NT + threadIdx.x;
-    const bool row = c < half * (g.jm - 2);
-    const int j = row ? 1 + c / half : 1, k2 = row ? c - (j - 1) * half : 0;
-    const int si = g.jm * g.kp, sj = g.kp;
+    const bool row = c < sx.half * (g.jm - 2);
+    const int j = row ? 1 + c / sx.half : 1, h = row ? c - (j - 1) * sx.half : 0;
+    const int si = g.jm * sx.hp, sj = sx.hp;
     const bool jlo = j == 1, jhi = j == g.jm - 2;
+    T* const own = E2 + colour * sx.fsh;
+    const T* const oth = E2 + (1 - colour) * sx.fsh;
     bool on[COLOUR_CH];
-    size_t o[COLOUR_CH];
+    int o[COLOUR_CH];
     double rr[COLOUR_CH], inv[COLOUR_CH], diag[COLOUR_CH], w3[COLOUR_CH];
     double wim[COLOUR_CH], wip[COLOUR_CH], wjm[COLOUR_CH], wjp[COLOUR_CH];
     const int i0 = 1 + blockIdx.y * COLOUR_CH;
 #pragma unroll
     for(int q = 0; q < COLOUR_CH; q++){
         const int i = min(i0 + q, g.im - 2);
-        int k = 2 * k2 + ((i + j + colour) & 1);
-        on[q] = row && i0 + q <= g.im - 2 && k <= g.km - 2;
-        if(k > g.km - 2) k = 0;
-        o[q] = gidx(g, i, j, k);
+        on[q] = row && i0 + q <= g.im - 2;
+        o[q] = (i * g.jm + j) * sx.hp + h;
         const bool ilo = i == 1, ihi = i == g.im - 2;
         const RBW4 W = ldw(w + i * g.jm + j);
         double d = W.den;
@@ -472,26 +515,27 @@ __global__ void __launch_bounds__(COLOUR_NT, COLOUR_MB) sor_colour_kernel(Grid g
             wjm[q] = jlo ? -C13 * W.num2 : W.num2;
             wjp[q] = jhi ? -C13 * W.num2 : W.num2;
         }
-        rr[q] = (double)__ldg(R + o[q]);
+        rr[q] = (double)__ldg(R2 + colour * sx.fsh + o[q]);
     }
     const bool done = *stop != 0;
     chain_wait();
     cudaTriggerProgrammaticLaunchCompletion();
     if(done) return;
-    // where a neighbour is folded, the other one's address (TR, of weight 0: the cell's own), so that
-    // no boundary value is read that the row does not hold
+    // where a neighbour is folded, the other one's address (TR, of weight 0: the cell at the same place), so
+    // that no boundary value is read that the row does not hold
     const int ojm = jlo ? (TR ? 0 : sj) : -sj, ojp = jhi ? (TR ? 0 : -sj) : sj;
     T pim[COLOUR_CH], pip[COLOUR_CH], pjm[COLOUR_CH], pjp[COLOUR_CH], pe[COLOUR_CH], pw[COLOUR_CH], p0[COLOUR_CH];
 #pragma unroll
     for(int q = 0; q < COLOUR_CH; q++){
-        const T* const p = E + o[q];
         const int i = min(i0 + q, g.im - 2);
-        int k = 2 * k2 + ((i + j + colour) & 1);
-        if(k > g.km - 2) k = 0;
+        const T* const p = oth + o[q];
+        // k = 2 h + odd: its phi neighbours are half-meridian h of the other colour and the one before or behind
+        const bool odd = (i + j + colour) & 1;
+        const int step = odd ? (h == sx.half - 1 ? 1 - sx.half : 1) : (h == 0 ? sx.half - 1 : -1);
         pim[q] = p[i == 1 ? (TR ? 0 : si) : -si]; pip[q] = p[i == g.im - 2 ? (TR ? 0 : -si) : si];
         pjm[q] = p[ojm]; pjp[q] = p[ojp];
-        pe[q] = *(p - k + phi_wrap(k + 1, g.km)); pw[q] = *(p - k + phi_wrap(k - 1, g.km));
-        p0[q] = *p;
+        pe[q] = p[odd ? step : 0]; pw[q] = p[odd ? 0 : step];
+        p0[q] = own[o[q]];
     }
 #pragma unroll
     for(int q = 0; q < COLOUR_CH; q++){
@@ -500,7 +544,7 @@ __global__ void __launch_bounds__(COLOUR_NT, COLOUR_MB) sor_colour_kernel(Grid g
         const double y = x * inv[q];
         const double pn = fma(fma(-y, diag[q], x), inv[q], y);
         const double e0 = (double)p0[q];
-        if(on[q]) E[o[q]] = (T)(e0 + omega * (pn - e0));
+        if(on[q]) own[o[q]] = (T)(e0 + omega * (pn - e0));
     }
 }
 
