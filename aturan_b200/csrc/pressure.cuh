@@ -35,7 +35,7 @@ struct RBW {
 };
 
 struct PressConst {
-    double inv_2dr, inv_2dthe, inv_2dphi, two_dr, two_dthe, two_dphi, src_scale;
+    double inv_2dr, inv_2dthe, inv_2dphi, two_dr, two_dthe, two_dphi, src_scale;   // inv_x: 1 / two_x
     int press_incr;
 };
 
@@ -47,11 +47,16 @@ __global__ void gs_aux_bc_kernel(Grid g, S* au, S* av, S* aw){
     const int j = 1 + blockIdx.y;
     if(k > g.km - 2 || j > g.jm - 2) return;
     S* A[3] = {au, av, aw};
+    // every load before the first store (which each of them would otherwise wait for)
+    S lo[3], hi[3];
+#pragma unroll
     for(int q = 0; q < 3; q++){
-        S* a = A[q];
-        a[gidx(g, 0, j, k)]        = (S)(C43 * (double)a[gidx(g, 1, j, k)] - C13 * (double)a[gidx(g, 2, j, k)]);
-        a[gidx(g, g.im - 1, j, k)] = (S)(C43 * (double)a[gidx(g, g.im - 2, j, k)] - C13 * (double)a[gidx(g, g.im - 3, j, k)]);
+        const S* a = A[q];
+        lo[q] = (S)(C43 * (double)a[gidx(g, 1, j, k)] - C13 * (double)a[gidx(g, 2, j, k)]);
+        hi[q] = (S)(C43 * (double)a[gidx(g, g.im - 2, j, k)] - C13 * (double)a[gidx(g, g.im - 3, j, k)]);
     }
+#pragma unroll
+    for(int q = 0; q < 3; q++){ A[q][gidx(g, 0, j, k)] = lo[q]; A[q][gidx(g, g.im - 1, j, k)] = hi[q]; }
 }
 
 // ---- PressureSolverUran.h:139-175: incr_src = src_scale div(rhs) + Lc(p_old), the radial
@@ -71,10 +76,13 @@ __global__ void gs_incr_kernel(Grid g, const S* ru, const S* rv, const S* rw, co
         if(ii == g.im - 1) return C43 * (double)ru[gidx(g, g.im - 2, j, k)] - C13 * (double)ru[gidx(g, g.im - 3, j, k)];
         return (double)ru[gidx(g, ii, j, k)];
     };
-    const double div_rhs =
-          (RU(i + 1) - RU(i - 1)) / c.two_dr
-        + ((double)rv[gidx(g, i, j + 1, k)] - (double)rv[gidx(g, i, j - 1, k)]) / c.two_dthe * W.inv_rm
-        + ((double)rw[gidx(g, i, j, ke)] - (double)rw[gidx(g, i, j, kw)]) / c.two_dphi * W.inv_rmsinthe;
+    const double du = RU(i + 1) - RU(i - 1);
+    const double dv = (double)rv[gidx(g, i, j + 1, k)] - (double)rv[gidx(g, i, j - 1, k)];
+    const double dw = (double)rw[gidx(g, i, j, ke)] - (double)rw[gidx(g, i, j, kw)];
+    double div_rhs = div_by(du, c.two_dr, c.inv_2dr) + div_by(dv, c.two_dthe, c.inv_2dthe) * W.inv_rm
+                   + div_by(dw, c.two_dphi, c.inv_2dphi) * W.inv_rmsinthe;
+    if(!isfinite(div_rhs))                    // an infinity's quotient (div_by makes it a NaN)
+        div_rhs = du / c.two_dr + dv / c.two_dthe * W.inv_rm + dw / c.two_dphi * W.inv_rmsinthe;
     const double lc_old =
           (P[gidx(g, i + 1, j, k)] + P[gidx(g, i - 1, j, k)]) * W.n1
         + (P[gidx(g, i, j + 1, k)] + P[gidx(g, i, j - 1, k)]) * W.n2
@@ -484,7 +492,11 @@ __global__ void prep_seam_kernel(Grid g, S* au, S* av, S* aw, S* ru, S* rv, S* r
     if(c >= g.im * g.jm) return;
     const int i = c / g.jm, j = c - i * g.jm;
     S* A[6] = {au, av, aw, ru, rv, rw};
-    for(int q = 0; q < 6; q++) A[q][gidx(g, i, j, g.km - 1)] = A[q][gidx(g, i, j, 0)];
+    S v[6];
+#pragma unroll
+    for(int q = 0; q < 6; q++) v[q] = A[q][gidx(g, i, j, 0)];
+#pragma unroll
+    for(int q = 0; q < 6; q++) A[q][gidx(g, i, j, g.km - 1)] = v[q];
 }
 
 // ---- PressureSolver.h:370-487: div(aux) source, clamped, non-finite guard ----

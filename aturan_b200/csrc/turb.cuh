@@ -223,11 +223,15 @@ __global__ void __launch_bounds__(128) turb_edges_kernel(TurbArgs<S> a){
         return seam_src(i == im - 1 ? im - 2 : i, j, k);
     };
     S* f[8] = {a.tke, a.dis, a.tken, a.disn, a.nue, a.prod, a.tks, a.dss};
+    // the eight fields' loads before the first store (which each of them would otherwise wait for)
+    S x[8], y[8];
     if(t < nseam){
         const int i = (int)(t / (jm - 2)), j = 1 + (int)(t % (jm - 2));
         const size_t d = gidx(g, i, j, km - 1), s = gidx(g, i, j, 0);
 #pragma unroll
-        for(int n = 0; n < 8; n++) f[n][d] = f[n][s];
+        for(int n = 0; n < 8; n++) x[n] = f[n][s];
+#pragma unroll
+        for(int n = 0; n < 8; n++) f[n][d] = x[n];
         return;
     }
     t -= nseam;
@@ -235,7 +239,9 @@ __global__ void __launch_bounds__(128) turb_edges_kernel(TurbArgs<S> a){
         const int j = 1 + (int)(t / km), k = (int)(t % km);
         const size_t d = gidx(g, im - 1, j, k), s = lid_src(im - 1, j, k);
 #pragma unroll
-        for(int n = 0; n < 8; n++) f[n][d] = f[n][s];
+        for(int n = 0; n < 8; n++) x[n] = f[n][s];
+#pragma unroll
+        for(int n = 0; n < 8; n++) f[n][d] = x[n];
         return;
     }
     t -= nlid;
@@ -244,7 +250,9 @@ __global__ void __launch_bounds__(128) turb_edges_kernel(TurbArgs<S> a){
         const size_t d0 = gidx(g, i, 0, k), s0 = lid_src(i, 1, k);
         const size_t d1 = gidx(g, i, jm - 1, k), s1 = lid_src(i, jm - 2, k);
 #pragma unroll
-        for(int n = 0; n < 8; n++){ f[n][d0] = f[n][s0]; f[n][d1] = f[n][s1]; }
+        for(int n = 0; n < 8; n++){ x[n] = f[n][s0]; y[n] = f[n][s1]; }
+#pragma unroll
+        for(int n = 0; n < 8; n++){ f[n][d0] = x[n]; f[n][d1] = y[n]; }
     }
 }
 
