@@ -42,6 +42,18 @@ struct PrecipArgs {
 __device__ __forceinline__ double pr_max(double a, double b){ return (a < b) ? b : a; }   // std::max
 __device__ __forceinline__ double pr_min(double a, double b){ return (b < a) ? b : a; }   // std::min
 
+// x / d from d's reciprocal y, the division's bits (div_by; what that cannot divide, infinities, is divided).
+__device__ __noinline__ static double pr_div_plain(double x, double d){ return x / d; }
+__device__ __forceinline__ double pr_div(double x, double d, double y){
+    const double q = div_by(x, d, y);
+    return isfinite(q) ? q : pr_div_plain(x, d);
+}
+// pow(x, e), which is 1 at the flux cap (x = 1)
+__device__ __forceinline__ double pr_pow(double x, double e){ return x == 1.0 ? 1.0 : pow(x, e); }
+
+// A level's march is one dependent chain, so what it does not need is left out: the quotients by the
+// layer's thickness, its fall time and the reference flux come from one reciprocal, and the powers of the
+// rain flux are formed where they are used (warm cells; evaporation).
 // Lane 4c + n of a warp: species n of the warp's column c (k = 8 * warp + c of the block's 32).
 template <typename S>
 __global__ void __launch_bounds__(128) precip_kernel(const __grid_constant__ PrecipArgs<S> a){
@@ -108,12 +120,14 @@ __global__ void __launch_bounds__(128) precip_kernel(const __grid_constant__ Pre
                 const double E_r = exp(s.C + (-s.L0 / T + s.del_alf * log(T) + s.del_bet * T) / s.den);   // ATPhys.h:49-52
                 const double q_sat = (p_u > E_r) ? rho * s.ep * E_r / p_u : q_v;
                 const double F_r_in = Pr, F_s_in = Ps, F_g_in = Pg;
-                const double Rain = pr_min(ratio_cap, F_r_in / P_ref);
-                const double Snow = pr_min(ratio_cap, F_s_in / P_ref);
-                const double Graupel = pr_min(ratio_cap, F_g_in / P_ref);
-                const double Rain_79 = (Rain > 0.0) ? pow(Rain, 7.0 / 9.0) : 0.0;
-                const double Rain_49 = (Rain > 0.0) ? pow(Rain, 4.0 / 9.0) : 0.0;
-                const bool warm = (T >= s.t_frz);
+                const double Rain = pr_min(ratio_cap, div_by(F_r_in, P_ref, 1.0 / P_ref));
+                const double Snow = pr_min(ratio_cap, div_by(F_s_in, P_ref, 1.0 / P_ref));
+                const double Graupel = pr_min(ratio_cap, div_by(F_g_in, P_ref, 1.0 / P_ref));
+                const bool warm = (T >= s.t_frz), evap = warm && Rain > 0.0 && q_v < q_sat;
+                const double Rain_79 = (warm && Rain > 0.0) ? pr_pow(Rain, 7.0 / 9.0) : 0.0;
+                const double Rain_49 = evap ? pr_pow(Rain, 4.0 / 9.0) : 0.0;
+                const double ydz = 1.0 / dz;
+                auto by_dz = [&](double x){ return pr_div(x, dz, ydz); };
                 const double S_c_au = (warm && q_c > q_c_crit) ? (rs * c_c_au) * (q_c - q_c_crit) : 0.0;
                 const double S_i_au = (!warm && T >= s.t_low) ? (rs * c_i_au) * q_i : 0.0;
                 const double S_ac = warm ? (rs * c_ac) * q_c * Rain_79 : 0.0;
@@ -126,20 +140,20 @@ __global__ void __launch_bounds__(128) precip_kernel(const __grid_constant__ Pre
                 const double F_g_melt = f_melt * F_g_in;
                 const double F_r_frz = f_frz * F_r_in;
                 const double F_r_avail = pr_max(0.0, F_r_in - F_r_frz + F_s_melt + F_g_melt + (S_c_au + S_ac) * dz);
-                const double S_ev_raw = (warm && Rain > 0.0 && q_v < q_sat) ? a_ev * (q_sat - q_v) * Rain_49 : 0.0;
+                const double S_ev_raw = evap ? a_ev * (q_sat - q_v) * Rain_49 : 0.0;
                 const double F_ev_sat = pr_max(0.0, q_sat - q_v) * v_fall;
                 const double F_ev = pr_min(pr_min(S_ev_raw * dz, F_r_avail), F_ev_sat);
-                const double S_ev = F_ev / dz;
+                const double S_ev = by_dz(F_ev);
                 term = s.Lf * (S_s_rim + S_g_rim + S_csg)
-                     + s.Lf * (F_r_frz - F_s_melt - F_g_melt) / dz
-                     - s.lv * F_ev / dz;
+                     + by_dz(s.Lf * (F_r_frz - F_s_melt - F_g_melt))
+                     - by_dz(s.lv * F_ev);
                 added = true;
-                const double tau = dz / v_fall;
+                const double tau = dz / v_fall, ytau = ydz * v_fall;     // v_fall = 2: both exact
                 const double d_c = pr_min(dep_frac * q_c, (S_c_au + S_ac + S_s_rim + S_g_rim + S_csg) * tau);
                 const double d_i = pr_min(dep_frac * q_i, S_i_au * tau);
                 if(a.coupling){
-                    sc[q] = (S)(-pr_max(0.0, d_c) / tau * a.nd);
-                    si[q] = (S)(-pr_max(0.0, d_i) / tau * a.nd);
+                    sc[q] = (S)(-pr_div(pr_max(0.0, d_c), tau, ytau) * a.nd);
+                    si[q] = (S)(-pr_div(pr_max(0.0, d_i), tau, ytau) * a.nd);
                     sv[q] = (S)(+S_ev * a.nd);
                 } else {
                     fc[q] = (S)(q_c - pr_max(0.0, d_c));
