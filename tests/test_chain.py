@@ -32,7 +32,7 @@ def test_every_chained_kernel_waits_first(f):
         name = re.search(r"(\w+_kernel)\s*\(", s[m.start():i]).group(1)
         body = s[i + 1:i + 4000]
         if name in LATE:
-            assert 0 < body.find("chain_wait();") < body.find("E + ")
+            assert 0 < body.find("chain_wait();") < body.find("oth + o[q]")
         elif body.lstrip().startswith("chain_wait();"):
             continue
         else:
