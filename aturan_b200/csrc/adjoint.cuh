@@ -437,32 +437,42 @@ __global__ void __launch_bounds__(128) adj_satadj_kernel(Grid g, const double* p
     if(K.local_rho){ const double r_ = rho_mix[q]; rho_c = (r_ > 0.0 && isfinite(r_)) ? r_ : K.r_mix; }
     const double hc = K.cp_mix * rho_c, t_ref = K.t_ref;
     const int base[4] = {ATURAN_H2O, ATURAN_H2S, ATURAN_NH3, ATURAN_CH4};
+    // every value of the cell up front (the loops over the gases would load a gas's behind the work, and the
+    // stores, of the one before it): state on entry, cloud and ice after, adjoints
+    double pv[4][3], qv[4][2], yv[4][3];
+#pragma unroll
+    for(int gi = 0; gi < 4; gi++){
+        const size_t f = (size_t)base[gi] * fs + q;
+#pragma unroll
+        for(int n = 0; n < 3; n++){ pv[gi][n] = __ldg(pre + f + n * fs); yv[gi][n] = ybar[f + n * fs]; }
+        qv[gi][0] = __ldg(post + f + fs); qv[gi][1] = __ldg(post + f + 2 * fs);
+    }
+    const double yt = ybar[q];
     // forward replay: each gas's entry record and the temperature after it
     SatEntry ent[4];
     double Tout[4];
     double T = pre[q] * t_ref;
     for(int gi = 0; gi < 4; gi++){
         const GasConst& G = K.gas[gi];
-        const size_t f = (size_t)base[gi] * fs + q;
-        ent[gi] = sat_entry(K, G, rho_c, p_u, T, pre[f], pre[f + fs], pre[f + 2 * fs]);
+        ent[gi] = sat_entry(K, G, rho_c, p_u, T, pv[gi][0], pv[gi][1], pv[gi][2]);
         const SatEntry& e = ent[gi];
         if(e.skip){ Tout[gi] = T; continue; }
         if(e.go){
             const double E = hc * e.t_u - G.lv * e.cloud - G.ls * e.ice;
-            T = (E + G.lv * post[f + fs] + G.ls * post[f + 2 * fs]) / hc;
+            T = (E + G.lv * qv[gi][0] + G.ls * qv[gi][1]) / hc;
         } else T = e.t_u;
         Tout[gi] = T;
     }
     // reverse
-    double Tb = ybar[q] / t_ref;
+    double Tb = yt / t_ref;
     for(int gi = 3; gi >= 0; gi--){
         const GasConst& G = K.gas[gi];
         const size_t f = (size_t)base[gi] * fs + q;
         const SatEntry& e = ent[gi];
         if(e.skip) continue;
-        double cb = ybar[f], clb = ybar[f + fs], ib = ybar[f + 2 * fs];
+        double cb = yv[gi][0], clb = yv[gi][1], ib = yv[gi][2];
         if(e.go){
-            const double qc = post[f + fs], qi = post[f + 2 * fs], Tp = Tout[gi];
+            const double qc = qv[gi][0], qi = qv[gi][1], Tp = Tout[gi];
             double Eb, Wb;
             if(qc > 0.0 && qi > 0.0){
                 const double r = qc / (qc + qi), L = r * G.lv + (1.0 - r) * G.ls;
