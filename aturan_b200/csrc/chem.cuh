@@ -84,7 +84,7 @@ __device__ __forceinline__ double nh4sh_df(double x, double T0, double heat, dou
 // r comes from safeguarded Newton (a step that leaves the bracket is replaced by its midpoint),
 // and f itself is evaluated, as the reference does, at the ~3 midpoints inside the band instead
 // of at all ~50 (41 x 181 x 361, FP64-bound: 960 us with 14 Newton steps a cell and the evaluations
-// at each lane's own step, 438 so). The final bracket is checked with f at both ends; a bracket that does not hold
+// at each lane's own step, 417 so). The final bracket is checked with f at both ends; a bracket that does not hold
 // (no single root, or Newton astray) is bisected again with f at every midpoint.
 __device__ __forceinline__ void nh4sh_bisect(double& lo, double& hi, double stop, double T0, double heat,
                                              double a, double b, double x0){

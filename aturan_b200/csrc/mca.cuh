@@ -27,7 +27,7 @@
 //     and the upper cell's equilibrium are one solve and their difference is exactly zero; a segment's
 //     edge pairs were tested with the values they still have; every other pair was stable at the start
 //     and has not changed. The reference's further sweep finds nothing, so there is none here.
-// Measured at 41x181x361 (mixed, synthetic state): 4.3 ms -- prep 0.14, tests 1.18, growth 2.50, finish
+// Measured at 41x181x361 (mixed, synthetic state): 4.2 ms -- prep 0.10, tests 1.18, growth 2.48, finish
 // 0.46 -- against 44.7 ms for one warp per column running the whole sweep with every settle and a
 // verifying sweep; 1.1 against 8.1 ms at 37x83x167, 0.34 against 0.88 ms at 21x37x73. Same bits. (With
 // every quotient a division and a column's whole state in shared memory: 6.0, 1.28 and 0.63 ms.)

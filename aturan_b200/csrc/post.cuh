@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(128) post_filter_i_kernel(Grid g, S* x, float*
 }
 
 // ---- damp_wiggles along k, j and i in one pass, out of place (x -> y) ----
-// The three 1-2-1 passes of damp_wiggles with all axes on, fused over a tile of FT_I x FT_J x FT_K
+// The three 1-2-1 passes of damp_wiggles with all axes on, fused over li levels of FT_J x FT_K
 // outputs: the k pass of the tile and its one-cell i and j halo is formed from global memory (the
 // k neighbours are the row's own, L1 hits), the j pass of the tile and its i halo from that, the i
 // pass from that. The halo rows and planes are the clamped ones the passes use at the poles and
