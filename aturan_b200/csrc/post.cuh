@@ -120,14 +120,6 @@ __global__ void __launch_bounds__(128) post_filter_i_kernel(Grid g, S* x, float*
 // and eight copies back of 10 us at 41 x 181 x 361 (FP64).
 constexpr int FT_N = 4;
 template <typename S> struct Filter3 { const S* x[FT_N]; S* y[FT_N]; };
-//
-// A block takes FT_K meridians x FT_J rows and walks up li levels: the k pass of a level's rows
-// (and the halo row on each side) goes to shared memory, double-buffered so that a level costs one
-// barrier; the thread of a column forms the j pass from it and keeps the last three levels' j passes
-// in registers for the i pass. The next level is in flight in registers meanwhile (two or four ahead
-// cost warps and were slower). Four FP64 fields of 41 x 181 x 361: 83 us with tiles of 4 levels staged
-// whole, 58 so (172 MB: 26 us).
-//
 // A block takes FT_K meridians x FT_J rows and walks up li levels: the k pass of a level's rows
 // (and the halo row on each side) goes to shared memory, double-buffered so that a level costs one
 // barrier; the thread of a column forms the j pass from it and keeps the last three levels' j passes
