@@ -42,7 +42,8 @@ struct AdjArgs {
     double* kbar_out;           // the previous stage's kbar and pe
     double* pe_out;
     const double* auxbar;       // stage 3 only, else null: adjoint of aux_u, aux_v, aux_w (the tendencies
-                                // of u, v, w without the p_dyn gradient, RHS_Uran_Turb.cpp:1020-1022), 0 off the interior
+                                // of u, v, w without the p_dyn gradient, RHS_Uran_Turb.cpp:1020-1022), used on
+                                // the interior alone
     const double* pdyn;
     const double* nt;           // the eddy viscosity as the tendencies use it (adj_nue)
     const GeoIJ<double>* geo;
@@ -91,9 +92,12 @@ struct AdjRow { double r2, t1, t2, t3, t4, p1, p3, p4, p5; };
 // One reverse stage of the NF fields (RHS_Uran_Turb.cpp:92-850): per cell (every row, every distinct
 // meridian; the seam copy k = km-1 is read by no stencil and receives nothing) the sum of what the cells
 // whose stencils contain it send; added into ybar, phbar and pdbar; and the previous stage's kbar and pe on
-// the interior. A neighbour off the interior sends nothing: its weights are zero and the cell's own place is
-// read instead, so that every load is unconditional and issued before the first use (branches made each
-// neighbour's loads wait for the one before). A cell sends its tendency adjoint times
+// the interior. A neighbour off the interior sends nothing: the cell (0, 0, 0), where every kbar and pe is 0,
+// is read in its place, so that every load is unconditional and issued before the first use (branches made
+// each neighbour's loads wait for the one before; one around the species' sums, 40 us a moist stage). What
+// else is read there counts as 0 by a select, not by a zero weight: it may be a NaN (the boundary rows of a
+// stage input are never written, those of the aux adjoint are the caller's). A cell sends its tendency
+// adjoint times
 //   transport: -wind * (r1, t1 or p1);  diffusion: D * (first- and second-order weights of its row),
 // the same weight for every field but its D (and u's own radial term), so a neighbour costs one weight per
 // D and one multiply-add per field. The rows' weights are formed once per block in shared memory.
@@ -135,8 +139,8 @@ __global__ void __launch_bounds__(128, NF == ADJ_NF ? 4 : 2) adj_stage_kernel(co
     const bool ini = i >= 1 && i <= g.im - 2, inj = j >= 1 && j <= g.jm - 2;
     const bool in = ini && inj;
     const bool nb[6] = {inj && i >= 2, inj && i <= g.im - 3, ini && j >= 2, ini && j <= g.jm - 3, in, in};
-    const int on[6] = {nb[0] ? o - si : o, nb[1] ? o + si : o, nb[2] ? o - sj : o, nb[3] ? o + sj : o,
-                       o - k + phi_wrap(k - 1, g.km), o - k + phi_wrap(k + 1, g.km)};
+    const int on[6] = {nb[0] ? o - si : 0, nb[1] ? o + si : 0, nb[2] ? o - sj : 0, nb[3] ? o + sj : 0,
+                       in ? o - k + phi_wrap(k - 1, g.km) : 0, in ? o - k + phi_wrap(k + 1, g.km) : 0};
     // the stencil's own places (boundary rows from the step's input)
     const int oc[4] = {in ? o - si : o, in ? o + si : o, in ? o - sj : o, in ? o + sj : o};
     const double* const kb[ADJ_NF] = {a.kbar, a.kbar + (size_t)fs, a.kbar + 2 * (size_t)fs, a.kbar + 3 * (size_t)fs};
@@ -148,7 +152,8 @@ __global__ void __launch_bounds__(128, NF == ADJ_NF ? 4 : 2) adj_stage_kernel(co
         at[d] = __ldg(kb[0] + q); au[d] = __ldg(kb[1] + q); av[d] = __ldg(kb[2] + q); aw[d] = __ldg(kb[3] + q);
         nt[d] = __ldg(a.nt + q);
         if(d < 6){
-            wn[d] = __ldg(a.X + (size_t)(1 + d / 2) * fs + q);
+            const double wx = __ldg(a.X + (size_t)(1 + d / 2) * fs + q);
+            wn[d] = nb[d] ? wx : 0.0;
             pe[d] = __ldg(a.pe + q);
             a0[d] = d < 2 ? au[d] : (d < 4 ? av[d] : aw[d]);
         }
@@ -170,7 +175,9 @@ __global__ void __launch_bounds__(128, NF == ADJ_NF ? 4 : 2) adj_stage_kernel(co
 #pragma unroll
         for(int d = 0; d < 7; d++){
             const int q = d < 6 ? on[d] : o;
-            au[d] += __ldg(a.auxbar + q); av[d] += __ldg(a.auxbar + (size_t)fs + q); aw[d] += __ldg(a.auxbar + 2 * (size_t)fs + q);
+            const double bu = __ldg(a.auxbar + q), bv = __ldg(a.auxbar + (size_t)fs + q), bw = __ldg(a.auxbar + 2 * (size_t)fs + q);
+            const bool use = d < 6 ? nb[d] : in;
+            au[d] += use ? bu : 0.0; av[d] += use ? bv : 0.0; aw[d] += use ? bw : 0.0;
         }
     }
     const double ire = K.inv_re_eff, irp = K.inv_re_pr, i09 = 1.0 / 0.9;
@@ -217,20 +224,19 @@ __global__ void __launch_bounds__(128, NF == ADJ_NF ? 4 : 2) adj_stage_kernel(co
     for(int d = 0; d < 6; d++){
         const AdjRow& R = rows[d == 0 ? 6 + tj : (d == 1 ? 10 + tj : (d == 2 ? tj : (d == 3 ? 2 + tj : 1 + tj)))];
         const double sg = (d & 1) ? -1.0 : 1.0;         // the first differences' sign: + from the lower neighbour
-        const double m = nb[d] ? 1.0 : 0.0;
         const double D = ire + nt[d], Dt = irp + nt[d] * i09;
-        const double c = m * sg * (d < 2 ? K.inv_2dr : (d < 4 ? R.t1 : R.p1));
+        const double c = sg * (d < 2 ? K.inv_2dr : (d < 4 ? R.t1 : R.p1));
         cw[d] = -wn[d] * c;
-        cd[d] = d < 2 ? m * (sg * R.r2 + K.inv_dr2) : (d < 4 ? m * (sg * R.t2 + R.t3) : m * R.p3);
+        cd[d] = d < 2 ? sg * R.r2 + K.inv_dr2 : (d < 4 ? sg * R.t2 + R.t3 : R.p3);
         const double WT = cw[d] + Dt * cd[d], WD = cw[d] + D * cd[d];
         xt += at[d] * WT; xv += av[d] * WD; xw += aw[d] * WD;
-        if(d < 2) xu += au[d] * (WD + D * (m * sg * R.r2));
+        if(d < 2) xu += au[d] * (WD + D * (sg * R.r2));
         else {
             xu += au[d] * WD;
-            if(d < 4){ xu += av[d] * (m * sg * R.t4 * D); h -= av[d] * c; }
+            if(d < 4){ xu += av[d] * (sg * R.t4 * D); h -= av[d] * c; }
             else {
-                const double c5 = m * sg * R.p5 * D;
-                xu += aw[d] * (m * sg * R.p4 * D); xv += aw[d] * c5; xw -= av[d] * c5;
+                const double c5 = sg * R.p5 * D;
+                xu += aw[d] * (sg * R.p4 * D); xv += aw[d] * c5; xw -= av[d] * c5;
                 h -= aw[d] * c;
             }
         }
@@ -267,10 +273,10 @@ __global__ void __launch_bounds__(128, NF == ADJ_NF ? 4 : 2) adj_stage_kernel(co
             for(int n = 0; n < 3; n++){
                 const size_t f = (size_t)(ADJ_NF + 3 * gi + n) * fs;
                 double x = aq[n] * W0;
-                // inv_rm and inv_rs are 0 off the interior, where aq is 0 too
-                xu -= aq[n] * ((rq[n].rp - rq[n].rm) * K.inv_2dr);
-                xv -= aq[n] * inv_rm * ((rq[n].tp - rq[n].tm) * K.inv_2dthe);
-                xw -= aq[n] * inv_rs * ((rq[n].pe - rq[n].pw) * K.inv_2dphi);
+                const double sr = rq[n].rp - rq[n].rm, st = rq[n].tp - rq[n].tm, sp = rq[n].pe - rq[n].pw;
+                xu -= aq[n] * ((in ? sr : 0.0) * K.inv_2dr);
+                xv -= aq[n] * inv_rm * ((in ? st : 0.0) * K.inv_2dthe);
+                xw -= aq[n] * inv_rs * ((in ? sp : 0.0) * K.inv_2dphi);
 #pragma unroll
                 for(int d = 0; d < 6; d++) x += an[n][d] * W[d];
                 a.ybar[f + o] = yb[n] + x;

@@ -1708,7 +1708,7 @@ int aturan_tape(aturan_ctx* ctx, int on){
     const size_t bytes = (nf * fs + (1 + 2 * ADJ_LB) * (size_t)g.im) * sizeof(double);
     void* mem = nullptr;
     if(cudaMalloc(&mem, bytes) != cudaSuccess){ cudaGetLastError(); return fail(ctx, ATURAN_E_NOMEM, "tape allocation"); }
-    CK(cudaMemsetAsync(mem, 0, bytes, ctx->st));      // kbar, pe and the aux adjoint stay zero off the interior
+    CK(cudaMemsetAsync(mem, 0, bytes, ctx->st));      // kbar and pe stay zero off the interior
     double* cur = reinterpret_cast<double*>(mem);
     auto take = [&](size_t n){ double* r = cur; cur += n; return r; };
     ctx->tape = reinterpret_cast<double*>(mem);
