@@ -126,6 +126,8 @@ __global__ void __launch_bounds__(128, NF == ADJ_NF ? 4 : 2) adj_stage_kernel(co
             w.t3 = G.inv_rm2 * K.inv_dthe2; w.t4 = 2.0 * G.inv_rm2 * K.inv_2dthe;
             w.p1 = G.inv_rmsinthe * K.inv_2dphi; w.p3 = G.inv_rm2sinthe2 * K.inv_dphi2;
             w.p4 = 2.0 * G.inv_rm2sinthe * K.inv_2dphi; w.p5 = 2.0 * G.costhe * G.inv_rm2sinthe2 * K.inv_2dphi;
+            // no cell of a row off the interior sends anything, and a pole's metric may be infinite
+            if(ri < 1 || ri > g.im - 2 || rj < 1 || rj > g.jm - 2) w = AdjRow{};
             rows[r] = w;
         }
         __syncthreads();

@@ -18,9 +18,11 @@ def _boundary(a, value):
     return a
 
 
-def _gradient(shape, moist, aux_off=0.0, leftovers=False):
+def _gradient(shape, moist, aux_off=0.0, leftovers=False, **params):
     """xbar and pbar of one taped step with random cotangents; aux_off: the aux cotangent off the interior."""
     p = P.default_params(*shape)
+    for n, v in params.items():
+        setattr(p, n, v)
     st = S.synthetic_state(p, seed=71)
     names = MOIST if moist else DRY
     ctx = api.Context(p)
@@ -70,3 +72,13 @@ def test_aux_cotangent_off_the_interior_is_not_read(shape, moist):
 @pytest.mark.parametrize("shape", SHAPES)
 def test_leftovers_in_the_stage_buffers_are_not_read(shape, moist):
     _same(_gradient(shape, moist), _gradient(shape, moist, leftovers=True))
+
+
+@pytest.mark.parametrize("moist", [False, True])
+@pytest.mark.parametrize("shape", SHAPES)
+def test_a_pole_without_a_metric_floor(shape, moist):
+    """sin = 0 on the pole's row and no floor: its weights are infinite, and nothing reads them."""
+    p = P.default_params(*shape)
+    assert p.the0 == 0.0
+    for n, x in _gradient(shape, moist, sinthe_min=0.0).items():
+        assert np.isfinite(x).all(), n
