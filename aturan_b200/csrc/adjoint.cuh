@@ -151,33 +151,33 @@ __global__ void __launch_bounds__(128, NF == ADJ_NF ? 4 : 2) adj_stage_kernel(co
 #pragma unroll
     for(int d = 0; d < 7; d++){
         const int q = d < 6 ? on[d] : o;
-        at[d] = __ldg(kb[0] + q); au[d] = __ldg(kb[1] + q); av[d] = __ldg(kb[2] + q); aw[d] = __ldg(kb[3] + q);
-        nt[d] = __ldg(a.nt + q);
+        at[d] = ldr(kb[0] + q); au[d] = ldr(kb[1] + q); av[d] = ldr(kb[2] + q); aw[d] = ldr(kb[3] + q);
+        nt[d] = ldr(a.nt + q);
         if(d < 6){
-            const double wx = __ldg(a.X + (size_t)(1 + d / 2) * fs + q);
+            const double wx = ldr(a.X + (size_t)(1 + d / 2) * fs + q);
             wn[d] = nb[d] ? wx : 0.0;
-            pe[d] = __ldg(a.pe + q);
+            pe[d] = ldr(a.pe + q);
             a0[d] = d < 2 ? au[d] : (d < 4 ? av[d] : aw[d]);
         }
     }
     auto stencil = [&](int q) -> R7<double> {
         const size_t f = (size_t)q * fs;
         R7<double> r;
-        r.c  = __ldg(a.X + f + o);
-        r.rm = __ldg(xsrc[0] + f + oc[0]); r.rp = __ldg(xsrc[1] + f + oc[1]);
-        r.tm = __ldg(xsrc[2] + f + oc[2]); r.tp = __ldg(xsrc[3] + f + oc[3]);
-        r.pw = __ldg(a.X + f + on[4]);     r.pe = __ldg(a.X + f + on[5]);
+        r.c  = ldr(a.X + f + o);
+        r.rm = ldr(xsrc[0] + f + oc[0]); r.rp = ldr(xsrc[1] + f + oc[1]);
+        r.tm = ldr(xsrc[2] + f + oc[2]); r.tp = ldr(xsrc[3] + f + oc[3]);
+        r.pw = ldr(a.X + f + on[4]);     r.pe = ldr(a.X + f + on[5]);
         return r;
     };
     const R7<double> rT = stencil(0), rU = stencil(1), rV = stencil(2), rW = stencil(3);
     const double* P = a.pdyn;
-    const double p_im = __ldg(P + oc[0]), p_ip = __ldg(P + oc[1]), p_jm = __ldg(P + oc[2]), p_jp = __ldg(P + oc[3]);
-    const double p_kw = __ldg(P + on[4]), p_ke = __ldg(P + on[5]);
+    const double p_im = ldr(P + oc[0]), p_ip = ldr(P + oc[1]), p_jm = ldr(P + oc[2]), p_jp = ldr(P + oc[3]);
+    const double p_kw = ldr(P + on[4]), p_ke = ldr(P + on[5]);
     if(a.auxbar){                                       // the aux adjoint joins every partial but those in p_dyn
 #pragma unroll
         for(int d = 0; d < 7; d++){
             const int q = d < 6 ? on[d] : o;
-            const double bu = __ldg(a.auxbar + q), bv = __ldg(a.auxbar + (size_t)fs + q), bw = __ldg(a.auxbar + 2 * (size_t)fs + q);
+            const double bu = ldr(a.auxbar + q), bv = ldr(a.auxbar + (size_t)fs + q), bw = ldr(a.auxbar + 2 * (size_t)fs + q);
             const bool use = d < 6 ? nb[d] : in;
             au[d] += use ? bu : 0.0; av[d] += use ? bv : 0.0; aw[d] += use ? bw : 0.0;
         }
@@ -267,9 +267,9 @@ __global__ void __launch_bounds__(128, NF == ADJ_NF ? 4 : 2) adj_stage_kernel(co
                 const size_t f = (size_t)(ADJ_NF + 3 * gi + n) * fs;
                 const double* kq = a.kbar + f;
 #pragma unroll
-                for(int d = 0; d < 6; d++) an[n][d] = __ldg(kq + on[d]);
+                for(int d = 0; d < 6; d++) an[n][d] = ldr(kq + on[d]);
                 rq[n] = stencil(ADJ_NF + 3 * gi + n);
-                aq[n] = __ldg(kq + o); yb[n] = a.ybar[f + o]; g0[n] = __ldg(a.g0 + f + o);
+                aq[n] = ldr(kq + o); yb[n] = a.ybar[f + o]; g0[n] = ldr(a.g0 + f + o);
             }
 #pragma unroll
             for(int n = 0; n < 3; n++){
@@ -296,8 +296,8 @@ __global__ void __launch_bounds__(128, NF == ADJ_NF ? 4 : 2) adj_stage_kernel(co
     double tp = 0.0;
     if(prev){
 #pragma unroll
-        for(int q = 0; q < ADJ_NF; q++) gb[q] = __ldg(a.g0 + (size_t)q * fs + o);
-        tp = __ldg(a.Xprev + o);
+        for(int q = 0; q < ADJ_NF; q++) gb[q] = ldr(a.g0 + (size_t)q * fs + o);
+        tp = ldr(a.Xprev + o);
     }
 #pragma unroll
     for(int q = 0; q < ADJ_NF; q++) a.ybar[(size_t)q * fs + o] = yb[q] + x[q];
@@ -452,8 +452,8 @@ __global__ void __launch_bounds__(128) adj_satadj_kernel(Grid g, const double* p
     for(int gi = 0; gi < 4; gi++){
         const size_t f = (size_t)base[gi] * fs + q;
 #pragma unroll
-        for(int n = 0; n < 3; n++){ pv[gi][n] = __ldg(pre + f + n * fs); yv[gi][n] = ybar[f + n * fs]; }
-        qv[gi][0] = __ldg(post + f + fs); qv[gi][1] = __ldg(post + f + 2 * fs);
+        for(int n = 0; n < 3; n++){ pv[gi][n] = ld(pre + f + n * fs); yv[gi][n] = ybar[f + n * fs]; }
+        qv[gi][0] = ld(post + f + fs); qv[gi][1] = ld(post + f + 2 * fs);
     }
     const double yt = ybar[q];
     // forward replay: each gas's entry record and the temperature after it
@@ -643,7 +643,7 @@ __global__ void __launch_bounds__(128) adj_level_apply_kernel(Grid g, const doub
     const int m = blockIdx.z;
     double R = 0.0, W = 0.0;
 #pragma unroll
-    for(int b = 0; b < ADJ_LB; b++){ R += __ldg(lev + 2 * (m * ADJ_LB + b)); W += __ldg(lev + 2 * (m * ADJ_LB + b) + 1); }
+    for(int b = 0; b < ADJ_LB; b++){ R += ld(lev + 2 * (m * ADJ_LB + b)); W += ld(lev + 2 * (m * ADJ_LB + b) + 1); }
     if(k >= g.km) return;
     const size_t o = gidx(g, m, j, k);
     const double T = t[o];

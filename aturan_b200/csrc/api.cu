@@ -1798,8 +1798,8 @@ int rk4_adjoint_impl(aturan_ctx* ctx, int nf, const double* const* ybar, const d
         a.auxbar = (stage == 3 && auxbar) ? ctx->aaux : nullptr;   // aux is stage 3's output
         a.w_prev = prev >= 0 ? dt / 6.0 * ((prev == 0 || prev == 3) ? 1.0 : 2.0) : 0.0;
         a.c_prev = prev >= 0 ? ((prev == 0 || prev == 1) ? 0.5 * dt : (prev == 2 ? dt : 0.0)) : 0.0;
-        if(nf == ADJ_NF_MOIST) chain(adj_stage_kernel<ADJ_NF_MOIST>, gs, dim3(32, 4), 0, ctx->st, a);
-        else chain(adj_stage_kernel<ADJ_NF>, gs, dim3(32, 4), 0, ctx->st, a);
+        if(nf == ADJ_NF_MOIST) adj_stage_kernel<ADJ_NF_MOIST><<<gs, dim3(32, 4), 0, ctx->st>>>(a);
+        else adj_stage_kernel<ADJ_NF><<<gs, dim3(32, 4), 0, ctx->st>>>(a);
         CK_LAUNCH("adjoint stage"); nl++;
     }
     const double* t0 = ctx->tX;

@@ -28,12 +28,12 @@ __host__ __device__ __forceinline__ double div_by(double a, double d, double y){
 // Launches of one stream follow one another by programmatic stream serialisation: the next kernel's
 // blocks are placed once the last block of the kernel before has exited, beside the flush of its
 // writes and the launch's own latency, and every kernel waits (chain_wait, its first statement) until
-// that flush is done before it touches memory. An empty kernel launched after another in a stream
+// that flush is done before it touches what another launch writes. An empty kernel launched after another in a stream
 // took 4.1 us and takes 2.0 so; eight dependent loads a thread, 600 blocks: 6.2 and 3.5. Only the point passes of
 // the pressure solves let their successor in before they end (sor_colour_kernel): elsewhere that was no
 // faster (3.5 to 4.6 us), and so a block never starts while one that may hold the successor's input in
-// its L1 still reads. A kernel that does not begin with chain_wait, or follows a point pass, is
-// launched the plain way.
+// its L1 still reads. A kernel that does not begin with chain_wait, reads what launches write by the read-only
+// path (ldr below), or follows a point pass, is launched the plain way.
 __device__ __forceinline__ void chain_wait(){ cudaGridDependencySynchronize(); }
 
 template <typename... E, typename... A>
@@ -55,6 +55,18 @@ inline cudaError_t chain(void (*kernel)(E...), dim3 grid, dim3 block, size_t sme
     return chain_if(true, kernel, grid, block, smem, st, std::forward<A>(args)...);
 }
 
+// A value that a launch writes, by a plain load. The read-only path (__ldg, or a const pointer with
+// __restrict__) wants memory that nobody writes while the kernel lives, and a chained kernel lives before
+// the one ahead of it has flushed its writes: the wait holds back neither a read-only load that the compiler
+// moves ahead of it nor one's cache. That path is for the tables formed with the context, for what the point
+// pass reads before its wait, and for kernels launched the plain way (ldr). Two of them gain more by it than
+// the chaining gave them: the FP64 momentum stage (the RK4 step at 41x181x361 with its transfers: 2.75 ms
+// chained with plain loads, 2.69 so) and the adjoint's reverse stage (dry gradient: 1.34 and 1.33 ms). The
+// others take the same time with either load.
+template <typename T>
+__device__ __forceinline__ T ld(const T* p){ return *p; }
+template <typename T>
+__device__ __forceinline__ T ldr(const T* p){ return __ldg(p); }
 
 struct Grid {
     int im, jm, km, kp;

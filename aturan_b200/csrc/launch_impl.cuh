@@ -60,7 +60,7 @@ void launch_momentum(const StageArgs<S, C>& a, dim3 grid2, cudaStream_t st){
     } else {
         const Grid& g = a.g;
         const dim3 grid((g.km - 1 + 31) / 32, (g.jm - 2 + 3) / 4, g.im - 2);
-        chain(rk_stage_kernel<S, C, StageCfg<S>::MINB1>, grid, dim3(32, 4), 0, st, a);
+        rk_stage_kernel<S, C, StageCfg<S>::MINB1><<<grid, dim3(32, 4), 0, st>>>(a);
     }
 }
 // damp_wiggles (lib/Utils.cpp:224-317) on x along the axes selected, k then j then i; lo: the low

@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(FT_K * FT_J) post_filter3_kernel(Grid g, const
     chain_wait();
     __shared__ double YK[2][FT_J + 2][FT_K];
     const int n = blockIdx.z / ni;
-    const S* __restrict__ x = f.x[n];
+    const S* x = f.x[n];
     const int tk = threadIdx.x, ty = threadIdx.y;              // 32 x 8
     const int k = blockIdx.x * FT_K + tk, j = blockIdx.y * FT_J + ty, i0 = (blockIdx.z - n * ni) * li;
     const int km = g.km;
@@ -160,8 +160,8 @@ __global__ void __launch_bounds__(FT_K * FT_J) post_filter3_kernel(Grid g, const
     S c, w, e, hc = S(0), hw = S(0), he = S(0);
     auto fetch = [&](int i){
         const size_t o = (size_t)min(max(i, 0), g.im - 1) * pl;
-        c = __ldg(row + o + kc); w = __ldg(row + o + km1); e = __ldg(row + o + kp1);
-        if(edge){ hc = __ldg(halo + o + kc); hw = __ldg(halo + o + km1); he = __ldg(halo + o + kp1); }
+        c = ld(row + o + kc); w = ld(row + o + km1); e = ld(row + o + kp1);
+        if(edge){ hc = ld(halo + o + kc); hw = ld(halo + o + km1); he = ld(halo + o + kp1); }
     };
     double ym = 0.0, y0 = 0.0;                                  // j passes of levels i - 2 and i - 1
     fetch(i0 - 1);

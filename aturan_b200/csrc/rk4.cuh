@@ -47,9 +47,6 @@ struct StageArgs {
     const float* tnlo;
 };
 
-template <typename S>
-__device__ __forceinline__ S ld(const S* p){ return __ldg(p); }
-
 template <typename C>
 __device__ __forceinline__ C cmax(C a, C b){ return (a < b) ? b : a; }   // std::max
 // x / d: the reference's division in the FP64 form; in the mixed form x times the reciprocal of
@@ -134,10 +131,10 @@ template <typename S, typename C>
 __device__ __forceinline__ R7<C> load7c(const S* X, const Cell& c, int q){
     const int f = q * c.fs;
     R7<C> r;
-    r.c  = (C)ld(X + (f + c.o));
-    r.rp = (C)ld(X + (f + c.oip)); r.rm = (C)ld(X + (f + c.oim));
-    r.tp = (C)ld(X + (f + c.ojp)); r.tm = (C)ld(X + (f + c.ojm));
-    r.pe = (C)ld(X + (f + c.oke)); r.pw = (C)ld(X + (f + c.okw));
+    r.c  = (C)ldr(X + (f + c.o));
+    r.rp = (C)ldr(X + (f + c.oip)); r.rm = (C)ldr(X + (f + c.oim));
+    r.tp = (C)ldr(X + (f + c.ojp)); r.tm = (C)ldr(X + (f + c.ojm));
+    r.pe = (C)ldr(X + (f + c.oke)); r.pw = (C)ldr(X + (f + c.okw));
     return r;
 }
 
@@ -165,7 +162,7 @@ __device__ __forceinline__ AccNc<C> load_acc_nc(const StageArgs<S, C>& a, const 
     const int off = q * c.fs + c.o;
     AccNc<C> v;
     v.acc = (a.stage == 0) ? C(0.0) : (C)X[c.dacc + off];
-    v.nc = (C)ld(X + (c.dnc + off));
+    v.nc = (C)ldr(X + (c.dnc + off));
     return v;
 }
 
@@ -270,16 +267,16 @@ __device__ __forceinline__ void load_momentum(MomIn<C>& in, const StageArgs<S, C
     const double* P = a.pdyn;                   // FP64, no boundary substitution: offsets from the cell
     const double* PH = a.phydro;
     const int JK = a.g.jm * a.g.kp, kp = a.g.kp;
-    in.p_ip = ld(P + (c.o + JK)); in.p_im = ld(P + (c.o - JK)); in.p_jp = ld(P + (c.o + kp)); in.p_jm = ld(P + (c.o - kp));
-    in.p_ke = ld(P + c.oke); in.p_kw = ld(P + c.okw);
-    in.ph_jp = ld(PH + (c.o + kp)); in.ph_jm = ld(PH + (c.o - kp)); in.ph_ke = ld(PH + c.oke); in.ph_kw = ld(PH + c.okw);
+    in.p_ip = ldr(P + (c.o + JK)); in.p_im = ldr(P + (c.o - JK)); in.p_jp = ldr(P + (c.o + kp)); in.p_jm = ldr(P + (c.o - kp));
+    in.p_ke = ldr(P + c.oke); in.p_kw = ldr(P + c.okw);
+    in.ph_jp = ldr(PH + (c.o + kp)); in.ph_jm = ldr(PH + (c.o - kp)); in.ph_ke = ldr(PH + c.oke); in.ph_kw = ldr(PH + c.okw);
     in.rU = load7c<S, C>(X, c, ATURAN_U); in.rV = load7c<S, C>(X, c, ATURAN_V); in.rW = load7c<S, C>(X, c, ATURAN_W);
     in.rT = load7c<S, C>(X, c, ATURAN_T);
     in.anU = load_acc_nc(a, X, c, ATURAN_U); in.anV = load_acc_nc(a, X, c, ATURAN_V);
     in.anW = load_acc_nc(a, X, c, ATURAN_W); in.anT = load_acc_nc(a, X, c, ATURAN_T);
     const S* F = X + (c.dforc + c.o);
-    in.f_tmf = (K.tmf != C(0.0)) ? (C)ld(F + (ATURAN_THERMALMASSFLUX - ATURAN_NUE) * c.fs) : C(0.0);
-    in.f_qp = (K.precip_coupling != C(0.0)) ? (C)ld(F + (ATURAN_Q_PRECIP - ATURAN_NUE) * c.fs) : C(0.0);
+    in.f_tmf = (K.tmf != C(0.0)) ? (C)ldr(F + (ATURAN_THERMALMASSFLUX - ATURAN_NUE) * c.fs) : C(0.0);
+    in.f_qp = (K.precip_coupling != C(0.0)) ? (C)ldr(F + (ATURAN_Q_PRECIP - ATURAN_NUE) * c.fs) : C(0.0);
 }
 
 // The tendencies of u, v, w and t of one cell (RHS_Uran_Turb.cpp:117-175, :208-331, :382-391,
@@ -379,7 +376,7 @@ template <> struct Pair<double> { using T = double2; };
 
 template <typename S, typename C>
 __device__ __forceinline__ void ld2(const S* p, C& x, C& y){
-    const typename Pair<S>::T v = __ldg(reinterpret_cast<const typename Pair<S>::T*>(p));
+    const typename Pair<S>::T v = ld(reinterpret_cast<const typename Pair<S>::T*>(p));
     x = (C)v.x; y = (C)v.y;
 }
 template <typename S, typename C>
@@ -658,7 +655,7 @@ __global__ void __launch_bounds__(128, MINB) rk_stage_kernel(const StageArgs<S, 
     S* W = const_cast<S*>(a.X);
     const Cell c = make_cell(a, i, j, k, 1);
 
-    const C nue_c = (C)ld(X + (c.dforc + c.o));                 // ATURAN_NUE, the forcing group's first
+    const C nue_c = (C)ldr(X + (c.dforc + c.o));                // ATURAN_NUE, the forcing group's first
     const C nue_t = (K.turb_coupling != C(0.0) && isfinite(nue_c)) ? K.turb_coupling * cmax(C(0.0), nue_c) : C(0.0);
     const C nue_t_s = qdiv(nue_t, C(0.9), C(1.0 / 0.9));
 
@@ -714,7 +711,7 @@ __device__ __forceinline__ void load_momentum2(MomIn<C>& A, MomIn<C>& B, const S
     const double* PH = a.phydro;
     const int JK = a.g.jm * a.g.kp, kp = a.g.kp;
     auto ldd2 = [](const double* p, double& x, double& y){
-        const double2 v = __ldg(reinterpret_cast<const double2*>(p)); x = v.x; y = v.y;
+        const double2 v = ld(reinterpret_cast<const double2*>(p)); x = v.x; y = v.y;
     };
     ldd2(P + (c.o + JK), A.p_ip, B.p_ip); ldd2(P + (c.o - JK), A.p_im, B.p_im);
     ldd2(P + (c.o + kp), A.p_jp, B.p_jp); ldd2(P + (c.o - kp), A.p_jm, B.p_jm);
@@ -795,9 +792,9 @@ __global__ void __launch_bounds__(256) buoy_partial_kernel(Grid g, const S* t, c
     for(int c = blockIdx.x * blockDim.x + threadIdx.x; c < ncell; c += nblk * blockDim.x){
         const int j = c / g.km, k = c - j * g.km;
         const size_t o = gidx(g, lev, j, k);
-        const double T = (double)__ldg(t + o);
+        const double T = (double)ld(t + o);
         if(!(T > 0.0)) continue;
-        const double b = h.g * (double)__ldg(ps + o) / (h.rR * T * h.t_ref);
+        const double b = h.g * (double)ld(ps + o) / (h.rR * T * h.t_ref);
         if(!isfinite(b)) continue;
         const double wg = wsin[j];
         s += wg * b;
@@ -856,9 +853,9 @@ __global__ void __launch_bounds__(BX_CH) buoy_terms_kernel(Grid g, const S* t, c
     if(c < ncell){
         const int j = c / g.km, k = c - j * g.km;
         const size_t o = gidx(g, lev, j, k);
-        const double T = (double)__ldg(t + o);
+        const double T = (double)ld(t + o);
         if(T > 0.0){
-            const double b = h.g * (double)__ldg(ps + o) / (h.rR * T * h.t_ref);
+            const double b = h.g * (double)ld(ps + o) / (h.rR * T * h.t_ref);
             if(isfinite(b)){ const double wg = wsin[j]; bv = wg * b; wv = wg; }
         }
         double* xb = terms + (size_t)lev * 2 * ncell;
@@ -1106,12 +1103,9 @@ constexpr int HYD_CH = 48;          // levels per chunk (41 levels: one chunk)
 
 // ROWS threads per column in phases 1 and 3 (HYD_CH / ROWS levels each); MINB resident blocks.
 template <typename S, int ROWS, int MINB>
-__global__ void __launch_bounds__(32 * ROWS, MINB) hydro_kernel(Grid g, const S* __restrict__ t, const S* __restrict__ ps,
-                                                    const S* __restrict__ v, const S* __restrict__ w,
-                                                    const double* __restrict__ ref, const double* __restrict__ rm_i,
-                                                    const double* __restrict__ cor_j, const double* __restrict__ pbaro,
-                                                    const double* __restrict__ pb0, double* __restrict__ pbf,
-                                                    double* __restrict__ ph, HydroConst h, int advance){
+__global__ void __launch_bounds__(32 * ROWS, MINB) hydro_kernel(Grid g, const S* t, const S* ps, const S* v, const S* w, const double* ref,
+                                                    const double* rm_i, const double* cor_j, const double* pbaro,
+                                                    const double* pb0, double* __restrict__ pbf, double* __restrict__ ph, HydroConst h, int advance){
     chain_wait();
     constexpr int HYD_PER = HYD_CH / ROWS;
     static_assert(HYD_CH % ROWS == 0, "a chunk splits evenly over the rows");
@@ -1139,7 +1133,7 @@ __global__ void __launch_bounds__(32 * ROWS, MINB) hydro_kernel(Grid g, const S*
                 const int r = ty + q * ROWS;
                 if(r < n){
                     const size_t o = gidx(g, i0 + r, j, k);
-                    tv[q] = __ldg(t + o); pv[q] = __ldg(ps + o); vv[q] = __ldg(v + o); wv[q] = __ldg(w + o);
+                    tv[q] = ld(t + o); pv[q] = ld(ps + o); vv[q] = ld(v + o); wv[q] = ld(w + o);
                 }
             }
 #pragma unroll

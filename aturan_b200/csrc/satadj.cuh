@@ -107,9 +107,9 @@ __global__ void __launch_bounds__(NT, 1024 / NT) satadj_kernel(const SatArgs<S> 
         const size_t q = gidx(g, i, j, k);
         const SatConst& K = a.k;
         double tt = t_ld(a.t, a.tlo, q);
-        const double p_u = (double)__ldg(a.ps + q);
+        const double p_u = (double)ld(a.ps + q);
         double rho_c = K.r_mix;                               // rho_at, cUranusModel.h:526-531
-        if(K.local_rho){ const double r_ = (double)__ldg(a.rho_mix + q); rho_c = (r_ > 0.0 && isfinite(r_)) ? r_ : K.r_mix; }
+        if(K.local_rho){ const double r_ = (double)ld(a.rho_mix + q); rho_c = (r_ > 0.0 && isfinite(r_)) ? r_ : K.r_mix; }
         const double cp_mix = K.cp_mix, t_ref = K.t_ref;
         // latent heat to temperature: x / (cp_mix rho_c), a multiplication in the mixed form
         const double inv_hc = FAST ? 1.0 / (cp_mix * rho_c) : 0.0;

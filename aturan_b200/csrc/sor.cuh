@@ -60,7 +60,7 @@ __device__ __forceinline__ double folded_acc(const Grid& g, const T* P, size_t o
                                              const RBW4& W, double* diag){
     const size_t si = (size_t)g.jm * g.kp, sj = g.kp;
     const int kw = phi_wrap(k - 1, g.km), ke = phi_wrap(k + 1, g.km);
-    auto p = [&](size_t q){ return (double)__ldg(P + q); };
+    auto p = [&](size_t q){ return (double)ld(P + q); };
     double d = W.den;
     double aim, aip, ajm, ajp;
     if(i == 1)        { d -= C43 * W.num1; aim = -C13 * p(o + si); } else aim = p(o - si);
@@ -88,7 +88,7 @@ __device__ __forceinline__ double folded_accT(const Grid& g, const T* P, size_t 
     if(j == 1)        d -= C43 * W.num2;
     if(j == g.jm - 2) d -= C43 * W.num2;
     *diag = d;
-    auto p = [&](size_t q){ return (double)__ldg(P + q); };
+    auto p = [&](size_t q){ return (double)ld(P + q); };
     double acc = (p(o - k + ke) + p(o - k + kw)) * W.num3;
     if(i - 1 >= 1)        acc += __ldg(&w[(i - 1) * g.jm + j].num1) * (i - 1 == 1 ? 1.0 - C13 : 1.0) * p(o - si);
     if(i + 1 <= g.im - 2) acc += __ldg(&w[(i + 1) * g.jm + j].num1) * (i + 1 == g.im - 2 ? 1.0 - C13 : 1.0) * p(o + si);
@@ -149,9 +149,9 @@ __global__ void __launch_bounds__(256) sor_colsum_kernel(Grid g, const T* P, con
                     const size_t o = gidx(g, i, j, k);
                     double diag;
                     const double acc = row_acc<TR, T>(g, P, o, i, j, k, w, &diag);
-                    const double lc = acc - diag * (double)__ldg(P + o);
+                    const double lc = acc - diag * (double)ld(P + o);
                     // the same subtraction as sor_shift_kernel
-                    const double s = shift ? (double)src[o] - sh : (double)__ldg(src + o);
+                    const double s = shift ? (double)src[o] - sh : (double)ld(src + o);
                     sv[c] = s;
                     rv[c] = s - lc;
                 }
@@ -615,9 +615,9 @@ __global__ void __launch_bounds__(256, 4) sor_line_kernel(Grid g, T* P, const T*
                 const int i = i0 + 8 * q;
                 if(i <= n && valid[h]){
                     const size_t o = gidx(g, i, j, k);
-                    vjm[q] = __ldg(P + (o - sj)); vjp[q] = __ldg(P + (o + sj));
-                    vke[q] = __ldg(P + (o - k + ke)); vkw[q] = __ldg(P + (o - k + kw));
-                    vr[q] = __ldg(R + o);
+                    vjm[q] = ld(P + (o - sj)); vjp[q] = ld(P + (o + sj));
+                    vke[q] = ld(P + (o - k + ke)); vkw[q] = ld(P + (o - k + kw));
+                    vr[q] = ld(R + o);
                     n2[q] = __ldg(&w[i * g.jm + j].num2); n3[q] = __ldg(&w[i * g.jm + j].num3);
                     if constexpr(TR){
                         n2m[q] = (j - 1 >= 1) ? __ldg(&w[i * g.jm + j - 1].num2) : 0.0;
