@@ -333,17 +333,55 @@ float* t_lo_of(aturan_ctx* c, int id){
     return nullptr;
 }
 
-// n contiguous FP64 arrays into (in) or out of consecutive padded FP64 fields from pad on, fs apart.
-cudaError_t pack_doubles(const Grid& g, int n, const double* const* flat, double* pad, size_t fs, bool in, cudaStream_t st){
+// How a caller's buffer of n bytes may be touched: by a kernel (memory of the context's device, doubles on
+// 8-byte boundaries), only by a copy (another device's memory, any alignment), or not at all.
+enum Reach { REACH_NONE, REACH_COPY, REACH_KERNEL };
+Reach reach(const aturan_ctx* ctx, const void* p, size_t n){
+    Reach r = (reinterpret_cast<uintptr_t>(p) & 7) == 0 ? REACH_KERNEL : REACH_COPY;
+    for(const char* q : {(const char*)p, (const char*)p + n - 1}){
+        cudaPointerAttributes a;
+        if(cudaPointerGetAttributes(&a, q) != cudaSuccess){ cudaGetLastError(); return REACH_NONE; }
+        if(a.type == cudaMemoryTypeUnregistered) return REACH_NONE;
+        if(a.type != cudaMemoryTypeDevice || a.device != ctx->device) r = REACH_COPY;
+    }
+    return r;
+}
+
+// n of the caller's contiguous FP64 arrays into (in) or out of consecutive padded FP64 fields from pad on:
+// one launch where a kernel reaches them all, else (and where outputs overlap: the later field is then
+// what stays) a copy per field.
+int pack_doubles(aturan_ctx* ctx, int n, const double* const* flat, double* pad, bool in){
+    const Grid& g = ctx->g;
+    const size_t rows = (size_t)g.im * g.jm, bytes = rows * g.km * 8;
+    bool direct = true;
+    for(int q = 0; q < n; q++){
+        const Reach r = reach(ctx, flat[q], bytes);
+        if(r == REACH_NONE) return fail(ctx, ATURAN_E_INVALID, "not a device buffer of im*jm*km doubles");
+        direct = direct && r == REACH_KERNEL;
+        for(int o = 0; !in && o < q; o++){
+            const uintptr_t a = reinterpret_cast<uintptr_t>(flat[q]), b = reinterpret_cast<uintptr_t>(flat[o]);
+            if((a > b ? a - b : b - a) < bytes) direct = false;
+        }
+    }
+    if(!direct){
+        for(int q = 0; q < n; q++){
+            double* const f = pad + q * g.fstride;
+            double* const c = const_cast<double*>(flat[q]);
+            if(in) CK(cudaMemcpy2DAsync(f, g.kp * 8, c, g.km * 8, g.km * 8, rows, cudaMemcpyDeviceToDevice, ctx->st));
+            else   CK(cudaMemcpy2DAsync(c, g.km * 8, f, g.kp * 8, g.km * 8, rows, cudaMemcpyDeviceToDevice, ctx->st));
+        }
+        return ATURAN_OK;
+    }
     PackBatch p;
     for(int q = 0; q < n; q++){
         p.flat[q] = flat[q];
-        p.dev[q] = pad + q * fs;
+        p.dev[q] = pad + q * g.fstride;
         p.lo[q] = nullptr;
         p.kind[q] = PACK_F64;
     }
-    launch_pack(p, n, g.km, g.kp, (size_t)g.im * g.jm, in, st);
-    return cudaGetLastError();
+    launch_pack(p, n, g.km, g.kp, rows, in, ctx->st);
+    CK_LAUNCH(in ? "layout in" : "layout out");
+    return ATURAN_OK;
 }
 
 template <typename S>
@@ -1763,8 +1801,8 @@ int rk4_adjoint_impl(aturan_ctx* ctx, int nf, const double* const* ybar, const d
     Region reg(ctx, ATURAN_K_ADJOINT, 0);
     long nl = 0;
     // the caller's ybar' (and the aux adjoint) into the padded layout
-    CK(pack_doubles(g, nf, ybar, ctx->ag0, fs, true, ctx->st));
-    if(auxbar) CK(pack_doubles(g, 3, auxbar, ctx->aaux, fs, true, ctx->st));
+    int rc = pack_doubles(ctx, nf, ybar, ctx->ag0, true); if(rc) return rc;
+    if(auxbar){ rc = pack_doubles(ctx, 3, auxbar, ctx->aaux, true); if(rc) return rc; }
     const RhsConst<double>& K = ctx->k64;
     const double t_min = K.t_min, t_max = K.t_max;
     const dim3 gc((g.km + 127) / 128, g.jm, g.im);
@@ -1818,8 +1856,8 @@ int rk4_adjoint_impl(aturan_ctx* ctx, int nf, const double* const* ybar, const d
         CK_LAUNCH("adjoint saturation adjustment"); nl++;
     }
     reg.n = nl;
-    CK(pack_doubles(g, nf, xbar, ctx->aybar, fs, false, ctx->st));
-    if(pbar) CK(pack_doubles(g, 1, &pbar, ctx->apdbar, fs, false, ctx->st));
+    rc = pack_doubles(ctx, nf, xbar, ctx->aybar, false); if(rc) return rc;
+    if(pbar){ rc = pack_doubles(ctx, 1, &pbar, ctx->apdbar, false); if(rc) return rc; }
     if(heatbar){
         chain(adj_heat_reduce_kernel, (g.jm * g.km + 255) / 256, 256, 0, ctx->st, g, ctx->ahacc, K.heat_scale, heatbar);
         CK_LAUNCH("heating adjoint");
@@ -1880,7 +1918,7 @@ int aturan_pressure_adjoint(aturan_ctx* ctx, int kind, double omega, int max_swe
     double* lam = ctx->akbar + fs;          // the source's adjoint
     double* sbar = ctx->akbar + 2 * fs;
     CK(cudaMemsetAsync(B, 0, 3 * fs * 8, ctx->st));
-    CK(pack_doubles(g, 1, &pbar, B, fs, true, ctx->st));
+    rc = pack_doubles(ctx, 1, &pbar, B, true); if(rc) return rc;
     // the boundary passes' adjoint, in reverse order
     chain(adj_pbc_p_kernel, (g.im * g.jm + 255) / 256, 256, 0, ctx->st, g, B);
     chain(adj_pbc_t_kernel, dim3((g.km + 127) / 128, g.im), 128, 0, ctx->st, g, B);
@@ -1904,7 +1942,7 @@ int aturan_pressure_adjoint(aturan_ctx* ctx, int kind, double omega, int max_swe
         g, sbar, ctx->rbw, ctx->pc, ctx->p.rigid_lid, aub, aub + fs, aub + 2 * fs);
     CK_LAUNCH("pressure adjoint: source");
     nl += 4;
-    CK(pack_doubles(g, 3, auxbar, aub, fs, false, ctx->st));
+    rc = pack_doubles(ctx, 3, auxbar, aub, false); if(rc) return rc;
     CK(cudaStreamSynchronize(ctx->st));
     reg.n = nl;
     if(sweeps_done) *sweeps_done = s;
@@ -2019,12 +2057,11 @@ int aturan_pressure_solve(aturan_ctx* ctx, int kind, int transposed, double omeg
     const bool line = kind == ATURAN_PRESS_RB_LINE;
     int rc = sor_check_sizes(ctx, omega, line); if(rc) return rc;
     if(max_sweeps < 1) max_sweeps = 1;
-    const Grid g = ctx->g;
     long nl = 0;
     Region reg(ctx, ATURAN_K_RB, 0);
     // working copies in the padded layout: the right-hand side in scratch, the iterate in stage64
-    CK(pack_doubles(g, 1, &b, ctx->scratch, g.fstride, true, ctx->st));
-    CK(pack_doubles(g, 1, &x, ctx->stage64, g.fstride, true, ctx->st));
+    rc = pack_doubles(ctx, 1, &b, ctx->scratch, true); if(rc) return rc;
+    rc = pack_doubles(ctx, 1, &x, ctx->stage64, true); if(rc) return rc;
     sor_compat(ctx, ctx->scratch, transposed != 0);
     CK_LAUNCH("solve right-hand side");
     nl += 3;
@@ -2038,7 +2075,7 @@ int aturan_pressure_solve(aturan_ctx* ctx, int kind, int transposed, double omeg
         : (transposed ? solve_fp64<true>(ctx, X, B, omega, max_sweeps, tol, line, &s, &r, nl)
                       : solve_fp64<false>(ctx, X, B, omega, max_sweeps, tol, line, &s, &r, nl));
     if(status < 0) return status;
-    CK(pack_doubles(g, 1, &x, ctx->stage64, g.fstride, false, ctx->st));
+    rc = pack_doubles(ctx, 1, &x, ctx->stage64, false); if(rc) return rc;
     CK(cudaStreamSynchronize(ctx->st));
     reg.n = nl;
     if(sweeps_done) *sweeps_done = s;
