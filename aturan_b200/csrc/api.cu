@@ -1609,21 +1609,30 @@ void* aturan_stream(aturan_ctx* ctx){ return ctx ? (void*)ctx->st : nullptr; }
 
 // The layout change of n fields to or from contiguous device buffers, on stream st: a launch per
 // PACK_MAX fields. At 41x181x361 a batch of FP64 fields moves at 6.5 TB/s, 6.6 us a field (13.6 us before).
+// A batch ends before a field, or an output buffer, that it already writes: the later one is what stays.
 static int pack_fields(aturan_ctx* ctx, int n, const int* fields, void* const* flat, bool in, cudaStream_t st){
     const Grid& g = ctx->g;
-    const size_t rows = (size_t)g.im * g.jm;
-    for(int q0 = 0; q0 < n; q0 += PACK_MAX){
+    const size_t rows = (size_t)g.im * g.jm, bytes = rows * g.km * 8;
+    auto again = [&](int q, int q0){
+        for(int o = q0; o < q; o++){
+            const uintptr_t a = reinterpret_cast<uintptr_t>(flat[q]), b = reinterpret_cast<uintptr_t>(flat[o]);
+            if(in ? fields[q] == fields[o] : (a > b ? a - b : b - a) < bytes) return true;
+        }
+        return false;
+    };
+    for(int q0 = 0; q0 < n;){
         PackBatch p;
-        const int m = std::min(PACK_MAX, n - q0);
-        for(int q = 0; q < m; q++){
+        int m = 0;
+        for(int q = q0; q < n && m < PACK_MAX && !again(q, q0); q++, m++){
             bool is64;
-            p.dev[q] = field_ptr(ctx, fields[q0 + q], &is64);
-            p.lo[q] = is64 ? nullptr : t_lo_of(ctx, fields[q0 + q]);
-            p.kind[q] = is64 ? PACK_F64 : (p.lo[q] ? PACK_PAIR : PACK_F32);
-            p.flat[q] = reinterpret_cast<const double*>(flat[q0 + q]);
+            p.dev[m] = field_ptr(ctx, fields[q], &is64);
+            p.lo[m] = is64 ? nullptr : t_lo_of(ctx, fields[q]);
+            p.kind[m] = is64 ? PACK_F64 : (p.lo[m] ? PACK_PAIR : PACK_F32);
+            p.flat[m] = reinterpret_cast<const double*>(flat[q]);
         }
         launch_pack(p, m, g.km, g.kp, rows, in, st);
         CK_LAUNCH(in ? "layout in" : "layout out");
+        q0 += m;
     }
     return ATURAN_OK;
 }
