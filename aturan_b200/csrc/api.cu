@@ -598,7 +598,7 @@ int sor_residual(aturan_ctx* ctx, const T* P, const T* src, bool want_col, int s
     const Grid g = ctx->g;
     double* src_w = nullptr;
     if constexpr(std::is_same<T, double>::value) src_w = shift ? const_cast<double*>(src) : nullptr;
-    chain(sor_colsum_kernel<T, TR>, dim3((g.km - 1 + 31) / 32, g.jm - 2), dim3(32, 8), 0, ctx->st, 
+    chain(sor_colsum_kernel<T, TR>, dim3((g.km - 1 + 31) / 32, g.jm - 2), dim3(32, 8), 0, ctx->st,
         g, P, src, ctx->rbw, ctx->sor_colR, ctx->sor_part, want_col ? 1 : 0, SorCheckArg{ctx->sor_check, slot, first, tol},
         fill32 ? ctx->r32 : nullptr, fill32 ? ctx->e32 : nullptr, src_w, src_w ? shift : nullptr);
     CK_LAUNCH("residual");
@@ -634,7 +634,9 @@ int sor_correct(aturan_ctx* ctx, T* P, T* x2){
                                             ctx->sor_Ac, ctx->sor_As, 1, c.J, kcf, sz_ac, stop);
     ModeLU lu = TR ? ModeLU{ctx->mluT_a, ctx->mluT_cf, ctx->mluT_idn} : ModeLU{ctx->mlu_a, ctx->mlu_cf, ctx->mlu_idn};
     const int pm = ctx->sor_pm;
-    chain(sor_tridiag_kernel, (c.NM + 1 + pm - 1) / pm, 128, (size_t)8 * c.J * (5 * pm + 4), ctx->st, 
+    const size_t tri = (size_t)8 * c.J * (5 * pm + 4);
+    smem_opt_in(sor_tridiag_kernel, tri);
+    chain(sor_tridiag_kernel, (c.NM + 1 + pm - 1) / pm, 128, tri, ctx->st,
         c, lu, ctx->sor_Ac, ctx->sor_As, pm, TR ? 1 : 0, SOR_KSPLIT, sz_ac, stop);
     const int kci = ((c.NM + 1 + SOR_KSPLIT - 1) / SOR_KSPLIT + 31) / 32 * 32;
     const dim3 gi((c.N + 31) / 32, (c.J + 31) / 32, SOR_KSPLIT);
@@ -650,14 +652,6 @@ int sor_correct(aturan_ctx* ctx, T* P, T* x2){
 // row's three factor arrays, per level, in the kernel's arithmetic type.
 template <typename T>
 inline size_t line_smem(const Grid& g){ return (size_t)(g.im - 2) * (LINE_COLS + 3) * sizeof(typename LineArith<T>::A); }
-
-// Allow sor_line_kernel above the default 48 KB of dynamic shared memory (once per instance).
-template <typename T, bool TR>
-bool line_smem_attr(){
-    static const bool ok = cudaFuncSetAttribute(sor_line_kernel<T, TR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                227 * 1024) == cudaSuccess || (cudaGetLastError(), false);
-    return ok;
-}
 
 // The point sweeps' work fields, free outside the RK4 step and the adjustment: the iterate and the
 // right-hand side split by colour (sor_colour_kernel).
@@ -682,10 +676,10 @@ template <typename T, bool TR = false>
 int sor_sweep(aturan_ctx* ctx, T* E, const T* R, double omega, bool line, bool chained){
     const Grid g = ctx->g;
     const int* stop = &ctx->sor_check->stop;
-    if(line && line_smem<T>(g) > 48 * 1024) line_smem_attr<T, TR>();
+    if(line) smem_opt_in(sor_line_kernel<T, TR>, line_smem<T>(g));
     for(int colour = 0; colour < 2; colour++){
         if(line){
-            chain(sor_line_kernel<T, TR>, dim3((g.km / 2 + LINE_COLS - 1) / LINE_COLS, g.jm - 2), 256, line_smem<T>(g), ctx->st, 
+            chain(sor_line_kernel<T, TR>, dim3((g.km / 2 + LINE_COLS - 1) / LINE_COLS, g.jm - 2), 256, line_smem<T>(g), ctx->st,
                 g, E, R, ctx->rbw, TR ? ctx->lluT_a : ctx->llu_a, TR ? ctx->lluT_cf : ctx->llu_cf,
                 TR ? ctx->lluT_idn : ctx->llu_idn, colour, omega, stop);
             continue;
@@ -699,9 +693,9 @@ int sor_sweep(aturan_ctx* ctx, T* E, const T* R, double omega, bool line, bool c
 int sor_check_sizes(aturan_ctx* ctx, double omega, bool line){
     const Grid& g = ctx->g;
     if(!(omega > 0.0 && omega < 2.0)) return fail(ctx, ATURAN_E_INVALID, "omega must lie in (0, 2)");
-    if(8 * ctx->sorc.J * (5 * ctx->sor_pm + 4) > 227 * 1024)
+    if(8 * ctx->sorc.J * (5 * ctx->sor_pm + 4) > SMEM_BLOCK_MAX)
         return fail(ctx, ATURAN_E_UNSUPPORTED, "the column correction needs jm <= 2900");
-    if(line && line_smem<double>(g) > 227 * 1024)
+    if(line && line_smem<double>(g) > SMEM_BLOCK_MAX)
         return fail(ctx, ATURAN_E_UNSUPPORTED, "line relaxation needs im <= 435");
     return ATURAN_OK;
 }
@@ -1504,15 +1498,6 @@ int aturan_ctx_create(const aturan_params* p, aturan_ctx** out){
         A2y += ((i == 1 || i == g.im - 2) ? 1.5 : 1.0) / (rm * rm);
     }
     ctx->sorc.J = sJ; ctx->sorc.N = sN; ctx->sorc.NM = sNM; ctx->sorc.inv_dthe2 = inv_dthe2; ctx->sorc.A2y = A2y;
-    {
-        const size_t tri = (size_t)8 * sJ * (5 * ctx->sor_pm + 4);   // the tridiagonal kernel's shared memory
-        if(tri > 48 * 1024 && tri <= 227 * 1024 &&
-           cudaFuncSetAttribute(sor_tridiag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tri) != cudaSuccess){
-            cudaGetLastError();
-            aturan_ctx_destroy(ctx);
-            return ATURAN_E_CUDA;
-        }
-    }
 
     auto up = [&](void* dst, const void* src, size_t n) -> int {
         return cudaMemcpyAsync(dst, src, n, cudaMemcpyHostToDevice, ctx->st) == cudaSuccess ? 0 : 1;
@@ -1850,7 +1835,7 @@ int rk4_adjoint_impl(aturan_ctx* ctx, int nf, const double* const* ybar, const d
         CK_LAUNCH("adjoint stage"); nl++;
     }
     const double* t0 = ctx->tX;
-    chain(adj_hydro_kernel, (g.jm * g.km + 31) / 32, dim3(32, 8), 0, ctx->st, 
+    chain(adj_hydro_kernel, (g.jm * g.km + 31) / 32, dim3(32, 8), 0, ctx->st,
         g, t0, reinterpret_cast<const double*>(ctx->pstat), t0 + 2 * fs, t0 + 3 * fs, ctx->tref, ctx->rm_i, ctx->cor_j,
         ctx->aphbar, ctx->aybar, ctx->arbar, ctx->hc);
     chain(adj_level_sum_kernel, dim3(ADJ_LB, g.im), 256, 0, ctx->st, g, t0, reinterpret_cast<const double*>(ctx->pstat), ctx->wsin,
@@ -1944,10 +1929,10 @@ int aturan_pressure_adjoint(aturan_ctx* ctx, int kind, double omega, int max_swe
     chain(sor_shift_finish_kernel, 1, 256, 0, ctx->st, ctx->sor_part, ny, ctx->sor_part + 2 * ny);
     const double n_int = (double)(g.im - 2) * (g.jm - 2) * (g.km - 1);
     const double sum_w = (double)(g.im - 1) * (g.jm - 1) * (g.km - 1);   // sum of y_i y_j over the interior
-    chain(adj_compat_mask_kernel, dim3((g.km - 1 + 127) / 128, g.jm - 2, g.im - 2), 128, 0, ctx->st, 
+    chain(adj_compat_mask_kernel, dim3((g.km - 1 + 127) / 128, g.jm - 2, g.im - 2), 128, 0, ctx->st,
         g, lam, ctx->sor_part + 2 * ny, n_int / sum_w, ctx->tSrc, ctx->rbw, sbar);
     double* aub = ctx->ag0;
-    chain(adj_div_kernel, dim3((g.km + 127) / 128, g.jm, g.im), 128, 0, ctx->st, 
+    chain(adj_div_kernel, dim3((g.km + 127) / 128, g.jm, g.im), 128, 0, ctx->st,
         g, sbar, ctx->rbw, ctx->pc, ctx->p.rigid_lid, aub, aub + fs, aub + 2 * fs);
     CK_LAUNCH("pressure adjoint: source");
     nl += 4;

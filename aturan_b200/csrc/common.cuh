@@ -55,6 +55,20 @@ inline cudaError_t chain(void (*kernel)(E...), dim3 grid, dim3 block, size_t sme
     return chain_if(true, kernel, grid, block, smem, st, std::forward<A>(args)...);
 }
 
+// Lets a kernel be launched with `bytes` of dynamic shared memory. Above the default 48 KB the kernel has to be
+// given a higher limit, which belongs to it on the current device, whatever context or thread asked for it
+// last. So every launch that needs it asks for the most a block can have, and nothing remembers that it did:
+// a flag per process would leave the kernels of a second device without it, and a limit fitted to one
+// context would take it from a larger one. False: the device does not allow it.
+constexpr int SMEM_BLOCK_MAX = 227 * 1024;
+template <typename... E>
+inline bool smem_opt_in(void (*kernel)(E...), size_t bytes){
+    if(bytes <= 48 * 1024) return true;
+    if(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BLOCK_MAX) == cudaSuccess) return true;
+    cudaGetLastError();
+    return false;
+}
+
 // A value that a launch writes, by a plain load. The read-only path (__ldg, or a const pointer with
 // __restrict__) wants memory that nobody writes while the kernel lives, and a chained kernel lives before
 // the one ahead of it has flushed its writes: the wait holds back neither a read-only load that the compiler

@@ -45,9 +45,7 @@ void launch_scalars(const StageArgs<S, C>& a, dim3 grid2, cudaStream_t st){
         constexpr int D = StageCfg<S>::AD;
         auto kern = rk_scalar_async_kernel<S, C, D, StageCfg<S>::AMINB>;
         const int sm = D * (int)sizeof(AsyncSlot<S>);
-        static const bool attr = (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, sm) == cudaSuccess)
-                                 || (cudaGetLastError(), false);
-        (void)attr;
+        smem_opt_in(kern, sm);
         chain(kern, grid2, dim3(32, 4), sm, st, a);
     } else {
         chain(rk_scalar_pair_kernel<S, C, StageCfg<S>::PD, StageCfg<S>::MINB2>, grid2, dim3(32, 4), 0, st, a);
@@ -77,9 +75,7 @@ int launch_filter(const Grid& g, S* x, float* lo, bool ai, bool aj, bool ak, dou
         // with the opt-in size (rows of up to 8192 values)
         const int R = 4 * g.km * (int)sizeof(double) <= 48 * 1024 ? 4 : 1;
         const int sm = R * g.km * (int)sizeof(double), rows = g.im * g.jm;
-        static const bool big = (cudaFuncSetAttribute(post_filter_k_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                      8192 * (int)sizeof(double)) == cudaSuccess) || (cudaGetLastError(), false);
-        (void)big;
+        smem_opt_in(post_filter_k_kernel<S>, sm);
         chain(post_filter_k_kernel<S>, (rows + R - 1) / R, dim3(32, R), sm, st, g, x, lo, coeff, phi_periodic && g.km > 2, rows);
         n++;
     }
@@ -168,10 +164,7 @@ int launch_mca_grow(const McaArgs<S>& a, cudaStream_t st){
     const size_t sm = (32 / G) * mca_col_bytes(a.g.im);
     if(sm > MCA_SMEM_MAX) return -1;
     auto kern = mca_grow_kernel<S, G>;
-    if(sm > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) != cudaSuccess){
-        cudaGetLastError();
-        return -1;
-    }
+    if(!smem_opt_in(kern, sm)) return -1;
     int per_sm = 0;
     if(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32, sm) != cudaSuccess || per_sm < 1){
         cudaGetLastError();
@@ -202,9 +195,7 @@ template <> struct HydCfg<float> { static constexpr int ROWS = 16, MINB = 2; };
 template <int NC>
 static int gs_wave_as(Grid g, double* P, const double* src, const GSW* w, const GsPlan& pl, GsEdge* edge, unsigned* ticket,
                       unsigned base, unsigned tag, int* err, cudaStream_t st){
-    static const bool ok = cudaFuncSetAttribute(gs_wave_kernel<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                GS_SMEM_MAX) == cudaSuccess || (cudaGetLastError(), false);
-    if(!ok) return -1;
+    if(!smem_opt_in(gs_wave_kernel<NC>, pl.smem)) return -1;
     chain(gs_wave_kernel<NC>, pl.nb, gs_threads(pl), pl.smem, st, g, P, src, w, pl, edge, ticket, base, tag, err);
     return cudaPeekAtLastError() == cudaSuccess ? 1 : -1;
 }

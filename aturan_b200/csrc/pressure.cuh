@@ -134,7 +134,6 @@ __global__ void gs_src_kernel(Grid g, const S* au, const S* av, const S* aw, con
 constexpr int GSR = 32;                           // ring: values per row, and steps of the incoming edge
 constexpr int GSC = 16;                           // values per chunk
 constexpr int GSB_MAX = 8;
-constexpr int GS_SMEM_MAX = 227 * 1024;
 struct GsEdge { unsigned lo, tag_lo, hi, tag_hi; };
 constexpr int GS_MOVERS = 128;                    // threads of the mover warps
 struct GsPlan { int ipad, B, nb, steps, nc; size_t smem; };   // nb = 0: a column does not fit, no plan
@@ -147,7 +146,7 @@ inline GsPlan gs_plan(const Grid& g){
     p.ipad = (g.im + GSC - 1) / GSC * GSC;
     auto smem = [&](int B){ return (size_t)p.ipad * (2 * B + 1) * GSR * 8 + (size_t)p.ipad * GSR * 8 + 256; };
     int B = GSB_MAX;
-    while(B > 0 && (smem(B) > GS_SMEM_MAX || p.ipad * B > 384)) B--;
+    while(B > 0 && (smem(B) > SMEM_BLOCK_MAX || p.ipad * B > 384)) B--;
     if(B == 0) return p;
     if(B > g.jm - 2) B = g.jm - 2;
     p.B = B; p.nb = (g.jm - 2 + B - 1) / B; p.steps = g.im + B + g.km; p.smem = smem(B);
