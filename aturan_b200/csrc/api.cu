@@ -143,17 +143,17 @@ int cuda_check(aturan_ctx* c, cudaError_t e, const char* what){
 #define CK(call) do { int rc_ = cuda_check(ctx, (call), #call); if(rc_) return rc_; } while(0)
 #define CK_LAUNCH(what) do { int rc_ = cuda_check(ctx, cudaGetLastError(), what); if(rc_) return rc_; } while(0)
 
-// Whether every bounded wait of the GS sweeps since the last call ended in time (gs_wave_kernel): read
-// where a caller waits for the stream or takes p_dyn. Synchronizes when there is something to read.
-int gs_waits_held(aturan_ctx* ctx){
-    if(!ctx->gs_unread) return ATURAN_OK;
+// Waits for the context's stream on behalf of a caller that takes results, and says whether every bounded
+// wait of the GS sweeps since the last such call ended in time (gs_wave_kernel): everything formed from their
+// p_dyn since then is in doubt, so whatever is taken first reports it, once.
+int wait_done(aturan_ctx* ctx){
     int e = 0;
-    CK(cudaMemcpyAsync(&e, ctx->gs_err, sizeof e, cudaMemcpyDeviceToHost, ctx->st));
+    if(ctx->gs_unread) CK(cudaMemcpyAsync(&e, ctx->gs_err, sizeof e, cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
     ctx->gs_unread = false;
     if(!e) return ATURAN_OK;
     CK(cudaMemsetAsync(ctx->gs_err, 0, sizeof e, ctx->st));
-    return fail(ctx, ATURAN_E_CUDA, "GS sweep: a wait between bands ran out; p_dyn is not valid");
+    return fail(ctx, ATURAN_E_CUDA, "GS sweep: a wait between bands ran out; p_dyn and what was formed from it since are not valid");
 }
 
 size_t round_up(size_t x, size_t a){ return (x + a - 1) / a * a; }
@@ -930,7 +930,7 @@ int run_post(aturan_ctx* ctx, const aturan_post_params* pp, double* clamp_added,
         double h[2 * POST_NSP] = {0.0};
         if(pp->species_clamp){
             CK(cudaMemcpyAsync(h, pl.out, sizeof h, cudaMemcpyDeviceToHost, ctx->st));
-            CK(cudaStreamSynchronize(ctx->st));
+            const int rc = wait_done(ctx); if(rc) return rc;
         }
         for(int n = 0; n < POST_NSP; n++){
             if(clamp_added) clamp_added[n] = h[n];
@@ -1637,8 +1637,9 @@ static int xfer(aturan_ctx* ctx, int field, void* other, bool up, bool other_is_
     const int rc = pack_fields(ctx, 1, &field, &ptr, up, ctx->st);
     if(rc) return rc;
     if(!up && !other_is_device) CK(cudaMemcpyAsync(other, flat, n * 8, cudaMemcpyDeviceToHost, ctx->st));
-    if(!up || !other_is_device) CK(cudaStreamSynchronize(ctx->st));
-    return !up && field == ATURAN_P_DYN ? gs_waits_held(ctx) : ATURAN_OK;
+    if(!up) return wait_done(ctx);
+    if(!other_is_device) CK(cudaStreamSynchronize(ctx->st));
+    return ATURAN_OK;
 }
 
 // Several fields in one call. With host buffers the DMA copies run on the side stream and the
@@ -1652,16 +1653,11 @@ static int xfer_many(aturan_ctx* ctx, int n, const int* fields, void* const* ptr
         if(fields[q] < 0 || fields[q] >= ATURAN_NFIELDS) return fail(ctx, ATURAN_E_INVALID, "field id out of range");
         if(!ptrs[q]) return fail(ctx, ATURAN_E_INVALID, "null buffer");
     }
-    bool takes_pdyn = false;
-    for(int q = 0; q < n && !up; q++) takes_pdyn |= fields[q] == ATURAN_P_DYN;
     const Grid& g = ctx->g;
     const size_t nval = (size_t)g.im * g.jm * g.km;
     if(on_device){
         const int rc = pack_fields(ctx, n, fields, ptrs, up, ctx->st);
-        if(rc || up) return rc;
-        if(takes_pdyn && ctx->gs_unread) return gs_waits_held(ctx);
-        CK(cudaStreamSynchronize(ctx->st));
-        return ATURAN_OK;
+        return rc || up ? rc : wait_done(ctx);
     }
     double* buf[2] = {ctx->stage64, ctx->scratch};
     // the staging fields are free only once the work already queued on the main stream is done
@@ -1689,8 +1685,9 @@ static int xfer_many(aturan_ctx* ctx, int n, const int* fields, void* const* ptr
     }
     CK(cudaEventRecord(ctx->ev_join, ctx->st2));
     CK(cudaStreamWaitEvent(ctx->st, ctx->ev_join, 0));
+    if(!up) return wait_done(ctx);
     CK(cudaStreamSynchronize(ctx->st));
-    return takes_pdyn ? gs_waits_held(ctx) : ATURAN_OK;
+    return ATURAN_OK;
 }
 
 int aturan_upload(aturan_ctx* ctx, int field, const double* host){ return xfer(ctx, field, (void*)host, true, false); }
@@ -1707,8 +1704,7 @@ int aturan_download_device(aturan_ctx* ctx, int field, double* dev){ return xfer
 int aturan_download_buoy_ref(aturan_ctx* ctx, double* host){
     if(!ctx || !host) return ATURAN_E_INVALID;
     CK(cudaMemcpyAsync(host, ctx->ref_level, ctx->g.im * 8, cudaMemcpyDeviceToHost, ctx->st));
-    CK(cudaStreamSynchronize(ctx->st));
-    return ATURAN_OK;
+    return wait_done(ctx);
 }
 
 int aturan_rk4_step(aturan_ctx* ctx){
@@ -1856,8 +1852,7 @@ int rk4_adjoint_impl(aturan_ctx* ctx, int nf, const double* const* ybar, const d
         chain(adj_heat_reduce_kernel, (g.jm * g.km + 255) / 256, 256, 0, ctx->st, g, ctx->ahacc, K.heat_scale, heatbar);
         CK_LAUNCH("heating adjoint");
     }
-    CK(cudaStreamSynchronize(ctx->st));
-    return ATURAN_OK;
+    return wait_done(ctx);
 }
 
 }  // namespace
@@ -1937,7 +1932,7 @@ int aturan_pressure_adjoint(aturan_ctx* ctx, int kind, double omega, int max_swe
     CK_LAUNCH("pressure adjoint: source");
     nl += 4;
     rc = pack_doubles(ctx, 3, auxbar, aub, false); if(rc) return rc;
-    CK(cudaStreamSynchronize(ctx->st));
+    rc = wait_done(ctx); if(rc) return rc;
     reg.n = nl;
     if(sweeps_done) *sweeps_done = s;
     if(resid) *resid = r;
@@ -1955,7 +1950,7 @@ int aturan_satadj(aturan_ctx* ctx, int gas_mask, long* n_adjusted, long* n_nocon
     if(count){
         unsigned long long h[2];
         CK(cudaMemcpyAsync(h, ctx->counters, sizeof h, cudaMemcpyDeviceToHost, ctx->st));
-        CK(cudaStreamSynchronize(ctx->st));
+        rc = wait_done(ctx); if(rc) return rc;
         if(n_adjusted) *n_adjusted = (long)h[0];
         if(n_noconv) *n_noconv = (long)h[1];
     }
@@ -2159,7 +2154,7 @@ int aturan_chemistry(aturan_ctx* ctx, const aturan_chem_params* cp, int what, lo
     if(count){
         unsigned long long h[2];
         CK(cudaMemcpyAsync(h, ctx->counters + 4, sizeof h, cudaMemcpyDeviceToHost, ctx->st));
-        CK(cudaStreamSynchronize(ctx->st));
+        const int done = wait_done(ctx); if(done) return done;
         if(n_formed) *n_formed = (long)h[0];
         if(n_decomposed) *n_decomposed = (long)h[1];
     }
@@ -2321,8 +2316,7 @@ int aturan_profile_read(aturan_ctx* ctx, double* ms, long* launches, int nkinds)
 
 int aturan_sync(aturan_ctx* ctx){
     if(!ctx) return ATURAN_E_INVALID;
-    CK(cudaStreamSynchronize(ctx->st));
-    return gs_waits_held(ctx);
+    return wait_done(ctx);
 }
 
 }  // extern "C"

@@ -258,7 +258,11 @@ int aturan_pressure_adjoint(aturan_ctx* ctx, int kind, double omega, int max_swe
 
 /* The pressure solve.
  *   GS_LEX:    replaces PressureSolverUran(m).run() (PressureSolverUran.h:33-250); omega,
- *              max_sweeps and tol are ignored (exactly one sweep, as the reference).
+ *              max_sweeps and tol are ignored (exactly one sweep, as the reference). The sweep's
+ *              blocks wait for one another for a bounded time. Should a wait run out, p_dyn is not
+ *              valid, and the next call that takes results from the context (a download, counts or
+ *              sums, an adjoint, aturan_sync) returns ATURAN_E_CUDA, once. While the context's
+ *              stream is being captured into a graph the sweep is refused (ATURAN_E_UNSUPPORTED).
  *   RB_SHARED: replaces PressureSolver<cUranusModel>(m).run() (PressureSolver.h:145-766) with
  *              ATURAN_PRESS_SWEEPS = max_sweeps; omega and tol ignored.
  *   RB_SOR:    the shared solver's equation (its source, clamp and boundary folds) solved with
