@@ -1217,15 +1217,15 @@ int aturan_ctx_create(const aturan_params* p, aturan_ctx** out){
     for(int n = 0; n < 6; n++) add((size_t)(sNM + 1) * sJ * 8);        // mode factorisations (Lc, Lc^T)
     for(int n = 0; n < 6; n++) add(nij * 8);                           // line factorisations (Lc, Lc^T)
     add(fs * 4); add(fs * 4);
-    ctx->gsp = gs_plan(g);
-    add(gs_edge_bytes(ctx->gsp)); add(4); add(4); add(sizeof(SorCheck));
     if(ctx->mixed) add(2 * fs * 4);                                    // the temperature pair's low parts
-    ctx->mem_bytes = bytes;
-    // the stage kernels address every buffer of the allocation by 32-bit element offsets
+    // the stage kernels address every buffer of the allocation up to here by 32-bit element offsets
     if(bytes / e >= (size_t)INT32_MAX){
         std::fprintf(stderr, "aturan_ctx_create: grid too large (%zu elements of context memory, limit 2^31)\n", bytes / e);
         delete ctx; return ATURAN_E_UNSUPPORTED;
     }
+    ctx->gsp = gs_plan(g);
+    add(gs_edge_bytes(ctx->gsp)); add(4); add(4); add(sizeof(SorCheck));
+    ctx->mem_bytes = bytes;
     int prio_lo = 0, prio_hi = 0;                         // least and most urgent
     if(cudaDeviceGetStreamPriorityRange(&prio_lo, &prio_hi) != cudaSuccess){ cudaGetLastError(); prio_lo = prio_hi = 0; }
     if(cudaStreamCreateWithPriority(&ctx->st, cudaStreamNonBlocking, prio_hi) != cudaSuccess){
@@ -1295,11 +1295,11 @@ int aturan_ctx_create(const aturan_params* p, aturan_ctx** out){
     ctx->mluT_idn = carve<double>(cur, (size_t)(sNM + 1) * sJ);
     ctx->lluT_a = carve<double>(cur, nij); ctx->lluT_cf = carve<double>(cur, nij); ctx->lluT_idn = carve<double>(cur, nij);
     ctx->r32 = carve<float>(cur, fs); ctx->e32 = carve<float>(cur, fs);
+    ctx->tlo = ctx->mixed ? carve<float>(cur, 2 * fs) : nullptr;
     ctx->gs_edge = reinterpret_cast<GsEdge*>(carve<char>(cur, gs_edge_bytes(ctx->gsp)));
     ctx->gs_ticket = carve<unsigned>(cur, 1);
     ctx->gs_err = carve<int>(cur, 1);
     ctx->sor_check = carve<SorCheck>(cur, 1);
-    ctx->tlo = ctx->mixed ? carve<float>(cur, 2 * fs) : nullptr;
 
     // zero everything once: padding columns and unused planes read as 0, never as garbage
     if(cudaMemsetAsync(ctx->mem, 0, bytes, ctx->st) != cudaSuccess){ aturan_ctx_destroy(ctx); return ATURAN_E_CUDA; }
