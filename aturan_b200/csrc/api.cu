@@ -264,7 +264,7 @@ RhsConst<C> make_rhs_const(const aturan_params& p){
 
 int validate(const aturan_params* p, std::string& why){
     if(p->abi_version != ATURAN_ABI_VERSION){ why = "abi_version mismatch"; return ATURAN_E_INVALID; }
-    if(p->im < 5 || p->jm < 5 || p->km < 5 || p->im > 512 || p->jm > 4096 || p->km > 8192){ why = "grid size out of range"; return ATURAN_E_INVALID; }
+    if(p->im < 5 || p->jm < 5 || p->km < 5 || p->im > IM_MAX || p->jm > 4096 || p->km > 8192){ why = "grid size out of range"; return ATURAN_E_INVALID; }
     if((p->km - 1) % 2){ why = "km-1 must be even (the red-black colours must alternate across the seam)"; return ATURAN_E_UNSUPPORTED; }
     if(p->precision != ATURAN_FP64 && p->precision != ATURAN_MIXED){ why = "unknown precision"; return ATURAN_E_INVALID; }
     if(!(p->dt > 0.0) || !(p->dr > 0.0) || !(p->dthe > 0.0) || !(p->dphi > 0.0)){ why = "non-positive step"; return ATURAN_E_INVALID; }
@@ -673,7 +673,7 @@ int sor_split(aturan_ctx* ctx, T* x, T* x2, bool to){
 // (line = false; of the split fields) or radial line. chained: the launch before is a point pass of the
 // same solve, so that a point pass may read what none writes before it waits for it (sor_colour_kernel).
 template <typename T, bool TR = false>
-int sor_sweep(aturan_ctx* ctx, T* E, const T* R, double omega, bool line, bool chained){
+void sor_sweep(aturan_ctx* ctx, T* E, const T* R, double omega, bool line, bool chained){
     const Grid g = ctx->g;
     const int* stop = &ctx->sor_check->stop;
     if(line) smem_opt_in(sor_line_kernel<T, TR>, line_smem<T>(g));
@@ -687,7 +687,6 @@ int sor_sweep(aturan_ctx* ctx, T* E, const T* R, double omega, bool line, bool c
         const dim3 grid(((g.km - 1) / 2 * (g.jm - 2) + COLOUR_NT - 1) / COLOUR_NT, (g.im - 2 + COLOUR_CH - 1) / COLOUR_CH);
         chain_if(chained || colour == 1, sor_colour_kernel<T, TR>, grid, COLOUR_NT, 0, ctx->st, g, sor_x2<T>(ctx), sor_r2<T>(ctx), ctx->rbw, colour, omega, stop);
     }
-    return ATURAN_OK;
 }
 
 int sor_check_sizes(aturan_ctx* ctx, double omega, bool line){
@@ -771,7 +770,7 @@ int solve_fp64(aturan_ctx* ctx, double* P, const double* src, double omega, int 
         [&](int s, int* next){
             int rc;
             for(int n = 0; n < check_every && s < max_sweeps; n++, s++){
-                rc = sor_sweep<double, TR>(ctx, P, src, omega, line, n > 0); if(rc) return rc;
+                sor_sweep<double, TR>(ctx, P, src, omega, line, n > 0);
                 nl += 2;
             }
             CK_LAUNCH("SOR sweeps");
@@ -820,7 +819,7 @@ int solve_mixed(aturan_ctx* ctx, double* P, const double* src, double omega, int
                     rc = sor_correct<float, TR>(ctx, ctx->e32, line ? nullptr : sor_x2<float>(ctx)); if(rc) return rc;
                     nl += 5;
                 }
-                rc = sor_sweep<float, TR>(ctx, ctx->e32, ctx->r32, omega, line, n > 0 && !now); if(rc) return rc;
+                sor_sweep<float, TR>(ctx, ctx->e32, ctx->r32, omega, line, n > 0 && !now);
                 nl += 2;
             }
             if(!line){ rc = sor_split(ctx, ctx->e32, sor_x2<float>(ctx), false); if(rc) return rc; nl++; }
@@ -1069,7 +1068,6 @@ template <typename S>
 int run_mca(aturan_ctx* ctx){
     const Grid& g = ctx->g;
     const aturan_params& p = ctx->p;
-    if(mca_col_bytes(g.im) > MCA_SMEM_MAX) return fail(ctx, ATURAN_E_UNSUPPORTED, "column too deep for the shared memory");
     int nl = 0;
     if(!ctx->mca_H_ready){
         // the cp table's running integral, formed once; ready only once its kernel has launched
@@ -1120,7 +1118,7 @@ int run_mca(aturan_ctx* ctx){
     }
     Region reg(ctx, ATURAN_K_MCA, 0);
     const int n = launch_mca(a, ctx->st);
-    if(n < 0) return fail(ctx, ATURAN_E_UNSUPPORTED, "mca: the column's shared memory");
+    if(n < 0) return fail(ctx, ATURAN_E_CUDA, "moist convective adjustment: launch");
     reg.n = nl + n;
     CK_LAUNCH("moist convective adjustment");
     return ATURAN_OK;
@@ -2190,8 +2188,6 @@ int aturan_iteration(aturan_ctx* ctx, const aturan_iter_params* ip, int iter_n){
                           ip->turb.buoy != 0 || ip->turb.abl_taper != 0))
         return fail(ctx, ATURAN_E_UNSUPPORTED, "turbulence: only the default knobs are implemented");
     const bool mca = ip->mca_stride > 0 && iter_n % ip->mca_stride == 0;
-    if(ip->mca_stride > 0 && mca_col_bytes(ctx->g.im) > MCA_SMEM_MAX)
-        return fail(ctx, ATURAN_E_UNSUPPORTED, "moist convective adjustment: column too deep for the shared memory");
     int rc;
     if(iter_n % 2 == 0){
         // the saturation adjustment and what follows it up to the chemistry forcing touch no field

@@ -82,6 +82,7 @@ __device__ __forceinline__ T ld(const T* p){ return *p; }
 template <typename T>
 __device__ __forceinline__ T ldr(const T* p){ return __ldg(p); }
 
+constexpr int IM_MAX = 512;        // levels of a context's grid
 struct Grid {
     int im, jm, km, kp;
     size_t fstride;            // elements per field (im * jm * kp)

@@ -156,15 +156,13 @@ int launch_precip_impl(const PrecipArgs<S>& a, cudaStream_t st){
     chain(precip_kernel<S>, dim3((a.g.km + 31) / 32, a.g.jm), 128, 0, st, a);
     return 1;
 }
-// The moist convective adjustment (mca.cuh); returns the launches, or -1 if a warp's columns do not fit
-// the shared memory. Lanes per column of the growth: 4 where the columns fill the chip's resident warps
-// so, 8 below that (MCA_SMALL_COLUMNS).
+// The moist convective adjustment (mca.cuh); returns the launches, or -1 on an error. Lanes per column of
+// the growth: 4 where the columns fill the chip's resident warps so, 8 below that (MCA_SMALL_COLUMNS).
 template <typename S, int G>
 int launch_mca_grow(const McaArgs<S>& a, cudaStream_t st){
     const size_t sm = (32 / G) * mca_col_bytes(a.g.im);
-    if(sm > MCA_SMEM_MAX) return -1;
+    static_assert((32 / G) * mca_col_bytes(IM_MAX) <= 48 * 1024, "a warp's columns fit the default shared memory");
     auto kern = mca_grow_kernel<S, G>;
-    if(!smem_opt_in(kern, sm)) return -1;
     int per_sm = 0;
     if(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32, sm) != cudaSuccess || per_sm < 1){
         cudaGetLastError();
@@ -177,7 +175,6 @@ int launch_mca_grow(const McaArgs<S>& a, cudaStream_t st){
 template <typename S>
 int launch_mca_impl(const McaArgs<S>& a, cudaStream_t st){
     const Grid& g = a.g;
-    if(mca_col_bytes(g.im) > MCA_SMEM_MAX) return -1;
     const dim3 b((g.km + 127) / 128, g.jm);
     if(cudaMemsetAsync(a.next, 0, sizeof(unsigned), st) != cudaSuccess) return -1;
     chain(mca_prep_kernel<S>, dim3(b.x, b.y, g.im), 128, 0, st, a);

@@ -300,8 +300,7 @@ __global__ void __launch_bounds__(128, 4) mca_test_kernel(const __grid_constant_
 
 // What a group keeps of its column in shared memory, and its bytes: the weights and a flag per level.
 struct McaCol { double* w; unsigned char* flag; };
-constexpr size_t MCA_SMEM_MAX = 227 * 1024;
-__host__ __device__ inline size_t mca_col_bytes(int im){ return (size_t)im * sizeof(double) + ((size_t)im + 7) / 8 * 8; }
+__host__ __device__ constexpr size_t mca_col_bytes(int im){ return (size_t)im * sizeof(double) + ((size_t)im + 7) / 8 * 8; }
 
 // Blocks of one warp, G (4 to 16) lanes per column. A group walks up its column from unstable pair to unstable
 // pair; every turn of the loop is one growth step of each group's segment, its three solves on three

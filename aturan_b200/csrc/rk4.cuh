@@ -83,25 +83,6 @@ struct D6 { C c, d1r, d2r, d1t, d2t, d1p, d2p; };
 template <typename C>
 struct R7 { C c, rp, rm, tp, tm, pe, pw; };
 
-// Neighbour addressing of one cell: offsets and, per direction, the array a neighbour is read
-// from (the stage input, or the state on a boundary row).
-template <typename S>
-struct Nbr {
-    size_t o, oim, oip, ojm, ojp, okw, oke, fs;
-    const S *X, *xim, *xip, *xjm, *xjp;
-};
-
-template <typename S, typename C>
-__device__ __forceinline__ R7<C> load7(const Nbr<S>& n, int q){
-    const size_t f = (size_t)q * n.fs;
-    R7<C> r;
-    r.c  = (C)ld(n.X + f + n.o);
-    r.rp = (C)ld(n.xip + f + n.oip); r.rm = (C)ld(n.xim + f + n.oim);
-    r.tp = (C)ld(n.xjp + f + n.ojp); r.tm = (C)ld(n.xjm + f + n.ojm);
-    r.pe = (C)ld(n.X + f + n.oke);   r.pw = (C)ld(n.X + f + n.okw);
-    return r;
-}
-
 // The forward stage's addressing of one cell: offsets in elements from the stage input X -- of the
 // cell and its six stencil neighbours (a neighbour on a boundary row lies in the state St, reached
 // through the same base), of a field (fs), and of the accumulator, n-copy, forcing and stage-output
