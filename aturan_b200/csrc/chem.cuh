@@ -109,6 +109,10 @@ __device__ __forceinline__ void nh4sh_bisect(double& lo, double& hi, double stop
     }
     // With u = a - x, v = b - x, the computed sign of f is unreliable within its rounding, ~8e-16 K_p,
     // of the root: 8e-16 uv / (u + v) <= 8e-16 min(u, v) in x, below stop; r adds a quarter of that.
+    // Besides, K_p as computed is a step function of x: where T0 + heat x passes to its next double it
+    // jumps by ~1e-14 of itself. The jump has the sign of f's slope (more NH4SH is warmer, K_p grows and f
+    // falls), so f changes sign once with it as without; and a bracket with an inferred end is checked with
+    // f there before it is used.
     const double band = 4.0 * stop;
     // whether the sign of f at each end was evaluated (the initial ends' signs are the caller's
     // tests: f(lo) > 0, and f(hi) <= 0 at x = 0 or x = min(a, b), where f = -K_p) or inferred

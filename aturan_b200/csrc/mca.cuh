@@ -29,7 +29,8 @@
 //     and has not changed. The reference's further sweep finds nothing, so there is none here.
 // Measured at 41x181x361 (mixed, synthetic state): 4.2 ms -- prep 0.10, tests 1.18, growth 2.48, finish
 // 0.46 -- against 44.7 ms for one warp per column running the whole sweep with every settle and a
-// verifying sweep; 1.1 against 8.1 ms at 37x83x167, 0.34 against 0.88 ms at 21x37x73. Same bits. (With
+// verifying sweep; 1.1 against 8.1 ms at 37x83x167, 0.34 against 0.88 ms at 21x37x73. Same bits in FP64; the
+// mixed form, whose multiply-adds contract, moved by 1e-15 of a field's maximum with the expressions. (With
 // every quotient a division and a column's whole state in shared memory: 6.0, 1.28 and 0.63 ms.)
 // The growth chain is what is left of the serial part: bound by the latency of its solves on small
 // grids, by that and FP64 issue on large ones, so it takes as many warps an SM as 128 registers allow

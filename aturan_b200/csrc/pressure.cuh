@@ -112,8 +112,9 @@ __global__ void gs_src_kernel(Grid g, const S* au, const S* av, const S* aw, con
 // The sweep's dependency chain is (im-2)+(jm-2)+(km-1) cells long, so what bounds it is the time of
 // one hyperplane. As a launch per hyperplane that was 2.3 us (576 launches, 1.31 ms at 41x181x361);
 // here a hyperplane step is one block barrier and one trip through shared memory: 0.235 ms (0.041
-// against 0.244 ms at 21x37x73). A step takes 0.17 us with 4 sweeping warps per block and 0.32 us
-// with 12 (the shared-memory pipe is then 60 % busy), and each band starts ~2 us after the one before.
+// against 0.244 ms at 21x37x73). A step takes 0.17 us with 4 sweeping warps per block, 0.23 us with 8
+// and 0.32 us with 12 (the shared-memory pipe is then 60 % busy). A band lags the one before by its own
+// rows' steps and a hand-over of ~2 us, so at 41x181x361 the chain is 577 steps and 22 hand-overs.
 //
 // A block owns a band of B rows j and all levels i; its thread (i, j) walks its row along k, at step
 // s on cell k = s - i - j. The rows lie in a ring of 32 values in shared memory, the new value

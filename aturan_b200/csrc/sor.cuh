@@ -110,7 +110,7 @@ __device__ __forceinline__ double row_acc(const Grid& g, const T* P, size_t o, i
 // the solve has reached its tolerance. Every later kernel of the solve does nothing once `stop` is
 // set, so the host enqueues the next sweeps before it knows the last check's answer and the device
 // never waits for it; it reads slot n while check n + 1 fills the other. (A line solve of five checks at
-// 41 x 181 x 361, mixed: 0.73 ms with a host round trip after each, 0.69 without.)
+// 41 x 181 x 361, mixed, with transfers: the round trips cost 0.04 ms of what then was 0.73, now 0.55.)
 struct SorCheck { double rr[2], ss[2]; int stop; unsigned ticket; };
 __host__ __device__ inline double rel_residual(double rr, double ss){ return ss > 0.0 ? sqrt(rr / ss) : sqrt(rr); }
 struct SorCheckArg { SorCheck* c; int slot; bool first; double tol; };   // slot < 0: column sums only

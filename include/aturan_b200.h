@@ -184,7 +184,8 @@ int aturan_download_device(aturan_ctx* ctx, int field, double* dev);
  * device buffers with on_device = 1. The host copies of field q overlap the on-device layout
  * change of field q-1, and the call waits once instead of once per field (what a driver that
  * exchanges the fields its CPU modules touch each iteration uses). Same return conditions as the
- * one-field calls, except that a device upload is asynchronous. */
+ * one-field calls, except that a device upload is asynchronous. A field given twice, and outputs that
+ * overlap, end as if the fields were moved one after the other. */
 int aturan_upload_many(aturan_ctx* ctx, int n, const int* fields, const double* const* src, int on_device);
 int aturan_download_many(aturan_ctx* ctx, int n, const int* fields, double* const* dst, int on_device);
 /* buoy_ref_level[im] of the last RK4 step (cUranusModel.h:1431). */
@@ -200,11 +201,12 @@ int aturan_rk4_step(aturan_ctx* ctx);
  * tendencies of t, u, v, w.
  * aturan_tape(ctx, 1): every later aturan_rk4_step and RB_SOR / RB_LINE aturan_pressure keeps what
  *   its adjoint needs (the stage inputs of t, u, v, w, the new T, p_dyn, the clamped pressure
- *   source and the level means: 19 fields, plus 56 fields of work arrays, of device memory);
+ *   source and the level means: 19 fields, plus 26 fields of work arrays, of device memory);
  *   aturan_tape(ctx, 2): the moist tape (aturan_moist_adjoint); aturan_tape(ctx, 0) frees either.
  *   ATURAN_E_UNSUPPORTED on a mixed context.
  * aturan_rk4_adjoint(ctx, ybar, xbar): ybar[4] and xbar[4] are device pointers to contiguous
- *   [im][jm][km] FP64 arrays in the order t, u, v, w. Given the adjoint ybar of those fields after
+ *   [im][jm][km] FP64 arrays in the order t, u, v, w (a buffer that is no device memory:
+ *   ATURAN_E_INVALID; so in the adjoint and solve calls below). Given the adjoint ybar of those fields after
  *   the last taped aturan_rk4_step, writes xbar = J^T ybar, J the step's Jacobian with respect to
  *   the fields before it, taken as the state and its start-of-step copies together (as after
  *   aturan_sync_ncopies). p_dyn, p_stat, p_baro, p_b0, p_bfollow, the forcing and the other
@@ -225,7 +227,7 @@ int aturan_rk4_adjoint_ex(aturan_ctx* ctx, const double* const* ybar, const doub
 /* The moist step's adjoint (no counterpart in the reference). aturan_tape(ctx, 2) switches on the
  * moist tape (the dry one's contents over sixteen fields -- t, u, v, w and the twelve condensable
  * species ATURAN_CH4 .. ATURAN_NH3_ICE -- plus the state an aturan_satadj of all four gases, or
- * aturan_step's adjustment, had on entry: 16 more fields and 84 more work fields; replaces a dry
+ * aturan_step's adjustment, had on entry: 83 fields, plus 74 fields of work arrays; replaces a dry
  * tape). Given ybar[16], the adjoint of those sixteen fields after the last taped
  * aturan_rk4_step, writes xbar[16]: the RK4 step's adjoint over the sixteen fields (the species'
  * transport and diffusion by the taped u, v, w, their forcing held fixed) and, when an adjustment
