@@ -646,6 +646,22 @@ def cpu_reference_step_time(nsteps, press, budget_s=120.0):
     return dt, kind, cores, f"{n} full steps (pressure: {ptxt} + 4 SatAdj + sync + RK4) of {what}, 41x181x361", n
 
 
+# What the line on stdout holds: the headline, what it was measured on and how, and its checks. The rest (the
+# timings of the other calls, kernel by kernel and accuracy tables, ~15 KB) goes to stderr as a JSON line of
+# its own: whoever keeps only the last few KB of stdout lost the headline with them.
+HEADLINE = ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better", "scaling",
+            "vs_baseline", "dtype", "data", "config", "gpu_launches", "roofline", "e2e", "clocks", "cpu_baseline")
+
+
+def report(line):
+    head = {k: line[k] for k in HEADLINE}
+    rest = {k: v for k, v in line.items() if k not in HEADLINE}
+    head["roofline"] = {k: v for k, v in line["roofline"].items() if k != "step"}
+    rest["roofline_step"] = line["roofline"].get("step")
+    print(json.dumps({"details": rest}), file=sys.stderr, flush=True)
+    print(json.dumps(head), flush=True)
+
+
 def run_reference_arm(args, rank, world):
     if rank != 0:
         return
@@ -945,7 +961,7 @@ def main():
         }
         if accuracy is not None:
             line["accuracy_vs_fp64"] = accuracy
-        print(json.dumps(line), flush=True)
+        report(line)
     ctx.close()
     if dist is not None:
         dist.barrier()
