@@ -356,7 +356,10 @@ int pack_doubles(aturan_ctx* ctx, int n, const double* const* flat, double* pad,
     bool direct = true;
     for(int q = 0; q < n; q++){
         const Reach r = reach(ctx, flat[q], bytes);
-        if(r == REACH_NONE) return fail(ctx, ATURAN_E_INVALID, "not a device buffer of im*jm*km doubles");
+        if(r == REACH_NONE){
+            CK(cudaStreamSynchronize(ctx->st));       // what this call has enqueued reads the other buffers
+            return fail(ctx, ATURAN_E_INVALID, "not a device buffer of im*jm*km doubles");
+        }
         direct = direct && r == REACH_KERNEL;
         for(int o = 0; !in && o < q; o++){
             const uintptr_t a = reinterpret_cast<uintptr_t>(flat[q]), b = reinterpret_cast<uintptr_t>(flat[o]);
